@@ -208,6 +208,61 @@ def work(case):
             "flops": pairs * product * (3 if case["pass"] == "train" else 1)}
 
 
+def _product64(x, w, sizes):
+    """Rows of ``x`` grouped by ``sizes`` times ``w[i]`` each, in 64 bits; idle experts are skipped."""
+    out = torch.empty(x.shape[0], w.shape[2], dtype=torch.float64, device=x.device)
+    start = 0
+    for i, size in enumerate(sizes):
+        if size:
+            torch.mm(x[start:start + size].double(), w[i].double(), out=out[start:start + size])
+        start += size
+    return out
+
+
+def _weight_grad64(x, grad, sizes, transposed):
+    shape = (len(sizes), grad.shape[1], x.shape[1]) if transposed else (len(sizes), x.shape[1], grad.shape[1])
+    out = torch.zeros(shape, dtype=torch.float64, device=x.device)
+    start = 0
+    for i, size in enumerate(sizes):
+        if size:
+            rows, cols = (grad, x) if transposed else (x, grad)
+            torch.mm(rows[start:start + size].double().t(), cols[start:start + size].double(), out=out[i])
+        start += size
+    return out
+
+
+def exact(case, seed):
+    """What ``run`` returns, computed in 64 bits from the same bf16 inputs."""
+    state = prepare(case, seed)
+    state = {key: v.detach() if isinstance(v, torch.Tensor) else v for key, v in state.items()}
+    op, x, trans_b = state["op"], state["x"], state["trans_b"]
+    sizes = [int(s) for s in state["sizes"].tolist()]
+    # weights as [z, in, out]
+    b, b2, down = (state[key].transpose(1, 2) if trans_b and key in state else state.get(key) for key in ("b", "b2", "down"))
+    rows = x.index_select(0, state["source"]) if op in ("gather", "layer") else x
+    out = _product64(rows, b, sizes)
+    if op in ("swiglu", "layer"):
+        gate, up = out, _product64(rows, b2, sizes)
+        out = torch.nn.functional.silu(gate) * up
+    if op == "layer":
+        y = _product64(out, down, sizes) * state["row_weight"].double()[:, None]
+        return torch.zeros(x.shape, dtype=torch.float64, device=x.device).index_add_(0, state["source"], y)
+    if case["pass"] != "train":
+        return out
+    grad = state["grad"]
+    if op == "swiglu":
+        s = torch.sigmoid(gate)
+        d_up = grad * gate * s
+        d_gate = grad * up * s * (1.0 + gate * (1.0 - s))
+        del s, gate, up
+        x_grad = _product64(d_gate, b.transpose(1, 2), sizes) + _product64(d_up, b2.transpose(1, 2), sizes)
+        return out, x_grad, _weight_grad64(rows, d_gate, sizes, trans_b), _weight_grad64(rows, d_up, sizes, trans_b)
+    x_grad = _product64(grad, b.transpose(1, 2), sizes)
+    if op == "gather":
+        x_grad = torch.zeros(x.shape, dtype=torch.float64, device=x.device).index_add_(0, state["source"], x_grad)
+    return out, x_grad, _weight_grad64(rows, grad, sizes, trans_b)
+
+
 def tolerance(case):
     """Four times the distance from the same path in 64 bits.  A single product is one
     rounding to bf16 of an fp32 sum (1.66e-3; largest element 3.9e-3).  The other paths
