@@ -294,6 +294,13 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   // by streaming their weights from HBM either way, and measured end to end the
   // launch was not faster with them (B200GMM_LIGHT=1 switches them on).
   p->light = (p->mode != kTN && ctas == 1 && !f.gather && !f.swiglu) ? env_int("B200GMM_LIGHT", 0) : 0;
+  // Tiles of at most half their rows run with their operands swapped (schedule.cuh).
+  // Nearer to a full tile the swapped form saves no tensor time (N = 112 twice against
+  // 256 once, bound by the shared-memory reads of the operands) and its epilogue, which
+  // transposes, is the longer one: 3001 rows in 7 experts, k = 1000, n = 2504 took 33.9 us
+  // up to 64 rows and without, 34.7 us up to 112; 256 experts of at most 118 rows,
+  // k = 7168, n = 2048: 992 us without, 925 up to 32, 932 up to 64, 950 up to 112.
+  p->swap_rows = (p->mode != kTN && !(f.swiglu && ctas == 2)) ? p->tile_m / 2 : 0;
   const int64_t wait_ns = env_int64("B200GMM_WAIT_LIMIT_NS", static_cast<int64_t>(ptx::kWaitLimitNs));
   p->wait_ns = wait_ns > 0 ? wait_ns : static_cast<int64_t>(ptx::kWaitLimitNs);
   // Upper bound on the tile count must fit the kernel's 32-bit tile index (twice:
@@ -467,6 +474,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   // N: columns of b (and of b2, and of c); the Problem's n is twice that for the gated product.
   const uint64_t T = uint64_t(tokens), D1 = uint64_t(dim_a1), N = uint64_t(n_out), Z = uint64_t(z);
   const bool gather = (a_rows != nullptr);  // a is then fetched row by row, without a tensor map
+  const bool swap_maps = !gather && (p.swap_rows > 0 || p.light);
   if (p.mode == kNN) {
     const uint64_t da[2] = {D1, T};
     const uint32_t ba[2] = {kBlockK, uint32_t(kBlockM)};
@@ -478,7 +486,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     if (swiglu && (rc = encode_map(&map_b2, b2, 3, db, bb)) != 0) return rc;
     if (gather) map_a = map_b;
     else if ((rc = encode_map(&map_a, a, 2, da, ba)) != 0) return rc;
-    if (p.light) {  // transposed tiles fetch their few rows of a in boxes of 32
+    if (swap_maps) {  // swapped and transposed tiles fetch their few rows of a in boxes of 32
       const uint32_t bl[2] = {kBlockK, 32};
       if ((rc = encode_map(&map_a2, a, 2, da, bl)) != 0) return rc;
     }
@@ -492,10 +500,12 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     if (swiglu && (rc = encode_map(&map_b2, b2, 3, db, bb)) != 0) return rc;
     if (gather) map_a = map_b;
     else if ((rc = encode_map(&map_a, a, 2, da, ba)) != 0) return rc;
-    if (p.light) {  // transposed tiles: rows of a in boxes of 32, 128 rows of b[i] as the M operand
+    if (swap_maps) {
       const uint32_t bl[2] = {kBlockK, 32};
-      const uint32_t bw[3] = {kBlockK, uint32_t(kLightCols), 1};
       if ((rc = encode_map(&map_a2, a, 2, da, bl)) != 0) return rc;
+    }
+    if (p.light) {  // transposed tiles: 128 rows of b[i] as the M operand
+      const uint32_t bw[3] = {kBlockK, uint32_t(kLightCols), 1};
       if ((rc = encode_map(&map_b2, b, 3, db, bw)) != 0) return rc;
       have_b2 = true;
     }
@@ -516,7 +526,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   }
 
   if (!have_b2) map_b2 = map_b;  // unused by the kernel, but a valid map
-  if (!p.light) map_a2 = map_a;
+  if (!swap_maps) map_a2 = map_a;
 
   // Output map for the epilogue's TMA stores: 32 x 32 boxes, 64-byte swizzle; for
   // wgrad, whose c[z, m, n] is addressed as z*m rows, 64 x 32 boxes with 128-byte

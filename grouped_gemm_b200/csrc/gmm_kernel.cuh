@@ -102,7 +102,7 @@ struct Geometry {
 constexpr uint32_t kLightWBytes = kLightCols * kLightK * 2;        // 32 KiB
 constexpr uint32_t kLightWHalf = kLightWBytes / 2;                 // 16 KiB per 64 of k
 constexpr uint32_t kLightXHalf = kLightRows * kBlockK * 2;         // 8 KiB per 64 of k
-constexpr uint32_t kLightXBox = 32 * kBlockK * 2;                  // one 32-row TMA box: 4 KiB
+constexpr uint32_t kRowBoxBytes = 32 * kBlockK * 2;                // one 32-row TMA box of activations: 4 KiB
 static_assert(kLightWBytes + 2 * kLightXHalf <= Geometry<1>::kStageBytes, "a transposed stage must fit a ring slot");
 
 // The gather variant adds one warp per ring stage; each fetches the rows of A for
@@ -381,6 +381,10 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   // (map_a2: the activations with 32-row boxes; NT also uses map_b2: b with
   // 128-row boxes).
   constexpr bool kLight = (MODE != kTN) && (CTAS == 1) && !GATHER && !SWIGLU;
+  // Swapped tiles (schedule.cuh) exist wherever the rows of a tile are independent and
+  // one CTA holds all that an output element needs: not in the pair form of the gated
+  // product, whose gate and up columns lie in different CTAs.
+  constexpr bool kSwap = (MODE != kTN) && !(SWIGLU && CTAS == 2);
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = ptx::smem_u32(smem_raw);
@@ -402,7 +406,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       ptx::prefetch_tensormap(&map_a);
       ptx::prefetch_tensormap(&map_b);
       if (SWIGLU || (kLight && MODE == kNT)) ptx::prefetch_tensormap(&map_b2);
-      if (kLight) ptx::prefetch_tensormap(&map_a2);
+      if (kSwap && !GATHER) ptx::prefetch_tensormap(&map_a2);
       ptx::prefetch_tensormap(&map_c);
       for (int s = 0; s < kStages; ++s) {
         // the producer's expect_tx arrival, plus one arrival by the gather warp that owns
@@ -468,8 +472,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       Tile t;
       uint32_t s = 0, ph = 0;
       bool ok = true;
-      // Bytes this CTA's TMA loads bring per stage: the gather warps fetch A themselves.
-      constexpr uint32_t kTmaBytes = GATHER ? G::kBBytes : G::kStageBytes;
       const CUtensorMap* tn_a = my_maps;
       const CUtensorMap* tn_b = my_maps + 1;
       while (ok) {
@@ -482,7 +484,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           // operand) and the tile's rows x 128 k of a (the UMMA B operand, K-major,
           // fetched in boxes of 32 rows; rows past the tile's last are never stored).
           const int row_boxes = (t.valid_rows + 31) >> 5;
-          const uint32_t bytes = kLightWBytes + 2u * uint32_t(row_boxes) * kLightXBox;
+          const uint32_t bytes = kLightWBytes + 2u * uint32_t(row_boxes) * kRowBoxBytes;
           for (int kb = 0; kb < nkb; ++kb) {
             if (!ptx::mbar_wait(ptx::smem_u32(&tail->empty[s]), ph ^ 1u, wait)) { ok = false; break; }
             const uint32_t bar = ptx::smem_u32(&tail->full[s]);
@@ -499,7 +501,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
                 ptx::tma_load_3d(sw + h * kLightWHalf, &map_b2, bar, k0, t.col0, t.expert);
               }
               for (int i = 0; i < row_boxes; ++i)
-                ptx::tma_load_2d(sx + h * kLightXHalf + i * kLightXBox, &map_a2, bar, k0, t.row0 + i * 32);
+                ptx::tma_load_2d(sx + h * kLightXHalf + i * kRowBoxBytes, &map_a2, bar, k0, t.row0 + i * 32);
             }
             if (++s == kStages) { s = 0; ph ^= 1u; }
           }
@@ -517,6 +519,25 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             ptx::fence_tensormap_acquire(tn_b);
           }
         }
+        // A swapped tile fetches its rows in boxes of 32; in a pair each CTA stages half of them.
+        const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
+        const int sw_boxes = (sw_rows / CTAS + 31) >> 5;
+        const int a_row = t.row0 + (sw_rows != 0 ? static_cast<int>(cta_rank) * (sw_rows / CTAS) : row_off);
+        // Bytes this CTA's TMA loads bring per stage: the gather warps fetch A themselves.
+        const uint32_t tma_bytes =
+            G::kBBytes + (GATHER ? 0u : (sw_rows != 0 ? uint32_t(sw_boxes) * kRowBoxBytes : G::kABytes));
+        auto load_rows = [&](uint32_t dst, uint32_t bar, int k0) {  // A of a forward / dgrad stage
+          if (GATHER) return;
+          if (kSwap && sw_rows != 0) {
+            for (int i = 0; i < sw_boxes; ++i) {
+              if (kPair) ptx::tma_load_2d_pair(dst + i * kRowBoxBytes, &map_a2, bar, k0, a_row + i * 32);
+              else ptx::tma_load_2d(dst + i * kRowBoxBytes, &map_a2, bar, k0, a_row + i * 32);
+            }
+          } else {
+            if (kPair) ptx::tma_load_2d_pair(dst, &map_a, bar, k0, a_row);
+            else ptx::tma_load_2d(dst, &map_a, bar, k0, a_row);
+          }
+        };
         for (int kb = 0; kb < nkb; ++kb) {
           if (!ptx::mbar_wait(ptx::smem_u32(&tail->empty[s]), ph ^ 1u, wait)) { ok = false; break; }
           const uint32_t local_bar = ptx::smem_u32(&tail->full[s]);
@@ -524,9 +545,9 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           const uint32_t sb = sa + G::kABytes;
           const int k0 = kb * kBlockK;
           if (!kPair) {
-            ptx::mbar_arrive_expect_tx(local_bar, kTmaBytes);
+            ptx::mbar_arrive_expect_tx(local_bar, tma_bytes);
             if (MODE == kNN) {
-              if (!GATHER) ptx::tma_load_2d(sa, &map_a, local_bar, k0, t.row0);
+              load_rows(sa, local_bar, k0);
 #pragma unroll
               for (int j = 0; j < G::kBCols / 64; ++j)
                 if (SWIGLU)
@@ -535,7 +556,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
                 else
                   ptx::tma_load_3d(sb + j * kBoxBytes, &map_b, local_bar, t.col0 + j * 64, k0, t.expert);
             } else if (MODE == kNT) {
-              if (!GATHER) ptx::tma_load_2d(sa, &map_a, local_bar, k0, t.row0);
+              load_rows(sa, local_bar, k0);
               if (SWIGLU) {  // the maps' boxes are 128 rows of b high
                 ptx::tma_load_3d(sb, &map_b, local_bar, k0, t.col0 / 2, t.expert);
                 ptx::tma_load_3d(sb + G::kBBytes / 2, &map_b2, local_bar, k0, t.col0 / 2, t.expert);
@@ -565,10 +586,10 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             // Pair: this CTA stages rows [row0+row_off, +128) of A and columns
             // [col0+col_off, +128) of B.
             // Both CTAs' loads complete on the leader's barrier (shared::cluster address).
-            if (leader) ptx::mbar_arrive_expect_tx(local_bar, 2 * kTmaBytes);
+            if (leader) ptx::mbar_arrive_expect_tx(local_bar, 2 * tma_bytes);
             const uint32_t bar = ptx::mapa(local_bar, 0);
             if (MODE == kNN) {
-              if (!GATHER) ptx::tma_load_2d_pair(sa, &map_a, bar, k0, t.row0 + row_off);
+              load_rows(sa, bar, k0);
 #pragma unroll
               for (int j = 0; j < G::kBCols / 64; ++j)
                 if (SWIGLU)  // the leader stages the gate columns, its peer the up columns
@@ -578,7 +599,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
                   ptx::tma_load_3d_pair(sb + j * kBoxBytes, &map_b, bar, t.col0 + col_off + j * 64, k0,
                                         t.expert);
             } else if (MODE == kNT) {
-              if (!GATHER) ptx::tma_load_2d_pair(sa, &map_a, bar, k0, t.row0 + row_off);
+              load_rows(sa, bar, k0);
               if (SWIGLU) ptx::tma_load_3d_pair(sb, leader ? &map_b : &map_b2, bar, k0, t.col0 / 2, t.expert);
               else ptx::tma_load_3d_pair(sb, &map_b, bar, k0, t.col0 + col_off, t.expert);
             } else {
@@ -662,6 +683,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         __syncwarp();
         continue;
       }
+      const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
       for (int kb = 0; kb < nkb; ++kb) {
         const uint32_t f_bar = ptx::smem_u32(&tail->full[s]);
         // (gather variant of a pair: one arrival is the other CTA's gather warp)
@@ -669,7 +691,30 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         ptx::tc_fence_after_sync();
         const uint32_t sa = stage_base + s * G::kStageBytes;
         const uint32_t sb = sa + G::kABytes;
-        if (lane == 0) {
+        if (kSwap && sw_rows != 0) {
+          // D[weight columns, rows] = W^T x X^T: the staged B tile is the UMMA A operand
+          // (128 columns a CTA per MMA), the staged rows are the UMMA B operand.
+          if (lane == 0) {
+            const uint32_t idesc = ptx::make_idesc_bf16(kBlockM * CTAS, sw_rows, kBMn ? 1 : 0, 0);
+            const uint64_t xdesc = ptx::make_smem_desc(sa, 16u, 1024u);
+            constexpr uint64_t w_step = kBMn ? (2048u >> 4) : (32u >> 4);
+#pragma unroll
+            for (int k = 0; k < kBlockK / 16; ++k) {
+#pragma unroll
+              for (int h = 0; h < 2 / CTAS; ++h) {  // one CTA: the tile's two halves of 128 columns
+                const uint32_t sw = sb + uint32_t(h) * (G::kBBytes / 2);
+                const uint64_t wdesc = kBMn ? ptx::make_smem_desc(sw, kBoxBytes, 1024u)
+                                            : ptx::make_smem_desc(sw, 16u, 1024u);
+                const uint32_t d = d_tmem + uint32_t(h) * (kBlockN / 2);
+                const uint32_t acc = (kb | k) != 0 ? 1u : 0u;
+                if (kPair) ptx::mma_bf16_ss_pair(d, wdesc + k * w_step, xdesc + k * (32u >> 4), idesc, acc);
+                else ptx::mma_bf16_ss(d, wdesc + k * w_step, xdesc + k * (32u >> 4), idesc, acc);
+              }
+            }
+            if (kPair) ptx::mma_commit_pair(ptx::smem_u32(&tail->empty[s]), 0x3);
+            else ptx::mma_commit(ptx::smem_u32(&tail->empty[s]));
+          }
+        } else if (lane == 0) {
           // K-major SW128 operand: 8-row groups 1024 B apart, +32 B per 16-wide k step.
           // MN-major SW128 operand: 64-wide boxes 8 KiB apart (LBO), 8-k-row groups
           // 1024 B apart (SBO), +2048 B per 16-deep k step.
@@ -950,14 +995,18 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         continue;
       }
       if (next < base + nkb) {
+        // a swapped tile's rows are split evenly over the CTAs of a pair (kSwap)
+        const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
+        const int own_rows = sw_rows != 0 ? sw_rows / CTAS : kBlockM;
+        const int own_off = static_cast<int>(cta_rank) * own_rows;
         int idx[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          const int r = row_off + j * 4 + sub;  // row inside the (pair) tile
+          const int r = own_off + j * 4 + sub;  // row inside the (pair) tile
           // rows that do not exist are filled with zeros and never stored; so is a
           // row whose index lies outside a_src, which is also reported
           idx[j] = -1;
-          if (r < t.valid_rows) {
+          if (r < t.valid_rows && j * 4 + sub < own_rows) {
             const int ix = a_rows[t.row0 + r];
             if (ix >= 0 && ix < a_src_rows) idx[j] = ix;
             else bad_index = true;
@@ -1120,11 +1169,141 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       }
     };
 
+    // Swapped tile: 32 rows x 32 columns held transposed, v[i] = row i, this lane's
+    // column.  The values go through the staging buffer (row i at 64 i, so a warp's
+    // store of one row is 64 consecutive bytes) and leave as a TMA store when all 32
+    // rows exist, else row by row: lane i sends row i.
+    auto emit_swapped = [&](const uint32_t (&v)[32], int rows, int64_t row, int col, int out_n) {
+      const uint32_t buf = scatter_rows ? my_out : stage_buf();
+      if (scatter_rows) {
+        if (stores > 0) ptx::bulk_wait_group_read<0>();  // this lane's previous copy
+      } else if (lane == 0 && stores > 0) {
+        ptx::bulk_wait_group_read<G::kOutBufs - 1>();
+      }
+      __syncwarp();
+      // 64-byte swizzle as in emit(); a scattered row is read linearly by its copy
+      const uint32_t piece = uint32_t(lane) >> 3;
+      const uint32_t at = buf + (uint32_t(lane) & 7u) * 2u;
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        const uint32_t sw = scatter_rows ? piece : (piece ^ ((uint32_t(i) >> 1) & 3u));
+        const __nv_bfloat16 h = __float2bfloat16_rn(__uint_as_float(v[i]));
+        asm volatile("st.shared.b16 [%0], %1;" ::"r"(at + uint32_t(i) * 64u + (sw << 4)), "h"(__bfloat16_as_ushort(h))
+                     : "memory");
+      }
+      if (scatter_rows) {
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane < rows) {
+          const int64_t addr = row_dest[row + lane];
+          if (dest_ok(addr)) {
+            const int left = out_n - col;
+            const uint32_t bytes = left < 32 ? uint32_t(left) * 2u : 64u;
+            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(addr) + col;
+            const uint32_t src = buf + uint32_t(lane) * 64u;
+            if (reduce_add) ptx::bulk_reduce_add_bf16_1d(dst, src, bytes);
+            else ptx::bulk_store_1d(dst, src, bytes);
+            ptx::bulk_commit_group();
+          } else {
+            bad_dest = true;
+          }
+        }
+        ++stores;
+      } else if (rows >= 32) {
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          ptx::tma_store_2d(&map_c, buf, col, static_cast<int>(row));
+          ptx::bulk_commit_group();
+        }
+        ++stores;
+      } else {
+        __syncwarp();
+        if (lane < rows) {
+          uint4* dst = reinterpret_cast<uint4*>(c + (row + lane) * out_n + col);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint4 o;
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
+                         : "r"(buf + uint32_t(lane) * 64u + ((uint32_t(j) ^ ((uint32_t(lane) >> 1) & 3u)) << 4))
+                         : "memory");
+            if (col + j * 8 < out_n) dst[j] = o;
+          }
+        }
+      }
+    };
+
     while (ok) {
       const int pos = feed.take(true, lane);
       if (pos == kNoTile) { ok = false; break; }
       if (!walk.decode(pos, &t)) break;
       const int nkb = tile_stages(t);
+      const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
+      if (kSwap && sw_rows != 0) {
+        // TMEM lane = output column, TMEM column = output row.  One CTA: this warp's
+        // half of the tile's columns is an accumulator of its own (for the gated
+        // product the two are gate and up of the same 128 output columns).  A pair:
+        // each CTA holds 128 of the columns.  Where both warps of a lane quadrant
+        // serve the same columns they take the 32-row chunks in turn.
+        constexpr bool kShareColumns = kPair || SWIGLU;
+        const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
+        ++it;
+        if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), aph, wait)) { ok = false; break; }
+        ptx::tc_fence_after_sync();
+        const int out_n = static_cast<int>(SWIGLU ? (p.n >> 1) : p.n);
+        const int col = (SWIGLU ? (t.col0 >> 1) : t.col0) + (kPair ? col_off : (SWIGLU ? 0 : col_base)) + q * 32;
+        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + (kShareColumns ? 0 : col_base);
+        if (col < out_n) {
+          for (int r0 = kShareColumns ? half * 32 : 0; r0 < t.valid_rows; r0 += kShareColumns ? 64 : 32) {
+            const int rows = t.valid_rows - r0;
+            const int64_t row = int64_t(t.row0) + r0;
+            uint32_t va[32], vb[32];
+            ptx::tmem_ld_32x32(taddr + uint32_t(r0), va);
+            if (SWIGLU) ptx::tmem_ld_32x32(taddr + kBlockN / 2 + uint32_t(r0), vb);
+            ptx::tmem_ld_wait();
+            if (SWIGLU && gate_grad != nullptr) {
+              // as in the plain tile's backward epilogue below
+              const __nv_bfloat16* src = gate_grad + row * out_n + col + lane;
+              const bool col_ok = col + lane < out_n;
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                const float dh = (col_ok && i < rows) ? __bfloat162float(src[int64_t(i) * out_n]) : 0.0f;
+                const float g = __uint_as_float(va[i]);
+                const float u = __uint_as_float(vb[i]);
+                const float sg = __fdividef(1.0f, 1.0f + __expf(-g));
+                va[i] = __float_as_uint(dh * u * sg * (1.0f + g * (1.0f - sg)));
+                vb[i] = __float_as_uint(dh * g * sg);
+              }
+              emit_swapped(va, rows, row, col, out_n);
+              emit_swapped(vb, rows, row + p.tokens, col, out_n);
+              continue;
+            }
+            if (SWIGLU) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) {
+                const float g = __uint_as_float(va[i]);
+                va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * __uint_as_float(vb[i]));
+              }
+            }
+            if (scatter_rows && row_scale != nullptr) {
+              const float w = lane < rows ? row_scale[row + lane] : 1.0f;
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                va[i] = __float_as_uint(__uint_as_float(va[i]) * __shfl_sync(0xffffffffu, w, i));
+            }
+            emit_swapped(va, rows, row, col, out_n);
+          }
+        }
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
+          if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(te_bar, 0));
+          else ptx::mbar_arrive(te_bar);
+        }
+        continue;
+      }
       if (kLight && t.kind) {
         // Transposed tile: TMEM lane = output column, TMEM column = output row.  This
         // warp reads the 32 output columns of its lane quadrant for its half of the
