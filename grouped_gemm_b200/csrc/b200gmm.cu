@@ -99,7 +99,7 @@ template <int MODE, int CTAS, bool GATHER, bool SWIGLU, bool PUSH = false>
 cudaError_t launch_gmm(const LaunchArgs& a) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.grid);
-  cfg.blockDim = dim3(GATHER ? gather_threads<CTAS, MODE>() : (PUSH ? kGemmPushThreads : kThreads));
+  cfg.blockDim = dim3(GATHER ? GatherWarps<CTAS>::kBlockThreads : (PUSH ? kGemmPushThreads : kThreads));
   cfg.dynamicSmemBytes = PUSH ? kSmemBytesPush : kSmemBytes;
   cfg.stream = a.stream;
   cudaLaunchAttribute attr[1];
@@ -529,14 +529,15 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   if (!swap_maps) map_a2 = map_a;
 
   // Output map for the epilogue's TMA stores: 32 x 32 boxes, 64-byte swizzle; for
-  // wgrad, whose c[z, m, n] is addressed as z*m rows, 64 x 32 boxes with 128-byte
+  // plain wgrad (c[z, m, n] is addressed as z*m rows) 64 x 32 boxes with 128-byte
   // swizzle.  Unused (left zeroed) when the rows are scattered through row_dest.
   CUtensorMap map_c = {};
   if (row_dest == nullptr) {
     const uint64_t dc[2] = {N, p.mode == kTN ? Z * D1 : (gate_grad != nullptr ? 2 * T : T)};
-    const uint32_t bc[2] = {p.mode == kTN ? 64u : 32u, 32};
+    const bool wide = p.mode == kTN && !gather;  // Geometry::kWideOut
+    const uint32_t bc[2] = {wide ? 64u : 32u, 32};
     if (dc[1] >= (uint64_t(1) << 31)) return B200GMM_ELIMIT;
-    if ((rc = encode_map(&map_c, c, 2, dc, bc, p.mode == kTN ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B)) != 0)
+    if ((rc = encode_map(&map_c, c, 2, dc, bc, wide ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B)) != 0)
       return rc;
   }
 

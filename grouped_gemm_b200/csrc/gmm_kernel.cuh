@@ -33,9 +33,9 @@
 //               multicast is used anywhere.
 //
 // Optional template variants:
-//   GATHER      row i of A is row a_rows[i] of another tensor: one extra warp per
-//               ring stage fetches the rows with cp.async in place of the TMA box
-//               loads of A (B still comes by TMA); also for wgrad, where the
+//   GATHER      row i of A is row a_rows[i] of another tensor: extra warps fetch
+//               the rows with cp.async in place of the TMA box loads of A (B still
+//               comes by TMA); also for wgrad, where the
 //               gathered rows are the contraction;
 //   SWIGLU      (forward / dgrad layouts) two right operands; the accumulator holds
 //               128 gate and 128 up columns and the epilogue writes silu(gate) * up.
@@ -82,12 +82,15 @@ constexpr int kSchedSlots = 8;
 // speed of its output stores.  Each epilogue warp has two buffers of 32 rows x 64
 // columns there (128-byte rows), used in turn, so that a warp fills one while
 // the TMA store of the other still reads; the forward / dgrad layouts have one
-// buffer of 32 x 32 per warp.
-template <int CTAS, int MODE = kNN>
+// buffer of 32 x 32 per warp.  So has the gathered wgrad: a warp that fetches rows
+// with cp.async needs over a microsecond from a free stage to a full one, and four
+// stages of a pair (0.28 us of MMAs each) do not cover that.
+template <int CTAS, int MODE = kNN, bool GATHER = false>
 struct Geometry {
-  static constexpr int kStages = (MODE == kTN) ? ((CTAS == 1) ? 3 : 4) : ((CTAS == 1) ? 4 : 6);
-  static constexpr int kOutBufs = (MODE == kTN) ? 2 : 1;  // staging buffers per epilogue warp
-  static constexpr uint32_t kOutBufBytes = (MODE == kTN) ? 4096u : 2048u;
+  static constexpr bool kWideOut = (MODE == kTN) && !GATHER;  // 64-column stores from double buffers
+  static constexpr int kStages = kWideOut ? ((CTAS == 1) ? 3 : 4) : ((CTAS == 1) ? 4 : 6);
+  static constexpr int kOutBufs = kWideOut ? 2 : 1;  // staging buffers per epilogue warp
+  static constexpr uint32_t kOutBufBytes = kWideOut ? 4096u : 2048u;
   static constexpr int kBCols = kBlockN / CTAS;                 // B columns staged by one CTA
   static constexpr uint32_t kABytes = kBlockM * kBlockK * 2;    // 16 KiB
   static constexpr uint32_t kBBytes = kBCols * kBlockK * 2;     // 32 or 16 KiB
@@ -105,10 +108,15 @@ constexpr uint32_t kLightXHalf = kLightRows * kBlockK * 2;         // 8 KiB per 
 constexpr uint32_t kRowBoxBytes = 32 * kBlockK * 2;                // one 32-row TMA box of activations: 4 KiB
 static_assert(kLightWBytes + 2 * kLightXHalf <= Geometry<1>::kStageBytes, "a transposed stage must fit a ring slot");
 
-// The gather variant adds one warp per ring stage; each fetches the rows of A for
-// the k-blocks that land in its stage.
-template <int CTAS, int MODE = kNN>
-constexpr int gather_threads() { return kThreads + 32 * Geometry<CTAS, MODE>::kStages; }
+// The gather variant adds warps that fetch the rows of A, a k-block each, in turn.
+// Four beside the four stages of the one-CTA ring, five beside the six of a pair: with
+// 11 + 5 = 16 warps a thread may use 128 registers, a 17th would leave 96 (an SM
+// quarter then holds five warps) and spill, and the sixth stage is the one being used.
+template <int CTAS>
+struct GatherWarps {
+  static constexpr int kWarps = CTAS == 1 ? 4 : 5;
+  static constexpr int kBlockThreads = kThreads + 32 * kWarps;
+};
 
 // The push variant adds four warps that move rows between GPUs while the tensor
 // cores work (in the default, bulk-copy form of the transfer only one of their
@@ -357,7 +365,7 @@ struct TileFeed {
 };
 
 template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false>
-__global__ void __launch_bounds__(GATHER ? gather_threads<CTAS, MODE>() : (PUSH ? kGemmPushThreads : kThreads), 1)
+__global__ void __launch_bounds__(GATHER ? GatherWarps<CTAS>::kBlockThreads : (PUSH ? kGemmPushThreads : kThreads), 1)
 gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
            const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_c,
            const __grid_constant__ CUtensorMap map_a2, __nv_bfloat16* __restrict__ c,
@@ -374,7 +382,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   // [0,128) are a @ b[:, c0 .. c0+128), columns [128,256) are a @ b2[:, c0 ..
   // c0+128) with c0 = col0 / 2, and the epilogue writes the 128 output columns
   // silu(gate) * up.
-  using G = Geometry<CTAS, MODE>;
+  using G = Geometry<CTAS, MODE, GATHER>;
   constexpr int kStages = G::kStages;
   constexpr bool kPair = (CTAS == 2);
   // Transposed tiles exist in the plain one-CTA forward / dgrad kernels only
@@ -409,7 +417,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       if (kSwap && !GATHER) ptx::prefetch_tensormap(&map_a2);
       ptx::prefetch_tensormap(&map_c);
       for (int s = 0; s < kStages; ++s) {
-        // the producer's expect_tx arrival, plus one arrival by the gather warp that owns
+        // the producer's expect_tx arrival, plus one arrival by the gather warp that fills
         // this stage in each CTA
         ptx::mbar_init(ptx::smem_u32(&tail->full[s]), 1 + (GATHER ? CTAS : 0));
         ptx::mbar_init(ptx::smem_u32(&tail->empty[s]), 1);
@@ -420,7 +428,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       }
       // Takers of a published tile position: per CTA the producer thread, the epilogue
       // warps and the gather warps, plus the leader's MMA warp.
-      constexpr uint32_t kTakers = CTAS * (1 + kEpilogueWarps + (GATHER ? kStages : 0)) + 1;
+      constexpr uint32_t kTakers = CTAS * (1 + kEpilogueWarps + (GATHER ? GatherWarps<CTAS>::kWarps : 0)) + 1;
       for (int i = 0; i < kSchedSlots; ++i) {
         ptx::mbar_init(ptx::smem_u32(&tail->sched_full[i]), 1);
         ptx::mbar_init(ptx::smem_u32(&tail->sched_empty[i]), kTakers);
@@ -913,27 +921,45 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   } else if (GATHER && warp > kSchedWarp) {
     // ---------------------------------------------------------- A-row gather
     // The caller's sort-by-expert fused into the load: row i of the grouped
-    // operand is row a_rows[i] of a_src (rows of p.d1 elements).  Gather warp w
-    // owns ring stage w: it fills it for every k-block that lands there (every
-    // kStages-th of the stream of k-blocks, which runs on across tiles), waits for
-    // its own copies and reports the stage full, so that as with the TMA loads
-    // every stage can be in flight at once.  A warp copies this CTA's 128 x 64
+    // operand is row a_rows[i] of a_src (rows of p.d1 elements).  The gather
+    // warps take the k-blocks in turn (the stream of k-blocks, and of ring stages, runs
+    // on across tiles); each waits for its stage to be free, fills it, waits for its own
+    // copies and reports the stage full, so that as many stages are in flight as there
+    // are gather warps.  A warp copies this CTA's 128 x 64
     // tile with 16-byte cp.async: eight neighbouring lanes cover the 128 bytes of
     // one row, a lane serves rows sub, sub + 4, .. sub + 124, and writes the
     // K-major 128-byte-swizzled layout a TMA box load would leave (16-byte chunk
     // index ^= row % 8).
-    const int w = warp - (kSchedWarp + 1);  // the stage this warp owns
+    constexpr int kGatherWarps = GatherWarps<CTAS>::kWarps;
     const int chunk = lane & 7;
     const int sub = lane >> 3;
-    const uint32_t stage_addr = stage_base + uint32_t(w) * G::kStageBytes;
-    const uint32_t full_bar = kPair ? ptx::mapa(ptx::smem_u32(&tail->full[w]), 0) : ptx::smem_u32(&tail->full[w]);
-    const uint32_t empty_bar = ptx::smem_u32(&tail->empty[w]);
+    // Row 4 i + sub of a 64- or 128-row block lands at 512 i + row_dst[i & 1]: the
+    // swizzle of a row depends on its last three bits only.  With one 32 x 32 -> 64 bit
+    // multiply-add per row that is all the arithmetic a copy needs; with it spelled out
+    // per copy a warp was busy issuing for longer than its copies were in flight.  What
+    // is left bounds the variant by latency, not by power as the plain kernels: gathered
+    // wgrad of 16384 rows, 4096 x 14336: 2.73 ms with four stages, 2.37 with six, 2.0 to
+    // 2.1 with this; without the gather 1.66.
+    const uint32_t row_dst[2] = {uint32_t(sub) * 128u + (uint32_t(chunk ^ sub) << 4),
+                                 uint32_t(sub) * 128u + (uint32_t(chunk ^ (sub + 4)) << 4)};
+    const uint32_t row_bytes = static_cast<uint32_t>(p.d1) * 2u;
+    auto row_offset = [&](int row) { return static_cast<uint64_t>(static_cast<uint32_t>(row)) * row_bytes; };
+    const uint32_t full_bar0 = kPair ? ptx::mapa(ptx::smem_u32(&tail->full[0]), 0) : ptx::smem_u32(&tail->full[0]);
+    const uint32_t empty_bar0 = ptx::smem_u32(&tail->empty[0]);
     TileWalker walk(p, tail);
     TileFeed<kPair> feed(tail, wait, !leader);
     Tile t;
-    uint32_t ph = 0;  // parity of this stage's current use
-    int next = w;     // position in the stream of k-blocks of this warp's next one
+    // position in the stream of k-blocks of this warp's next one, the ring stage it
+    // lands in and the parity of that stage's use
+    int next = warp - (kSchedWarp + 1);
+    int stage = next;
+    uint32_t ph = 0;
     int base = 0;     // k-blocks of the stream before the current tile
+    auto advance = [&]() {
+      next += kGatherWarps;
+      stage += kGatherWarps;
+      if (stage >= kStages) { stage -= kStages; ph ^= 1u; }
+    };
     bool ok = true;
     bool bad_index = false;
     while (ok) {
@@ -962,26 +988,41 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           }
         };
         if (next < base + nkb) load_idx(next - base);
-        for (; next < base + nkb; next += kStages) {
-          if (lane == 0) ok = ptx::mbar_wait(empty_bar, ph ^ 1u, wait);
+        for (; next < base + nkb; advance()) {
+          if (lane == 0) ok = ptx::mbar_wait(empty_bar0 + uint32_t(stage) * 8u, ph ^ 1u, wait);
           ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
           if (!ok) break;
+          const uint32_t stage_addr = stage_base + uint32_t(stage) * G::kStageBytes;
+          const uint32_t full_bar = full_bar0 + uint32_t(stage) * 8u;
+          // (the box's 128 bytes lie next to each other: the same row offset serves both)
+          const int col = t.row0 + row_off + chunk * 8;  // column of a_src in the first box
+          const char* src0 = reinterpret_cast<const char*>(a_src) + int64_t(col) * 2;
+          bool whole = col + 64 < p.d1;  // d1 is a multiple of 8: a piece is all in or all out
 #pragma unroll
-          for (int j = 0; j < kBlockM / 64; ++j) {
-            const int col = t.row0 + row_off + j * 64 + chunk * 8;  // column of a_src
-            const bool in_m = col < p.d1;  // d1 is a multiple of 8
+          for (int i = 0; i < 16; ++i) whole = whole && idx[i] >= 0;
+          if (__all_sync(0xffffffffu, whole)) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-              const int r = i * 4 + sub;
-              const uint32_t dst = stage_addr + uint32_t(j) * kBoxBytes + uint32_t(r) * 128u +
-                                   (uint32_t(chunk ^ (r & 7)) << 4);
-              const bool live = in_m && idx[i] >= 0;
-              ptx::cp_async_16(dst, live ? static_cast<const void*>(a_src + int64_t(idx[i]) * p.d1 + col) : a_src,
-                               live ? 16u : 0u);
+              const char* src = src0 + row_offset(idx[i]);
+              const uint32_t dst = stage_addr + row_dst[i & 1] + uint32_t(i) * 512u;
+              ptx::cp_async_16(dst, src);
+              ptx::cp_async_16(dst + kBoxBytes, src + 128);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < kBlockM / 64; ++j) {
+              const bool in_m = col + j * 64 < p.d1;
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const bool live = in_m && idx[i] >= 0;
+                ptx::cp_async_16(stage_addr + uint32_t(j) * kBoxBytes + row_dst[i & 1] + uint32_t(i) * 512u,
+                                 live ? src0 + row_offset(idx[i]) + j * 128 : reinterpret_cast<const char*>(a_src),
+                                 live ? 16u : 0u);
+              }
             }
           }
           // the indices of this warp's next k-block of the tile arrive while the copies fly
-          if (next + kStages < base + nkb) load_idx(next + kStages - base);
+          if (next + kGatherWarps < base + nkb) load_idx(next + kGatherWarps - base);
           ptx::cp_async_wait_all();
           ptx::fence_proxy_async_smem();
           __syncwarp();
@@ -989,7 +1030,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             if (kPair) ptx::mbar_arrive_cluster(full_bar);
             else ptx::mbar_arrive(full_bar);
           }
-          ph ^= 1u;
         }
         base += nkb;
         continue;
@@ -1000,6 +1040,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         const int own_rows = sw_rows != 0 ? sw_rows / CTAS : kBlockM;
         const int own_off = static_cast<int>(cta_rank) * own_rows;
         int idx[32];
+        bool all_rows = true;  // every row of this lane exists
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           const int r = own_off + j * 4 + sub;  // row inside the (pair) tile
@@ -1011,20 +1052,28 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             if (ix >= 0 && ix < a_src_rows) idx[j] = ix;
             else bad_index = true;
           }
+          all_rows = all_rows && idx[j] >= 0;
         }
-        for (; next < base + nkb; next += kStages) {
-          if (lane == 0) ok = ptx::mbar_wait(empty_bar, ph ^ 1u, wait);
+        for (; next < base + nkb; advance()) {
+          if (lane == 0) ok = ptx::mbar_wait(empty_bar0 + uint32_t(stage) * 8u, ph ^ 1u, wait);
           ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
           if (!ok) break;
+          const uint32_t stage_addr = stage_base + uint32_t(stage) * G::kStageBytes;
+          const uint32_t full_bar = full_bar0 + uint32_t(stage) * 8u;
           const int kcol = (next - base) * kBlockK + chunk * 8;
-          const bool in_k = kcol < p.d1;  // d1 is a multiple of 8: a chunk is all in or all out
+          const bool in_k = kcol < p.d1;  // d1 is a multiple of 8: a piece is all in or all out
+          const char* src0 = reinterpret_cast<const char*>(a_src) + int64_t(kcol) * 2;
+          if (__all_sync(0xffffffffu, in_k && all_rows)) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int r = j * 4 + sub;
-            const uint32_t dst = stage_addr + uint32_t(r) * 128u + (uint32_t(chunk ^ (r & 7)) << 4);
-            const bool live = in_k && idx[j] >= 0;
-            ptx::cp_async_16(dst, live ? static_cast<const void*>(a_src + int64_t(idx[j]) * p.d1 + kcol) : a_src,
-                             live ? 16u : 0u);
+            for (int j = 0; j < 32; ++j)
+              ptx::cp_async_16(stage_addr + row_dst[j & 1] + uint32_t(j) * 512u, src0 + row_offset(idx[j]));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const bool live = in_k && idx[j] >= 0;
+              ptx::cp_async_16(stage_addr + row_dst[j & 1] + uint32_t(j) * 512u,
+                               live ? src0 + row_offset(idx[j]) : reinterpret_cast<const char*>(a_src), live ? 16u : 0u);
+            }
           }
           ptx::cp_async_wait_all();
           // this lane's copies are complete: make them visible to the tensor core's
@@ -1035,7 +1084,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             if (kPair) ptx::mbar_arrive_cluster(full_bar);
             else ptx::mbar_arrive(full_bar);
           }
-          ph ^= 1u;
         }
       }
       base += nkb;
@@ -1118,7 +1166,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       if (col >= cols_left) return;  // chunk lies entirely past the last column
       uint4 o[4];
       pack(v, o);
-      if (MODE != kTN && warp_full) {
+      if (!G::kWideOut && warp_full) {
         // The store that last read this buffer must be done reading.
         const uint32_t buf = stage_buf();
         if (lane == 0 && stores > 0) ptx::bulk_wait_group_read<G::kOutBufs - 1>();
@@ -1384,7 +1432,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       uint32_t va[32], vb[32];
       if (MODE == kTN && nkb == 0) {  // (forward and dgrad tiles always have k > 0)
         // Empty wgrad expert: its block of the output is zeros.
-        if (warp_full) {
+        if (G::kWideOut && warp_full) {
           // Zeros need staging once: every store of this tile reads the same buffer,
           // so none of them waits for the one before.
           const uint32_t buf = stage_buf();
@@ -1480,7 +1528,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         continue;
       }
       const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + col_base;
-      if (MODE == kTN && warp_full) {
+      if (G::kWideOut && warp_full) {
 #pragma unroll 1
         for (int ch = 0; ch < kBlockN / 64; ch += 2) {
           ptx::tmem_ld_32x32(taddr + ch * 32, va);
