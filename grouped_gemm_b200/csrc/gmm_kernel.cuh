@@ -16,9 +16,9 @@
 //               store; a warp whose 32 rows do not all exist (ragged last tile of
 //               an expert) stores its valid rows directly;
 //   warp 10     scheduler (leader CTA): draws tile positions from a global counter,
-//               several tiles ahead of the other roles, and hands them over through
-//               a small ring in shared memory (in both CTAs of a pair); for wgrad
-//               it also prepares, ahead of time, the tensor maps clipped to the
+//               several tiles ahead of the other roles, works out the tile of each and
+//               hands it over through a small ring in shared memory (in both CTAs of a
+//               pair); for wgrad it also prepares, ahead of time, the tensor maps clipped to the
 //               expert a tile belongs to.
 //
 // Two variants, chosen on the host:
@@ -71,7 +71,7 @@ constexpr uint32_t kBoxBytes = 64 * kBlockK * 2;  // one 64-wide MN-major TMA bo
 // MMA warp counts finished tiles).
 constexpr int kMapSlots = 8;
 constexpr int kMaxCtas = 256;  // workspace is sized for this many CTAs
-// Ring through which the scheduler hands tile positions to the other roles.  Deep
+// Ring through which the scheduler hands tiles to the other roles.  Deep
 // enough that the producer can run ahead by a ring of one-stage tiles plus both
 // accumulators, and that the scheduler's own latencies (the counter's round trip,
 // a tensor-map edit) stay hidden behind tiles already handed out.
@@ -147,15 +147,30 @@ constexpr int kPushChunks = 3;
 constexpr uint32_t kPushStageBytes = kPushChunkBytes * kPushChunks;
 
 
-struct __align__(8) SmemTail {
+// One slot of the scheduler's ring: a position of the launch order and its tile,
+// worked out once by the scheduler.  (Every role decoding positions for itself, three
+// integer divisions and a chain of shared-memory reads per tile, cost the epilogue of
+// a tile of one or two k-blocks as much time as reading its accumulator.)
+struct __align__(16) TileRecord {
+  int pos;
+  int map;          // wgrad: map slot of the tile (kMapFresh: edited for this tile), else 0
+  int expert;       // -1: the launch order is exhausted
+  int kind;
+  int row0, col0;
+  int valid_rows;
+  int k_len;
+  int k_row0;
+  int pad[3];
+};
+
+struct __align__(16) SmemTail {
   uint64_t full[kMaxStages];
   uint64_t empty[kMaxStages];
   uint64_t tmem_full[2];
   uint64_t tmem_empty[2];
   uint64_t sched_full[kSchedSlots];
   uint64_t sched_empty[kSchedSlots];
-  int sched_tile[kSchedSlots];      // position of the launch order
-  int sched_map[kSchedSlots];       // wgrad: map slot of the tile (bit 30: freshly edited), else 0
+  TileRecord sched_tile[kSchedSlots];
   uint32_t tiles_done;              // tiles of this cluster whose loads have all landed
   uint32_t tmem_base;
   uint32_t abort_flag;
@@ -269,8 +284,8 @@ __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* 
   }
 }
 
-// Position of the launch order -> tile.  Every role keeps its own copy; positions
-// arrive in increasing order, so the expert cursor only ever moves forward.
+// Position of the launch order -> tile (the scheduler's).  Positions come in
+// increasing order, so the expert cursor only ever moves forward.
 struct TileWalker {
   const Problem& p;
   const SmemTail* tail;
@@ -287,21 +302,20 @@ struct TileWalker {
   }
 };
 
-// Where a role's tile positions come from: the leader CTA's scheduler thread
-// publishes each position (and, for wgrad, the tile's map slot) through
-// sched_tile / sched_map / sched_full, in its own CTA and in its peer; every other
+// Where a role's tiles come from: the leader CTA's scheduler thread publishes each
+// tile through sched_tile / sched_full, in its own CTA and in its peer; every other
 // role takes them from there and releases the slot on the leader's sched_empty.
-constexpr int kNoTile = -1;  // a wait was abandoned
-constexpr int kMapFresh = 1 << 30;  // sched_map flag: the slot was edited for this tile
+enum Taken { kTile, kEndOfOrder, kAbandoned };  // kAbandoned: a wait gave up
+constexpr int kMapFresh = 1 << 30;  // TileRecord::map flag: the slot was edited for this tile
 
 template <bool kPair>
 struct TileFeed {
   SmemTail* tail;
   ptx::WaitCtx wait;
   uint32_t taken;   // positions taken (or published) so far
-  int map;          // sched_map entry of the position taken last
+  int map;          // map slot of the tile taken last
   bool remote;      // this role sits in the peer CTA: what it reads was written from the leader
-  int last;         // position taken last (-1: none yet)
+  int last;         // launch-order position taken last (-1: none yet)
   uint32_t sum;     // sum of the positions taken
 
   __device__ TileFeed(SmemTail* tail_, const ptx::WaitCtx& w, bool in_peer = false)
@@ -314,16 +328,19 @@ struct TileFeed {
   }
 
   // Consumer side, called by every lane of a warp (warp_wide) or by one thread.
-  __device__ __forceinline__ int take(bool warp_wide, int lane) {
+  __device__ __forceinline__ Taken take(bool warp_wide, int lane, Tile* tile) {
     const uint32_t slot = taken % kSchedSlots;
     const uint32_t parity = (taken / kSchedSlots) & 1u;
     ++taken;
     const uint32_t full = ptx::smem_u32(&tail->sched_full[slot]);
     const bool got = (kPair && remote) ? ptx::mbar_wait<true, 32>(full, parity, wait)
                                        : ptx::mbar_wait<false, 32>(full, parity, wait);
-    if (!got) return kNoTile;
-    const int t = *reinterpret_cast<volatile int*>(&tail->sched_tile[slot]);
-    map = *reinterpret_cast<volatile int*>(&tail->sched_map[slot]);
+    if (!got) return kAbandoned;
+    const uint32_t rec = ptx::smem_u32(&tail->sched_tile[slot]);
+    int t, unused[3];
+    ptx::ld_shared_v4(rec, &t, &map, &tile->expert, &tile->kind);
+    ptx::ld_shared_v4(rec + 16, &tile->row0, &tile->col0, &tile->valid_rows, &tile->k_len);
+    ptx::ld_shared_v4(rec + 32, &tile->k_row0, &unused[0], &unused[1], &unused[2]);
     // Self-check of the hand-off: positions reach every role in strictly
     // increasing order.  One that does not is never used: the fault is recorded,
     // the launch is told to drain, and this role stops (warp-uniformly).
@@ -332,32 +349,37 @@ struct TileFeed {
     if (bad) {
       tail->handoff_fault = 1u;
       *wait.abort_flag = 1u;
-      return kNoTile;
+      return kAbandoned;
     }
     last = t;
     sum += static_cast<uint32_t>(t);
     if (warp_wide) __syncwarp();
     if (!warp_wide || lane == 0) {
-      // Both values are in registers: the slot may be overwritten from here on.
+      // The record is in registers: the slot may be overwritten from here on.
       const uint32_t bar = ptx::smem_u32(&tail->sched_empty[slot]);
       if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(bar, 0));
       else ptx::mbar_arrive(bar);
     }
-    return t;
+    return tile->expert < 0 ? kEndOfOrder : kTile;
   }
 
-  // Scheduler side (one thread of the leader CTA): hand position t to everyone.
-  __device__ __forceinline__ bool publish(int t, int map_entry) {
+  // Scheduler side (one thread of the leader CTA): hand position t and its tile
+  // (expert -1: the end) to everyone.
+  __device__ __forceinline__ bool publish(int t, int map_entry, const Tile& tile) {
     const uint32_t slot = taken % kSchedSlots;
     const uint32_t parity = (taken / kSchedSlots) & 1u;
     ++taken;
     if (!ptx::mbar_wait<kPair, 0>(ptx::smem_u32(&tail->sched_empty[slot]), parity ^ 1u, wait)) return false;
-    *reinterpret_cast<volatile int*>(&tail->sched_tile[slot]) = t;
-    *reinterpret_cast<volatile int*>(&tail->sched_map[slot]) = map_entry;
+    const uint32_t rec = ptx::smem_u32(&tail->sched_tile[slot]);
+    ptx::st_shared_v4(rec, t, map_entry, tile.expert, tile.kind);
+    ptx::st_shared_v4(rec + 16, tile.row0, tile.col0, tile.valid_rows, tile.k_len);
+    ptx::st_shared_v4(rec + 32, tile.k_row0, 0, 0, 0);
     ptx::mbar_arrive(ptx::smem_u32(&tail->sched_full[slot]));
     if (kPair) {
-      ptx::st_shared_cluster_u32(ptx::mapa(ptx::smem_u32(&tail->sched_tile[slot]), 1), static_cast<uint32_t>(t));
-      ptx::st_shared_cluster_u32(ptx::mapa(ptx::smem_u32(&tail->sched_map[slot]), 1), static_cast<uint32_t>(map_entry));
+      const uint32_t peer = ptx::mapa(rec, 1);
+      ptx::st_shared_cluster_v4(peer, t, map_entry, tile.expert, tile.kind);
+      ptx::st_shared_cluster_v4(peer + 16, tile.row0, tile.col0, tile.valid_rows, tile.k_len);
+      ptx::st_shared_cluster_v4(peer + 32, tile.k_row0, 0, 0, 0);
       ptx::mbar_arrive_release_cluster(ptx::mapa(ptx::smem_u32(&tail->sched_full[slot]), 1));
     }
     return true;
@@ -475,7 +497,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   if (warp == 0) {
     // ---------------------------------------------------------- TMA producer
     if (lane == 0) {
-      TileWalker walk(p, tail);
       TileFeed<kPair> feed(tail, wait, !leader);
       Tile t;
       uint32_t s = 0, ph = 0;
@@ -483,9 +504,9 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       const CUtensorMap* tn_a = my_maps;
       const CUtensorMap* tn_b = my_maps + 1;
       while (ok) {
-        const int pos = feed.take(false, 0);
-        if (pos == kNoTile) { ok = false; break; }
-        if (!walk.decode(pos, &t)) break;
+        const Taken got = feed.take(false, 0, &t);
+        if (got == kAbandoned) { ok = false; break; }
+        if (got == kEndOfOrder) break;
         const int nkb = tile_stages(t);
         if (kLight && t.kind) {
           // Transposed tile: per stage 128 columns x 128 k of b[expert] (the UMMA A
@@ -638,7 +659,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     __syncwarp();
   } else if (warp == 1 && leader) {
     // ---------------------------------------------------------- MMA issuer
-    TileWalker walk(p, tail);
     TileFeed<kPair> feed(tail, wait, !leader);
     Tile t;
     uint32_t s = 0, ph = 0, it = 0;
@@ -649,9 +669,9 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       if (MODE == kTN && lane == 0) *reinterpret_cast<volatile uint32_t*>(&tail->tiles_done) = feed.taken;
     };
     while (ok) {
-      const int pos = feed.take(true, lane);
-      if (pos == kNoTile) { ok = false; break; }
-      if (!walk.decode(pos, &t)) break;
+      const Taken got = feed.take(true, lane, &t);
+      if (got == kAbandoned) { ok = false; break; }
+      if (got == kEndOfOrder) break;
       const int nkb = tile_stages(t);
       if (nkb == 0) { loads_landed(); continue; }  // empty wgrad expert: the epilogue writes zeros
       const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
@@ -774,7 +794,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       if (lane == 0) {
         TileWalker walk(p, tail);
         TileFeed<kPair> feed(tail, wait, !leader);
-        Tile t;
+        Tile t = {};
         // wgrad: the map slot clipped to the current expert, and for every slot the
         // index (in this cluster's sequence of tiles) of the last tile that loads
         // through it.
@@ -791,6 +811,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         while (ok) {
           int entry = 0;
           const bool live = walk.decode(pos, &t);
+          if (!live) t.expert = -1;
           if (MODE == kTN && live && t.k_len > 0) {
             if (held_expert != t.expert) {
               // New expert: clip the row extent of a and b at its last row, in the next
@@ -822,7 +843,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             entry |= held_slot;
             last_tile[held_slot] = static_cast<int>(feed.taken);
           }
-          if (!feed.publish(pos, entry)) { ok = false; break; }
+          if (!feed.publish(pos, entry, t)) { ok = false; break; }
           if (!live) break;  // the end of the order has been handed to everyone
           pos = static_cast<int>(drawn) + tile_stride;
           if (pos < walk.total) drawn = atomicAdd(sched_counter, 1u);
@@ -946,7 +967,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     auto row_offset = [&](int row) { return static_cast<uint64_t>(static_cast<uint32_t>(row)) * row_bytes; };
     const uint32_t full_bar0 = kPair ? ptx::mapa(ptx::smem_u32(&tail->full[0]), 0) : ptx::smem_u32(&tail->full[0]);
     const uint32_t empty_bar0 = ptx::smem_u32(&tail->empty[0]);
-    TileWalker walk(p, tail);
     TileFeed<kPair> feed(tail, wait, !leader);
     Tile t;
     // position in the stream of k-blocks of this warp's next one, the ring stage it
@@ -963,9 +983,9 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     bool ok = true;
     bool bad_index = false;
     while (ok) {
-      const int pos = feed.take(true, lane);
-      if (pos == kNoTile) { ok = false; break; }
-      if (!walk.decode(pos, &t)) break;
+      const Taken got = feed.take(true, lane, &t);
+      if (got == kAbandoned) { ok = false; break; }
+      if (got == kEndOfOrder) break;
       const int nkb = tile_stages(t);
       if (MODE == kTN) {
         // wgrad: the gathered rows are the contraction.  A k-block is 64 grouped rows
@@ -1096,7 +1116,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     const int half = (warp - 2) >> 2;  // which 128 of the tile's 256 columns
     const int col_base = half * (kBlockN / 2);
     const uint32_t my_out = out_base + uint32_t(warp - 2) * (G::kOutBufBytes * G::kOutBufs);
-    TileWalker walk(p, tail);
     TileFeed<kPair> feed(tail, wait, !leader);
     Tile t;
     uint32_t it = 0;
@@ -1283,9 +1302,9 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     };
 
     while (ok) {
-      const int pos = feed.take(true, lane);
-      if (pos == kNoTile) { ok = false; break; }
-      if (!walk.decode(pos, &t)) break;
+      const Taken got = feed.take(true, lane, &t);
+      if (got == kAbandoned) { ok = false; break; }
+      if (got == kEndOfOrder) break;
       const int nkb = tile_stages(t);
       const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
       if (kSwap && sw_rows != 0) {

@@ -295,10 +295,17 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 // (Same instruction; the name used where ordinary stores to the other CTA's
-// shared memory, st_shared_cluster_u32, are being published.)
+// shared memory, st_shared_cluster_v4, are being published.)
 __device__ __forceinline__ void mbar_arrive_release_cluster(uint32_t cluster_bar) { mbar_arrive_cluster(cluster_bar); }
-__device__ __forceinline__ void st_shared_cluster_u32(uint32_t cluster_addr, uint32_t v) {
-  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+__device__ __forceinline__ void st_shared_cluster_v4(uint32_t cluster_addr, int a, int b, int c, int d) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d)
+               : "memory");
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, int a, int b, int c, int d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void ld_shared_v4(uint32_t addr, int* a, int* b, int* c, int* d) {
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(*a), "=r"(*b), "=r"(*c), "=r"(*d) : "r"(addr) : "memory");
 }
 
 // TMA loads issued by either CTA of a pair; the mbarrier operand is a
