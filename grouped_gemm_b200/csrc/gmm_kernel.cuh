@@ -206,6 +206,14 @@ __device__ __forceinline__ T warp_inclusive_scan(T v, int lane) {
   return v;
 }
 
+// batch_sizes that travel as a kernel argument (host batch_sizes of few experts): no
+// copy to the device precedes the launch.  Values are clamped to [-1, tokens + 1], which
+// the schedule treats as it would the originals.
+constexpr int kInlineExperts = 64;
+struct InlineSizes {
+  int32_t v[kInlineExperts];
+};
+
 // One step of the exclusive prefix sum of batch_sizes: the 32 experts base ..
 // base + 31 (zeros past z), added to the running carry.  Returns this lane's
 // exclusive sum and advances the carry.  The scan every kernel of this library
@@ -227,8 +235,10 @@ __device__ __forceinline__ int64_t scan_step(int64_t v, int lane, int64_t* carry
 //               wgrad problems the same way, csrc/fill_arguments.cuh:80-86), so
 //               that the launch ends on the shortest tiles;
 //   tile_start  exclusive prefix sums of the per-expert tile counts in that order.
+//
+// batch_sizes == nullptr: the sizes are those of `inline_sizes`.
 __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* __restrict__ batch_sizes,
-                                               SmemTail* tail, uint32_t* status) {
+                                               const InlineSizes& inline_sizes, SmemTail* tail, uint32_t* status) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int scan_warp = (blockDim.x >= 96) ? 2 : 0;
@@ -238,7 +248,7 @@ __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* 
     uint32_t flags = 0;
     for (int base = 0; base < p.z; base += 32) {
       const int e = base + lane;
-      int64_t v = (e < p.z) ? batch_sizes[e] : 0;
+      int64_t v = (e >= p.z) ? 0 : (batch_sizes != nullptr ? batch_sizes[e] : inline_sizes.v[e]);
       if (v < 0) { v = 0; flags |= 0x2u; }
       int64_t start = scan_step(v, lane, &carry);
       if (start + v > p.tokens) flags |= 0x4u;
@@ -396,7 +406,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
            const int32_t* __restrict__ a_rows, const __nv_bfloat16* __restrict__ a_src,
            const int64_t a_src_rows, const float* __restrict__ row_scale, const int reduce_add,
            const int64_t dest_lo, const int64_t dest_hi, const __nv_bfloat16* __restrict__ gate_grad,
-           const PushArgs push) {
+           const PushArgs push, const __grid_constant__ InlineSizes inline_sizes) {
   static_assert(!SWIGLU || MODE != kTN, "the gated product is a forward product");
   static_assert(!PUSH || (!GATHER && !SWIGLU && MODE != kTN), "push warps exist in the plain forward / dgrad kernels");
   // SWIGLU: two right operands of n columns each, b (gate) and b2 (up).  The
@@ -473,7 +483,12 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       ptx::tmem_relinquish();
     }
   }
-  build_schedule(p, batch_sizes, tail, status);
+  // Everything above touches this SM only and overlaps the end of the kernel before
+  // this one in the stream (launch attribute, b200gmm.cu); global memory starts here.
+  // The kernel after this one may take over SMs as soon as they fall idle: it waits here too.
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+  build_schedule(p, batch_sizes, inline_sizes, tail, status);
   ptx::tc_fence_before_sync();
   __syncthreads();
   if (kPair) ptx::cluster_sync();  // the peer's barriers exist before anything arrives on them
@@ -806,7 +821,8 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         int pos = first_tile;
         // Positions after the first come from the global counter, drawn one tile
         // ahead of their use so that the atomic's round trip is never waited for.
-        uint32_t drawn = (pos < walk.total) ? atomicAdd(sched_counter, 1u) : 0u;
+        // (single_wave: there is no counter and no second tile.)
+        uint32_t drawn = (!p.single_wave && pos < walk.total) ? atomicAdd(sched_counter, 1u) : 0u;
         bool ok = true;
         while (ok) {
           int entry = 0;
@@ -845,7 +861,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           }
           if (!feed.publish(pos, entry, t)) { ok = false; break; }
           if (!live) break;  // the end of the order has been handed to everyone
-          pos = static_cast<int>(drawn) + tile_stride;
+          pos = p.single_wave ? walk.total : static_cast<int>(drawn) + tile_stride;
           if (pos < walk.total) drawn = atomicAdd(sched_counter, 1u);
         }
       }
@@ -1651,7 +1667,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 schedule_dump_kernel(const int64_t* __restrict__ batch_sizes, const Problem p, int32_t* __restrict__ out,
                      int max_tiles, int32_t* __restrict__ out_count, uint32_t* status) {
   __shared__ SmemTail tail;
-  build_schedule(p, batch_sizes, &tail, status);
+  build_schedule(p, batch_sizes, InlineSizes{}, &tail, status);
   __syncthreads();
   if (threadIdx.x == 0) {
     TileWalker walk(p, &tail);

@@ -57,6 +57,7 @@ struct Problem {
   int lt;          // column tiles of a transposed tile's width: ceil(n / 128)
   int wide_a;      // TN: a's columns are a multiple of 64, one TMA load brings all 64-column boxes of a stage
   int wide_b;      // TN: same for b
+  int single_wave; // every tile there can be is some cluster's first: no position is drawn from the counter
   int swap_rows;   // NN/NT: a tile of at most this many rows (rounded up, swapped_rows) runs with its operands swapped
 };
 
@@ -94,6 +95,12 @@ B200GMM_HD int light_rows(const Problem& p, int rows) {
 B200GMM_HD int expert_tiles(const Problem& p, int rows) {
   if (p.mode == kTN) return p.mt * p.nt;
   return heavy_row_tiles(p, rows) * p.nt + (light_rows(p, rows) > 0 ? p.lt : 0);
+}
+
+// Most tiles a launch can have, whatever batch_sizes holds (B200GMM_LIGHT off).
+B200GMM_HD int64_t max_tiles(const Problem& p) {
+  if (p.mode == kTN) return int64_t(p.z) * p.mt * p.nt;
+  return (p.tokens / p.tile_m + (p.z < p.tokens ? p.z : p.tokens)) * p.nt;
 }
 
 // Pipeline stages (ring slots) one tile consumes.
