@@ -48,12 +48,15 @@ def _load_extension():
 
 
 _ext = _load_extension()
-if not hasattr(_ext, "device_status"):
+if not hasattr(_ext, "gmm_autograd"):
     raise ImportError(f"the module {EXT_NAME} that is already imported ({getattr(_ext, '__file__', '?')}) is not "
                       "this library's binding")
 
 #: ``gmm(a, b, c, batch_sizes, trans_a, trans_b) -> None`` -- writes into ``c``.
 gmm = _ext.gmm
+
+#: ``gmm_autograd(a, b, batch_sizes, trans_b) -> c`` -- ``ops.GroupedGemm``, natively.
+gmm_autograd = _ext.gmm_autograd
 
 
 def device_status(device):
