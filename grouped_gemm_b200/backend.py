@@ -252,6 +252,12 @@ def gmm_swiglu_backward(a, b_gate, b_up, grad_out, batch_sizes, trans_b=False):
     the accumulator; returns ``(d_gate, d_up)``, bf16 [T, n] each (two halves of one
     [2, T, n] tensor), with ``d_gate = grad_out * up * silu'(gate)`` and
     ``d_up = grad_out * silu(gate)``.  Rows past ``sum(batch_sizes)`` are zeros."""
+    d = _swiglu_product_grads(a, b_gate, b_up, grad_out, batch_sizes, trans_b)
+    return d[0], d[1]
+
+
+def _swiglu_product_grads(a, b_gate, b_up, grad_out, batch_sizes, trans_b):
+    """Both gradients of ``gmm_swiglu_backward`` as the one [2, T, n] tensor they are made in."""
     assert a.ndim == 2 and b_gate.ndim == 3 and b_up.ndim == 3 and batch_sizes.ndim == 1 and grad_out.ndim == 2
     n = b_gate.shape[1] if trans_b else b_gate.shape[2]
     k = b_gate.shape[2] if trans_b else b_gate.shape[1]
@@ -266,19 +272,41 @@ def gmm_swiglu_backward(a, b_gate, b_up, grad_out, batch_sizes, trans_b=False):
         raise RuntimeError("gmm_swiglu_backward: shapes of a, b_gate, b_up, grad_out and batch_sizes do not fit together")
     if not (a.is_contiguous() and b_gate.is_contiguous() and b_up.is_contiguous() and grad_out.is_contiguous()):
         raise RuntimeError("gmm_swiglu_backward: a, b_gate, b_up and grad_out must be contiguous")
-    out = torch.zeros(2, tokens, n, device=a.device, dtype=a.dtype)
     lib = _capi.load()
     z = batch_sizes.shape[0]
+    # Every row is written by the kernel; with no experts there is no launch.
+    out = (torch.empty if z > 0 else torch.zeros)(2, tokens, n, device=a.device, dtype=a.dtype)
     with torch.cuda.device(a.device):
         ws_bytes = _capi.workspace_bytes(z)
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device)
         bs = _host_or_device_sizes(batch_sizes)
-        rc = lib.b200gmm_run_swiglu_backward(
+        rc = lib.b200gmm_run_swiglu_backward_full(
             a.data_ptr(), b_gate.data_ptr(), b_up.data_ptr(), grad_out.data_ptr(), out.data_ptr(), bs.data_ptr(),
             1 if bs.is_cuda else 0, z, tokens, k, n, 1 if trans_b else 0, ws.data_ptr(), ws_bytes,
             backend.device_status(a.device).data_ptr(), torch.cuda.current_stream(a.device).cuda_stream)
     _capi.check(rc, "b200gmm_run_swiglu_backward")
-    return out[0], out[1]
+    return out
+
+
+def _gmm_pair_sum(a_pair, b0, b1, batch_sizes, trans_b):
+    """``gmm(a_pair[0], b0) + gmm(a_pair[1], b1)`` in one launch and one accumulator:
+    the input gradient of the gated product, from operands that
+    ``_swiglu_product_grads`` has checked and made."""
+    tokens, k = a_pair.shape[1], a_pair.shape[2]
+    n = b0.shape[1] if trans_b else b0.shape[2]
+    c = torch.empty(tokens, n, device=a_pair.device, dtype=a_pair.dtype)
+    lib = _capi.load()
+    z = batch_sizes.shape[0]
+    with torch.cuda.device(a_pair.device):
+        ws_bytes = _capi.workspace_bytes(z)
+        ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a_pair.device)
+        bs = _host_or_device_sizes(batch_sizes)
+        rc = lib.b200gmm_run_pair_sum(
+            a_pair.data_ptr(), b0.data_ptr(), b1.data_ptr(), c.data_ptr(), bs.data_ptr(), 1 if bs.is_cuda else 0, z,
+            tokens, k, n, 1 if trans_b else 0, ws.data_ptr(), ws_bytes,
+            backend.device_status(a_pair.device).data_ptr(), torch.cuda.current_stream(a_pair.device).cuda_stream)
+    _capi.check(rc, "b200gmm_run_pair_sum")
+    return c
 
 
 def device_status(device="cuda"):

@@ -304,6 +304,8 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   // transposes, is the longer one: 3001 rows in 7 experts, k = 1000, n = 2504 took 33.9 us
   // up to 64 rows and without, 34.7 us up to 112; 256 experts of at most 118 rows,
   // k = 7168, n = 2048: 992 us without, 925 up to 32, 932 up to 64, 950 up to 112.
+  p->pair_sum = 0;
+  p->zero_rest = 0;
   p->single_wave = 0;  // decided where the grid is (run_impl)
   p->swap_rows = (p->mode != kTN && !(f.swiglu && ctas == 2)) ? p->tile_m / 2 : 0;
   const int64_t wait_ns = env_int64("B200GMM_WAIT_LIMIT_NS", static_cast<int64_t>(ptx::kWaitLimitNs));
@@ -389,7 +391,9 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
              const int32_t* a_rows = nullptr, int64_t a_source_rows = 0, const void* b2 = nullptr,
              const float* row_scale = nullptr, int reduce_add = 0, const void* dest_base = nullptr,
              int64_t dest_bytes = 0, const void* gate_grad = nullptr, const PushArgs* push = nullptr,
-             bool* push_launched = nullptr) {
+             bool* push_launched = nullptr, bool pair_sum = false, bool zero_rest = false) {
+  // pair_sum: a is [2, tokens, dim_a1], c = a[0] x b + a[1] x b2 (b2 is then no gate).
+  // zero_rest (with gate_grad): also the rows of c that belong to no expert are written.
   // push != nullptr: rows to move inside the same launch (plain forward / dgrad
   // kernels only); *push_launched tells the caller whether a launch took them.
   // gate_grad != nullptr: backward epilogue of the gated product; c is [2, tokens, n].
@@ -401,9 +405,10 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     return B200GMM_EINVAL;
   // b2 != nullptr: gated product silu(a @ b) * (a @ b2); n counts the columns of
   // each of b, b2 and c, the schedule runs over 2n virtual columns.
-  const bool swiglu = (b2 != nullptr);
+  const bool swiglu = (b2 != nullptr) && !pair_sum;
   if (swiglu && (trans_a || a_rows != nullptr)) return B200GMM_EINVAL;
-  if (swiglu && (reinterpret_cast<uintptr_t>(b2) & 15)) return B200GMM_EALIGN;
+  if (pair_sum && (trans_a || a_rows != nullptr || row_dest != nullptr)) return B200GMM_EINVAL;
+  if (b2 != nullptr && (reinterpret_cast<uintptr_t>(b2) & 15)) return B200GMM_EALIGN;
   if (swiglu && (n % 8) != 0) return B200GMM_EALIGN;
   const int64_t n_out = n;
   if (swiglu) n = 2 * n;
@@ -456,6 +461,14 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     if ((rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat)) != B200GMM_OK) return rc;
   }
 
+  p.pair_sum = pair_sum ? 1 : 0;
+  p.zero_rest = zero_rest ? 1 : 0;
+  if (pair_sum) {
+    if (b2 == nullptr) return B200GMM_EINVAL;
+    if (2 * tokens + p.tile_m >= (int64_t(1) << 31)) return B200GMM_ELIMIT;
+    p.light = 0;  // (transposed tiles know no second part)
+  }
+
   size_t need = 0;
   b200gmm_workspace_bytes(z, &need);
   if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 127))
@@ -496,20 +509,20 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   }
 
   CUtensorMap map_a, map_b, map_b2, map_a2;
-  bool have_b2 = swiglu;
+  bool have_b2 = (b2 != nullptr);
   // N: columns of b (and of b2, and of c); the Problem's n is twice that for the gated product.
   const uint64_t T = uint64_t(tokens), D1 = uint64_t(dim_a1), N = uint64_t(n_out), Z = uint64_t(z);
   const bool gather = (a_rows != nullptr);  // a is then fetched row by row, without a tensor map
   const bool swap_maps = !gather && (p.swap_rows > 0 || p.light);
   if (p.mode == kNN) {
-    const uint64_t da[2] = {D1, T};
+    const uint64_t da[2] = {D1, pair_sum ? 2 * T : T};
     const uint32_t ba[2] = {kBlockK, uint32_t(kBlockM)};
     const uint64_t db[3] = {N, D1, Z};
     const uint32_t bb[3] = {64, kBlockK, 1};
     // (One load per 64-column box: a single load of all the boxes of a stage through
     // a {64, k, n / 64, z} view of b measured 10-15 % slower in this layout.)
     if ((rc = encode_map(&map_b, b, 3, db, bb)) != 0) return rc;
-    if (swiglu && (rc = encode_map(&map_b2, b2, 3, db, bb)) != 0) return rc;
+    if (b2 != nullptr && (rc = encode_map(&map_b2, b2, 3, db, bb)) != 0) return rc;
     if (gather) map_a = map_b;
     else if ((rc = encode_map(&map_a, a, 2, da, ba)) != 0) return rc;
     if (swap_maps) {  // swapped and transposed tiles fetch their few rows of a in boxes of 32
@@ -517,13 +530,13 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
       if ((rc = encode_map(&map_a2, a, 2, da, bl)) != 0) return rc;
     }
   } else if (p.mode == kNT) {
-    const uint64_t da[2] = {D1, T};
+    const uint64_t da[2] = {D1, pair_sum ? 2 * T : T};
     const uint32_t ba[2] = {kBlockK, uint32_t(kBlockM)};
     const uint64_t db[3] = {D1, N, Z};
     // rows of b per box: a CTA's share of the tile; for the gated product half a tile from each of b, b2
     const uint32_t bb[3] = {kBlockK, uint32_t(swiglu ? kBlockN / 2 : kBlockN / ctas), 1};
     if ((rc = encode_map(&map_b, b, 3, db, bb)) != 0) return rc;
-    if (swiglu && (rc = encode_map(&map_b2, b2, 3, db, bb)) != 0) return rc;
+    if (b2 != nullptr && (rc = encode_map(&map_b2, b2, 3, db, bb)) != 0) return rc;
     if (gather) map_a = map_b;
     else if ((rc = encode_map(&map_a, a, 2, da, ba)) != 0) return rc;
     if (swap_maps) {
@@ -623,6 +636,25 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   if (with_push && push_launched != nullptr) *push_launched = true;
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return B200GMM_OK;
+}
+
+int swiglu_backward(const void* a, const void* b_gate, const void* b_up, const void* grad_out,
+                    void* grad_products, const int64_t* batch_sizes, int batch_sizes_on_device, int z,
+                    int64_t tokens, int64_t dim_a1, int64_t n, int trans_b, void* workspace,
+                    size_t workspace_bytes, uint32_t* device_status, void* cuda_stream, bool zero_rest) {
+  if (grad_products == nullptr || (grad_out == nullptr && tokens > 0 && n > 0)) return B200GMM_EINVAL;
+  if (b_up == nullptr && tokens > 0 && n > 0 && dim_a1 > 0 && z > 0) return B200GMM_EINVAL;
+  if (dim_a1 == 0 || tokens == 0 || n == 0 || z == 0) {
+    // g = u = 0 everywhere: dg = dh * 0 * silu'(0) = 0 and du = dh * silu(0) = 0
+    if (tokens > 0 && n > 0 && z > 0 &&
+        cudaMemsetAsync(grad_products, 0, size_t(2) * size_t(tokens) * size_t(n) * 2,
+                        static_cast<cudaStream_t>(cuda_stream)) != cudaSuccess)
+      return B200GMM_ECUDA;
+    return check_args_only(z, tokens, dim_a1, n, trans_b);
+  }
+  return run_impl(a, b_gate, grad_products, batch_sizes, batch_sizes_on_device, z, tokens, dim_a1, n, 0, trans_b,
+                  workspace, workspace_bytes, device_status, cuda_stream, nullptr, nullptr, 0, b_up, nullptr, 0, nullptr, 0,
+                  grad_out, nullptr, nullptr, false, zero_rest);
 }
 
 }  // namespace
@@ -737,19 +769,25 @@ int b200gmm_run_swiglu_backward(const void* a, const void* b_gate, const void* b
                                 void* grad_products, const int64_t* batch_sizes, int batch_sizes_on_device, int z,
                                 int64_t tokens, int64_t dim_a1, int64_t n, int trans_b, void* workspace,
                                 size_t workspace_bytes, uint32_t* device_status, void* cuda_stream) {
-  if (grad_products == nullptr || (grad_out == nullptr && tokens > 0 && n > 0)) return B200GMM_EINVAL;
-  if (b_up == nullptr && tokens > 0 && n > 0 && dim_a1 > 0 && z > 0) return B200GMM_EINVAL;
-  if (dim_a1 == 0 || tokens == 0 || n == 0 || z == 0) {
-    // g = u = 0 everywhere: dg = dh * 0 * silu'(0) = 0 and du = dh * silu(0) = 0
-    if (tokens > 0 && n > 0 && z > 0 &&
-        cudaMemsetAsync(grad_products, 0, size_t(2) * size_t(tokens) * size_t(n) * 2,
-                        static_cast<cudaStream_t>(cuda_stream)) != cudaSuccess)
-      return B200GMM_ECUDA;
-    return check_args_only(z, tokens, dim_a1, n, trans_b);
-  }
-  return run_impl(a, b_gate, grad_products, batch_sizes, batch_sizes_on_device, z, tokens, dim_a1, n, 0, trans_b,
-                  workspace, workspace_bytes, device_status, cuda_stream, nullptr, nullptr, 0, b_up, nullptr, 0, nullptr, 0,
-                  grad_out);
+  return swiglu_backward(a, b_gate, b_up, grad_out, grad_products, batch_sizes, batch_sizes_on_device, z, tokens, dim_a1,
+                         n, trans_b, workspace, workspace_bytes, device_status, cuda_stream, false);
+}
+
+int b200gmm_run_swiglu_backward_full(const void* a, const void* b_gate, const void* b_up, const void* grad_out,
+                                     void* grad_products, const int64_t* batch_sizes, int batch_sizes_on_device, int z,
+                                     int64_t tokens, int64_t dim_a1, int64_t n, int trans_b, void* workspace,
+                                     size_t workspace_bytes, uint32_t* device_status, void* cuda_stream) {
+  return swiglu_backward(a, b_gate, b_up, grad_out, grad_products, batch_sizes, batch_sizes_on_device, z, tokens, dim_a1,
+                         n, trans_b, workspace, workspace_bytes, device_status, cuda_stream, true);
+}
+
+int b200gmm_run_pair_sum(const void* a_pair, const void* b0, const void* b1, void* c, const int64_t* batch_sizes,
+                         int batch_sizes_on_device, int z, int64_t tokens, int64_t dim_a1, int64_t n, int trans_b,
+                         void* workspace, size_t workspace_bytes, uint32_t* device_status, void* cuda_stream) {
+  if (b1 == nullptr && tokens > 0 && n > 0 && dim_a1 > 0 && z > 0) return B200GMM_EINVAL;
+  return run_impl(a_pair, b0, c, batch_sizes, batch_sizes_on_device, z, tokens, dim_a1, n, 0, trans_b, workspace,
+                  workspace_bytes, device_status, cuda_stream, nullptr, nullptr, 0, b1, nullptr, 0, nullptr, 0, nullptr,
+                  nullptr, nullptr, true);
 }
 
 int b200gmm_run_static(const void* a, const void* b, void* c, const int64_t* batch_sizes,

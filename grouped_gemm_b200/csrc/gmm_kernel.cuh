@@ -424,6 +424,9 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   // Swapped tiles (schedule.cuh) exist wherever the rows of a tile are independent and
   // one CTA holds all that an output element needs: not in the pair form of the gated
   // product, whose gate and up columns lie in different CTAs.
+  // A sum of two products over one accumulator (Problem::pair_sum) is an option of the
+  // plain kernels.
+  constexpr bool kPairSum = (MODE != kTN) && !GATHER && !SWIGLU && !PUSH;
   constexpr bool kSwap = (MODE != kTN) && !(SWIGLU && CTAS == 2);
 
   extern __shared__ uint8_t smem_raw[];
@@ -494,6 +497,17 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   if (kPair) ptx::cluster_sync();  // the peer's barriers exist before anything arrives on them
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = tail->tmem_base;
+  if (SWIGLU && p.zero_rest) {
+    // Rows that belong to no expert, in both halves of c (usually there are none).
+    const int64_t row_vecs = (p.n >> 1) / 8;
+    const int64_t first = tail->row_start[p.z];
+    const int64_t vecs = (p.tokens - first) * row_vecs;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < 2 * vecs; i += int64_t(gridDim.x) * blockDim.x) {
+      const bool second = i >= vecs;
+      uint4* rest = reinterpret_cast<uint4*>(c) + (first + (second ? p.tokens : 0)) * row_vecs;
+      rest[second ? i - vecs : i] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
 
   constexpr bool kAMn = (MODE == kTN);                 // A operand MN-major (wgrad reads a^T)
   constexpr bool kBMn = (MODE == kNN || MODE == kTN);  // B operand MN-major
@@ -570,24 +584,32 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         // Bytes this CTA's TMA loads bring per stage: the gather warps fetch A themselves.
         const uint32_t tma_bytes =
             G::kBBytes + (GATHER ? 0u : (sw_rows != 0 ? uint32_t(sw_boxes) * kRowBoxBytes : G::kABytes));
+        int part_row = a_row;                // row of a the current part of the contraction starts at
+        const CUtensorMap* part_b = &map_b;  // and its weights
         auto load_rows = [&](uint32_t dst, uint32_t bar, int k0) {  // A of a forward / dgrad stage
           if (GATHER) return;
           if (kSwap && sw_rows != 0) {
             for (int i = 0; i < sw_boxes; ++i) {
-              if (kPair) ptx::tma_load_2d_pair(dst + i * kRowBoxBytes, &map_a2, bar, k0, a_row + i * 32);
-              else ptx::tma_load_2d(dst + i * kRowBoxBytes, &map_a2, bar, k0, a_row + i * 32);
+              if (kPair) ptx::tma_load_2d_pair(dst + i * kRowBoxBytes, &map_a2, bar, k0, part_row + i * 32);
+              else ptx::tma_load_2d(dst + i * kRowBoxBytes, &map_a2, bar, k0, part_row + i * 32);
             }
           } else {
-            if (kPair) ptx::tma_load_2d_pair(dst, &map_a, bar, k0, a_row);
-            else ptx::tma_load_2d(dst, &map_a, bar, k0, a_row);
+            if (kPair) ptx::tma_load_2d_pair(dst, &map_a, bar, k0, part_row);
+            else ptx::tma_load_2d(dst, &map_a, bar, k0, part_row);
           }
         };
+        int k0 = -kBlockK;
         for (int kb = 0; kb < nkb; ++kb) {
+          k0 += kBlockK;
+          if (kPairSum && p.pair_sum && 2 * kb == nkb) {  // second part
+            k0 = 0;
+            part_row += static_cast<int>(p.tokens);
+            part_b = &map_b2;
+          }
           if (!ptx::mbar_wait(ptx::smem_u32(&tail->empty[s]), ph ^ 1u, wait)) { ok = false; break; }
           const uint32_t local_bar = ptx::smem_u32(&tail->full[s]);
           const uint32_t sa = stage_base + s * G::kStageBytes;
           const uint32_t sb = sa + G::kABytes;
-          const int k0 = kb * kBlockK;
           if (!kPair) {
             ptx::mbar_arrive_expect_tx(local_bar, tma_bytes);
             if (MODE == kNN) {
@@ -598,14 +620,14 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
                   ptx::tma_load_3d(sb + j * kBoxBytes, j < 2 ? &map_b : &map_b2, local_bar,
                                    t.col0 / 2 + (j & 1) * 64, k0, t.expert);
                 else
-                  ptx::tma_load_3d(sb + j * kBoxBytes, &map_b, local_bar, t.col0 + j * 64, k0, t.expert);
+                  ptx::tma_load_3d(sb + j * kBoxBytes, part_b, local_bar, t.col0 + j * 64, k0, t.expert);
             } else if (MODE == kNT) {
               load_rows(sa, local_bar, k0);
               if (SWIGLU) {  // the maps' boxes are 128 rows of b high
                 ptx::tma_load_3d(sb, &map_b, local_bar, k0, t.col0 / 2, t.expert);
                 ptx::tma_load_3d(sb + G::kBBytes / 2, &map_b2, local_bar, k0, t.col0 / 2, t.expert);
               } else {
-                ptx::tma_load_3d(sb, &map_b, local_bar, k0, t.col0, t.expert);
+                ptx::tma_load_3d(sb, part_b, local_bar, k0, t.col0, t.expert);
               }
             } else {
               const int r0 = t.k_row0 + k0;
@@ -640,12 +662,12 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
                   ptx::tma_load_3d_pair(sb + j * kBoxBytes, leader ? &map_b : &map_b2, bar,
                                         t.col0 / 2 + j * 64, k0, t.expert);
                 else
-                  ptx::tma_load_3d_pair(sb + j * kBoxBytes, &map_b, bar, t.col0 + col_off + j * 64, k0,
+                  ptx::tma_load_3d_pair(sb + j * kBoxBytes, part_b, bar, t.col0 + col_off + j * 64, k0,
                                         t.expert);
             } else if (MODE == kNT) {
               load_rows(sa, bar, k0);
               if (SWIGLU) ptx::tma_load_3d_pair(sb, leader ? &map_b : &map_b2, bar, k0, t.col0 / 2, t.expert);
-              else ptx::tma_load_3d_pair(sb, &map_b, bar, k0, t.col0 + col_off, t.expert);
+              else ptx::tma_load_3d_pair(sb, part_b, bar, k0, t.col0 + col_off, t.expert);
             } else {
               const int r0 = t.k_row0 + k0;
               if (!GATHER) {

@@ -70,7 +70,8 @@ class GatedGroupedGemm(torch.autograd.Function):
       kernel and turns the output gradient into the gradients of the two products;
       from there on it is the reference's backward (ops.py:14-29) twice: the input
       gradient is the sum of two grouped products against the other orientation of
-      the weights, each weight gradient one ``trans_a`` product.
+      the weights (one launch, summed in the accumulator), each weight gradient one
+      ``trans_a`` product.
     """
 
     @staticmethod
@@ -85,11 +86,11 @@ class GatedGroupedGemm(torch.autograd.Function):
         want_a, want_g, want_u = ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.needs_input_grad[2]
         if not (want_a or want_g or want_u):
             return None, None, None, None, None
-        d_gate, d_up = backend.gmm_swiglu_backward(a, b_gate, b_up, grad.contiguous(), batch_sizes, trans_b=ctx.trans_b)
+        d = backend._swiglu_product_grads(a, b_gate, b_up, grad.contiguous(), batch_sizes, ctx.trans_b)
+        d_gate, d_up = d[0], d[1]
         agrad = ggrad = ugrad = None
         if want_a:
-            agrad = backend.gmm(d_gate, b_gate, batch_sizes, trans_b=not ctx.trans_b)
-            agrad += backend.gmm(d_up, b_up, batch_sizes, trans_b=not ctx.trans_b)
+            agrad = backend._gmm_pair_sum(d, b_gate, b_up, batch_sizes, not ctx.trans_b)
         def wgrad(d):  # in the weights' own layout (reference ops.py:24-28)
             lhs, rhs = (d, a) if ctx.trans_b else (a, d)
             return backend.gmm(lhs, rhs, batch_sizes, trans_a=True)
