@@ -83,7 +83,7 @@ struct LaunchArgs {
   Problem p;
   uint32_t* status = nullptr;
   CUtensorMap* slots = nullptr;
-  uint32_t* sched_counter = nullptr;       // zeroed on the stream before the launch (unused: single_wave)
+  uint32_t* sched_counter = nullptr;      // zeroed on the stream before the launch (unused: single_wave)
   InlineSizes inline_sizes;               // batch_sizes == nullptr: these
   bool overlap = false;                   // the prologue may overlap the kernel before it in the stream
   const int64_t* row_dest = nullptr;      // scatter / combine epilogue
@@ -116,6 +116,20 @@ cudaError_t launch_gmm(const LaunchArgs& a) {
   return cudaLaunchKernelEx(&cfg, gmm_kernel<MODE, CTAS, GATHER, SWIGLU, PUSH>, a.map_a, a.map_b, a.map_b2, a.map_c, a.map_a2, a.c,
                             a.batch_sizes, a.p, a.status, a.slots, a.sched_counter, a.row_dest, a.a_rows, a.a_src, a.a_src_rows,
                             a.row_scale, a.reduce_add, a.dest_lo, a.dest_hi, a.gate_grad, a.push, a.inline_sizes);
+}
+
+// The tile counter's zeros, as a kernel that overlaps its neighbours (gmm_kernel.cuh).
+cudaError_t zero_counter(uint32_t* sched_counter, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(32);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, zero_counter_kernel, sched_counter);
 }
 
 // The plain forward / dgrad kernels with push warps (a.push.src != nullptr).
@@ -303,7 +317,9 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   // 256 once, bound by the shared-memory reads of the operands) and its epilogue, which
   // transposes, is the longer one: 3001 rows in 7 experts, k = 1000, n = 2504 took 33.9 us
   // up to 64 rows and without, 34.7 us up to 112; 256 experts of at most 118 rows,
-  // k = 7168, n = 2048: 992 us without, 925 up to 32, 932 up to 64, 950 up to 112.
+  // k = 7168, n = 2048: 992 us without, 925 up to 32, 932 up to 64, 950 up to 112.  Without
+  // against up to 64 in separate processes: that case 869 -> 770 us, 64 rows over 8 experts
+  // of 4096 x 14336 149 -> 140 us, 65536 rows over 256 experts 7.56 -> 7.50 ms (a training step).
   p->pair_sum = 0;
   p->zero_rest = 0;
   p->single_wave = 0;  // decided where the grid is (run_impl)
@@ -487,13 +503,16 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   // experts of 4096 x 14336): 135.9 -> 129.4 us.
   const bool single_wave = !p.light && max_tiles(p) * ctas <= max_ctas;
   p.single_wave = single_wave ? 1 : 0;
-  if (!single_wave && cudaMemsetAsync(sched_counter, 0, 16, stream) != cudaSuccess) return B200GMM_ECUDA;
 
   // A capturing stream keeps the copy of host batch_sizes (a replay reads them again)
   // and full dependencies between its kernels.
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) return B200GMM_ECUDA;
   const bool capturing = capture != cudaStreamCaptureStatusNone;
+  if (!single_wave && (capturing ? cudaMemsetAsync(sched_counter, 0, 16, stream) : zero_counter(sched_counter, stream)) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return B200GMM_ECUDA;
+  }
   LaunchArgs la;
   la.overlap = !capturing;
   const int64_t* bs_dev = batch_sizes;

@@ -1666,6 +1666,16 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   }
 }
 
+// Zeroes the tile counter for the launch that follows.  A memset between two kernels
+// starts when the first has ended and keeps the second from being set up until then;
+// this is in place, waiting, while the first still runs, and lets the second queue up too
+// (training step of 3001 rows in 7 experts, 1000 x 2504, three such launches: 98.6 -> 92.6 us).
+__global__ void __launch_bounds__(32, 1) zero_counter_kernel(uint32_t* sched_counter) {
+  ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
+  if (threadIdx.x < 4) sched_counter[threadIdx.x] = 0u;
+}
+
 // Argument fill on its own (bit-exact tests, inspection): the same scan step the
 // GEMM kernels' schedule is built from, writing the reference's nine per-expert
 // values (schedule.cuh: fill_fields).
