@@ -89,24 +89,17 @@ def gmm_scatter(a, b, batch_sizes, out, row_index, trans_b=False, row_weight=Non
     lib = _capi.load()
     z = batch_sizes.shape[0]
     with torch.cuda.device(a.device):
-        dest = row_index * (n * 2) + out.data_ptr()          # byte address of every destination row
-        window = (out.data_ptr(), out.numel() * 2)           # the kernel refuses addresses outside ``out``
+        index = row_index.contiguous()
         ws_bytes = _capi.workspace_bytes(z)
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device)
         bs = _host_or_device_sizes(batch_sizes)
-        status = backend.device_status(a.device).data_ptr()
-        stream = torch.cuda.current_stream(a.device).cuda_stream
-        if row_weight is None and not accumulate:
-            rc = lib.b200gmm_run_scatter(
-                a.data_ptr(), b.data_ptr(), dest.data_ptr(), *window, bs.data_ptr(), 1 if bs.is_cuda else 0, z,
-                a.shape[0], a.shape[1], n, 1 if trans_b else 0, ws.data_ptr(), ws_bytes, status, stream)
-        else:
-            rc = lib.b200gmm_run_combine(
-                a.data_ptr(), b.data_ptr(), dest.data_ptr(), *window,
-                None if row_weight is None else row_weight.data_ptr(), 1 if accumulate else 0,
-                bs.data_ptr(), 1 if bs.is_cuda else 0, z,
-                a.shape[0], a.shape[1], n, 1 if trans_b else 0, ws.data_ptr(), ws_bytes, status, stream)
-    _capi.check(rc, "b200gmm_run_scatter")
+        rc = lib.b200gmm_run_combine_rows(
+            a.data_ptr(), b.data_ptr(), index.data_ptr(), out.data_ptr(), out.shape[0],
+            None if row_weight is None else row_weight.data_ptr(), 1 if accumulate else 0,
+            bs.data_ptr(), 1 if bs.is_cuda else 0, z, a.shape[0], a.shape[1], n, 1 if trans_b else 0,
+            ws.data_ptr(), ws_bytes, backend.device_status(a.device).data_ptr(),
+            torch.cuda.current_stream(a.device).cuda_stream)
+    _capi.check(rc, "b200gmm_run_combine_rows")
     return out
 
 

@@ -320,6 +320,8 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   // k = 7168, n = 2048: 992 us without, 925 up to 32, 932 up to 64, 950 up to 112.  Without
   // against up to 64 in separate processes: that case 869 -> 770 us, 64 rows over 8 experts
   // of 4096 x 14336 149 -> 140 us, 65536 rows over 256 experts 7.56 -> 7.50 ms (a training step).
+  p->dest_indexed = 0;
+  p->dest_rows = 0;
   p->pair_sum = 0;
   p->zero_rest = 0;
   p->single_wave = 0;  // decided where the grid is (run_impl)
@@ -407,7 +409,10 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
              const int32_t* a_rows = nullptr, int64_t a_source_rows = 0, const void* b2 = nullptr,
              const float* row_scale = nullptr, int reduce_add = 0, const void* dest_base = nullptr,
              int64_t dest_bytes = 0, const void* gate_grad = nullptr, const PushArgs* push = nullptr,
-             bool* push_launched = nullptr, bool pair_sum = false, bool zero_rest = false) {
+             bool* push_launched = nullptr, bool pair_sum = false, bool zero_rest = false,
+             int64_t dest_rows = -1) {
+  // dest_rows >= 0: row_dest holds rows of the [dest_rows, n] destination at
+  // dest_base instead of addresses.
   // pair_sum: a is [2, tokens, dim_a1], c = a[0] x b + a[1] x b2 (b2 is then no gate).
   // zero_rest (with gate_grad): also the rows of c that belong to no expert are written.
   // push != nullptr: rows to move inside the same launch (plain forward / dgrad
@@ -477,6 +482,8 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     if ((rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat)) != B200GMM_OK) return rc;
   }
 
+  p.dest_indexed = dest_rows >= 0 ? 1 : 0;
+  p.dest_rows = dest_rows;
   p.pair_sum = pair_sum ? 1 : 0;
   p.zero_rest = zero_rest ? 1 : 0;
   if (pair_sum) {
@@ -746,6 +753,18 @@ int b200gmm_run_combine(const void* a, const void* b, const int64_t* row_dest, c
   return run_impl(a, b, nullptr, batch_sizes, batch_sizes_on_device, z, tokens, dim_a1, n, 0, trans_b,
                   workspace, workspace_bytes, device_status, cuda_stream, row_dest, nullptr, 0, nullptr,
                   row_weight, accumulate ? 1 : 0, dest_base, dest_bytes);
+}
+
+int b200gmm_run_combine_rows(const void* a, const void* b, const int64_t* row_index, void* out, int64_t out_rows,
+                             const float* row_weight, int accumulate, const int64_t* batch_sizes,
+                             int batch_sizes_on_device, int z, int64_t tokens, int64_t dim_a1, int64_t n, int trans_b,
+                             void* workspace, size_t workspace_bytes, uint32_t* device_status, void* cuda_stream) {
+  if (row_index == nullptr || out_rows < 0 || (out == nullptr && out_rows > 0)) return B200GMM_EINVAL;
+  if (row_weight != nullptr && (reinterpret_cast<uintptr_t>(row_weight) & 3)) return B200GMM_EALIGN;
+  if (dim_a1 == 0) return accumulate ? B200GMM_OK : B200GMM_EINVAL;  // as b200gmm_run_combine
+  return run_impl(a, b, nullptr, batch_sizes, batch_sizes_on_device, z, tokens, dim_a1, n, 0, trans_b,
+                  workspace, workspace_bytes, device_status, cuda_stream, row_index, nullptr, 0, nullptr,
+                  row_weight, accumulate ? 1 : 0, out, out_rows * n * 2, nullptr, nullptr, nullptr, false, false, out_rows);
 }
 
 int b200gmm_run_gather(const void* x, int64_t x_rows, const int32_t* row_index, const void* b, void* c,

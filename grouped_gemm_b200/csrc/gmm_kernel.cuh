@@ -1167,6 +1167,17 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     auto dest_ok = [&](int64_t addr) {
       return (addr & 15) == 0 && (dest_hi == 0 || (addr >= dest_lo && addr + dest_row_bytes <= dest_hi));
     };
+    // Where row i of the result goes; false: nowhere.  (Rows given as indices become
+    // addresses here, not in two launches of their own before this one.)
+    auto dest_of = [&](int64_t i, int64_t* addr) {
+      const int64_t v = row_dest[i];
+      if (p.dest_indexed) {
+        *addr = dest_lo + v * dest_row_bytes;
+        return v >= 0 && v < p.dest_rows && (dest_lo & 15) == 0;
+      }
+      *addr = v;
+      return dest_ok(v);
+    };
     // Buffer for the next TMA store and the wait before it may be written: with two
     // buffers the store before last read this one.
     auto stage_buf = [&]() { return my_out + (G::kOutBufs == 2 ? (stores & 1u) * G::kOutBufBytes : 0u); };
@@ -1300,8 +1311,8 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         ptx::fence_proxy_async_smem();
         __syncwarp();
         if (lane < rows) {
-          const int64_t addr = row_dest[row + lane];
-          if (dest_ok(addr)) {
+          int64_t addr;
+          if (dest_of(row + lane, &addr)) {
             const int left = out_n - col;
             const uint32_t bytes = left < 32 ? uint32_t(left) * 2u : 64u;
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(addr) + col;
@@ -1437,8 +1448,8 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
               float f = __uint_as_float(v[u]);
               __nv_bfloat16* dst;
               if (row_dest != nullptr) {
-                const int64_t addr = row_dest[grow];
-                if (!dest_ok(addr)) { bad_dest = true; continue; }
+                int64_t addr;
+                if (!dest_of(grow, &addr)) { bad_dest = true; continue; }
                 if (row_scale != nullptr) f *= row_scale[grow];
                 dst = reinterpret_cast<__nv_bfloat16*>(addr) + col;
               } else {
@@ -1469,8 +1480,8 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       const int out_col0 = SWIGLU ? (t.col0 >> 1) : t.col0;
       __nv_bfloat16* crow = c + (out_row0 + r) * out_n + out_col0;
       if (scatter && row_ok) {
-        const int64_t addr = row_dest[out_row0 + r];
-        if (dest_ok(addr)) {
+        int64_t addr;
+        if (dest_of(out_row0 + r, &addr)) {
           crow = reinterpret_cast<__nv_bfloat16*>(addr) + out_col0;
         } else {  // never written: skipped and reported
           row_ok = false;

@@ -63,6 +63,8 @@ struct Problem {
                    // write, read back and add, and one rounding instead of three.  With zero_rest
                    // instead of a zeroed [2, tokens, n] a training step of 16384 rows, 8 experts of
                    // 4096 x 14336, went from 13.73 to 13.27 ms, the gradient's error from 3.0e-3 to 2.3e-3.)
+  int dest_indexed;  // row_dest holds rows of a [dest_rows, n] destination at dest_lo, not addresses
+  int64_t dest_rows;
   int zero_rest;   // gated backward: rows past the last expert's of both halves of c become zeros
   int swap_rows;   // NN/NT: a tile of at most this many rows (rounded up, swapped_rows) runs with its operands swapped
 };
