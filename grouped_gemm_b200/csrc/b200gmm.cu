@@ -280,6 +280,7 @@ int choose_ctas(int z, int64_t tokens, int64_t d1, int trans_a) {
 struct Features {
   bool gather = false;
   bool swiglu = false;
+  bool gated_backward = false;
 };
 
 int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b, int ctas,
@@ -312,20 +313,24 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   // by streaming their weights from HBM either way, and measured end to end the
   // launch was not faster with them (B200GMM_LIGHT=1 switches them on).
   p->light = (p->mode != kTN && ctas == 1 && !f.gather && !f.swiglu) ? env_int("B200GMM_LIGHT", 0) : 0;
-  // Tiles of at most half their rows run with their operands swapped (schedule.cuh).
-  // Nearer to a full tile the swapped form saves no tensor time (N = 112 twice against
-  // 256 once, bound by the shared-memory reads of the operands) and its epilogue, which
-  // transposes, is the longer one: 3001 rows in 7 experts, k = 1000, n = 2504 took 33.9 us
-  // up to 64 rows and without, 34.7 us up to 112; 256 experts of at most 118 rows,
-  // k = 7168, n = 2048: 992 us without, 925 up to 32, 932 up to 64, 950 up to 112.  Without
-  // against up to 64 in separate processes: that case 869 -> 770 us, 64 rows over 8 experts
-  // of 4096 x 14336 149 -> 140 us, 65536 rows over 256 experts 7.56 -> 7.50 ms (a training step).
+  // Token generation: where an expert has at most 16 rows on average and the contraction
+  // is long, tiles of at most half their rows run with their operands swapped
+  // (schedule.cuh).  Without and with, each in a process of its own: 1024 rows over 256
+  // experts, k = 7168, n = 2048: 869 and 770 us; 64 rows over 8 experts of 4096 x 14336: 149 and
+  // 140 us; a decode step of that expert layer (128 rows): 450 and 425 us.  Outside of that
+  // the transposing epilogue costs what the padded rows did, or more.  64 experts, n =
+  // 4096: 8 rows each, k = 512 and 2048: 50 and 50, 171 and 172 us; 64 rows each: 55.0 and 55.5, 183
+  // and 187 us; remainders of 32 experts of 300 rows, k = 2048: 207 and 220 us, gated 383 and
+  // 452 us.  The gated backward, which reads its gradient row by row there: 104 and 222 us
+  // (40 rows, k = 512).
+  constexpr int64_t kSwapMeanRows = 16, kSwapMinK = 4096;
+  p->swap_rows = (p->mode != kTN && !(f.swiglu && ctas == 2) && !f.gated_backward && tokens <= kSwapMeanRows * z &&
+                  d1 >= kSwapMinK) ? p->tile_m / 2 : 0;
   p->dest_indexed = 0;
   p->dest_rows = 0;
   p->pair_sum = 0;
   p->zero_rest = 0;
   p->single_wave = 0;  // decided where the grid is (run_impl)
-  p->swap_rows = (p->mode != kTN && !(f.swiglu && ctas == 2)) ? p->tile_m / 2 : 0;
   const int64_t wait_ns = env_int64("B200GMM_WAIT_LIMIT_NS", static_cast<int64_t>(ptx::kWaitLimitNs));
   p->wait_ns = wait_ns > 0 ? wait_ns : static_cast<int64_t>(ptx::kWaitLimitNs);
   // Upper bound on the tile count must fit the kernel's 32-bit tile index (twice:
@@ -441,6 +446,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   Features feat;
   feat.gather = (a_rows != nullptr);
   feat.swiglu = swiglu;
+  feat.gated_backward = gate_grad != nullptr;
   int ctas = choose_ctas(z, tokens, dim_a1, trans_a);
   int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat);
   if (rc != B200GMM_OK) return rc;

@@ -1378,23 +1378,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             ptx::tmem_ld_32x32(taddr + uint32_t(r0), va);
             if (SWIGLU) ptx::tmem_ld_32x32(taddr + kBlockN / 2 + uint32_t(r0), vb);
             ptx::tmem_ld_wait();
-            if (SWIGLU && gate_grad != nullptr) {
-              // as in the plain tile's backward epilogue below
-              const __nv_bfloat16* src = gate_grad + row * out_n + col + lane;
-              const bool col_ok = col + lane < out_n;
-#pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const float dh = (col_ok && i < rows) ? __bfloat162float(src[int64_t(i) * out_n]) : 0.0f;
-                const float g = __uint_as_float(va[i]);
-                const float u = __uint_as_float(vb[i]);
-                const float sg = __fdividef(1.0f, 1.0f + __expf(-g));
-                va[i] = __float_as_uint(dh * u * sg * (1.0f + g * (1.0f - sg)));
-                vb[i] = __float_as_uint(dh * g * sg);
-              }
-              emit_swapped(va, rows, row, col, out_n);
-              emit_swapped(vb, rows, row + p.tokens, col, out_n);
-              continue;
-            }
             if (SWIGLU) {
 #pragma unroll
               for (int i = 0; i < 32; ++i) {

@@ -116,15 +116,13 @@ B200GMM_HD int tile_stages(const Tile& t) {
   return t.kind ? (t.k_len + kLightK - 1) / kLightK : (t.k_len + kBlockK - 1) / kBlockK;
 }
 
-// Swapped tiles (NN/NT): a tile_m x 256 tile with few rows, that is a small expert or
-// the last rows of a larger one, is computed as its transpose, from the same loads.
-// The tile's 256 weight columns ride UMMA M (one CTA: two MMAs of 128 columns; a pair:
-// one MMA of 2 x 128) and its rows ride UMMA N, rounded up to the step N allows, so
-// that the tensor core works for the rows that exist and not for tile_m of them, and
-// only those rows are fetched.  A launch of small experts is bound by streaming their
-// weights; what the padded rows cost it was tensor time and power and a third of the
-// bytes that enter an SM.  Token generation over 256 experts (1024 rows, k = 7168,
-// n = 2048): 816 -> 735 us; down projection of 8 (128 rows, k = 14336): 144 -> 128 us.
+// Swapped tiles (NN/NT): a tile_m x 256 tile with few rows is computed as its transpose,
+// from the same loads.  The tile's 256 weight columns ride UMMA M (one CTA: two MMAs of
+// 128 columns; a pair: one MMA of 2 x 128) and its rows ride UMMA N, rounded up to the step N
+// allows, so that the tensor core works for the rows that exist and not for tile_m of
+// them, and only those rows are fetched.  Launches of small experts are bound by streaming
+// weights; what the padded rows cost them was tensor time and power and a third of the
+// bytes that enter an SM.  Which launches: Problem::swap_rows, decided by check_problem.
 // Returns the rounded row count, 0 for a plain tile.
 B200GMM_HD int swapped_rows(const Problem& p, const Tile& t) {
   if (p.swap_rows == 0 || t.kind != 0) return 0;
