@@ -389,6 +389,18 @@ int static_scratch_address(void** out) {
 size_t maps_offset(int z) { return round128(size_t(z) * sizeof(int64_t) + 16); }
 size_t maps_bytes() { return size_t(kMaxCtas) * kMapSlots * 2 * sizeof(CUtensorMap); }
 
+// Whether a copy from this host array reads it before the copy call returns.  A pinned
+// (or managed) array is read when the stream gets to the copy, and earlier work of the
+// stream may be what fills it.
+bool pageable(const void* host) {
+  cudaPointerAttributes attr;
+  if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return attr.type == cudaMemoryTypeUnregistered;
+}
+
 }  // namespace
 
 extern "C" {
@@ -529,7 +541,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   LaunchArgs la;
   la.overlap = !capturing;
   const int64_t* bs_dev = batch_sizes;
-  if (!batch_sizes_on_device && z <= kInlineExperts && !capturing) {
+  if (!batch_sizes_on_device && z <= kInlineExperts && !capturing && pageable(batch_sizes)) {
     for (int e = 0; e < z; ++e)
       la.inline_sizes.v[e] = static_cast<int32_t>(std::max<int64_t>(-1, std::min<int64_t>(batch_sizes[e], tokens + 1)));
     bs_dev = nullptr;
