@@ -520,7 +520,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   uint32_t* sched_counter = reinterpret_cast<uint32_t*>(static_cast<char*>(workspace) + size_t(z) * sizeof(int64_t));
   const int max_ctas = std::min(ctas == 2 ? dev->pair_ctas : dev->sm_count, kMaxCtas);
   // A launch whose every possible tile is the first of some cluster draws no positions:
-  // no counter to zero, and no more CTAs than tiles.  Together with the inline
+  // no counter to zero, and no more CTAs than tiles (below).  Together with the inline
   // batch_sizes below this leaves a small call with one operation on the stream instead
   // of two or three; its kernel can then also start while the one before it ends.
   // A training step of 512 rows (4 experts, 128 x 128, host batch_sizes): 108.9 -> 99.3 us,
@@ -624,7 +624,12 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
       return rc;
   }
 
-  la.grid = single_wave ? static_cast<int>(max_tiles(p)) * ctas : max_ctas;
+  const bool with_push = push != nullptr && push->src != nullptr && push->n_items > 0 && !gather && !swiglu &&
+                         p.mode != kTN;
+  // A launch that carries a row transfer keeps every CTA, however few its tiles: the
+  // items are dealt over the grid.  (6 rows in 4 experts, k = 64, n = 72, beside 4000 rows of
+  // 21504 bytes: 6466 us on the tiles' four CTAs, 196 us on all.)
+  la.grid = single_wave && !with_push ? static_cast<int>(max_tiles(p)) * ctas : max_ctas;
   la.stream = stream;
   la.map_a = map_a;
   la.map_b = map_b;
@@ -651,8 +656,6 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     la.a_src = static_cast<const __nv_bfloat16*>(a);
     la.a_src_rows = a_source_rows;
   }
-  const bool with_push = push != nullptr && push->src != nullptr && push->n_items > 0 && !gather && !swiglu &&
-                         p.mode != kTN;
   if (with_push) {
     la.push = *push;
     la.push.via_tma = env_int("B200GMM_PUSH_TMA", 1) ? 1 : 0;  // bulk copies measured faster than the register path

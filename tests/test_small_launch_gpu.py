@@ -97,3 +97,53 @@ def test_captured_call_reads_host_sizes_at_replay():
     graph.replay()
     torch.cuda.synchronize()
     assert bool((c == 128).all())
+
+
+def test_row_transfer_in_a_small_launch_uses_the_whole_device(monkeypatch):
+    """A product of six rows that carries 86 MB of row transfer.  The same transfer as a
+    launch of its own takes about 45 us, inside the product about 200; dealt over the
+    product's four thread blocks alone it took 6500.  The bound, about 1000, lies between."""
+    lib = _capi.load()
+    monkeypatch.setenv("B200GMM_PUSH_TMA", "1")
+    sizes, k, n, items, columns = [3, 1, 0, 2], 64, 72, 4000, 10752
+    z, rows = len(sizes), sum(sizes)
+    a = torch.randn(rows, k, device="cuda").bfloat16()
+    b = torch.randn(z, k, n, device="cuda").bfloat16()
+    want = backend.gmm(a, b, torch.tensor(sizes))
+    bs = torch.tensor(sizes, device="cuda")
+    out = torch.zeros(rows, n, device="cuda", dtype=torch.bfloat16)
+    dest = torch.arange(rows, device="cuda") * (n * 2) + out.data_ptr()
+    src = torch.randn(items, columns, device="cuda").bfloat16()
+    dst = torch.zeros_like(src)
+    row = torch.arange(items, device="cuda")
+    rank = torch.zeros(items, dtype=torch.int32, device="cuda")
+    table = torch.tensor([dst.data_ptr()], device="cuda")
+    nbytes = _capi.workspace_bytes(z)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    head = (a.data_ptr(), b.data_ptr(), dest.data_ptr(), out.data_ptr(), out.numel() * 2, bs.data_ptr(), 1, z, rows, k, n, 0)
+    push = (src.data_ptr(), columns * 2, items, None, rank.data_ptr(), row.data_ptr(), table.data_ptr())
+
+    def fused():
+        assert lib.b200gmm_run_scatter_push(*head, *push, ws.data_ptr(), nbytes, None, stream) == 0
+
+    def separate():
+        assert lib.b200gmm_run_scatter(*head, ws.data_ptr(), nbytes, None, stream) == 0
+        assert lib.b200gmm_push_rows(*push, 0, stream) == 0
+
+    def microseconds(launch):
+        times = []
+        for _ in range(8):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            begin.record()
+            launch()
+            end.record()
+            end.synchronize()
+            times.append(begin.elapsed_time(end) * 1e3)
+        return sorted(times)[len(times) // 2]
+
+    alone = microseconds(separate)
+    dst.zero_()
+    together = microseconds(fused)
+    assert torch.equal(out, want) and torch.equal(dst, src)
+    assert together < 20 * alone + 100, (together, alone)
