@@ -237,7 +237,7 @@ __device__ __forceinline__ int64_t scan_step(int64_t v, int lane, int64_t* carry
 //   tile_start  exclusive prefix sums of the per-expert tile counts in that order.
 //
 // batch_sizes == nullptr: the sizes are those of `inline_sizes`.
-__device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* __restrict__ batch_sizes,
+__device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* batch_sizes,
                                                const InlineSizes& inline_sizes, SmemTail* tail, uint32_t* status) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -396,16 +396,21 @@ struct TileFeed {
   }
 };
 
+// The inputs that ordinary loads read (batch_sizes, row_dest, a_rows, row_scale, gate_grad,
+// the rows of a push) may still be written by the kernel before this one while this one
+// sets up.  So none of them is `const __restrict__` or read through __ldg: either lets
+// the compiler take the read-only path, whose loads it need not keep behind the
+// grid_dependency_wait() below.
 template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false>
 __global__ void __launch_bounds__(GATHER ? GatherWarps<CTAS>::kBlockThreads : (PUSH ? kGemmPushThreads : kThreads), 1)
 gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
            const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_c,
            const __grid_constant__ CUtensorMap map_a2, __nv_bfloat16* __restrict__ c,
-           const int64_t* __restrict__ batch_sizes, const Problem p,
-           uint32_t* status, CUtensorMap* map_slots, uint32_t* sched_counter, const int64_t* __restrict__ row_dest,
-           const int32_t* __restrict__ a_rows, const __nv_bfloat16* __restrict__ a_src,
-           const int64_t a_src_rows, const float* __restrict__ row_scale, const int reduce_add,
-           const int64_t dest_lo, const int64_t dest_hi, const __nv_bfloat16* __restrict__ gate_grad,
+           const int64_t* batch_sizes, const Problem p,
+           uint32_t* status, CUtensorMap* map_slots, uint32_t* sched_counter, const int64_t* row_dest,
+           const int32_t* a_rows, const __nv_bfloat16* a_src,
+           const int64_t a_src_rows, const float* row_scale, const int reduce_add,
+           const int64_t dest_lo, const int64_t dest_hi, const __nv_bfloat16* gate_grad,
            const PushArgs push, const __grid_constant__ InlineSizes inline_sizes) {
   static_assert(!SWIGLU || MODE != kTN, "the gated product is a forward product");
   static_assert(!PUSH || (!GATHER && !SWIGLU && MODE != kTN), "push warps exist in the plain forward / dgrad kernels");
@@ -967,7 +972,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
 #pragma unroll
         for (int j = 0; j < kPushVecsInFlight; ++j) {
           const int64_t v = base + j * 32 + lane;
-          if (v < push.row_vecs) r[j] = __ldg(src + v);
+          if (v < push.row_vecs) r[j] = src[v];
         }
 #pragma unroll
         for (int j = 0; j < kPushVecsInFlight; ++j) {

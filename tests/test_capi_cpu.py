@@ -203,3 +203,17 @@ def test_variant_choice_depends_on_shapes_only(monkeypatch):
     small = _schedule([64] * 64, 4096, 512, 512, 0, 0, 0)
     assert int(big[:, 3].max()) == 256 and int(small[:, 3].max()) == 64
     assert (small[:, 5] == 1).all(), "64-row experts run as transposed tiles"
+
+
+def test_overlapped_kernel_has_no_read_only_inputs():
+    """gmm_kernel starts while the kernel before it may still write its inputs, so no input
+    that it reads with ordinary loads may take the read-only path: the output is the only
+    __restrict__ parameter, and neither it nor build_schedule uses __ldg."""
+    path = os.path.join(ROOT, "grouped_gemm_b200", "csrc", "gmm_kernel.cuh")
+    text = re.sub(r"//[^\n]*", "", open(path).read())
+    signature = re.search(r"\bgmm_kernel\((.*?)\)\s*\{", text, flags=re.S).group(1)
+    restricted = [p.strip() for p in signature.split(",") if "__restrict__" in p]
+    assert restricted == ["__nv_bfloat16* __restrict__ c"]
+    schedule = re.search(r"\bvoid build_schedule\((.*?)\)\s*\{", text, flags=re.S).group(1)
+    assert "__restrict__" not in schedule
+    assert "__ldg" not in text
