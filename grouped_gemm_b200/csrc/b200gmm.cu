@@ -487,6 +487,12 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     }
   }
   if (a == nullptr || b == nullptr) return B200GMM_EINVAL;
+  if (pair_sum) {
+    if (b2 == nullptr) return B200GMM_EINVAL;
+    // rows of a's second part and the length of both parts of the contraction, each
+    // rounded up to a k-block, are 32-bit numbers in the kernel (schedule.cuh: make_tile)
+    if (2 * tokens + p.tile_m >= (int64_t(1) << 31) || 2 * (dim_a1 + kBlockK) >= (int64_t(1) << 31)) return B200GMM_ELIMIT;
+  }
   if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(b) & 15) ||
       (reinterpret_cast<uintptr_t>(c) & 15))
     return B200GMM_EALIGN;
@@ -505,8 +511,6 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   p.pair_sum = pair_sum ? 1 : 0;
   p.zero_rest = zero_rest ? 1 : 0;
   if (pair_sum) {
-    if (b2 == nullptr) return B200GMM_EINVAL;
-    if (2 * tokens + p.tile_m >= (int64_t(1) << 31)) return B200GMM_ELIMIT;
     p.light = 0;  // (transposed tiles know no second part)
   }
 

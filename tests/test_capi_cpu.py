@@ -217,3 +217,24 @@ def test_overlapped_kernel_has_no_read_only_inputs():
     schedule = re.search(r"\bvoid build_schedule\((.*?)\)\s*\{", text, flags=re.S).group(1)
     assert "__restrict__" not in schedule
     assert "__ldg" not in text
+
+
+def test_pair_sum_refuses_what_its_32_bit_numbers_cannot_hold():
+    """Both parts of the contraction, each a whole number of k-blocks of 64, and the rows of
+    both parts of a_pair: below 2^31 each, refused before any CUDA call (the addresses
+    are dummies; sizes that fit would go on to ask for the device)."""
+    lib = _capi.load()
+    dummy = np.zeros(64, dtype=np.int64)
+    at = (dummy.ctypes.data + 15) // 16 * 16
+    bs = np.array([8], dtype=np.int64)
+
+    def run(tokens, d1, b1=at, n=8):
+        return lib.b200gmm_run_pair_sum(at, at, b1, at, bs.ctypes.data, 0, 1, tokens, d1, n, 0, None, 0, None, None)
+
+    assert run(8, 2 ** 30 - 64) == -3
+    assert run(8, 2 ** 31 - 264) == -3
+    assert run(2 ** 30 - 128, 64) == -3
+    assert run(8, 64, b1=None) == -1
+    assert run(8, 64, b1=at + 8) == -2
+    assert run(8, 60) == -2
+    assert run(0, 2 ** 30 - 64) == 0 and run(8, 2 ** 30 - 64, n=0) == 0     # nothing to do
