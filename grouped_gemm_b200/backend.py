@@ -287,6 +287,10 @@ def _gmm_pair_sum(a_pair, b0, b1, batch_sizes, trans_b):
     ``_swiglu_product_grads`` has checked and made."""
     tokens, k = a_pair.shape[1], a_pair.shape[2]
     n = b0.shape[1] if trans_b else b0.shape[2]
+    if tokens >= 2 ** 30 - 128:   # past what the one launch can address, not past what the two can
+        c = gmm(a_pair[0], b0, batch_sizes, trans_b=trans_b)
+        c += gmm(a_pair[1], b1, batch_sizes, trans_b=trans_b)
+        return c
     c = torch.empty(tokens, n, device=a_pair.device, dtype=a_pair.dtype)
     lib = _capi.load()
     z = batch_sizes.shape[0]

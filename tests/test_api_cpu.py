@@ -133,3 +133,22 @@ def test_fused_gather_autograd_plumbing(monkeypatch, trans_b):
     assert torch.allclose(y1, y2.detach(), rtol=1e-4, atol=1e-4)
     assert torch.allclose(x1.grad, x2.grad, rtol=1e-4, atol=1e-4)
     assert torch.allclose(b1.grad, b2.grad, rtol=1e-4, atol=1e-4)
+
+
+def test_gated_input_gradient_past_the_row_limit_of_one_launch(monkeypatch):
+    """Rows that the two products take and their sum in one launch does not (2^30 - 128 and
+    more): two products, added.  Tensors without storage stand in for the 34 GB."""
+    calls = []
+
+    def product(a, b, batch_sizes, trans_a=False, trans_b=False, c=None):
+        calls.append((tuple(a.shape), a.storage_offset(), b, trans_b))
+        return torch.empty(a.shape[0], b.shape[1] if trans_b else b.shape[2], device=a.device, dtype=a.dtype)
+
+    monkeypatch.setattr(backend, "gmm", product)
+    rows = 2 ** 30 - 128
+    pair = torch.empty(2, rows, 8, device="meta", dtype=torch.bfloat16)
+    b0, b1 = (torch.empty(1, 16, 8, device="meta", dtype=torch.bfloat16) for _ in range(2))
+    c = backend._gmm_pair_sum(pair, b0, b1, torch.tensor([rows]), True)
+    assert c.shape == (rows, 16)
+    assert [(shape, offset, tb) for shape, offset, _, tb in calls] == [((rows, 8), 0, True), ((rows, 8), rows * 8, True)]
+    assert calls[0][2] is b0 and calls[1][2] is b1
