@@ -281,7 +281,38 @@ struct Features {
   bool gather = false;
   bool swiglu = false;
   bool gated_backward = false;
+  bool scatter = false;  // row_dest: rows of the result go where a table says
 };
+
+// Which launches run their tiles of few rows with swapped operands (schedule.cuh), and up
+// to how many rows a tile.  What the form saves is tensor work on rows that do not exist,
+// that is, power: launches that stream weights for long run into the power cap, and the
+// clock follows.  What it costs is an epilogue that transposes.  Measured over 1 to 256
+// experts, k = 64 .. 7168, uniform and Zipf routing, both forms in turn, 40 ms each; time
+// without / with (under the power cap a figure moves by a tenth from run to run):
+//   rows an expert (mean)  plain products and scattered rows: 1.00 to 1.25 up to 64 (256
+//     experts, k = 7168, n = 2048, Zipf: 1128 / 908 us at 8 rows, 1457 / 1183 at 32, 1571 / 1339 at
+//     64), even from 80 to 128, 0.81 to 1.02 from 144 on, where remainders share their weights
+//     with whole tiles (192 rows each: 2172 / 2669 us).  Gated product: 1.04 up to 48 on
+//     average (same experts, 32 rows, Zipf: 3060 / 2361 us), 0.98 at 64, 0.79 to 1.0 from 96 on.
+//   contraction  scattered rows and the gated product gain most where it is short and the
+//     epilogue counts (64 experts of 8 rows, n = 4096, k = 64: 30.8 / 20.6 and 39.2 / 24.6 us).  A
+//     plain product's whole boxes leave as TMA stores in either form: 0.92 to 1.10 at k =
+//     64 and 128, even at 256 and 384; it takes the form from 512 on.
+//   tiles  where most SMs have none, one SM's pipeline is the bound, not HBM and not power:
+//     1 expert of 16 rows, k = 4096: plain 0.92 with 16 tiles, 0.97 with 48, 1.01 with 64;
+//     scattered 0.97, 1.02, 1.05; gated 0.84, 0.89, 0.92, and 1.06 with 100.
+// Not the gathered product (0.95 to 1.0 nearly everywhere: its copies are the bound, and
+// the rows that do not exist are not copied in either form), and not the gated backward,
+// which reads its gradient row by row there (104 and 222 us at 40 rows, k = 512).
+int swap_rows(const Problem& p, const Features& f, int ctas, int sm_count) {
+  constexpr int64_t kMeanRows = 64, kMeanRowsGated = 48, kPlainMinK = 512;
+  if (p.mode == kTN || ctas != 1 || f.gather || f.gated_backward) return 0;
+  const int64_t tiles = int64_t(p.nt) * std::min<int64_t>(p.z, p.tokens);  // experts with rows have one row tile, mostly
+  if (f.swiglu) return p.tokens <= kMeanRowsGated * p.z && 3 * tiles >= 2 * sm_count ? kBlockM / 2 : 0;
+  if (!f.scatter && p.d1 < kPlainMinK) return 0;
+  return p.tokens <= kMeanRows * p.z && 2 * tiles >= sm_count ? kBlockM / 2 : 0;
+}
 
 int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b, int ctas,
                   Problem* p, const Features& f = Features()) {
@@ -313,19 +344,7 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   // by streaming their weights from HBM either way, and measured end to end the
   // launch was not faster with them (B200GMM_LIGHT=1 switches them on).
   p->light = (p->mode != kTN && ctas == 1 && !f.gather && !f.swiglu) ? env_int("B200GMM_LIGHT", 0) : 0;
-  // Token generation: where an expert has at most 16 rows on average and the contraction
-  // is long, tiles of at most half their rows run with their operands swapped
-  // (schedule.cuh).  Without and with, each in a process of its own: 1024 rows over 256
-  // experts, k = 7168, n = 2048: 869 and 770 us; 64 rows over 8 experts of 4096 x 14336: 149 and
-  // 140 us; a decode step of that expert layer (128 rows): 450 and 425 us.  Outside of that
-  // the transposing epilogue costs what the padded rows did, or more.  64 experts, n =
-  // 4096: 8 rows each, k = 512 and 2048: 50 and 50, 171 and 172 us; 64 rows each: 55.0 and 55.5, 183
-  // and 187 us; remainders of 32 experts of 300 rows, k = 2048: 207 and 220 us, gated 383 and
-  // 452 us.  The gated backward, which reads its gradient row by row there: 104 and 222 us
-  // (40 rows, k = 512).
-  constexpr int64_t kSwapMeanRows = 16, kSwapMinK = 4096;
-  p->swap_rows = (p->mode != kTN && !(f.swiglu && ctas == 2) && !f.gated_backward && tokens <= kSwapMeanRows * z &&
-                  d1 >= kSwapMinK) ? p->tile_m / 2 : 0;
+  p->swap_rows = 0;  // decided where the device is known (run_impl)
   p->dest_indexed = 0;
   p->dest_rows = 0;
   p->pair_sum = 0;
@@ -459,6 +478,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   feat.gather = (a_rows != nullptr);
   feat.swiglu = swiglu;
   feat.gated_backward = gate_grad != nullptr;
+  feat.scatter = row_dest != nullptr;
   int ctas = choose_ctas(z, tokens, dim_a1, trans_a);
   int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat);
   if (rc != B200GMM_OK) return rc;
@@ -506,6 +526,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     if ((rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat)) != B200GMM_OK) return rc;
   }
 
+  p.swap_rows = swap_rows(p, feat, ctas, dev->sm_count);
   p.dest_indexed = dest_rows >= 0 ? 1 : 0;
   p.dest_rows = dest_rows;
   p.pair_sum = pair_sum ? 1 : 0;

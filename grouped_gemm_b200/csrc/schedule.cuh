@@ -122,7 +122,7 @@ B200GMM_HD int tile_stages(const Tile& t) {
 // allows, so that the tensor core works for the rows that exist and not for tile_m of
 // them, and only those rows are fetched.  Launches of small experts are bound by streaming
 // weights; what the padded rows cost them was tensor time and power and a third of the
-// bytes that enter an SM.  Which launches: Problem::swap_rows, decided by check_problem.
+// bytes that enter an SM.  Which launches: Problem::swap_rows (b200gmm.cu: swap_rows).
 // Returns the rounded row count, 0 for a plain tile.
 B200GMM_HD int swapped_rows(const Problem& p, const Tile& t) {
   if (p.swap_rows == 0 || t.kind != 0) return 0;
