@@ -582,7 +582,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   // N: columns of b (and of b2, and of c); the Problem's n is twice that for the gated product.
   const uint64_t T = uint64_t(tokens), D1 = uint64_t(dim_a1), N = uint64_t(n_out), Z = uint64_t(z);
   const bool gather = (a_rows != nullptr);  // a is then fetched row by row, without a tensor map
-  const bool swap_maps = !gather && (p.swap_rows > 0 || p.light);
+  const bool swap_maps = p.swap_rows > 0 || p.light;
   if (p.mode == kNN) {
     const uint64_t da[2] = {D1, pair_sum ? 2 * T : T};
     const uint32_t ba[2] = {kBlockK, uint32_t(kBlockM)};

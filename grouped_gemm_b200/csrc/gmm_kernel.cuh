@@ -426,13 +426,10 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   // (map_a2: the activations with 32-row boxes; NT also uses map_b2: b with
   // 128-row boxes).
   constexpr bool kLight = (MODE != kTN) && (CTAS == 1) && !GATHER && !SWIGLU;
-  // Swapped tiles (schedule.cuh) exist wherever the rows of a tile are independent and
-  // one CTA holds all that an output element needs: not in the pair form of the gated
-  // product, whose gate and up columns lie in different CTAs.
-  // A sum of two products over one accumulator (Problem::pair_sum) is an option of the
-  // plain kernels.
+  // So do swapped tiles (schedule.cuh), and in the gated product's.  A sum of two products
+  // over one accumulator (Problem::pair_sum) is an option of the plain kernels.
+  constexpr bool kSwap = (MODE != kTN) && (CTAS == 1) && !GATHER;
   constexpr bool kPairSum = (MODE != kTN) && !GATHER && !SWIGLU && !PUSH;
-  constexpr bool kSwap = (MODE != kTN) && !(SWIGLU && CTAS == 2);
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = ptx::smem_u32(smem_raw);
@@ -454,7 +451,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       ptx::prefetch_tensormap(&map_a);
       ptx::prefetch_tensormap(&map_b);
       if (SWIGLU || (kLight && MODE == kNT)) ptx::prefetch_tensormap(&map_b2);
-      if (kSwap && !GATHER) ptx::prefetch_tensormap(&map_a2);
+      if (kSwap) ptx::prefetch_tensormap(&map_a2);
       ptx::prefetch_tensormap(&map_c);
       for (int s = 0; s < kStages; ++s) {
         // the producer's expect_tx arrival, plus one arrival by the gather warp that fills
@@ -582,22 +579,18 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             ptx::fence_tensormap_acquire(tn_b);
           }
         }
-        // A swapped tile fetches its rows in boxes of 32; in a pair each CTA stages half of them.
-        const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
-        const int sw_boxes = (sw_rows / CTAS + 31) >> 5;
-        const int a_row = t.row0 + (sw_rows != 0 ? static_cast<int>(cta_rank) * (sw_rows / CTAS) : row_off);
+        // A swapped tile fetches its rows in boxes of 32.
+        const int sw_boxes = kSwap ? (swapped_rows(p, t) + 31) >> 5 : 0;
         // Bytes this CTA's TMA loads bring per stage: the gather warps fetch A themselves.
         const uint32_t tma_bytes =
-            G::kBBytes + (GATHER ? 0u : (sw_rows != 0 ? uint32_t(sw_boxes) * kRowBoxBytes : G::kABytes));
-        int part_row = a_row;                // row of a the current part of the contraction starts at
+            G::kBBytes + (GATHER ? 0u : (kSwap && sw_boxes != 0 ? uint32_t(sw_boxes) * kRowBoxBytes : G::kABytes));
+        int part_row = t.row0 + row_off;     // row of a the current part of the contraction starts at
         const CUtensorMap* part_b = &map_b;  // and its weights
         auto load_rows = [&](uint32_t dst, uint32_t bar, int k0) {  // A of a forward / dgrad stage
           if (GATHER) return;
-          if (kSwap && sw_rows != 0) {
-            for (int i = 0; i < sw_boxes; ++i) {
-              if (kPair) ptx::tma_load_2d_pair(dst + i * kRowBoxBytes, &map_a2, bar, k0, part_row + i * 32);
-              else ptx::tma_load_2d(dst + i * kRowBoxBytes, &map_a2, bar, k0, part_row + i * 32);
-            }
+          if (kSwap && sw_boxes != 0) {
+            for (int i = 0; i < sw_boxes; ++i)
+              ptx::tma_load_2d(dst + i * kRowBoxBytes, &map_a2, bar, k0, part_row + i * 32);
           } else {
             if (kPair) ptx::tma_load_2d_pair(dst, &map_a, bar, k0, part_row);
             else ptx::tma_load_2d(dst, &map_a, bar, k0, part_row);
@@ -763,26 +756,23 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         const uint32_t sb = sa + G::kABytes;
         if (kSwap && sw_rows != 0) {
           // D[weight columns, rows] = W^T x X^T: the staged B tile is the UMMA A operand
-          // (128 columns a CTA per MMA), the staged rows are the UMMA B operand.
+          // (its two halves of 128 columns in turn), the staged rows are the UMMA B operand.
           if (lane == 0) {
-            const uint32_t idesc = ptx::make_idesc_bf16(kBlockM * CTAS, sw_rows, kBMn ? 1 : 0, 0);
+            const uint32_t idesc = ptx::make_idesc_bf16(kBlockM, sw_rows, kBMn ? 1 : 0, 0);
             const uint64_t xdesc = ptx::make_smem_desc(sa, 16u, 1024u);
             constexpr uint64_t w_step = kBMn ? (2048u >> 4) : (32u >> 4);
 #pragma unroll
             for (int k = 0; k < kBlockK / 16; ++k) {
 #pragma unroll
-              for (int h = 0; h < 2 / CTAS; ++h) {  // one CTA: the tile's two halves of 128 columns
+              for (int h = 0; h < 2; ++h) {
                 const uint32_t sw = sb + uint32_t(h) * (G::kBBytes / 2);
                 const uint64_t wdesc = kBMn ? ptx::make_smem_desc(sw, kBoxBytes, 1024u)
                                             : ptx::make_smem_desc(sw, 16u, 1024u);
                 const uint32_t d = d_tmem + uint32_t(h) * (kBlockN / 2);
-                const uint32_t acc = (kb | k) != 0 ? 1u : 0u;
-                if (kPair) ptx::mma_bf16_ss_pair(d, wdesc + k * w_step, xdesc + k * (32u >> 4), idesc, acc);
-                else ptx::mma_bf16_ss(d, wdesc + k * w_step, xdesc + k * (32u >> 4), idesc, acc);
+                ptx::mma_bf16_ss(d, wdesc + k * w_step, xdesc + k * (32u >> 4), idesc, (kb | k) != 0 ? 1u : 0u);
               }
             }
-            if (kPair) ptx::mma_commit_pair(ptx::smem_u32(&tail->empty[s]), 0x3);
-            else ptx::mma_commit(ptx::smem_u32(&tail->empty[s]));
+            ptx::mma_commit(ptx::smem_u32(&tail->empty[s]));
           }
         } else if (lane == 0) {
           // K-major SW128 operand: 8-row groups 1024 B apart, +32 B per 16-wide k step.
@@ -1098,19 +1088,15 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         continue;
       }
       if (next < base + nkb) {
-        // a swapped tile's rows are split evenly over the CTAs of a pair (kSwap)
-        const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
-        const int own_rows = sw_rows != 0 ? sw_rows / CTAS : kBlockM;
-        const int own_off = static_cast<int>(cta_rank) * own_rows;
         int idx[32];
         bool all_rows = true;  // every row of this lane exists
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          const int r = own_off + j * 4 + sub;  // row inside the (pair) tile
+          const int r = row_off + j * 4 + sub;  // row inside the (pair) tile
           // rows that do not exist are filled with zeros and never stored; so is a
           // row whose index lies outside a_src, which is also reported
           idx[j] = -1;
-          if (r < t.valid_rows && j * 4 + sub < own_rows) {
+          if (r < t.valid_rows) {
             const int ix = a_rows[t.row0 + r];
             if (ix >= 0 && ix < a_src_rows) idx[j] = ix;
             else bad_index = true;
@@ -1362,21 +1348,19 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       const int nkb = tile_stages(t);
       const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
       if (kSwap && sw_rows != 0) {
-        // TMEM lane = output column, TMEM column = output row.  One CTA: this warp's
-        // half of the tile's columns is an accumulator of its own (for the gated
-        // product the two are gate and up of the same 128 output columns).  A pair:
-        // each CTA holds 128 of the columns.  Where both warps of a lane quadrant
-        // serve the same columns they take the 32-row chunks in turn.
-        constexpr bool kShareColumns = kPair || SWIGLU;
+        // TMEM lane = output column, TMEM column = output row.  This warp's half of the
+        // tile's columns is an accumulator of its own; for the gated product the two are
+        // gate and up of the same 128 output columns, and the two warps of a lane quadrant
+        // take the 32-row chunks in turn.
         const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
         ++it;
         if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), aph, wait)) { ok = false; break; }
         ptx::tc_fence_after_sync();
         const int out_n = static_cast<int>(SWIGLU ? (p.n >> 1) : p.n);
-        const int col = (SWIGLU ? (t.col0 >> 1) : t.col0) + (kPair ? col_off : (SWIGLU ? 0 : col_base)) + q * 32;
-        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + (kShareColumns ? 0 : col_base);
+        const int col = (SWIGLU ? (t.col0 >> 1) : t.col0) + (SWIGLU ? 0 : col_base) + q * 32;
+        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + (SWIGLU ? 0 : col_base);
         if (col < out_n) {
-          for (int r0 = kShareColumns ? half * 32 : 0; r0 < t.valid_rows; r0 += kShareColumns ? 64 : 32) {
+          for (int r0 = SWIGLU ? half * 32 : 0; r0 < t.valid_rows; r0 += SWIGLU ? 64 : 32) {
             const int rows = t.valid_rows - r0;
             const int64_t row = int64_t(t.row0) + r0;
             uint32_t va[32], vb[32];
@@ -1401,11 +1385,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         }
         ptx::tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) {
-          const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
-          if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(te_bar, 0));
-          else ptx::mbar_arrive(te_bar);
-        }
+        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&tail->tmem_empty[ab]));
         continue;
       }
       if (kLight && t.kind) {

@@ -116,18 +116,17 @@ B200GMM_HD int tile_stages(const Tile& t) {
   return t.kind ? (t.k_len + kLightK - 1) / kLightK : (t.k_len + kBlockK - 1) / kBlockK;
 }
 
-// Swapped tiles (NN/NT): a tile_m x 256 tile with few rows is computed as its transpose,
-// from the same loads.  The tile's 256 weight columns ride UMMA M (one CTA: two MMAs of
-// 128 columns; a pair: one MMA of 2 x 128) and its rows ride UMMA N, rounded up to the step N
-// allows, so that the tensor core works for the rows that exist and not for tile_m of
-// them, and only those rows are fetched.  Launches of small experts are bound by streaming
+// Swapped tiles (NN/NT, one CTA): a 128 x 256 tile with few rows is computed as its
+// transpose, from the same loads.  The tile's 256 weight columns ride UMMA M (two MMAs of
+// 128) and its rows ride UMMA N, rounded up to the step of 16 that N allows, so that the
+// tensor core works for the rows that exist and not for 128 of them, and only those
+// rows are fetched.  Launches of small experts are bound by streaming
 // weights; what the padded rows cost them was tensor time and power and a third of the
 // bytes that enter an SM.  Which launches: Problem::swap_rows (b200gmm.cu: swap_rows).
 // Returns the rounded row count, 0 for a plain tile.
 B200GMM_HD int swapped_rows(const Problem& p, const Tile& t) {
   if (p.swap_rows == 0 || t.kind != 0) return 0;
-  const int step = p.tile_m == kBlockM ? 16 : 32;
-  const int rows = (t.valid_rows + step - 1) / step * step;
+  const int rows = (t.valid_rows + 15) & ~15;
   return rows <= p.swap_rows ? rows : 0;
 }
 
