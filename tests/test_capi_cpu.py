@@ -238,3 +238,36 @@ def test_pair_sum_refuses_what_its_32_bit_numbers_cannot_hold():
     assert run(8, 64, b1=at + 8) == -2
     assert run(8, 60) == -2
     assert run(0, 2 ** 30 - 64) == 0 and run(8, 2 ** 30 - 64, n=0) == 0     # nothing to do
+
+
+def test_row_index_and_gated_backward_entries_reject_bad_arguments_before_cuda():
+    """The entry points that gmm_scatter and the gated backward use."""
+    lib = _capi.load()
+    bs = np.array([64, 64], dtype=np.int64)
+    room = np.zeros(64, dtype=np.int64)
+    at = (room.ctypes.data + 15) // 16 * 16   # any non-null, 16-byte aligned address
+
+    def rows(index=at, out=at, out_rows=128, weight=None, accumulate=0, tokens=128, k=64, n=64):
+        return lib.b200gmm_run_combine_rows(at, at, index, out, out_rows, weight, accumulate, bs.ctypes.data, 0, 2, tokens, k,
+                                            n, 0, None, 0, None, None)
+
+    assert rows(index=None) == -1
+    assert rows(out_rows=-1) == -1
+    assert rows(out=None) == -1
+    assert rows(weight=at + 2) == -2
+    assert rows(k=60) == -2 and rows(n=60) == -2
+    assert rows(k=0) == -1                      # nothing to overwrite the rows with
+    assert rows(k=0, accumulate=1) == 0         # adding nothing
+    assert rows(tokens=0) == 0 and rows(n=0) == 0
+
+    for entry in (lib.b200gmm_run_swiglu_backward, lib.b200gmm_run_swiglu_backward_full):
+        def gated(up=at, grad=at, products=at, tokens=128, k=64, n=64):
+            return entry(at, at, up, grad, products, bs.ctypes.data, 0, 2, tokens, k, n, 0, None, 0, None, None)
+
+        assert gated(products=None) == -1
+        assert gated(grad=None) == -1
+        assert gated(up=None) == -1
+        assert gated(up=at + 8) == -2
+        assert gated(grad=at + 8) == -1
+        assert gated(n=60) == -2 and gated(k=60) == -2
+        assert gated(tokens=0) == 0 and gated(n=0) == 0
