@@ -41,8 +41,8 @@ def gmm(a, b, batch_sizes, trans_a=False, trans_b=False, c=None):
 
 def _host_or_device_sizes(batch_sizes):
     """batch_sizes as the C ABI wants it: on the device as it is; on the host
-    contiguous and pageable (the library's asynchronous copy reads a pinned array
-    only when the stream gets there, by which time the caller may have changed it)."""
+    contiguous and pageable: that is read before the call returns, a pinned array only
+    when the stream gets there, by which time the caller may have changed it."""
     if batch_sizes.is_cuda:
         return batch_sizes
     bs = batch_sizes.contiguous()
@@ -277,7 +277,7 @@ def _swiglu_product_grads(a, b_gate, b_up, grad_out, batch_sizes, trans_b):
             a.data_ptr(), b_gate.data_ptr(), b_up.data_ptr(), grad_out.data_ptr(), out.data_ptr(), bs.data_ptr(),
             1 if bs.is_cuda else 0, z, tokens, k, n, 1 if trans_b else 0, ws.data_ptr(), ws_bytes,
             backend.device_status(a.device).data_ptr(), torch.cuda.current_stream(a.device).cuda_stream)
-    _capi.check(rc, "b200gmm_run_swiglu_backward")
+    _capi.check(rc, "b200gmm_run_swiglu_backward_full")
     return out
 
 

@@ -70,10 +70,10 @@ void gmm(at::Tensor a, at::Tensor b, at::Tensor c, at::Tensor batch_sizes, bool 
     TORCH_CHECK(batch_sizes.is_contiguous(), "batch_sizes must be contiguous");
   } else {
     batch_sizes = batch_sizes.contiguous();
-    // The library copies host batch sizes to the device with an asynchronous copy.
-    // From pageable memory the data is staged before that call returns; from pinned
-    // memory the copy reads the caller's buffer later, on the stream, when the
-    // caller may already have changed or freed it.  Take a pageable copy.
+    // The library reads host batch sizes in pageable memory before the call returns (as
+    // an argument of the launch, or staged by an asynchronous copy).  Pinned memory it
+    // reads later, on the stream, when the caller may already have changed or freed it.
+    // Take a pageable copy.
     if (batch_sizes.is_pinned()) batch_sizes = batch_sizes.clone();
   }
   TORCH_CHECK(z <= B200GMM_MAX_EXPERTS, b200gmm_strerror(B200GMM_ELIMIT));
