@@ -8,10 +8,10 @@
 //               TMEM), commits each stage back to the producer and each finished
 //               accumulator to the epilogue; two 256-column accumulators alternate
 //               so the epilogue of tile i overlaps the main loop of tile i+1;
-//   warps 2-9   epilogue: each warp owns 32 rows x 128 columns of the tile (TMEM
+//   warps 2-9   epilogue: each warp owns 32 rows x 128 columns of an accumulator (TMEM
 //               lane quadrant = warp % 4, column half = (warp - 2) / 4).  It
-//               tcgen05.ld's 32 columns at a time (the next load is in flight while
-//               the current one is converted), rounds to bf16, stages the 32x32
+//               tcgen05.ld's 32 columns at a time, rounds to bf16, and hands the
+//               accumulator back once all are in registers; then it stages each 32x32
 //               chunk in swizzled shared memory and writes it with a TMA tensor
 //               store; a warp whose 32 rows do not all exist (ragged last tile of
 //               an expert) stores its valid rows directly;
@@ -26,11 +26,17 @@
 //               last <= 64 rows of an expert run as a transposed tile instead: 128
 //               output columns on UMMA M, the rows on UMMA N (schedule.cuh);
 //   CTAS == 2   a pair of CTAs (a 2-CTA cluster on neighbouring SMs) owns
-//               256 x 256 tiles: each CTA stages its own 128 rows of A and HALF of
-//               the B tile, and the leader's tcgen05.mma.cta_group::2 reads both
-//               halves.  That cuts the L2 -> shared-memory traffic per flop by a
-//               third and shrinks a stage to 32 KiB, so six stages fit.  No TMA
-//               multicast is used anywhere.
+//               256 x 512 tiles: each CTA stages its own 128 rows of A and HALF of
+//               the B tile, the leader's tcgen05.mma.cta_group::2 reads both
+//               halves, and both accumulators belong to the tile.  A k-block of A is then
+//               staged once for 512 columns: 48 KiB enter an SM for 128 x 512 outputs, where
+//               32 KiB for 128 x 256 did before (a one-CTA tile: 48 KiB for 128 x 256).
+//               These launches run at the power cap, where bytes moved are time, and
+//               the row copies of the gathered product were its bound:
+//               16384 rows, 8 experts of 4096 x 14336, tiles of 256 against 512 columns:
+//               gathered product 1866 / 1633 us, gathered wgrad 2052 / 1783, scattered dgrad 1625 /
+//               1539; 32768 rows, plain: 2989 / 2943, dgrad 2995 / 2939, wgrad 3051 / 2912.
+//               No TMA multicast is used anywhere.
 //
 // Optional template variants:
 //   GATHER      row i of A is row a_rows[i] of another tensor: extra warps fetch
@@ -63,13 +69,17 @@ constexpr int kSchedWarp = 2 + kEpilogueWarps;        // warp 10
 constexpr int kThreads = 32 * (kSchedWarp + 1);       // 352
 constexpr int kMaxExperts = 1024;
 constexpr uint32_t kTmemCols = 512;
-constexpr int kMaxStages = 6;
+constexpr int kMaxStages = 4;
 constexpr uint32_t kBoxBytes = 64 * kBlockK * 2;  // one 64-wide MN-major TMA box: 8 KiB
 // wgrad keeps private, editable copies of its two tensor maps in the caller's
 // workspace: kMapSlots {a, b} pairs per cluster, edited in turn.  The scheduler
 // edits a slot only when every tile that used it has all its loads landed (the
 // MMA warp counts finished tiles).
 constexpr int kMapSlots = 8;
+// k-blocks by which the second accumulator of a wide tile trails the first at its ends
+// (gmm_kernel, wide_tile): 512 cycles of MMAs each.  One is 0.5 to 1.5 % slower (epilogue not
+// done reading).
+constexpr int kSkew = 2;
 constexpr int kMaxCtas = 256;  // workspace is sized for this many CTAs
 // Ring through which the scheduler hands tiles to the other roles.  Deep
 // enough that the producer can run ahead by a ring of one-stage tiles plus both
@@ -82,20 +92,20 @@ constexpr int kSchedSlots = 8;
 // speed of its output stores.  Each epilogue warp has two buffers of 32 rows x 64
 // columns there (128-byte rows), used in turn, so that a warp fills one while
 // the TMA store of the other still reads; the forward / dgrad layouts have one
-// buffer of 32 x 32 per warp.  So has the gathered wgrad: a warp that fetches rows
-// with cp.async needs over a microsecond from a free stage to a full one, and four
-// stages of a pair (0.28 us of MMAs each) do not cover that.
+// buffer of 32 x 32 per warp.  So has the gathered wgrad, which needs the stages: a warp
+// that fetches rows with cp.async takes over a microsecond from a free stage to a full one.
 template <int CTAS, int MODE = kNN, bool GATHER = false>
 struct Geometry {
   static constexpr bool kWideOut = (MODE == kTN) && !GATHER;  // 64-column stores from double buffers
-  static constexpr int kStages = kWideOut ? ((CTAS == 1) ? 3 : 4) : ((CTAS == 1) ? 4 : 6);
+  static constexpr int kStages = kWideOut ? 3 : 4;
+  static constexpr int kUnits = CTAS;  // accumulators a tile fills side by side: a pair's tile is 512 columns wide
   static constexpr int kOutBufs = kWideOut ? 2 : 1;  // staging buffers per epilogue warp
   static constexpr uint32_t kOutBufBytes = kWideOut ? 4096u : 2048u;
-  static constexpr int kBCols = kBlockN / CTAS;                 // B columns staged by one CTA
+  static constexpr int kBCols = kBlockN / CTAS;                 // B columns staged by one CTA, per accumulator
   static constexpr uint32_t kABytes = kBlockM * kBlockK * 2;    // 16 KiB
-  static constexpr uint32_t kBBytes = kBCols * kBlockK * 2;     // 32 or 16 KiB
-  static constexpr uint32_t kStageBytes = kABytes + kBBytes;
-  static constexpr uint32_t kRingBytes = kStages * kStageBytes;  // 192 KiB (wgrad: 128 or 144 KiB)
+  static constexpr uint32_t kBBytes = kBCols * kBlockK * 2;     // 32 or 16 KiB, per accumulator
+  static constexpr uint32_t kStageBytes = kABytes + kUnits * kBBytes;  // 48 KiB
+  static constexpr uint32_t kRingBytes = kStages * kStageBytes;  // 192 KiB (wgrad: 144 KiB)
   static constexpr uint32_t kOutBytes = kEpilogueWarps * kOutBufs * kOutBufBytes;  // 16 KiB (wgrad: 64 KiB)
 };
 
@@ -108,15 +118,10 @@ constexpr uint32_t kLightXHalf = kLightRows * kBlockK * 2;         // 8 KiB per 
 constexpr uint32_t kRowBoxBytes = 32 * kBlockK * 2;                // one 32-row TMA box of activations: 4 KiB
 static_assert(kLightWBytes + 2 * kLightXHalf <= Geometry<1>::kStageBytes, "a transposed stage must fit a ring slot");
 
-// The gather variant adds warps that fetch the rows of A, a k-block each, in turn.
-// Four beside the four stages of the one-CTA ring, five beside the six of a pair: with
-// 11 + 5 = 16 warps a thread may use 128 registers, a 17th would leave 96 (an SM
-// quarter then holds five warps) and spill, and the sixth stage is the one being used.
-template <int CTAS>
-struct GatherWarps {
-  static constexpr int kWarps = CTAS == 1 ? 4 : 5;
-  static constexpr int kBlockThreads = kThreads + 32 * kWarps;
-};
+// The gather variant adds warps that fetch the rows of A, a k-block each, in turn: as many
+// as the ring has stages.  With 11 + 4 = 15 warps a thread may use 128 registers.
+constexpr int kGatherWarps = 4;
+constexpr int kGatherThreads = kThreads + 32 * kGatherWarps;
 
 // The push variant adds four warps that move rows between GPUs while the tensor
 // cores work (in the default, bulk-copy form of the transfer only one of their
@@ -160,7 +165,8 @@ struct __align__(16) TileRecord {
   int valid_rows;
   int k_len;
   int k_row0;
-  int pad[3];
+  int units;
+  int pad[2];
 };
 
 struct __align__(16) SmemTail {
@@ -190,7 +196,7 @@ static_assert(kSmemBytes <= 232448, "exceeds the 227 KiB of shared memory a CTA 
 constexpr size_t kPushStageOffset = (sizeof(SmemTail) + 127) / 128 * 128;
 constexpr size_t kSmemBytesPush = kSmemBytes - sizeof(SmemTail) + kPushStageOffset + kPushStageBytes;
 static_assert(kSmemBytesPush <= 232448, "the push variant's staging must fit too");
-static_assert(Geometry<1>::kRingBytes == Geometry<2>::kRingBytes, "both variants use the same ring size");
+static_assert(Geometry<1>::kStageBytes == Geometry<2>::kStageBytes && Geometry<1>::kRingBytes == Geometry<2>::kRingBytes, "both variants use the same ring size");
 static_assert(Geometry<1, kTN>::kRingBytes + Geometry<1, kTN>::kOutBytes <= Geometry<1>::kRingBytes + Geometry<1>::kOutBytes &&
               Geometry<2, kTN>::kRingBytes + Geometry<2, kTN>::kOutBytes <= Geometry<1>::kRingBytes + Geometry<1>::kOutBytes,
               "the wgrad layout must fit the common size");
@@ -296,18 +302,41 @@ __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* 
 
 // Position of the launch order -> tile (the scheduler's).  Positions come in
 // increasing order, so the expert cursor only ever moves forward.
+//
+// Tiles two accumulators wide are coarse: what is left over after whole rounds of the
+// grid's `clusters` is taken as halves when the halves fit one round, which then lasts half as
+// long.  A half that does not exist (the last column tile may be one accumulator
+// wide) is a tile of no units.
 struct TileWalker {
   const Problem& p;
   const SmemTail* tail;
+  int whole;  // positions before the halves
   int total;
   int pos;
-  __device__ TileWalker(const Problem& p_, const SmemTail* tail_)
-      : p(p_), tail(tail_), total(tail_->tile_start[p_.z]), pos(0) {}
+  __device__ TileWalker(const Problem& p_, const SmemTail* tail_, int clusters)
+      : p(p_), tail(tail_), whole(tail_->tile_start[p_.z]), total(whole), pos(0) {
+    if (p.tile_n > kBlockN && clusters > 0) {
+      const int left = whole % clusters;
+      if (2 * left <= clusters) {
+        whole -= left;
+        total += left;
+      }
+    }
+  }
   __device__ __forceinline__ bool decode(int t, Tile* out) {
     if (t < 0 || t >= total) return false;
+    int half = -1;
+    if (t >= whole) {
+      half = (t - whole) & 1;
+      t = whole + ((t - whole) >> 1);
+    }
     while (t >= tail->tile_start[pos + 1]) ++pos;
     const int e = tail->perm[pos];
     *out = make_tile(p, e, t - tail->tile_start[pos], tail->row_start[e], tail->row_start[e + 1]);
+    if (half >= 0) {
+      out->units = half < out->units ? 1 : 0;
+      out->col0 += half * kBlockN;
+    }
     return true;
   }
 };
@@ -347,10 +376,10 @@ struct TileFeed {
                                        : ptx::mbar_wait<false, 32>(full, parity, wait);
     if (!got) return kAbandoned;
     const uint32_t rec = ptx::smem_u32(&tail->sched_tile[slot]);
-    int t, unused[3];
+    int t, unused[2];
     ptx::ld_shared_v4(rec, &t, &map, &tile->expert, &tile->kind);
     ptx::ld_shared_v4(rec + 16, &tile->row0, &tile->col0, &tile->valid_rows, &tile->k_len);
-    ptx::ld_shared_v4(rec + 32, &tile->k_row0, &unused[0], &unused[1], &unused[2]);
+    ptx::ld_shared_v4(rec + 32, &tile->k_row0, &tile->units, &unused[0], &unused[1]);
     // Self-check of the hand-off: positions reach every role in strictly
     // increasing order.  One that does not is never used: the fault is recorded,
     // the launch is told to drain, and this role stops (warp-uniformly).
@@ -383,13 +412,13 @@ struct TileFeed {
     const uint32_t rec = ptx::smem_u32(&tail->sched_tile[slot]);
     ptx::st_shared_v4(rec, t, map_entry, tile.expert, tile.kind);
     ptx::st_shared_v4(rec + 16, tile.row0, tile.col0, tile.valid_rows, tile.k_len);
-    ptx::st_shared_v4(rec + 32, tile.k_row0, 0, 0, 0);
+    ptx::st_shared_v4(rec + 32, tile.k_row0, tile.units, 0, 0);
     ptx::mbar_arrive(ptx::smem_u32(&tail->sched_full[slot]));
     if (kPair) {
       const uint32_t peer = ptx::mapa(rec, 1);
       ptx::st_shared_cluster_v4(peer, t, map_entry, tile.expert, tile.kind);
       ptx::st_shared_cluster_v4(peer + 16, tile.row0, tile.col0, tile.valid_rows, tile.k_len);
-      ptx::st_shared_cluster_v4(peer + 32, tile.k_row0, 0, 0, 0);
+      ptx::st_shared_cluster_v4(peer + 32, tile.k_row0, tile.units, 0, 0);
       ptx::mbar_arrive_release_cluster(ptx::mapa(ptx::smem_u32(&tail->sched_full[slot]), 1));
     }
     return true;
@@ -402,7 +431,7 @@ struct TileFeed {
 // the compiler take the read-only path, whose loads it need not keep behind the
 // grid_dependency_wait() below.
 template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false>
-__global__ void __launch_bounds__(GATHER ? GatherWarps<CTAS>::kBlockThreads : (PUSH ? kGemmPushThreads : kThreads), 1)
+__global__ void __launch_bounds__(GATHER ? kGatherThreads : (PUSH ? kGemmPushThreads : kThreads), 1)
 gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
            const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_c,
            const __grid_constant__ CUtensorMap map_a2, __nv_bfloat16* __restrict__ c,
@@ -465,7 +494,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       }
       // Takers of a published tile position: per CTA the producer thread, the epilogue
       // warps and the gather warps, plus the leader's MMA warp.
-      constexpr uint32_t kTakers = CTAS * (1 + kEpilogueWarps + (GATHER ? GatherWarps<CTAS>::kWarps : 0)) + 1;
+      constexpr uint32_t kTakers = CTAS * (1 + kEpilogueWarps + (GATHER ? kGatherWarps : 0)) + 1;
       for (int i = 0; i < kSchedSlots; ++i) {
         ptx::mbar_init(ptx::smem_u32(&tail->sched_full[i]), 1);
         ptx::mbar_init(ptx::smem_u32(&tail->sched_empty[i]), kTakers);
@@ -583,7 +612,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         const int sw_boxes = kSwap ? (swapped_rows(p, t) + 31) >> 5 : 0;
         // Bytes this CTA's TMA loads bring per stage: the gather warps fetch A themselves.
         const uint32_t tma_bytes =
-            G::kBBytes + (GATHER ? 0u : (kSwap && sw_boxes != 0 ? uint32_t(sw_boxes) * kRowBoxBytes : G::kABytes));
+            G::kBBytes * uint32_t(kPair ? t.units : 1) + (GATHER ? 0u : (kSwap && sw_boxes != 0 ? uint32_t(sw_boxes) * kRowBoxBytes : G::kABytes));
         int part_row = t.row0 + row_off;     // row of a the current part of the contraction starts at
         const CUtensorMap* part_b = &map_b;  // and its weights
         auto load_rows = [&](uint32_t dst, uint32_t bar, int k0) {  // A of a forward / dgrad stage
@@ -647,42 +676,40 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
               }
             }
           } else {
-            // Pair: this CTA stages rows [row0+row_off, +128) of A and columns
-            // [col0+col_off, +128) of B.
-            // Both CTAs' loads complete on the leader's barrier (shared::cluster address).
+            // Pair: this CTA stages rows [row0+row_off, +128) of A and half of the columns
+            // of B.  Both CTAs' loads complete on the leader's barrier (shared::cluster address).
             if (leader) ptx::mbar_arrive_expect_tx(local_bar, 2 * tma_bytes);
             const uint32_t bar = ptx::mapa(local_bar, 0);
-            if (MODE == kNN) {
+            const int r0 = t.k_row0 + k0;  // (wgrad)
+            if (MODE != kTN) {
               load_rows(sa, bar, k0);
+            } else if (!GATHER) {
+              if (p.wide_a) {
+                ptx::tma_load_3d_pair(sa, tn_a, bar, 0, r0, (t.row0 + row_off) >> 6);
+              } else {
 #pragma unroll
-              for (int j = 0; j < G::kBCols / 64; ++j)
-                if (SWIGLU)  // the leader stages the gate columns, its peer the up columns
-                  ptx::tma_load_3d_pair(sb + j * kBoxBytes, leader ? &map_b : &map_b2, bar,
-                                        t.col0 / 2 + j * 64, k0, t.expert);
-                else
-                  ptx::tma_load_3d_pair(sb + j * kBoxBytes, part_b, bar, t.col0 + col_off + j * 64, k0,
-                                        t.expert);
-            } else if (MODE == kNT) {
-              load_rows(sa, bar, k0);
-              if (SWIGLU) ptx::tma_load_3d_pair(sb, leader ? &map_b : &map_b2, bar, k0, t.col0 / 2, t.expert);
-              else ptx::tma_load_3d_pair(sb, part_b, bar, k0, t.col0 + col_off, t.expert);
-            } else {
-              const int r0 = t.k_row0 + k0;
-              if (!GATHER) {
-                if (p.wide_a) {
-                  ptx::tma_load_3d_pair(sa, tn_a, bar, 0, r0, (t.row0 + row_off) >> 6);
-                } else {
-#pragma unroll
-                  for (int j = 0; j < kBlockM / 64; ++j)
-                    ptx::tma_load_2d_pair(sa + j * kBoxBytes, tn_a, bar, t.row0 + row_off + j * 64, r0);
-                }
+                for (int j = 0; j < kBlockM / 64; ++j)
+                  ptx::tma_load_2d_pair(sa + j * kBoxBytes, tn_a, bar, t.row0 + row_off + j * 64, r0);
               }
-              if (p.wide_b) {
-                ptx::tma_load_3d_pair(sb, tn_b, bar, 0, r0, (t.col0 + col_off) >> 6);
+            }
+            // this CTA's 128 columns of each accumulator (gated: the leader stages the gate
+            // columns, its peer the up columns)
+            const CUtensorMap* b_map = SWIGLU ? (leader ? &map_b : &map_b2) : part_b;
+            for (int u = 0; u < t.units; ++u) {
+              const uint32_t dst = sb + uint32_t(u) * G::kBBytes;
+              const int c0 = SWIGLU ? t.col0 / 2 + u * (kBlockN / 2) : t.col0 + u * kBlockN + col_off;
+              if (MODE == kNN) {
+#pragma unroll
+                for (int j = 0; j < G::kBCols / 64; ++j)
+                  ptx::tma_load_3d_pair(dst + j * kBoxBytes, b_map, bar, c0 + j * 64, k0, t.expert);
+              } else if (MODE == kNT) {
+                ptx::tma_load_3d_pair(dst, b_map, bar, k0, c0, t.expert);
+              } else if (p.wide_b) {
+                ptx::tma_load_3d_pair(dst, tn_b, bar, 0, r0, c0 >> 6);
               } else {
 #pragma unroll
                 for (int j = 0; j < G::kBCols / 64; ++j)
-                  ptx::tma_load_2d_pair(sb + j * kBoxBytes, tn_b, bar, t.col0 + col_off + j * 64, r0);
+                  ptx::tma_load_2d_pair(dst + j * kBoxBytes, tn_b, bar, c0 + j * 64, r0);
               }
             }
           }
@@ -703,12 +730,102 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     auto loads_landed = [&]() {
       if (MODE == kTN && lane == 0) *reinterpret_cast<volatile uint32_t*>(&tail->tiles_done) = feed.taken;
     };
+    // Matrix instructions of a pair: k-block kb's 64 of k, from `stage` into accumulator `acc` (the
+    // unit-th of the tile).
+    constexpr uint64_t kAStep = kAMn ? (2048u >> 4) : (32u >> 4);
+    constexpr uint64_t kBStep = kBMn ? (2048u >> 4) : (32u >> 4);
+    auto a_desc = [&](uint32_t stage) {
+      const uint32_t sa = stage_base + stage * G::kStageBytes;
+      return kAMn ? ptx::make_smem_desc(sa, kBoxBytes, 1024u) : ptx::make_smem_desc(sa, 16u, 1024u);
+    };
+    auto b_desc = [&](uint32_t stage, uint32_t unit) {
+      const uint32_t sb = stage_base + stage * G::kStageBytes + G::kABytes + unit * G::kBBytes;
+      return kBMn ? ptx::make_smem_desc(sb, kBoxBytes, 1024u) : ptx::make_smem_desc(sb, 16u, 1024u);
+    };
+    auto issue_unit = [&](uint32_t stage, uint32_t unit, uint32_t acc, int kb) {
+      const uint64_t adesc = a_desc(stage), bdesc = b_desc(stage, unit);
+      const uint32_t d = tmem_base + acc * kBlockN;
+#pragma unroll
+      for (int k = 0; k < kBlockK / 16; ++k)
+        ptx::mma_bf16_ss_pair(d, adesc + k * kAStep, bdesc + k * kBStep, kIdesc, (kb | k) != 0 ? 1u : 0u);
+    };
+    // A tile of two accumulators: every k-block feeds both, so that A is staged once for 512
+    // columns.  All of TMEM is one tile then, and no accumulator is free for the next tile while the
+    // epilogue reads; so the second one runs kSkew k-blocks behind the first at both ends
+    // of the tile: while the first is read out the tensor core finishes the second, and
+    // while the second is read out it starts the next tile's first.
+    auto wide_tile = [&](int nkb) {
+      const uint32_t acc0 = it & 1u, par0 = (it >> 1) & 1u;
+      const uint32_t acc1 = (it + 1u) & 1u, par1 = ((it + 1u) >> 1) & 1u;
+      it += 2;
+      auto full_wait = [&](uint32_t stage, uint32_t parity) {
+        // (gather variant: one arrival is the other CTA's gather warp)
+        if (!ptx::mbar_wait<GATHER>(ptx::smem_u32(&tail->full[stage]), parity, wait)) return false;
+        ptx::tc_fence_after_sync();
+        return true;
+      };
+      auto next = [&](uint32_t* stage, uint32_t* parity) {
+        if (++*stage == kStages) { *stage = 0; *parity ^= 1u; }
+      };
+      auto acc_wait = [&](uint32_t acc, uint32_t parity) {
+        // (acquire at cluster scope: half of the arrivals come from the other CTA's epilogue warps)
+        if (!ptx::mbar_wait<true>(ptx::smem_u32(&tail->tmem_empty[acc]), parity ^ 1u, wait)) return false;
+        ptx::tc_fence_after_sync();
+        return true;
+      };
+      const int head = nkb < kSkew ? nkb : kSkew;
+      const int last = nkb - head < kSkew ? nkb - head : kSkew;
+      // both ends: `count` k-blocks into the first accumulator, then the same into the second
+      auto end_blocks = [&](int kb0, int count, bool first, bool done) {
+        uint32_t s1 = s, ph1 = ph;
+        if (first && !acc_wait(acc0, par0)) return false;
+        for (int i = 0; i < count; ++i) {
+          if (!full_wait(s1, ph1)) return false;
+          if (lane == 0) issue_unit(s1, 0, acc0, kb0 + i);
+          __syncwarp();
+          next(&s1, &ph1);
+        }
+        if (done && lane == 0) ptx::mma_commit_pair(ptx::smem_u32(&tail->tmem_full[acc0]), 0x3);
+        if (first && !acc_wait(acc1, par1)) return false;
+        for (int i = 0; i < count; ++i) {
+          if (lane == 0) {
+            issue_unit(s, 1, acc1, kb0 + i);
+            ptx::mma_commit_pair(ptx::smem_u32(&tail->empty[s]), 0x3);
+          }
+          __syncwarp();
+          next(&s, &ph);
+        }
+        if (done && lane == 0) ptx::mma_commit_pair(ptx::smem_u32(&tail->tmem_full[acc1]), 0x3);
+        return true;
+      };
+      if (!end_blocks(0, head, true, last == 0)) return false;
+      for (int kb = head; kb < nkb - last; ++kb) {
+        if (!full_wait(s, ph)) return false;
+        if (lane == 0) {
+          const uint64_t adesc = a_desc(s), bdesc0 = b_desc(s, 0), bdesc1 = b_desc(s, 1);
+#pragma unroll
+          for (int k = 0; k < kBlockK / 16; ++k) {
+            ptx::mma_bf16_ss_pair(tmem_base + acc0 * kBlockN, adesc + k * kAStep, bdesc0 + k * kBStep, kIdesc, 1u);
+            ptx::mma_bf16_ss_pair(tmem_base + acc1 * kBlockN, adesc + k * kAStep, bdesc1 + k * kBStep, kIdesc, 1u);
+          }
+          ptx::mma_commit_pair(ptx::smem_u32(&tail->empty[s]), 0x3);
+        }
+        __syncwarp();
+        next(&s, &ph);
+      }
+      return last == 0 || end_blocks(nkb - last, last, false, true);
+    };
     while (ok) {
       const Taken got = feed.take(true, lane, &t);
       if (got == kAbandoned) { ok = false; break; }
       if (got == kEndOfOrder) break;
       const int nkb = tile_stages(t);
       if (nkb == 0) { loads_landed(); continue; }  // empty wgrad expert: the epilogue writes zeros
+      if (kPair && t.units == 2) {
+        if (!(ok = wide_tile(nkb))) break;
+        loads_landed();
+        continue;
+      }
       const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
       ++it;
       const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
@@ -824,7 +941,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         __syncwarp();
       }
       if (lane == 0) {
-        TileWalker walk(p, tail);
+        TileWalker walk(p, tail, tile_stride);
         TileFeed<kPair> feed(tail, wait, !leader);
         Tile t = {};
         // wgrad: the map slot clipped to the current expert, and for every slot the
@@ -845,6 +962,11 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           int entry = 0;
           const bool live = walk.decode(pos, &t);
           if (!live) t.expert = -1;
+          if (live && t.units == 0) {  // a half that does not exist
+            pos = p.single_wave ? walk.total : static_cast<int>(drawn) + tile_stride;
+            if (pos < walk.total) drawn = atomicAdd(sched_counter, 1u);
+            continue;
+          }
           if (MODE == kTN && live && t.k_len > 0) {
             if (held_expert != t.expert) {
               // New expert: clip the row extent of a and b at its last row, in the next
@@ -984,7 +1106,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     // one row, a lane serves rows sub, sub + 4, .. sub + 124, and writes the
     // K-major 128-byte-swizzled layout a TMA box load would leave (16-byte chunk
     // index ^= row % 8).
-    constexpr int kGatherWarps = GatherWarps<CTAS>::kWarps;
     const int chunk = lane & 7;
     const int sub = lane >> 3;
     // Row 4 i + sub of a 64- or 128-row block lands at 512 i + row_dst[i & 1]: the
@@ -1173,7 +1294,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     // buffers the store before last read this one.
     auto stage_buf = [&]() { return my_out + (G::kOutBufs == 2 ? (stores & 1u) * G::kOutBufBytes : 0u); };
 
-    // One 32-column chunk `v` (fp32 bits) of this lane's row, starting at column
+    // One 32-column chunk `o` (rounded) of this lane's row, starting at column
     // `col` of the tile: through the staging buffer and a TMA store when the
     // whole warp's rows exist, else straight to global for the rows that do.
     const bool scatter_rows = (MODE != kTN) && (row_dest != nullptr);
@@ -1196,10 +1317,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     // staging buffer of 128-byte rows (128-byte swizzle: 16-byte piece index ^=
     // row % 8) and one TMA store of a 64 x 32 box; columns past the tensor's last
     // are clipped by the store.
-    auto emit64 = [&](const uint32_t (&v0)[32], const uint32_t (&v1)[32], int col, int tile_row, int col0) {
-      uint4 o[8];
-      pack(v0, o);
-      pack(v1, o + 4);
+    auto emit64 = [&](const uint4* o, int col, int tile_row, int col0) {
       const uint32_t buf = stage_buf();
       if (lane == 0 && stores > 0) ptx::bulk_wait_group_read<G::kOutBufs - 1>();
       __syncwarp();
@@ -1220,11 +1338,9 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       }
       ++stores;
     };
-    auto emit = [&](const uint32_t (&v)[32], int col, bool warp_full, bool row_ok,
+    auto emit = [&](const uint4* o, int col, bool warp_full, bool row_ok,
                     __nv_bfloat16* crow, int cols_left, int tile_row, int col0) {
       if (col >= cols_left) return;  // chunk lies entirely past the last column
-      uint4 o[4];
-      pack(v, o);
       if (!G::kWideOut && warp_full) {
         // The store that last read this buffer must be done reading.
         const uint32_t buf = stage_buf();
@@ -1434,6 +1550,10 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&tail->tmem_empty[ab]));
         continue;
       }
+      // one accumulator of 256 columns after the other
+#pragma unroll 1
+      for (int unit = 0; unit < (kPair ? t.units : 1); ++unit) {
+      const int unit_col0 = t.col0 + unit * kBlockN;
       const int r = row_off + q * 32 + lane;  // row inside the (pair) tile
       bool row_ok = r < t.valid_rows;
       // row_dest != nullptr (expert-parallel combine fused into this epilogue):
@@ -1445,7 +1565,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       const int64_t out_row0 = (MODE == kTN) ? (int64_t(t.expert) * p.d1 + t.row0) : int64_t(t.row0);
       // Output geometry: the gated product writes half as many columns as it schedules.
       const int64_t out_n = SWIGLU ? (p.n >> 1) : p.n;
-      const int out_col0 = SWIGLU ? (t.col0 >> 1) : t.col0;
+      const int out_col0 = SWIGLU ? (unit_col0 >> 1) : unit_col0;
       __nv_bfloat16* crow = c + (out_row0 + r) * out_n + out_col0;
       if (scatter && row_ok) {
         int64_t addr;
@@ -1465,7 +1585,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * row_w);
       };
-      uint32_t va[32], vb[32];
+      uint32_t va[32], vb[32];  // (vb: gated product)
       if (MODE == kTN && nkb == 0) {  // (forward and dgrad tiles always have k > 0)
         // Empty wgrad expert: its block of the output is zeros.
         if (G::kWideOut && warp_full) {
@@ -1485,58 +1605,60 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
 #pragma unroll 1
             for (int ch = 0; ch < kBlockN / 128; ++ch) {
               const int col = col_base + ch * 64;
-              if (col < cols_left) ptx::tma_store_2d(&map_c, buf, t.col0 + col, tile_row);
+              if (col < cols_left) ptx::tma_store_2d(&map_c, buf, unit_col0 + col, tile_row);
             }
             ptx::bulk_commit_group();
           }
           ++stores;
           continue;
         }
-#pragma unroll
-        for (int i = 0; i < 32; ++i) va[i] = 0u;
+        const uint4 zeros[4] = {};
 #pragma unroll 1
         for (int ch = 0; ch < kBlockN / 64; ++ch)
-          emit(va, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, t.col0);
+          emit(zeros, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
         continue;
+      }
+      uint4 d4[8] = {};  // gated backward: this lane's 64 values of the output gradient
+      if (SWIGLU && gate_grad != nullptr && row_ok) {
+        const int col = half * 64;
+        const uint4* src = reinterpret_cast<const uint4*>(gate_grad + (out_row0 + r) * out_n + out_col0 + col);
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (col + j * 8 < cols_left) d4[j] = src[j];
       }
       const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
       ++it;
       if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), aph, wait)) { ok = false; break; }
       ptx::tc_fence_after_sync();
+      // The accumulator is read and rounded as a whole and handed back; only then do its values
+      // leave through the staging buffer, where each chunk waits for the store before it.
+      auto release = [&]() {
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
+          if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(te_bar, 0));
+          else ptx::mbar_arrive(te_bar);
+        }
+      };
       if (SWIGLU) {
         // This warp's 64 of the tile's 128 output columns: gate from accumulator
         // columns [64 half, +64), up from the same columns of the second half.
         const uint32_t tg = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + half * 64;
-#pragma unroll 1
+        uint4 o[16];
+#pragma unroll
         for (int ch = 0; ch < 2; ++ch) {
           ptx::tmem_ld_32x32(tg + ch * 32, va);
           ptx::tmem_ld_32x32(tg + kBlockN / 2 + ch * 32, vb);
           ptx::tmem_ld_wait();
-          if (ch == 1) {
-            // Every column has been read: hand the accumulator back before the last stores.
-            ptx::tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) {
-              const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
-              if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(te_bar, 0));
-              else ptx::mbar_arrive(te_bar);
-            }
-          }
-          const int col = half * 64 + ch * 32;
+          if (ch == 1) release();
           if (gate_grad != nullptr) {
             // Backward of the gated product: with g, u recomputed in the accumulator and
-            // dh = gate_grad[row, col ..] read here, the gradients w.r.t. the two products
+            // dh = gate_grad[row, col ..] (read above), the gradients w.r.t. the two products
             //   dg = dh * u * silu'(g),  silu'(g) = s (1 + g (1 - s)),  s = 1 / (1 + exp(-g))
             //   du = dh * silu(g)
             // go to rows [0, T) and [T, 2T) of the output.
-            uint4 d4[4] = {};
-            if (row_ok) {
-              const uint4* src = reinterpret_cast<const uint4*>(gate_grad + (out_row0 + r) * out_n + out_col0 + col);
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (col + j * 8 < cols_left) d4[j] = src[j];
-            }
-            const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(d4);
+            const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(d4 + ch * 4);
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               const float g = __uint_as_float(va[i]);
@@ -1547,65 +1669,48 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
               va[i] = __float_as_uint(dh * u * sg * (1.0f + g * (1.0f - sg)));
               vb[i] = __float_as_uint(dh * g * sg);
             }
-            emit(va, col, warp_full, row_ok, crow, cols_left, tile_row, out_col0);
-            emit(vb, col, warp_full, row_ok, crow + p.tokens * out_n, cols_left, tile_row + static_cast<int>(p.tokens),
-                 out_col0);
-            continue;
-          }
+            pack(va, o + ch * 4);
+            pack(vb, o + 8 + ch * 4);
+          } else {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float g = __uint_as_float(va[i]);
-            const float u = __uint_as_float(vb[i]);
-            va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * u);  // silu(g) * u
+            for (int i = 0; i < 32; ++i) {
+              const float g = __uint_as_float(va[i]);
+              const float u = __uint_as_float(vb[i]);
+              va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * u);  // silu(g) * u
+            }
+            if (scaled) scale(va);
+            pack(va, o + ch * 4);
           }
-          if (scaled) scale(va);
-          emit(va, col, warp_full, row_ok, crow, cols_left, tile_row, out_col0);
+        }
+#pragma unroll
+        for (int ch = 0; ch < 2; ++ch) {
+          const int col = half * 64 + ch * 32;
+          emit(o + ch * 4, col, warp_full, row_ok, crow, cols_left, tile_row, out_col0);
+          if (gate_grad != nullptr)
+            emit(o + 8 + ch * 4, col, warp_full, row_ok, crow + p.tokens * out_n, cols_left,
+                 tile_row + static_cast<int>(p.tokens), out_col0);
         }
         continue;
       }
       const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + col_base;
+      uint4 o[16];
+#pragma unroll
+      for (int ch = 0; ch < kBlockN / 64; ++ch) {
+        ptx::tmem_ld_32x32(taddr + ch * 32, va);
+        ptx::tmem_ld_wait();
+        if (ch == kBlockN / 64 - 1) release();
+        if (scaled) scale(va);
+        pack(va, o + ch * 4);
+      }
       if (G::kWideOut && warp_full) {
-#pragma unroll 1
-        for (int ch = 0; ch < kBlockN / 64; ch += 2) {
-          ptx::tmem_ld_32x32(taddr + ch * 32, va);
-          ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
-          ptx::tmem_ld_wait();
-          if (ch + 2 >= kBlockN / 64) {
-            // Every column has been read: hand the accumulator back before the last store.
-            ptx::tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) {
-              const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
-              if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(te_bar, 0));
-              else ptx::mbar_arrive(te_bar);
-            }
-          }
-          if (col_base + ch * 32 < cols_left) emit64(va, vb, col_base + ch * 32, tile_row, t.col0);
-        }
+#pragma unroll
+        for (int ch = 0; ch < kBlockN / 64; ch += 2)
+          if (col_base + ch * 32 < cols_left) emit64(o + ch * 4, col_base + ch * 32, tile_row, unit_col0);
         continue;
       }
-      ptx::tmem_ld_32x32(taddr, va);
-#pragma unroll 1
-      for (int ch = 0; ch < kBlockN / 64; ch += 2) {
-        ptx::tmem_ld_wait();
-        ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
-        if (scaled) scale(va);
-        emit(va, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, t.col0);
-        ptx::tmem_ld_wait();
-        if (ch + 2 < kBlockN / 64) {
-          ptx::tmem_ld_32x32(taddr + (ch + 2) * 32, va);
-        } else {
-          // Every column has been read: hand the accumulator back before the last stores.
-          ptx::tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) {
-            const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
-            if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(te_bar, 0));
-            else ptx::mbar_arrive(te_bar);
-          }
-        }
-        if (scaled) scale(vb);
-        emit(vb, col_base + (ch + 1) * 32, warp_full, row_ok, crow, cols_left, tile_row, t.col0);
+#pragma unroll
+      for (int ch = 0; ch < kBlockN / 64; ++ch)
+        emit(o + ch * 4, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
       }
     }
     // Shared memory must outlive the stores that still read it.
@@ -1681,15 +1786,16 @@ schedule_dump_kernel(const int64_t* __restrict__ batch_sizes, const Problem p, i
   build_schedule(p, batch_sizes, InlineSizes{}, &tail, status);
   __syncthreads();
   if (threadIdx.x == 0) {
-    TileWalker walk(p, &tail);
+    TileWalker walk(p, &tail, 0);
     Tile t;
     int n = 0;
     for (int pos = 0; walk.decode(pos, &t); ++pos) {
-      if (n < max_tiles) {
+      for (int unit = 0; unit < t.units; ++unit, ++n) {
+        if (n >= max_tiles) continue;
         int32_t* o = out + int64_t(n) * 6;
-        o[0] = t.expert; o[1] = t.row0; o[2] = t.col0; o[3] = t.valid_rows; o[4] = tile_stages(t); o[5] = t.kind;
+        o[0] = t.expert; o[1] = t.row0; o[2] = t.col0 + unit * kBlockN;
+        o[3] = t.valid_rows; o[4] = tile_stages(t); o[5] = t.kind;
       }
-      ++n;
     }
     *out_count = n;
   }

@@ -47,12 +47,13 @@ struct Problem {
   int64_t d1;      // a.shape[1]: k for NN/NT, m for TN
   int64_t n;       // output columns
   int tile_m;      // output rows per scheduled tile: 128 (one CTA) or 256 (a CTA pair)
+  int tile_n;      // output columns per scheduled tile: 256, or 512 (a CTA pair: two accumulators of 256)
   int group_m;     // row-tiles swept together across the columns (L2 reuse of b)
   int light;       // 1: experts of <= kLightRows rows run as transposed tiles (NN/NT, tile_m 128)
   int order;       // 0: experts in index order.  1: experts sorted by rows, largest first
   int64_t wait_ns; // limit of every wait inside the kernel, in nanoseconds
   // Derived on the host so that decoding a tile needs no 64-bit division:
-  int nt;          // column tiles of kBlockN: ceil(n / 256)
+  int nt;          // column tiles: ceil(n / tile_n)
   int mt;          // TN: row tiles of c[i]: ceil(d1 / tile_m)
   int lt;          // column tiles of a transposed tile's width: ceil(n / 128)
   int wide_a;      // TN: a's columns are a multiple of 64, one TMA load brings all 64-column boxes of a stage
@@ -71,7 +72,7 @@ struct Problem {
 
 // Fills the derived fields of a Problem whose shape fields are set.
 B200GMM_HD void derive(Problem* p) {
-  p->nt = static_cast<int>((p->n + kBlockN - 1) / kBlockN);
+  p->nt = static_cast<int>((p->n + p->tile_n - 1) / p->tile_n);
   p->mt = static_cast<int>((p->d1 + p->tile_m - 1) / p->tile_m);
   p->lt = static_cast<int>((p->n + kLightCols - 1) / kLightCols);
 }
@@ -84,6 +85,7 @@ struct Tile {
   int k_row0;      // TN: first contraction row in a/b (global); else 0
   int k_len;       // contraction length (k, or batch_sizes[expert] for TN)
   int kind;        // 0: tile_m x 256 tile; 1: transposed tile (valid_rows <= kLightRows, kLightCols columns)
+  int units;       // accumulators of kBlockN columns: 1, or 2 (a CTA pair's tile of 512 columns; the last may be half)
 };
 
 B200GMM_HD int ceil_div_i(int a, int b) { return (a + b - 1) / b; }
@@ -107,8 +109,9 @@ B200GMM_HD int expert_tiles(const Problem& p, int rows) {
 
 // Most tiles a launch can have, whatever batch_sizes holds (B200GMM_LIGHT off).
 B200GMM_HD int64_t max_tiles(const Problem& p) {
-  if (p.mode == kTN) return int64_t(p.z) * p.mt * p.nt;
-  return (p.tokens / p.tile_m + (p.z < p.tokens ? p.z : p.tokens)) * p.nt;
+  const int64_t nt = (p.n + kBlockN - 1) / kBlockN;  // (a wide tile may be taken as two positions)
+  if (p.mode == kTN) return int64_t(p.z) * p.mt * nt;
+  return (p.tokens / p.tile_m + (p.z < p.tokens ? p.z : p.tokens)) * nt;
 }
 
 // Pipeline stages (ring slots) one tile consumes.
@@ -142,6 +145,11 @@ B200GMM_HD void decode_in_expert(int local, int row_tiles, int nt, int group_m, 
   *ni = r / gm;
 }
 
+// Accumulators that the tile at column col0 fills.
+B200GMM_HD int tile_units(const Problem& p, int col0) {
+  return p.tile_n > kBlockN && p.n - col0 > kBlockN ? 2 : 1;
+}
+
 // `local` = tile index relative to the expert's first tile; rs/re = row_start[expert],
 // row_start[expert+1] (already clamped to tokens).
 B200GMM_HD Tile make_tile(const Problem& p, int expert, int local, int rs, int re) {
@@ -157,7 +165,8 @@ B200GMM_HD Tile make_tile(const Problem& p, int expert, int local, int rs, int r
     t.valid_rows = left < p.tile_m ? left : p.tile_m;
     t.k_row0 = rs;
     t.k_len = re - rs;
-    t.col0 = ni * kBlockN;
+    t.col0 = ni * p.tile_n;
+    t.units = tile_units(p, t.col0);
     return t;
   }
   t.k_row0 = 0;
@@ -170,8 +179,10 @@ B200GMM_HD Tile make_tile(const Problem& p, int expert, int local, int rs, int r
     t.row0 = rs + mi * p.tile_m;
     const int left = re - t.row0;
     t.valid_rows = left < p.tile_m ? left : p.tile_m;
-    t.col0 = ni * kBlockN;
+    t.col0 = ni * p.tile_n;
+    t.units = tile_units(p, t.col0);
   } else {
+    t.units = 1;
     t.kind = 1;
     t.row0 = rs + mt * kBlockM;
     t.valid_rows = re - t.row0;
