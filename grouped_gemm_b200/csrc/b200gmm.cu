@@ -305,14 +305,31 @@ struct Features {
 // Not the gathered product (0.95 to 1.0 nearly everywhere: its copies are the bound, and
 // the rows that do not exist are not copied in either form), and not the gated backward,
 // which reads its gradient row by row there (104 and 222 us at 40 rows, k = 512).
+// A pair's tiles of up to 192 of 256 rows: the last row tile of an expert, and all of a small
+// expert.  Time without / with:
+//   256 experts of 256 rows on average, Zipf, 7168 x 2048: 2480 / 2244 us, dgrad 2486 / 2152 (one-CTA tiles:
+//     2383, 2322); 64 experts of 64 rows, 4088 x 8184: 942 / 815.
+//   large experts (8 of 1024 rows, 4096 x 14336): gated product 1676 / 1599 us, scattered rows 887 / 867,
+//     forward 815 / 822, dgrad 812 / 844; of 4096: forward 2910 / 2877, dgrad 2934 / 3055.  So NN up to 2048 rows
+//     and NT up to 512.
+//   few tiles: one pair's pipeline is the bound, as above (322 rows, one expert, 5976 x 4736: 37 us with
+//     one-CTA tiles, 63 with this): a tile for every SM.
 int swap_rows(const Problem& p, const Features& f, int ctas, int sm_count) {
   constexpr int64_t kMeanRows = 64, kMeanRowsGated = 48, kPlainMinK = 512;
-  if (p.mode == kTN || ctas != 1 || f.gather || f.gated_backward) return 0;
+  if (p.mode == kTN || f.gather || f.gated_backward) return 0;
+  if (ctas == 2) {
+    const int64_t pair_tiles = (2 * p.tokens / p.tile_m + std::min<int64_t>(p.z, p.tokens)) * p.nt / 2;
+    return pair_tiles >= sm_count && p.tokens < (p.mode == kNN ? 2048 : 512) * int64_t(p.z) ? 3 * kBlockM / 2 : 0;
+  }
   const int64_t tiles = int64_t(p.nt) * std::min<int64_t>(p.z, p.tokens);  // experts with rows have one row tile, mostly
   if (f.swiglu) return p.tokens <= kMeanRowsGated * p.z && 3 * tiles >= 2 * sm_count ? kBlockM / 2 : 0;
   if (!f.scatter && p.d1 < kPlainMinK) return 0;
   return p.tokens <= kMeanRows * p.z && 2 * tiles >= sm_count ? kBlockM / 2 : 0;
 }
+
+// Whether rows of an operand start at any 16 bytes: a k-block of such a row is five sectors in two
+// lines of L2 instead of four in one.  (b's rows are d1 long in the NT layout.)
+bool ragged_rows(int64_t d1, int64_t n, int trans_b) { return d1 % 16 != 0 || (!trans_b && n % 16 != 0); }
 
 int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b, int ctas,
                   Problem* p, const Features& f = Features()) {
@@ -349,6 +366,13 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   // by streaming their weights from HBM either way, and measured end to end the
   // launch was not faster with them (B200GMM_LIGHT=1 switches them on).
   p->light = (p->mode != kTN && ctas == 1 && !f.gather && !f.swiglu) ? env_int("B200GMM_LIGHT", 0) : 0;
+  // A pair's wide tiles are half as many.  wgrad's are as long as their expert has rows: with
+  // few a CTA the long ones end the launch (11 experts, 126529 rows, 4144 x 576: 712 us with tiles of 256
+  // columns, 872 with 512).  Forward and dgrad: few rounds lose more to the last one than the bytes
+  // save (3 experts, 3172 rows, 1936 x 4672: 62.3 / 66.3), unless rows start at any 16 bytes, when bytes
+  // are what bounds them (7 experts, 3001 rows, 1000 x 2504: 26.4 / 23.0).
+  p->narrow_rounds = trans_a ? 8 : (ragged_rows(d1, n, trans_b) ? 0 : 4);
+  p->swap_units = 1;
   p->swap_rows = 0;  // decided where the device is known (run_impl)
   p->dest_indexed = 0;
   p->dest_rows = 0;
@@ -516,7 +540,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     if (b2 == nullptr) return B200GMM_EINVAL;
     // rows of a's second part and the length of both parts of the contraction, each
     // rounded up to a k-block, are 32-bit numbers in the kernel (schedule.cuh: make_tile)
-    if (2 * tokens + p.tile_m >= (int64_t(1) << 31) || 2 * (dim_a1 + kBlockK) >= (int64_t(1) << 31)) return B200GMM_ELIMIT;
+    if (2 * tokens + 2 * kBlockM >= (int64_t(1) << 31) || 2 * (dim_a1 + kBlockK) >= (int64_t(1) << 31)) return B200GMM_ELIMIT;
   }
   if ((reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(b) & 15) ||
       (reinterpret_cast<uintptr_t>(c) & 15))
@@ -532,6 +556,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   }
 
   p.swap_rows = swap_rows(p, feat, ctas, dev->sm_count);
+  p.swap_units = swiglu ? ctas : 1;
   p.dest_indexed = dest_rows >= 0 ? 1 : 0;
   p.dest_rows = dest_rows;
   p.pair_sum = pair_sum ? 1 : 0;
@@ -647,7 +672,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   CUtensorMap map_c = {};
   if (row_dest == nullptr) {
     const uint64_t dc[2] = {N, p.mode == kTN ? Z * D1 : (gate_grad != nullptr ? 2 * T : T)};
-    const bool wide = p.mode == kTN && !gather;  // Geometry::kWideOut
+    const bool wide = p.mode == kTN && !gather && ctas == 1;  // Geometry::kWideOut
     const uint32_t bc[2] = {wide ? 64u : 32u, 32};
     if (dc[1] >= (uint64_t(1) << 31)) return B200GMM_ELIMIT;
     if ((rc = encode_map(&map_c, c, 2, dc, bc, wide ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B)) != 0)

@@ -59,6 +59,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "ptx.cuh"
 #include "schedule.cuh"
 
@@ -69,7 +71,7 @@ constexpr int kSchedWarp = 2 + kEpilogueWarps;        // warp 10
 constexpr int kThreads = 32 * (kSchedWarp + 1);       // 352
 constexpr int kMaxExperts = 1024;
 constexpr uint32_t kTmemCols = 512;
-constexpr int kMaxStages = 4;
+constexpr int kMaxStages = 6;
 constexpr uint32_t kBoxBytes = 64 * kBlockK * 2;  // one 64-wide MN-major TMA box: 8 KiB
 // wgrad keeps private, editable copies of its two tensor maps in the caller's
 // workspace: kMapSlots {a, b} pairs per cluster, edited in turn.  The scheduler
@@ -87,16 +89,15 @@ constexpr int kMaxCtas = 256;  // workspace is sized for this many CTAs
 // a tensor-map edit) stay hidden behind tiles already handed out.
 constexpr int kSchedSlots = 8;
 
-// wgrad gives up ring stages for larger epilogue staging: its tiles can be a single
-// k-block deep (few rows per expert, or none), and then the kernel runs at the
-// speed of its output stores.  Each epilogue warp has two buffers of 32 rows x 64
-// columns there (128-byte rows), used in turn, so that a warp fills one while
-// the TMA store of the other still reads; the forward / dgrad layouts have one
-// buffer of 32 x 32 per warp.  So has the gathered wgrad, which needs the stages: a warp
-// that fetches rows with cp.async takes over a microsecond from a free stage to a full one.
+// The one-CTA wgrad, which is what experts of few rows get, gives up ring stages for larger
+// epilogue staging: its tiles can be a single k-block deep (few rows per expert, or none), and
+// then the kernel runs at the speed of its output stores.  Each epilogue warp has two buffers of
+// 32 rows x 64 columns there (128-byte rows), used in turn, so that a warp fills one while
+// the TMA store of the other still reads; everywhere else there is one buffer of 32 x 32 per
+// warp, and the whole 192 KiB for the ring.
 template <int CTAS, int MODE = kNN, bool GATHER = false>
 struct Geometry {
-  static constexpr bool kWideOut = (MODE == kTN) && !GATHER;  // 64-column stores from double buffers
+  static constexpr bool kWideOut = (MODE == kTN) && !GATHER && CTAS == 1;  // 64-column stores from double buffers
   static constexpr int kStages = kWideOut ? 3 : 4;
   static constexpr int kUnits = CTAS;  // accumulators a tile fills side by side: a pair's tile is 512 columns wide
   static constexpr int kOutBufs = kWideOut ? 2 : 1;  // staging buffers per epilogue warp
@@ -105,7 +106,11 @@ struct Geometry {
   static constexpr uint32_t kABytes = kBlockM * kBlockK * 2;    // 16 KiB
   static constexpr uint32_t kBBytes = kBCols * kBlockK * 2;     // 32 or 16 KiB, per accumulator
   static constexpr uint32_t kStageBytes = kABytes + kUnits * kBBytes;  // 48 KiB
-  static constexpr uint32_t kRingBytes = kStages * kStageBytes;  // 192 KiB (wgrad: 144 KiB)
+  static constexpr uint32_t kRingBytes = kStages * kStageBytes;  // 192 KiB (one-CTA wgrad: 144 KiB)
+  // A pair's launch whose tiles all fill one accumulator divides the same ring into stages without
+  // the second one's half.
+  static constexpr uint32_t kNarrowStageBytes = kABytes + kBBytes;                    // 32 KiB
+  static constexpr int kNarrowStages = CTAS == 2 ? int(kRingBytes / kNarrowStageBytes) : kStages;  // 6
   static constexpr uint32_t kOutBytes = kEpilogueWarps * kOutBufs * kOutBufBytes;  // 16 KiB (wgrad: 64 KiB)
 };
 
@@ -303,8 +308,9 @@ __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* 
 // Position of the launch order -> tile (the scheduler's).  Positions come in
 // increasing order, so the expert cursor only ever moves forward.
 //
-// Tiles two accumulators wide are coarse: what is left over after whole rounds of the
-// grid's `clusters` is taken as halves when the halves fit one round, which then lasts half as
+// Tiles two accumulators wide are coarse.  A launch of few of them takes all as halves
+// (narrow_tiles); in others what is left over after whole rounds of the grid's
+// `clusters` is taken as halves when the halves fit one round, which then lasts half as
 // long.  A half that does not exist (the last column tile may be one accumulator
 // wide) is a tile of no units.
 struct TileWalker {
@@ -315,12 +321,12 @@ struct TileWalker {
   int pos;
   __device__ TileWalker(const Problem& p_, const SmemTail* tail_, int clusters)
       : p(p_), tail(tail_), whole(tail_->tile_start[p_.z]), total(whole), pos(0) {
-    if (p.tile_n > kBlockN && clusters > 0) {
-      const int left = whole % clusters;
-      if (2 * left <= clusters) {
-        whole -= left;
-        total += left;
-      }
+    if (p.tile_n > kBlockN && p.n > kBlockN && clusters > 0) {
+      int halves = whole % clusters;
+      if (2 * halves > clusters) halves = 0;
+      if (narrow_tiles(p, whole, clusters)) halves = whole;
+      whole -= halves;
+      total += halves;
     }
   }
   __device__ __forceinline__ bool decode(int t, Tile* out) {
@@ -449,7 +455,6 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   // c0+128) with c0 = col0 / 2, and the epilogue writes the 128 output columns
   // silu(gate) * up.
   using G = Geometry<CTAS, MODE, GATHER>;
-  constexpr int kStages = G::kStages;
   constexpr bool kPair = (CTAS == 2);
   // Transposed tiles exist in the plain one-CTA forward / dgrad kernels only
   // (map_a2: the activations with 32-row boxes; NT also uses map_b2: b with
@@ -457,7 +462,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   constexpr bool kLight = (MODE != kTN) && (CTAS == 1) && !GATHER && !SWIGLU;
   // So do swapped tiles (schedule.cuh), and in the gated product's.  A sum of two products
   // over one accumulator (Problem::pair_sum) is an option of the plain kernels.
-  constexpr bool kSwap = (MODE != kTN) && (CTAS == 1) && !GATHER;
+  constexpr bool kSwap = (MODE != kTN) && !GATHER;
   constexpr bool kPairSum = (MODE != kTN) && !GATHER && !SWIGLU && !PUSH;
 
   extern __shared__ uint8_t smem_raw[];
@@ -482,7 +487,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       if (SWIGLU || (kLight && MODE == kNT)) ptx::prefetch_tensormap(&map_b2);
       if (kSwap) ptx::prefetch_tensormap(&map_a2);
       ptx::prefetch_tensormap(&map_c);
-      for (int s = 0; s < kStages; ++s) {
+      for (int s = 0; s < G::kNarrowStages; ++s) {
         // the producer's expect_tx arrival, plus one arrival by the gather warp that fills
         // this stage in each CTA
         ptx::mbar_init(ptx::smem_u32(&tail->full[s]), 1 + (GATHER ? CTAS : 0));
@@ -547,6 +552,12 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
 
   const int first_tile = kPair ? (blockIdx.x >> 1) : blockIdx.x;
   const int tile_stride = kPair ? (gridDim.x >> 1) : gridDim.x;
+  // The ring.  A launch of few tiles is bound by the latency of its loads, one of narrow outputs by
+  // their bytes: stages in flight count (one expert of 5788 rows, 792 x 2224, wgrad: 62 us
+  // with three stages, 38 with four).
+  const bool narrow = kPair && narrow_tiles(p, tail->tile_start[p.z], tile_stride);
+  const uint32_t ring_stages = narrow ? G::kNarrowStages : G::kStages;
+  const uint32_t stage_bytes = narrow ? G::kNarrowStageBytes : G::kStageBytes;
   const int row_off = static_cast<int>(cta_rank) * kBlockM;  // this CTA's rows inside a pair tile
   const int col_off = static_cast<int>(cta_rank) * G::kBCols;  // this CTA's share of the B tile
 
@@ -577,7 +588,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           for (int kb = 0; kb < nkb; ++kb) {
             if (!ptx::mbar_wait(ptx::smem_u32(&tail->empty[s]), ph ^ 1u, wait)) { ok = false; break; }
             const uint32_t bar = ptx::smem_u32(&tail->full[s]);
-            const uint32_t sw = stage_base + s * G::kStageBytes;
+            const uint32_t sw = stage_base + s * stage_bytes;
             const uint32_t sx = sw + kLightWBytes;
             ptx::mbar_arrive_expect_tx(bar, bytes);
 #pragma unroll
@@ -592,7 +603,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
               for (int i = 0; i < row_boxes; ++i)
                 ptx::tma_load_2d(sx + h * kLightXHalf + i * kRowBoxBytes, &map_a2, bar, k0, t.row0 + i * 32);
             }
-            if (++s == kStages) { s = 0; ph ^= 1u; }
+            if (++s == ring_stages) { s = 0; ph ^= 1u; }
           }
           continue;
         }
@@ -608,18 +619,21 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             ptx::fence_tensormap_acquire(tn_b);
           }
         }
-        // A swapped tile fetches its rows in boxes of 32.
-        const int sw_boxes = kSwap ? (swapped_rows(p, t) + 31) >> 5 : 0;
+        // A swapped tile fetches its rows in boxes of 32, each CTA of a pair half of them.
+        const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
+        const int sw_boxes = (sw_rows / CTAS + 31) >> 5;
         // Bytes this CTA's TMA loads bring per stage: the gather warps fetch A themselves.
         const uint32_t tma_bytes =
             G::kBBytes * uint32_t(kPair ? t.units : 1) + (GATHER ? 0u : (kSwap && sw_boxes != 0 ? uint32_t(sw_boxes) * kRowBoxBytes : G::kABytes));
-        int part_row = t.row0 + row_off;     // row of a the current part of the contraction starts at
+        int part_row = t.row0 + (sw_rows != 0 ? static_cast<int>(cta_rank) * (sw_rows / CTAS) : row_off);  // row of a the current part of the contraction starts at
         const CUtensorMap* part_b = &map_b;  // and its weights
         auto load_rows = [&](uint32_t dst, uint32_t bar, int k0) {  // A of a forward / dgrad stage
           if (GATHER) return;
           if (kSwap && sw_boxes != 0) {
-            for (int i = 0; i < sw_boxes; ++i)
-              ptx::tma_load_2d(dst + i * kRowBoxBytes, &map_a2, bar, k0, part_row + i * 32);
+            for (int i = 0; i < sw_boxes; ++i) {
+              if (kPair) ptx::tma_load_2d_pair(dst + i * kRowBoxBytes, &map_a2, bar, k0, part_row + i * 32);
+              else ptx::tma_load_2d(dst + i * kRowBoxBytes, &map_a2, bar, k0, part_row + i * 32);
+            }
           } else {
             if (kPair) ptx::tma_load_2d_pair(dst, &map_a, bar, k0, part_row);
             else ptx::tma_load_2d(dst, &map_a, bar, k0, part_row);
@@ -635,7 +649,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           }
           if (!ptx::mbar_wait(ptx::smem_u32(&tail->empty[s]), ph ^ 1u, wait)) { ok = false; break; }
           const uint32_t local_bar = ptx::smem_u32(&tail->full[s]);
-          const uint32_t sa = stage_base + s * G::kStageBytes;
+          const uint32_t sa = stage_base + s * stage_bytes;
           const uint32_t sb = sa + G::kABytes;
           if (!kPair) {
             ptx::mbar_arrive_expect_tx(local_bar, tma_bytes);
@@ -692,12 +706,15 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
                   ptx::tma_load_2d_pair(sa + j * kBoxBytes, tn_a, bar, t.row0 + row_off + j * 64, r0);
               }
             }
-            // this CTA's 128 columns of each accumulator (gated: the leader stages the gate
-            // columns, its peer the up columns)
-            const CUtensorMap* b_map = SWIGLU ? (leader ? &map_b : &map_b2) : part_b;
+            // this CTA's 128 columns of each accumulator.  Gated: the leader stages the gate
+            // columns, its peer the up columns, of the same 128 outputs; in a swapped tile, whose
+            // lanes are columns, the first accumulator is gate and the second up of 256.
             for (int u = 0; u < t.units; ++u) {
               const uint32_t dst = sb + uint32_t(u) * G::kBBytes;
-              const int c0 = SWIGLU ? t.col0 / 2 + u * (kBlockN / 2) : t.col0 + u * kBlockN + col_off;
+              const bool across = SWIGLU && sw_rows != 0;
+              const CUtensorMap* b_map = SWIGLU ? ((across ? u == 0 : leader) ? &map_b : &map_b2) : part_b;
+              const int c0 = SWIGLU ? t.col0 / 2 + (across ? static_cast<int>(cta_rank) : u) * (kBlockN / 2)
+                                    : t.col0 + u * kBlockN + col_off;
               if (MODE == kNN) {
 #pragma unroll
                 for (int j = 0; j < G::kBCols / 64; ++j)
@@ -713,7 +730,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
               }
             }
           }
-          if (++s == kStages) { s = 0; ph ^= 1u; }
+          if (++s == ring_stages) { s = 0; ph ^= 1u; }
         }
       }
       feed.tally(warp);
@@ -735,26 +752,34 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     constexpr uint64_t kAStep = kAMn ? (2048u >> 4) : (32u >> 4);
     constexpr uint64_t kBStep = kBMn ? (2048u >> 4) : (32u >> 4);
     auto a_desc = [&](uint32_t stage) {
-      const uint32_t sa = stage_base + stage * G::kStageBytes;
+      const uint32_t sa = stage_base + stage * stage_bytes;
       return kAMn ? ptx::make_smem_desc(sa, kBoxBytes, 1024u) : ptx::make_smem_desc(sa, 16u, 1024u);
     };
     auto b_desc = [&](uint32_t stage, uint32_t unit) {
-      const uint32_t sb = stage_base + stage * G::kStageBytes + G::kABytes + unit * G::kBBytes;
+      const uint32_t sb = stage_base + stage * stage_bytes + G::kABytes + unit * G::kBBytes;
       return kBMn ? ptx::make_smem_desc(sb, kBoxBytes, 1024u) : ptx::make_smem_desc(sb, 16u, 1024u);
     };
-    auto issue_unit = [&](uint32_t stage, uint32_t unit, uint32_t acc, int kb) {
+    // (swapped: the staged columns of B are the first operand, the staged rows the second)
+    // Each form has code of its own: with the choice made per instruction the plain tiles
+    // took 12 % longer.
+    uint32_t sw_idesc = 0;
+    auto mma_pair = [&](auto swapped, uint32_t d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+      if constexpr (decltype(swapped)::value) ptx::mma_bf16_ss_pair(d, bdesc, adesc, sw_idesc, accumulate);
+      else ptx::mma_bf16_ss_pair(d, adesc, bdesc, kIdesc, accumulate);
+    };
+    auto issue_unit = [&](auto swapped, uint32_t stage, uint32_t unit, uint32_t acc, int kb) {
       const uint64_t adesc = a_desc(stage), bdesc = b_desc(stage, unit);
       const uint32_t d = tmem_base + acc * kBlockN;
 #pragma unroll
       for (int k = 0; k < kBlockK / 16; ++k)
-        ptx::mma_bf16_ss_pair(d, adesc + k * kAStep, bdesc + k * kBStep, kIdesc, (kb | k) != 0 ? 1u : 0u);
+        mma_pair(swapped, d, adesc + k * kAStep, bdesc + k * kBStep, (kb | k) != 0 ? 1u : 0u);
     };
     // A tile of two accumulators: every k-block feeds both, so that A is staged once for 512
     // columns.  All of TMEM is one tile then, and no accumulator is free for the next tile while the
     // epilogue reads; so the second one runs kSkew k-blocks behind the first at both ends
     // of the tile: while the first is read out the tensor core finishes the second, and
     // while the second is read out it starts the next tile's first.
-    auto wide_tile = [&](int nkb) {
+    auto wide_tile = [&](auto swapped, int nkb) {
       const uint32_t acc0 = it & 1u, par0 = (it >> 1) & 1u;
       const uint32_t acc1 = (it + 1u) & 1u, par1 = ((it + 1u) >> 1) & 1u;
       it += 2;
@@ -765,7 +790,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         return true;
       };
       auto next = [&](uint32_t* stage, uint32_t* parity) {
-        if (++*stage == kStages) { *stage = 0; *parity ^= 1u; }
+        if (++*stage == ring_stages) { *stage = 0; *parity ^= 1u; }
       };
       auto acc_wait = [&](uint32_t acc, uint32_t parity) {
         // (acquire at cluster scope: half of the arrivals come from the other CTA's epilogue warps)
@@ -781,7 +806,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         if (first && !acc_wait(acc0, par0)) return false;
         for (int i = 0; i < count; ++i) {
           if (!full_wait(s1, ph1)) return false;
-          if (lane == 0) issue_unit(s1, 0, acc0, kb0 + i);
+          if (lane == 0) issue_unit(swapped, s1, 0, acc0, kb0 + i);
           __syncwarp();
           next(&s1, &ph1);
         }
@@ -789,7 +814,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         if (first && !acc_wait(acc1, par1)) return false;
         for (int i = 0; i < count; ++i) {
           if (lane == 0) {
-            issue_unit(s, 1, acc1, kb0 + i);
+            issue_unit(swapped, s, 1, acc1, kb0 + i);
             ptx::mma_commit_pair(ptx::smem_u32(&tail->empty[s]), 0x3);
           }
           __syncwarp();
@@ -805,8 +830,8 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           const uint64_t adesc = a_desc(s), bdesc0 = b_desc(s, 0), bdesc1 = b_desc(s, 1);
 #pragma unroll
           for (int k = 0; k < kBlockK / 16; ++k) {
-            ptx::mma_bf16_ss_pair(tmem_base + acc0 * kBlockN, adesc + k * kAStep, bdesc0 + k * kBStep, kIdesc, 1u);
-            ptx::mma_bf16_ss_pair(tmem_base + acc1 * kBlockN, adesc + k * kAStep, bdesc1 + k * kBStep, kIdesc, 1u);
+            mma_pair(swapped, tmem_base + acc0 * kBlockN, adesc + k * kAStep, bdesc0 + k * kBStep, 1u);
+            mma_pair(swapped, tmem_base + acc1 * kBlockN, adesc + k * kAStep, bdesc1 + k * kBStep, 1u);
           }
           ptx::mma_commit_pair(ptx::smem_u32(&tail->empty[s]), 0x3);
         }
@@ -821,8 +846,12 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       if (got == kEndOfOrder) break;
       const int nkb = tile_stages(t);
       if (nkb == 0) { loads_landed(); continue; }  // empty wgrad expert: the epilogue writes zeros
+      const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
+      if (kSwap && kPair && sw_rows != 0) sw_idesc = ptx::make_idesc_bf16(kBlockM * CTAS, sw_rows, kBMn ? 1 : 0, 0);
       if (kPair && t.units == 2) {
-        if (!(ok = wide_tile(nkb))) break;
+        if constexpr (kSwap) ok = sw_rows != 0 ? wide_tile(std::true_type{}, nkb) : wide_tile(std::false_type{}, nkb);
+        else ok = wide_tile(std::false_type{}, nkb);
+        if (!ok) break;
         loads_landed();
         continue;
       }
@@ -840,7 +869,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         for (int kb = 0; kb < nkb; ++kb) {
           if (!ptx::mbar_wait(ptx::smem_u32(&tail->full[s]), ph, wait)) { ok = false; break; }
           ptx::tc_fence_after_sync();
-          const uint32_t sw = stage_base + s * G::kStageBytes;
+          const uint32_t sw = stage_base + s * stage_bytes;
           const uint32_t sx = sw + kLightWBytes;
           if (lane == 0) {
 #pragma unroll
@@ -857,21 +886,26 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             ptx::mma_commit(ptx::smem_u32(&tail->empty[s]));
           }
           __syncwarp();
-          if (++s == kStages) { s = 0; ph ^= 1u; }
+          if (++s == ring_stages) { s = 0; ph ^= 1u; }
         }
         if (ok && lane == 0) ptx::mma_commit(ptx::smem_u32(&tail->tmem_full[ab]));
         __syncwarp();
         continue;
       }
-      const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
       for (int kb = 0; kb < nkb; ++kb) {
         const uint32_t f_bar = ptx::smem_u32(&tail->full[s]);
         // (gather variant of a pair: one arrival is the other CTA's gather warp)
         if (!ptx::mbar_wait<kPair && GATHER>(f_bar, ph, wait)) { ok = false; break; }
         ptx::tc_fence_after_sync();
-        const uint32_t sa = stage_base + s * G::kStageBytes;
+        const uint32_t sa = stage_base + s * stage_bytes;
         const uint32_t sb = sa + G::kABytes;
-        if (kSwap && sw_rows != 0) {
+        if (kPair) {
+          if (lane == 0) {
+            if (kSwap && sw_rows != 0) issue_unit(std::true_type{}, s, 0, ab, kb);
+            else issue_unit(std::false_type{}, s, 0, ab, kb);
+            ptx::mma_commit_pair(ptx::smem_u32(&tail->empty[s]), 0x3);
+          }
+        } else if (kSwap && sw_rows != 0) {
           // D[weight columns, rows] = W^T x X^T: the staged B tile is the UMMA A operand
           // (its two halves of 128 columns in turn), the staged rows are the UMMA B operand.
           if (lane == 0) {
@@ -903,18 +937,12 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           constexpr uint64_t b_step = kBMn ? (2048u >> 4) : (32u >> 4);
 #pragma unroll
           for (int k = 0; k < kBlockK / 16; ++k) {
-            if (kPair)
-              ptx::mma_bf16_ss_pair(d_tmem, adesc + k * a_step, bdesc + k * b_step, kIdesc,
-                                    (kb | k) != 0 ? 1u : 0u);
-            else
-              ptx::mma_bf16_ss(d_tmem, adesc + k * a_step, bdesc + k * b_step, kIdesc,
-                               (kb | k) != 0 ? 1u : 0u);
+            ptx::mma_bf16_ss(d_tmem, adesc + k * a_step, bdesc + k * b_step, kIdesc, (kb | k) != 0 ? 1u : 0u);
           }
-          if (kPair) ptx::mma_commit_pair(ptx::smem_u32(&tail->empty[s]), 0x3);
-          else ptx::mma_commit(ptx::smem_u32(&tail->empty[s]));
+          ptx::mma_commit(ptx::smem_u32(&tail->empty[s]));
         }
         __syncwarp();
-        if (++s == kStages) { s = 0; ph ^= 1u; }
+        if (++s == ring_stages) { s = 0; ph ^= 1u; }
       }
       if (ok) loads_landed();
       if (ok && lane == 0) {
@@ -1132,7 +1160,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     auto advance = [&]() {
       next += kGatherWarps;
       stage += kGatherWarps;
-      if (stage >= kStages) { stage -= kStages; ph ^= 1u; }
+      if (stage >= static_cast<int>(ring_stages)) { stage -= static_cast<int>(ring_stages); ph ^= 1u; }
     };
     bool ok = true;
     bool bad_index = false;
@@ -1166,7 +1194,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           if (lane == 0) ok = ptx::mbar_wait(empty_bar0 + uint32_t(stage) * 8u, ph ^ 1u, wait);
           ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
           if (!ok) break;
-          const uint32_t stage_addr = stage_base + uint32_t(stage) * G::kStageBytes;
+          const uint32_t stage_addr = stage_base + uint32_t(stage) * stage_bytes;
           const uint32_t full_bar = full_bar0 + uint32_t(stage) * 8u;
           // (the box's 128 bytes lie next to each other: the same row offset serves both)
           const int col = t.row0 + row_off + chunk * 8;  // column of a_src in the first box
@@ -1228,7 +1256,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           if (lane == 0) ok = ptx::mbar_wait(empty_bar0 + uint32_t(stage) * 8u, ph ^ 1u, wait);
           ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
           if (!ok) break;
-          const uint32_t stage_addr = stage_base + uint32_t(stage) * G::kStageBytes;
+          const uint32_t stage_addr = stage_base + uint32_t(stage) * stage_bytes;
           const uint32_t full_bar = full_bar0 + uint32_t(stage) * 8u;
           const int kcol = (next - base) * kBlockK + chunk * 8;
           const bool in_k = kcol < p.d1;  // d1 is a multiple of 8: a piece is all in or all out
@@ -1392,11 +1420,11 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       }
     };
 
-    // Swapped tile: 32 rows x 32 columns held transposed, v[i] = row i, this lane's
-    // column.  The values go through the staging buffer (row i at 64 i, so a warp's
-    // store of one row is 64 consecutive bytes) and leave as a TMA store when all 32
-    // rows exist, else row by row: lane i sends row i.
-    auto emit_swapped = [&](const uint32_t (&v)[32], int rows, int64_t row, int col, int out_n) {
+    // Swapped tile: 32 rows x 32 columns held transposed, f[c][l] = this lane's fragment of rows
+    // 8 c .. 8 c + 7, columns 8 l .. 8 l + 7 (stmatrix_x4_trans turns it).  The values go through
+    // the staging buffer (row i at 64 i) and leave as a TMA store when all 32 rows exist, as
+    // bulk copies of a row when they are scattered, else as 64 bytes of a row by four lanes.
+    auto emit_swapped = [&](const uint32_t (&f)[4][4], int rows, int64_t row, int col, int out_n) {
       const uint32_t buf = scatter_rows ? my_out : stage_buf();
       if (scatter_rows) {
         if (stores > 0) ptx::bulk_wait_group_read<0>();  // this lane's previous copy
@@ -1404,16 +1432,13 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         ptx::bulk_wait_group_read<G::kOutBufs - 1>();
       }
       __syncwarp();
-      // 64-byte swizzle as in emit(); a scattered row is read linearly by its copy
+      // this lane gives the address of row 8 c + lane % 8, columns 8 (lane / 8) and on: 64-byte
+      // swizzle as in emit(); a scattered row is read linearly by its copy
       const uint32_t piece = uint32_t(lane) >> 3;
-      const uint32_t at = buf + (uint32_t(lane) & 7u) * 2u;
+      const uint32_t sw = scatter_rows ? piece : (piece ^ ((uint32_t(lane) >> 1) & 3u));
+      const uint32_t at = buf + (uint32_t(lane) & 7u) * 64u + (sw << 4);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const uint32_t sw = scatter_rows ? piece : (piece ^ ((uint32_t(i) >> 1) & 3u));
-        const __nv_bfloat16 h = __float2bfloat16_rn(__uint_as_float(v[i]));
-        asm volatile("st.shared.b16 [%0], %1;" ::"r"(at + uint32_t(i) * 64u + (sw << 4)), "h"(__bfloat16_as_ushort(h))
-                     : "memory");
-      }
+      for (int c4 = 0; c4 < 4; ++c4) ptx::stmatrix_x4_trans(at + uint32_t(c4) * 512u, f[c4][0], f[c4][1], f[c4][2], f[c4][3]);
       if (scatter_rows) {
         ptx::fence_proxy_async_smem();
         __syncwarp();
@@ -1442,18 +1467,18 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         ++stores;
       } else {
         __syncwarp();
-        if (lane < rows) {
-          uint4* dst = reinterpret_cast<uint4*>(c + (row + lane) * out_n + col);
+        const int cj = (lane & 3) * 8;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint4 o;
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
-                         : "r"(buf + uint32_t(lane) * 64u + ((uint32_t(j) ^ ((uint32_t(lane) >> 1) & 3u)) << 4))
-                         : "memory");
-            if (col + j * 8 < out_n) dst[j] = o;
-          }
+        for (int i = 0; i < 4; ++i) {
+          const int r = i * 8 + (lane >> 2);
+          uint4 o;
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
+                       : "r"(buf + uint32_t(r) * 64u + (((uint32_t(lane) & 3u) ^ ((uint32_t(r) >> 1) & 3u)) << 4))
+                       : "memory");
+          if (r < rows && col + cj < out_n) *reinterpret_cast<uint4*>(c + (row + r) * out_n + col + cj) = o;
         }
+        __syncwarp();
       }
     };
 
@@ -1464,44 +1489,73 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       const int nkb = tile_stages(t);
       const int sw_rows = kSwap ? swapped_rows(p, t) : 0;
       if (kSwap && sw_rows != 0) {
-        // TMEM lane = output column, TMEM column = output row.  This warp's half of the
-        // tile's columns is an accumulator of its own; for the gated product the two are
-        // gate and up of the same 128 output columns, and the two warps of a lane quadrant
-        // take the 32-row chunks in turn.
-        const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
-        ++it;
-        if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), aph, wait)) { ok = false; break; }
-        ptx::tc_fence_after_sync();
+        // TMEM lane = output column, TMEM column = output row.  One CTA: the two halves of the
+        // accumulator hold 128 columns each (gated: gate and up of the same 128).  A pair: an
+        // accumulator holds 128 columns of each CTA (gated: the first gate, the second up).  Where
+        // both warps of a lane quadrant serve the same columns they take 32-row chunks in turn.
+        constexpr bool kShared = kPair || SWIGLU;
         const int out_n = static_cast<int>(SWIGLU ? (p.n >> 1) : p.n);
-        const int col = (SWIGLU ? (t.col0 >> 1) : t.col0) + (SWIGLU ? 0 : col_base) + q * 32;
-        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + (SWIGLU ? 0 : col_base);
-        if (col < out_n) {
-          for (int r0 = SWIGLU ? half * 32 : 0; r0 < t.valid_rows; r0 += SWIGLU ? 64 : 32) {
-            const int rows = t.valid_rows - r0;
-            const int64_t row = int64_t(t.row0) + r0;
-            uint32_t va[32], vb[32];
-            ptx::tmem_ld_32x32(taddr + uint32_t(r0), va);
-            if (SWIGLU) ptx::tmem_ld_32x32(taddr + kBlockN / 2 + uint32_t(r0), vb);
-            ptx::tmem_ld_wait();
-            if (SWIGLU) {
+        const int r_first = kShared ? half * 32 : 0, r_step = kShared ? 64 : 32;
+#pragma unroll 1
+        for (int unit = 0; unit < (kPair && !SWIGLU ? t.units : 1); ++unit) {
+          const uint32_t ab = it & 1u, ab2 = kPair ? (it + 1u) & 1u : ab;  // (ab2: up columns)
+          if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), (it >> 1) & 1u, wait)) { ok = false; break; }
+          if (kPair && SWIGLU &&
+              !ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab2]), ((it + 1u) >> 1) & 1u, wait)) { ok = false; break; }
+          it += (kPair && SWIGLU) ? 2 : 1;
+          ptx::tc_fence_after_sync();
+          const int col = (SWIGLU ? (t.col0 >> 1) : t.col0) + (kPair ? unit * kBlockN + static_cast<int>(cta_rank) * (kBlockN / 2)
+                                                                     : (SWIGLU ? 0 : col_base)) + q * 32;
+          const uint32_t lane_base = uint32_t(q * 32) << 16;
+          const uint32_t ta = tmem_base + lane_base + ab * kBlockN + (kShared ? 0 : col_base);
+          const uint32_t tb = tmem_base + lane_base + ab2 * kBlockN + (kPair ? 0 : kBlockN / 2);
+          const bool live = col < out_n;
+          bool held = true;  // the accumulator(s)
+          auto release = [&]() {
+            held = false;
+            ptx::tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+              const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
+              if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(te_bar, 0));
+              else ptx::mbar_arrive(te_bar);
+              if (kPair && SWIGLU) ptx::mbar_arrive_cluster(ptx::mapa(ptx::smem_u32(&tail->tmem_empty[ab2]), 0));
+            }
+          };
+#pragma unroll 1
+          for (int r0 = r_first; live && r0 < t.valid_rows; r0 += r_step) {
+            uint32_t f[4][4];
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const float g = __uint_as_float(va[i]);
-                va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * __uint_as_float(vb[i]));
+            for (int h = 0; h < 2; ++h) {  // 16 lanes at a time: columns 16 h .. 16 h + 15 of the chunk
+              uint32_t va[16], vb[16];
+              ptx::tmem_ld_16x32_frag(ta + uint32_t(r0) + (uint32_t(h * 16) << 16), va);
+              if (SWIGLU) ptx::tmem_ld_16x32_frag(tb + uint32_t(r0) + (uint32_t(h * 16) << 16), vb);
+              ptx::tmem_ld_wait();
+              if (h == 1 && r0 + r_step >= t.valid_rows) release();
+              if (SWIGLU) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                  const float g = __uint_as_float(va[i]);
+                  va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * __uint_as_float(vb[i]));
+                }
+              }
+              if (scatter_rows && row_scale != nullptr) {
+                const float w = r0 + lane < t.valid_rows ? row_scale[int64_t(t.row0) + r0 + lane] : 1.0f;
+#pragma unroll
+                for (int i = 0; i < 16; ++i)  // value i: row 8 (i / 4) + 2 (lane % 4) + i % 2
+                  va[i] = __float_as_uint(__uint_as_float(va[i]) *
+                                          __shfl_sync(0xffffffffu, w, (i >> 2) * 8 + (lane & 3) * 2 + (i & 1)));
+              }
+#pragma unroll
+              for (int i = 0; i < 16; i += 2) {
+                __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(va[i]), __uint_as_float(va[i + 1]));
+                f[i >> 2][h * 2 + ((i >> 1) & 1)] = *reinterpret_cast<uint32_t*>(&v);
               }
             }
-            if (scatter_rows && row_scale != nullptr) {
-              const float w = lane < rows ? row_scale[row + lane] : 1.0f;
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                va[i] = __float_as_uint(__uint_as_float(va[i]) * __shfl_sync(0xffffffffu, w, i));
-            }
-            emit_swapped(va, rows, row, col, out_n);
+            emit_swapped(f, t.valid_rows - r0, int64_t(t.row0) + r0, col, out_n);
           }
+          if (held) release();
         }
-        ptx::tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&tail->tmem_empty[ab]));
         continue;
       }
       if (kLight && t.kind) {
@@ -1585,7 +1639,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * row_w);
       };
-      uint32_t va[32], vb[32];  // (vb: gated product)
+      uint32_t va[32], vb[32];
       if (MODE == kTN && nkb == 0) {  // (forward and dgrad tiles always have k > 0)
         // Empty wgrad expert: its block of the output is zeros.
         if (G::kWideOut && warp_full) {
@@ -1618,19 +1672,24 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           emit(zeros, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
         continue;
       }
-      uint4 d4[8] = {};  // gated backward: this lane's 64 values of the output gradient
-      if (SWIGLU && gate_grad != nullptr && row_ok) {
-        const int col = half * 64;
+      // Gated backward: a chunk (a pair: both) of this lane's values of the output gradient.  (A pair reads both
+      // before it waits for the accumulator, which is then held for less time.)
+      constexpr int kGradChunks = kPair ? 2 : 1;
+      uint4 d4[4 * kGradChunks] = {};
+      auto load_grad = [&](int first) {
+        if (gate_grad == nullptr || !row_ok) return;
+        const int col = half * 64 + first * 32;
         const uint4* src = reinterpret_cast<const uint4*>(gate_grad + (out_row0 + r) * out_n + out_col0 + col);
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < 4 * kGradChunks; ++j)
           if (col + j * 8 < cols_left) d4[j] = src[j];
-      }
+      };
+      if (SWIGLU && kPair) load_grad(0);
       const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
       ++it;
       if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), aph, wait)) { ok = false; break; }
       ptx::tc_fence_after_sync();
-      // The accumulator is read and rounded as a whole and handed back; only then do its values
+      // A pair's accumulator is read and rounded as a whole and handed back; only then do its values
       // leave through the staging buffer, where each chunk waits for the store before it.
       auto release = [&]() {
         ptx::tc_fence_before_sync();
@@ -1645,20 +1704,30 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         // This warp's 64 of the tile's 128 output columns: gate from accumulator
         // columns [64 half, +64), up from the same columns of the second half.
         const uint32_t tg = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + half * 64;
-        uint4 o[16];
-#pragma unroll
+        uint4 o[8 * kGradChunks];  // per chunk: the result, or both gradients
+        auto emit_chunk = [&](int ch) {
+          const int col = half * 64 + ch * 32;
+          const uint4* oc = o + (kPair ? ch * 8 : 0);
+          emit(oc, col, warp_full, row_ok, crow, cols_left, tile_row, out_col0);
+          if (gate_grad != nullptr)
+            emit(oc + 4, col, warp_full, row_ok, crow + p.tokens * out_n, cols_left,
+                 tile_row + static_cast<int>(p.tokens), out_col0);
+        };
+#pragma unroll(kPair ? 2 : 1)
         for (int ch = 0; ch < 2; ++ch) {
           ptx::tmem_ld_32x32(tg + ch * 32, va);
           ptx::tmem_ld_32x32(tg + kBlockN / 2 + ch * 32, vb);
           ptx::tmem_ld_wait();
           if (ch == 1) release();
+          uint4* oc = o + (kPair ? ch * 8 : 0);
           if (gate_grad != nullptr) {
+            if (!kPair) load_grad(ch);
             // Backward of the gated product: with g, u recomputed in the accumulator and
-            // dh = gate_grad[row, col ..] (read above), the gradients w.r.t. the two products
+            // dh = gate_grad[row, col ..], the gradients w.r.t. the two products
             //   dg = dh * u * silu'(g),  silu'(g) = s (1 + g (1 - s)),  s = 1 / (1 + exp(-g))
             //   du = dh * silu(g)
             // go to rows [0, T) and [T, 2T) of the output.
-            const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(d4 + ch * 4);
+            const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(d4 + (kPair ? ch * 4 : 0));
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               const float g = __uint_as_float(va[i]);
@@ -1669,8 +1738,8 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
               va[i] = __float_as_uint(dh * u * sg * (1.0f + g * (1.0f - sg)));
               vb[i] = __float_as_uint(dh * g * sg);
             }
-            pack(va, o + ch * 4);
-            pack(vb, o + 8 + ch * 4);
+            pack(va, oc);
+            pack(vb, oc + 4);
           } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
@@ -1679,38 +1748,56 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
               va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * u);  // silu(g) * u
             }
             if (scaled) scale(va);
-            pack(va, o + ch * 4);
+            pack(va, oc);
           }
+          if (!kPair) emit_chunk(ch);
         }
-#pragma unroll
-        for (int ch = 0; ch < 2; ++ch) {
-          const int col = half * 64 + ch * 32;
-          emit(o + ch * 4, col, warp_full, row_ok, crow, cols_left, tile_row, out_col0);
-          if (gate_grad != nullptr)
-            emit(o + 8 + ch * 4, col, warp_full, row_ok, crow + p.tokens * out_n, cols_left,
-                 tile_row + static_cast<int>(p.tokens), out_col0);
+        if (kPair) {
+          emit_chunk(0);
+          emit_chunk(1);
         }
         continue;
       }
       const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + col_base;
-      uint4 o[16];
-#pragma unroll
-      for (int ch = 0; ch < kBlockN / 64; ++ch) {
-        ptx::tmem_ld_32x32(taddr + ch * 32, va);
-        ptx::tmem_ld_wait();
-        if (ch == kBlockN / 64 - 1) release();
-        if (scaled) scale(va);
-        pack(va, o + ch * 4);
+      uint4 o[kPair ? 16 : 8];
+      auto emit_chunks = [&](int ch) {  // two of 32 columns
+        const int col = col_base + ch * 32;
+        const uint4* oc = o + (kPair ? ch * 4 : 0);
+        if (G::kWideOut && warp_full) {
+          if (col < cols_left) emit64(oc, col, tile_row, unit_col0);
+        } else {
+          emit(oc, col, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
+          emit(oc + 4, col + 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
+        }
+      };
+#pragma unroll(kPair ? 2 : 1)
+      for (int ch = 0; ch < kBlockN / 64; ch += 2) {
+        uint4* oc = o + (kPair ? ch * 4 : 0);
+        if (GATHER || PUSH) {  // (128 registers)
+          ptx::tmem_ld_32x32(taddr + ch * 32, va);
+          ptx::tmem_ld_wait();
+          if (scaled) scale(va);
+          pack(va, oc);
+          ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, va);
+          ptx::tmem_ld_wait();
+          if (ch + 2 == kBlockN / 64) release();
+          if (scaled) scale(va);
+          pack(va, oc + 4);
+        } else {
+          ptx::tmem_ld_32x32(taddr + ch * 32, va);
+          ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
+          ptx::tmem_ld_wait();
+          if (ch + 2 == kBlockN / 64) release();
+          if (scaled) { scale(va); scale(vb); }
+          pack(va, oc);
+          pack(vb, oc + 4);
+        }
+        if (!kPair) emit_chunks(ch);
       }
-      if (G::kWideOut && warp_full) {
-#pragma unroll
-        for (int ch = 0; ch < kBlockN / 64; ch += 2)
-          if (col_base + ch * 32 < cols_left) emit64(o + ch * 4, col_base + ch * 32, tile_row, unit_col0);
-        continue;
+      if (kPair) {
+        emit_chunks(0);
+        emit_chunks(2);
       }
-#pragma unroll
-      for (int ch = 0; ch < kBlockN / 64; ++ch)
-        emit(o + ch * 4, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
       }
     }
     // Shared memory must outlive the stores that still read it.

@@ -68,6 +68,8 @@ struct Problem {
   int64_t dest_rows;
   int zero_rest;   // gated backward: rows past the last expert's of both halves of c become zeros
   int swap_rows;   // NN/NT: a tile of at most this many rows (rounded up, swapped_rows) runs with its operands swapped
+  int narrow_rounds;  // a pair's launch of fewer rounds of wide tiles than this runs halves of them
+  int swap_units;  // ... if it has this many accumulators (a pair's gated tile: 2, gate and up, else 1)
 };
 
 // Fills the derived fields of a Problem whose shape fields are set.
@@ -119,17 +121,17 @@ B200GMM_HD int tile_stages(const Tile& t) {
   return t.kind ? (t.k_len + kLightK - 1) / kLightK : (t.k_len + kBlockK - 1) / kBlockK;
 }
 
-// Swapped tiles (NN/NT, one CTA): a 128 x 256 tile with few rows is computed as its
-// transpose, from the same loads.  The tile's 256 weight columns ride UMMA M (two MMAs of
-// 128) and its rows ride UMMA N, rounded up to the step of 16 that N allows, so that the
-// tensor core works for the rows that exist and not for 128 of them, and only those
-// rows are fetched.  Launches of small experts are bound by streaming
-// weights; what the padded rows cost them was tensor time and power and a third of the
-// bytes that enter an SM.  Which launches: Problem::swap_rows (b200gmm.cu: swap_rows).
+// Swapped tiles (NN/NT): a tile with few rows is computed as its transpose, from the same
+// loads.  The tile's weight columns ride UMMA M (one CTA: two MMAs of 128 columns; a pair: one
+// MMA of 2 x 128 for each accumulator) and its rows ride UMMA N, rounded up to the step that N
+// allows, so that the tensor core works for the rows that exist and not for tile_m of
+// them, and only those rows are fetched.  Which launches, and up to how many rows a tile:
+// Problem::swap_rows (b200gmm.cu: swap_rows).
 // Returns the rounded row count, 0 for a plain tile.
 B200GMM_HD int swapped_rows(const Problem& p, const Tile& t) {
-  if (p.swap_rows == 0 || t.kind != 0) return 0;
-  const int rows = (t.valid_rows + 15) & ~15;
+  if (p.swap_rows == 0 || t.kind != 0 || t.units < p.swap_units) return 0;
+  const int step = p.tile_m == kBlockM ? 16 : 32;
+  const int rows = (t.valid_rows + step - 1) / step * step;
   return rows <= p.swap_rows ? rows : 0;
 }
 
@@ -143,6 +145,15 @@ B200GMM_HD void decode_in_expert(int local, int row_tiles, int nt, int group_m, 
   const int r = local - g * group_span;
   *mi = first + r % gm;
   *ni = r / gm;
+}
+
+// Whether a pair's launch of `tiles` wide tiles on `clusters` pairs takes all of them as
+// halves of one accumulator: where they are all that wide, where the halves fit one
+// round, or (Problem::narrow_rounds) where there are few rounds.  (single_wave: a pair has no
+// second tile, so only what fits one round may be halved.)
+B200GMM_HD bool narrow_tiles(const Problem& p, int tiles, int clusters) {
+  if (p.n <= kBlockN || 2 * tiles <= clusters) return true;
+  return !p.single_wave && tiles < p.narrow_rounds * clusters;
 }
 
 // Accumulators that the tile at column col0 fills.
