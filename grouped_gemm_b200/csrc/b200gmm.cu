@@ -266,14 +266,55 @@ int encode_blocked(CUtensorMap* map, const void* base, uint64_t cols, uint64_t r
   return encode_map(map, base, experts > 0 ? 4 : 3, dims, box, CU_TENSOR_MAP_SWIZZLE_128B, strides);
 }
 
+// Whether rows of an operand start at any 16 bytes: a k-block of such a row is five sectors in two
+// lines of L2 instead of four in one.  (b's rows are d1 long in the NT layout.)
+bool ragged_rows(int64_t d1, int64_t n, int trans_b) { return d1 % 16 != 0 || (!trans_b && n % 16 != 0); }
+
 // Which variant a problem runs on.  Only shapes known on the host may decide
-// (batch_sizes can live on the device): a CTA pair pays off when an expert has,
-// on average, at least a couple of 256-row tiles.  B200GMM_CTAS=1|2 overrides.
-int choose_ctas(int z, int64_t tokens, int64_t d1, int trans_a) {
+// (batch_sizes can live on the device).  B200GMM_CTAS=1|2 overrides.
+//
+// What bounds the choice is bytes into the SMs: per k-block an SM loads 48 KiB for 128 x 256
+// outputs (one CTA), 48 KiB for 128 x 512 (a pair's tile) or 32 KiB for 128 x 256 (half of one).
+// rounds_one and rounds_pair are these bytes (/ 16 KiB) over the rounds of tiles that the
+// grid makes, for experts of even size, half a row tile of each idle.  Times of the kernels
+// follow their ratio, times a factor for the path (8 or 64 experts, 64 to 1024 rows each):
+//   rows that start at any 16 bytes (a row is then two lines of L2 where it could be one):
+//     about 0.8; z = 64, 128 rows, 4088 x 8184: ratio 1.5, forward 1351 / 933 us; 512 rows: 1.8, 3769 /
+//     2282; z = 8, 128 rows, 1000 x 2504: 1.0, 17.4 / 21.5.
+//   others: 0.55, the L2 being no bound; z = 64, 512 rows, 2048 x 4096: 1.81, 564 / 608 us; z = 8,
+//     1024 rows: 2.0, 135 / 129; z = 8, 512 rows, dgrad: 1.2, 68 / 90.
+// Many experts (128 and more) are hardly ever of even size, and swapped tiles take the
+// small ones: z = 256, 256 rows, 7168 x 2048, Zipf routing: ratio 1.67, 2383 / 2244 us, dgrad
+// 2322 / 2152 (even sizes: 3 % slower).
+// A short contraction leaves an accumulator little time to be read out while the other one
+// fills, which a pair's tile does not have: one CTA below 416 (any 16 bytes) and 512 (49 experts, 98681
+// rows, 72 x 2000: 159 / 101 us; 173, 110139, 128 x 856: 113 / 77; 81, 68558, 432 x 2608: 240 / 223).
+// Few tiles: where one-CTA tiles fill no more than one round, experts of less than 384 rows leave
+// too much of a pair's tile idle (one of 322 rows, 5976 x 4736: 37 / 63 us; of 428: 30 / 25).
+// wgrad loads its operands for as many k-blocks as an expert has rows, and writes as much in
+// either form: the line lies at 384 rows (any 16 bytes: 0.98 at 256, 1.17 at 512) and 512
+// (0.9 and 1.02).
+int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b) {
   const int forced = env_int("B200GMM_CTAS", 0);
   if (forced == 1 || forced == 2) return forced;
-  if (z <= 0 || tokens / z < 512) return 1;
-  return (!trans_a || d1 >= 256) ? 2 : 1;
+  if (z <= 0 || tokens <= 0 || d1 <= 0 || n <= 0) return 1;
+  constexpr int64_t kSms = 148, kPairs = kSms / 2;
+  const bool ragged = ragged_rows(d1, n, trans_b);
+  const int64_t nt = (n + kBlockN - 1) / kBlockN;
+  const auto tiles = [&](int64_t tile_m, int64_t cols) {
+    return trans_a ? z * ((d1 + tile_m - 1) / tile_m) * cols
+                   : (2 * tokens / tile_m + std::min<int64_t>(z, tokens)) * cols / 2;
+  };
+  const int64_t one = tiles(kBlockM, nt), pair = tiles(2 * kBlockM, (nt + 1) / 2);
+  const int64_t left = pair % kPairs;
+  const int64_t rounds_one = 3 * ((one + kSms - 1) / kSms);
+  const int64_t rounds_pair = nt == 1 ? 2 * ((pair + kPairs - 1) / kPairs)
+                                      : 3 * (pair / kPairs) + (left == 0 ? 0 : (2 * left <= kPairs ? 2 : 3));
+  const double ratio = double(rounds_one) / double(std::max<int64_t>(rounds_pair, 1));
+  if (trans_a) return tokens >= (ragged ? 384 : 512) * int64_t(z) && d1 >= 256 && ratio >= 1.5 ? 2 : 1;
+  if (d1 < (ragged ? 416 : 512) || (one <= kSms && tokens < 384 * int64_t(z))) return 1;
+  if (nt == 1) return ratio >= 1.25 && (ragged || tokens >= 512 * int64_t(z)) ? 2 : 1;
+  return ratio >= (ragged ? 1.25 : (z >= 128 ? 1.6 : 1.85)) ? 2 : 1;
 }
 
 // Which kernel features a plain, gathered or gated launch uses (schedule.cuh: Problem).
@@ -326,10 +367,6 @@ int swap_rows(const Problem& p, const Features& f, int ctas, int sm_count) {
   if (!f.scatter && p.d1 < kPlainMinK) return 0;
   return p.tokens <= kMeanRows * p.z && 2 * tiles >= sm_count ? kBlockM / 2 : 0;
 }
-
-// Whether rows of an operand start at any 16 bytes: a k-block of such a row is five sectors in two
-// lines of L2 instead of four in one.  (b's rows are d1 long in the NT layout.)
-bool ragged_rows(int64_t d1, int64_t n, int trans_b) { return d1 % 16 != 0 || (!trans_b && n % 16 != 0); }
 
 int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b, int ctas,
                   Problem* p, const Features& f = Features()) {
@@ -508,7 +545,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   feat.swiglu = swiglu;
   feat.gated_backward = gate_grad != nullptr;
   feat.scatter = row_dest != nullptr;
-  int ctas = choose_ctas(z, tokens, dim_a1, trans_a);
+  int ctas = choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b);
   int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat);
   if (rc != B200GMM_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
@@ -986,7 +1023,7 @@ int b200gmm_schedule_host(const int64_t* batch_sizes_host, int z, int64_t tokens
                           int64_t n, int trans_a, int trans_b, int cluster_ctas, int64_t* out,
                           int64_t max_tiles, int64_t* n_tiles) {
   Problem p;
-  if (cluster_ctas == 0) cluster_ctas = choose_ctas(z, tokens, dim_a1, trans_a);
+  if (cluster_ctas == 0) cluster_ctas = choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b);
   const int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, cluster_ctas, &p);
   if (rc != B200GMM_OK) return rc;
   if (n_tiles == nullptr || (z > 0 && batch_sizes_host == nullptr)) return B200GMM_EINVAL;
@@ -1034,7 +1071,7 @@ int b200gmm_schedule_device(const int64_t* batch_sizes_device, int z, int64_t to
                             int64_t max_tiles, int32_t* n_tiles_device, uint32_t* device_status,
                             void* cuda_stream) {
   Problem p;
-  if (cluster_ctas == 0) cluster_ctas = choose_ctas(z, tokens, dim_a1, trans_a);
+  if (cluster_ctas == 0) cluster_ctas = choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b);
   const int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, cluster_ctas, &p);
   if (rc != B200GMM_OK) return rc;
   if (n_tiles_device == nullptr || (z > 0 && batch_sizes_device == nullptr) || max_tiles < 0 ||
