@@ -101,7 +101,7 @@ template <int MODE, int CTAS, bool GATHER, bool SWIGLU, bool PUSH = false>
 cudaError_t launch_gmm(const LaunchArgs& a) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.grid);
-  cfg.blockDim = dim3(GATHER ? kGatherThreads : (PUSH ? kGemmPushThreads : kThreads));
+  cfg.blockDim = dim3(GATHER ? GatherWarps<CTAS>::kBlockThreads : (PUSH ? kGemmPushThreads : kThreads));
   cfg.dynamicSmemBytes = PUSH ? kSmemBytesPush : kSmemBytes;
   cfg.stream = a.stream;
   cudaLaunchAttribute attr[2];
@@ -270,6 +270,14 @@ int encode_blocked(CUtensorMap* map, const void* base, uint64_t cols, uint64_t r
 // lines of L2 instead of four in one.  (b's rows are d1 long in the NT layout.)
 bool ragged_rows(int64_t d1, int64_t n, int trans_b) { return d1 % 16 != 0 || (!trans_b && n % 16 != 0); }
 
+// Which kernel features a plain, gathered or gated launch uses (schedule.cuh: Problem).
+struct Features {
+  bool gather = false;
+  bool swiglu = false;
+  bool gated_backward = false;
+  bool scatter = false;  // row_dest: rows of the result go where a table says
+};
+
 // Which variant a problem runs on.  Only shapes known on the host may decide
 // (batch_sizes can live on the device).  B200GMM_CTAS=1|2 overrides.
 //
@@ -279,51 +287,52 @@ bool ragged_rows(int64_t d1, int64_t n, int trans_b) { return d1 % 16 != 0 || (!
 // grid makes, for experts of even size, half a row tile of each idle.  Times of the kernels
 // follow their ratio, times a factor for the path (8 or 64 experts, 64 to 1024 rows each):
 //   rows that start at any 16 bytes (a row is then two lines of L2 where it could be one):
-//     about 0.8; z = 64, 128 rows, 4088 x 8184: ratio 1.5, forward 1351 / 933 us; 512 rows: 1.8, 3769 /
-//     2282; z = 8, 128 rows, 1000 x 2504: 1.0, 17.4 / 21.5.
+//     about 0.8 to 1; z = 64, 128 rows, 4088 x 8184: ratio 1.5, forward 1351 / 933 us; 512 rows: 1.8, 3769 /
+//     2282; z = 7, 428 rows, 1000 x 2504: 1.2, 28.0 / 23.0 or, other sizes, 31.5; z = 8, 128 rows: 1.0,
+//     17.4 / 21.5.
 //   others: 0.55, the L2 being no bound; z = 64, 512 rows, 2048 x 4096: 1.81, 564 / 608 us; z = 8,
-//     1024 rows: 2.0, 135 / 129; z = 8, 512 rows, dgrad: 1.2, 68 / 90.
+//     1024 rows: 2.0, 135 / 129; z = 8, 512 rows, dgrad: 1.2, 68 / 90.  From 1024 rows on the power
+//     cap adds to it (17 experts of 1548 rows, dgrad 7344 -> 520: 1.67, 309 / 248).
 // Many experts (128 and more) are hardly ever of even size, and swapped tiles take the
 // small ones: z = 256, 256 rows, 7168 x 2048, Zipf routing: ratio 1.67, 2383 / 2244 us, dgrad
-// 2322 / 2152 (even sizes: 3 % slower).
+// 2322 / 2152 (even sizes: 3 % slower).  The gathered product has no swapped tiles: from 256 rows on
+// (146 experts of 126 rows, 6712 x 2496: 1185 / 1487).
 // A short contraction leaves an accumulator little time to be read out while the other one
 // fills, which a pair's tile does not have: one CTA below 416 (any 16 bytes) and 512 (49 experts, 98681
-// rows, 72 x 2000: 159 / 101 us; 173, 110139, 128 x 856: 113 / 77; 81, 68558, 432 x 2608: 240 / 223).
+// rows, 72 x 2000: 159 / 101 us; 173, 110139, 128 x 856: 113 / 77; 81, 68558, 432 x 2608: 240 / 223),
+// and below 128 rows an expert up to 2048 (123 experts, 11149 rows, 528 x 1624: 64 / 81).  Scattered rows
+// run in halves there (narrow_rounds): from 512 rows on.
 // Few tiles: where one-CTA tiles fill no more than one round, experts of less than 384 rows leave
 // too much of a pair's tile idle (one of 322 rows, 5976 x 4736: 37 / 63 us; of 428: 30 / 25).
 // wgrad loads its operands for as many k-blocks as an expert has rows, and writes as much in
 // either form: the line lies at 384 rows (any 16 bytes: 0.98 at 256, 1.17 at 512) and 512
 // (0.9 and 1.02).
-int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b) {
+int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b, const Features& f = Features()) {
   const int forced = env_int("B200GMM_CTAS", 0);
   if (forced == 1 || forced == 2) return forced;
   if (z <= 0 || tokens <= 0 || d1 <= 0 || n <= 0) return 1;
   constexpr int64_t kSms = 148, kPairs = kSms / 2;
-  const bool ragged = ragged_rows(d1, n, trans_b);
+  const bool ragged = ragged_rows(d1, f.swiglu ? n / 2 : n, trans_b);
   const int64_t nt = (n + kBlockN - 1) / kBlockN;
   const auto tiles = [&](int64_t tile_m, int64_t cols) {
     return trans_a ? z * ((d1 + tile_m - 1) / tile_m) * cols
                    : (2 * tokens / tile_m + std::min<int64_t>(z, tokens)) * cols / 2;
   };
+  const auto rows_from = [&](int64_t mean) { return tokens >= mean * int64_t(z); };
   const int64_t one = tiles(kBlockM, nt), pair = tiles(2 * kBlockM, (nt + 1) / 2);
   const int64_t left = pair % kPairs;
   const int64_t rounds_one = 3 * ((one + kSms - 1) / kSms);
   const int64_t rounds_pair = nt == 1 ? 2 * ((pair + kPairs - 1) / kPairs)
                                       : 3 * (pair / kPairs) + (left == 0 ? 0 : (2 * left <= kPairs ? 2 : 3));
   const double ratio = double(rounds_one) / double(std::max<int64_t>(rounds_pair, 1));
-  if (trans_a) return tokens >= (ragged ? 384 : 512) * int64_t(z) && d1 >= 256 && ratio >= 1.5 ? 2 : 1;
-  if (d1 < (ragged ? 416 : 512) || (one <= kSms && tokens < 384 * int64_t(z))) return 1;
-  if (nt == 1) return ratio >= 1.25 && (ragged || tokens >= 512 * int64_t(z)) ? 2 : 1;
-  return ratio >= (ragged ? 1.25 : (z >= 128 ? 1.6 : 1.85)) ? 2 : 1;
+  if (trans_a) return rows_from(ragged ? 384 : 512) && d1 >= 256 && ratio >= 1.5 ? 2 : 1;
+  if (d1 < (ragged ? 416 : 512) || (one <= kSms && !rows_from(384))) return 1;
+  if (!rows_from(f.gather || f.gated_backward ? 256 : (d1 < 2048 ? 128 : 64))) return 1;
+  if (f.scatter && d1 < 8192) return rows_from(512) ? 2 : 1;
+  if (nt == 1) return ratio >= 1.25 && (ragged || rows_from(512)) ? 2 : 1;
+  if (ragged) return ratio >= 1.25 ? 2 : 1;
+  return ratio >= (rows_from(1024) || (z >= 128 && !f.gather && !f.gated_backward) ? 1.6 : 1.85) ? 2 : 1;
 }
-
-// Which kernel features a plain, gathered or gated launch uses (schedule.cuh: Problem).
-struct Features {
-  bool gather = false;
-  bool swiglu = false;
-  bool gated_backward = false;
-  bool scatter = false;  // row_dest: rows of the result go where a table says
-};
 
 // Which launches run their tiles of few rows with swapped operands (schedule.cuh), and up
 // to how many rows a tile.  What the form saves is tensor work on rows that do not exist,
@@ -404,11 +413,13 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   // launch was not faster with them (B200GMM_LIGHT=1 switches them on).
   p->light = (p->mode != kTN && ctas == 1 && !f.gather && !f.swiglu) ? env_int("B200GMM_LIGHT", 0) : 0;
   // A pair's wide tiles are half as many.  wgrad's are as long as their expert has rows: with
-  // few a CTA the long ones end the launch (11 experts, 126529 rows, 4144 x 576: 712 us with tiles of 256
-  // columns, 872 with 512).  Forward and dgrad: few rounds lose more to the last one than the bytes
-  // save (3 experts, 3172 rows, 1936 x 4672: 62.3 / 66.3), unless rows start at any 16 bytes, when bytes
-  // are what bounds them (7 experts, 3001 rows, 1000 x 2504: 26.4 / 23.0).
-  p->narrow_rounds = trans_a ? 8 : (ragged_rows(d1, n, trans_b) ? 0 : 4);
+  // few a CTA and experts of 2048 rows and more the long ones end the launch (11 experts, 126529 rows, 4144 x 576: 712 us with tiles of 256
+  // columns, 872 with 512).  Forward and dgrad: one or two rounds lose more to the last one than the
+  // bytes save (3 experts, 3172 rows, 1936 x 4672: 62.3 / 66.3), unless rows start at any 16 bytes, when
+  // bytes are what bounds them (7 experts, 3001 rows, 1000 x 2504: 26.4 / 23.0).  Scattered rows leave in
+  // 64-byte copies: while an accumulator's are sent the other one has to wait, unless the contraction
+  // is long (16384 rows, 8 experts, 4096 x 14336: 1573 / 1660; 14336 x 4096, 8192 rows: 892 / 855).
+  p->narrow_rounds = trans_a ? (tokens >= 2048 * int64_t(z) ? 8 : 0) : (f.scatter && d1 < 8192 ? 1 << 20 : (ragged_rows(d1, f.swiglu ? n / 2 : n, trans_b) ? 0 : 2));
   p->swap_units = 1;
   p->swap_rows = 0;  // decided where the device is known (run_impl)
   p->dest_indexed = 0;
@@ -545,7 +556,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   feat.swiglu = swiglu;
   feat.gated_backward = gate_grad != nullptr;
   feat.scatter = row_dest != nullptr;
-  int ctas = choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b);
+  int ctas = choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b, feat);
   int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat);
   if (rc != B200GMM_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);

@@ -123,10 +123,14 @@ constexpr uint32_t kLightXHalf = kLightRows * kBlockK * 2;         // 8 KiB per 
 constexpr uint32_t kRowBoxBytes = 32 * kBlockK * 2;                // one 32-row TMA box of activations: 4 KiB
 static_assert(kLightWBytes + 2 * kLightXHalf <= Geometry<1>::kStageBytes, "a transposed stage must fit a ring slot");
 
-// The gather variant adds warps that fetch the rows of A, a k-block each, in turn: as many
-// as the ring has stages.  With 11 + 4 = 15 warps a thread may use 128 registers.
-constexpr int kGatherWarps = 4;
-constexpr int kGatherThreads = kThreads + 32 * kGatherWarps;
+// The gather variant adds warps that fetch the rows of A, a k-block each, in turn: four beside
+// rings of four stages, five beside the six of a pair's narrow tiles.  With 11 + 5 = 16 warps a thread may
+// use 128 registers, a 17th would leave 96 and spill.
+template <int CTAS>
+struct GatherWarps {
+  static constexpr int kWarps = CTAS == 1 ? 4 : 5;
+  static constexpr int kBlockThreads = kThreads + 32 * kWarps;
+};
 
 // The push variant adds four warps that move rows between GPUs while the tensor
 // cores work (in the default, bulk-copy form of the transfer only one of their
@@ -437,7 +441,7 @@ struct TileFeed {
 // the compiler take the read-only path, whose loads it need not keep behind the
 // grid_dependency_wait() below.
 template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false>
-__global__ void __launch_bounds__(GATHER ? kGatherThreads : (PUSH ? kGemmPushThreads : kThreads), 1)
+__global__ void __launch_bounds__(GATHER ? GatherWarps<CTAS>::kBlockThreads : (PUSH ? kGemmPushThreads : kThreads), 1)
 gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
            const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_c,
            const __grid_constant__ CUtensorMap map_a2, __nv_bfloat16* __restrict__ c,
@@ -499,7 +503,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
       }
       // Takers of a published tile position: per CTA the producer thread, the epilogue
       // warps and the gather warps, plus the leader's MMA warp.
-      constexpr uint32_t kTakers = CTAS * (1 + kEpilogueWarps + (GATHER ? kGatherWarps : 0)) + 1;
+      constexpr uint32_t kTakers = CTAS * (1 + kEpilogueWarps + (GATHER ? GatherWarps<CTAS>::kWarps : 0)) + 1;
       for (int i = 0; i < kSchedSlots; ++i) {
         ptx::mbar_init(ptx::smem_u32(&tail->sched_full[i]), 1);
         ptx::mbar_init(ptx::smem_u32(&tail->sched_empty[i]), kTakers);
@@ -1165,13 +1169,16 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     Tile t;
     // position in the stream of k-blocks of this warp's next one, the ring stage it
     // lands in and the parity of that stage's use
+    // (with fewer stages than warps the last warp only passes tiles on)
+    const int active_warps = min(GatherWarps<CTAS>::kWarps, static_cast<int>(ring_stages));
     int next = warp - (kSchedWarp + 1);
     int stage = next;
+    if (next >= active_warps) next = 1 << 30;
     uint32_t ph = 0;
     int base = 0;     // k-blocks of the stream before the current tile
     auto advance = [&]() {
-      next += kGatherWarps;
-      stage += kGatherWarps;
+      next += active_warps;
+      stage += active_warps;
       if (stage >= static_cast<int>(ring_stages)) { stage -= static_cast<int>(ring_stages); ph ^= 1u; }
     };
     bool ok = true;
@@ -1236,7 +1243,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
             }
           }
           // the indices of this warp's next k-block of the tile arrive while the copies fly
-          if (next + kGatherWarps < base + nkb) load_idx(next + kGatherWarps - base);
+          if (next + active_warps < base + nkb) load_idx(next + active_warps - base);
           ptx::cp_async_wait_all();
           ptx::fence_proxy_async_smem();
           __syncwarp();

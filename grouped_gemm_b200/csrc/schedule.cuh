@@ -111,7 +111,8 @@ B200GMM_HD int expert_tiles(const Problem& p, int rows) {
 
 // Most tiles a launch can have, whatever batch_sizes holds (B200GMM_LIGHT off).
 B200GMM_HD int64_t max_tiles(const Problem& p) {
-  const int64_t nt = (p.n + kBlockN - 1) / kBlockN;  // (a wide tile may be taken as two positions)
+  // (a wide tile may be taken as two positions, whether or not both halves exist)
+  const int64_t nt = p.tile_n > kBlockN && p.n > kBlockN ? 2 * int64_t(p.nt) : (p.n + kBlockN - 1) / kBlockN;
   if (p.mode == kTN) return int64_t(p.z) * p.mt * nt;
   return (p.tokens / p.tile_m + (p.z < p.tokens ? p.z : p.tokens)) * nt;
 }
@@ -153,7 +154,7 @@ B200GMM_HD void decode_in_expert(int local, int row_tiles, int nt, int group_m, 
 // second tile, so only what fits one round may be halved.)
 B200GMM_HD bool narrow_tiles(const Problem& p, int tiles, int clusters) {
   if (p.n <= kBlockN || 2 * tiles <= clusters) return true;
-  return !p.single_wave && tiles < p.narrow_rounds * clusters;
+  return !p.single_wave && tiles < int64_t(p.narrow_rounds) * clusters;
 }
 
 // Accumulators that the tile at column col0 fills.
