@@ -34,6 +34,10 @@ SIGNATURES = {
         _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int,
         _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int, _c.c_int,
         _c.c_void_p, _c.c_size_t, _c.c_void_p, _c.c_void_p]),
+    "b200gmm_run_gradients": (_c.c_int, [
+        _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int,
+        _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int,
+        _c.c_void_p, _c.c_size_t, _c.c_void_p, _c.c_void_p]),
     "b200gmm_run_static": (_c.c_int, [
         _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_void_p, _c.c_int, _c.c_int,
         _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int, _c.c_int,

@@ -132,6 +132,24 @@ cudaError_t zero_counter(uint32_t* sched_counter, cudaStream_t stream) {
   return cudaLaunchKernelEx(&cfg, zero_counter_kernel, sched_counter);
 }
 
+// The two gradients of a small product (gmm_kernel.cuh: gmm_gradients_kernel), as two launches prepared
+// them.
+template <int MODE>
+cudaError_t launch_gradients(const LaunchArgs& d, const LaunchArgs& w) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(d.grid + w.grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = kSmemBytes;
+  cfg.stream = d.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  auto args = [](const LaunchArgs& a) { return ProductArgs{a.map_a, a.map_b, a.map_c, a.c, a.p, a.grid}; };
+  return cudaLaunchKernelEx(&cfg, gmm_gradients_kernel<MODE>, args(d), args(w), d.batch_sizes, d.status, d.slots, d.inline_sizes);
+}
+
 // The plain forward / dgrad kernels with push warps (a.push.src != nullptr).
 cudaError_t launch_with_push(const LaunchArgs& a, int ctas) {
   if (a.p.mode == kNN)
@@ -187,6 +205,9 @@ int device_info(DeviceInfo** out) {
         set_smem_attr<kNN, 2, false, true>() != cudaSuccess || set_smem_attr<kNT, 2, false, true>() != cudaSuccess ||
         set_smem_attr<kNN, 1, false, false, true>() != cudaSuccess || set_smem_attr<kNT, 1, false, false, true>() != cudaSuccess ||
         set_smem_attr<kNN, 2, false, false, true>() != cudaSuccess || set_smem_attr<kNT, 2, false, false, true>() != cudaSuccess)
+      return B200GMM_ECUDA;
+    if (cudaFuncSetAttribute(gmm_gradients_kernel<kNN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)) != cudaSuccess ||
+        cudaFuncSetAttribute(gmm_gradients_kernel<kNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)) != cudaSuccess)
       return B200GMM_ECUDA;
     // How many 2-CTA clusters of this kernel the device can hold at once (a GPC
     // with an odd number of free SMs leaves one out).
@@ -523,7 +544,9 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
              const float* row_scale = nullptr, int reduce_add = 0, const void* dest_base = nullptr,
              int64_t dest_bytes = 0, const void* gate_grad = nullptr, const PushArgs* push = nullptr,
              bool* push_launched = nullptr, bool pair_sum = false, bool zero_rest = false,
-             int64_t dest_rows = -1) {
+             int64_t dest_rows = -1, LaunchArgs* prepared = nullptr) {
+  // prepared != nullptr: the launch is described there and left to the caller (plain products of one
+  // wave of tiles).
   // dest_rows >= 0: row_dest holds rows of the [dest_rows, n] destination at
   // dest_base instead of addresses.
   // pair_sum: a is [2, tokens, dim_a1], c = a[0] x b + a[1] x b2 (b2 is then no gate).
@@ -556,7 +579,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   feat.swiglu = swiglu;
   feat.gated_backward = gate_grad != nullptr;
   feat.scatter = row_dest != nullptr;
-  int ctas = choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b, feat);
+  int ctas = prepared != nullptr ? 1 : choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b, feat);
   int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat);
   if (rc != B200GMM_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
@@ -775,6 +798,10 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     // (the pacing is a wait like any other: all of it stays inside the wait limit)
     if (la.push.interval_ns * items_per_warp > p.wait_ns) la.push.interval_ns = p.wait_ns / items_per_warp;
   }
+  if (prepared != nullptr) {
+    *prepared = la;
+    return B200GMM_OK;
+  }
   const cudaError_t err = gather      ? launch_variant<true, false>(la, ctas)
                           : swiglu    ? launch_variant<false, true>(la, ctas)
                           : with_push ? launch_with_push(la, ctas)
@@ -817,6 +844,42 @@ int b200gmm_run(const void* a, const void* b, void* c, const int64_t* batch_size
                 uint32_t* device_status, void* cuda_stream) {
   return run_impl(a, b, c, batch_sizes, batch_sizes_on_device, z, tokens, dim_a1, n, trans_a, trans_b,
                   workspace, workspace_bytes, device_status, cuda_stream, nullptr);
+}
+
+int b200gmm_run_gradients(const void* a, const void* b, const void* grad, void* a_grad, void* b_grad,
+                          const int64_t* batch_sizes, int batch_sizes_on_device, int z, int64_t tokens, int64_t dim_a1,
+                          int64_t n, int trans_b, void* workspace, size_t workspace_bytes, uint32_t* device_status,
+                          void* cuda_stream) {
+  const void *lhs = trans_b ? grad : a, *rhs = trans_b ? a : grad;
+  const int64_t lhs_cols = trans_b ? n : dim_a1, rhs_cols = trans_b ? dim_a1 : n;
+  // One launch of one-CTA tiles where all tiles of both products fit the SMs at once and the input
+  // gradient's are plain.  Side by side they take the time of the longer; two launches
+  // of a few microseconds each cost the host about as much as all of their preparation.
+  bool together = z > 0 && tokens > 0 && dim_a1 > 0 && n > 0 && env_int("B200GMM_CTAS", 1) == 1;
+  DeviceInfo* dev = nullptr;
+  Problem d, w;
+  together = together && check_problem(z, tokens, n, dim_a1, 0, !trans_b, 1, &d) == B200GMM_OK &&
+             check_problem(z, tokens, lhs_cols, rhs_cols, 1, 0, 1, &w) == B200GMM_OK && !d.light &&
+             device_info(&dev) == B200GMM_OK && max_tiles(d) + max_tiles(w) <= std::min(dev->sm_count, kMaxCtas) &&
+             swap_rows(d, Features(), 1, dev->sm_count) == 0;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (together && cudaStreamIsCapturing(static_cast<cudaStream_t>(cuda_stream), &capture) != cudaSuccess) return B200GMM_ECUDA;
+  together = together && capture == cudaStreamCaptureStatusNone;  // (a captured product keeps its own full dependencies)
+  LaunchArgs ld, lw;
+  int rc = run_impl(grad, b, a_grad, batch_sizes, batch_sizes_on_device, z, tokens, n, dim_a1, 0, !trans_b, workspace,
+                    workspace_bytes, device_status, cuda_stream, nullptr, nullptr, 0, nullptr, nullptr, 0, nullptr, 0, nullptr,
+                    nullptr, nullptr, false, false, -1, together ? &ld : nullptr);
+  if (rc != B200GMM_OK) return rc;
+  rc = run_impl(lhs, rhs, b_grad, batch_sizes, batch_sizes_on_device, z, tokens, lhs_cols, rhs_cols, 1, 0, workspace,
+                workspace_bytes, device_status, cuda_stream, nullptr, nullptr, 0, nullptr, nullptr, 0, nullptr, 0, nullptr,
+                nullptr, nullptr, false, false, -1, together ? &lw : nullptr);
+  if (rc != B200GMM_OK || !together) return rc;
+  if ((trans_b ? launch_gradients<kNN>(ld, lw) : launch_gradients<kNT>(ld, lw)) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return B200GMM_ECUDA;
+  }
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return B200GMM_OK;
 }
 
 int b200gmm_run_scatter(const void* a, const void* b, const int64_t* row_dest, const void* dest_base,

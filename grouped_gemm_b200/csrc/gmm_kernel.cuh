@@ -440,17 +440,19 @@ struct TileFeed {
 // sets up.  So none of them is `const __restrict__` or read through __ldg: either lets
 // the compiler take the read-only path, whose loads it need not keep behind the
 // grid_dependency_wait() below.
-template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false>
-__global__ void __launch_bounds__(GATHER ? GatherWarps<CTAS>::kBlockThreads : (PUSH ? kGemmPushThreads : kThreads), 1)
-gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-           const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_c,
-           const __grid_constant__ CUtensorMap map_a2, __nv_bfloat16* __restrict__ c,
-           const int64_t* batch_sizes, const Problem p,
-           uint32_t* status, CUtensorMap* map_slots, uint32_t* sched_counter, const int64_t* row_dest,
-           const int32_t* a_rows, const __nv_bfloat16* a_src,
-           const int64_t a_src_rows, const float* row_scale, const int reduce_add,
-           const int64_t dest_lo, const int64_t dest_hi, const __nv_bfloat16* gate_grad,
-           const PushArgs push, const __grid_constant__ InlineSizes inline_sizes) {
+// What one CTA of a launch does: CTA `block` of `blocks`.
+template <int MODE, int CTAS, bool GATHER, bool SWIGLU, bool PUSH>
+__device__ __forceinline__ void
+gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
+          const CUtensorMap& map_b2, const CUtensorMap& map_c,
+          const CUtensorMap& map_a2, __nv_bfloat16* __restrict__ c,
+          const int64_t* batch_sizes, const Problem& p,
+          uint32_t* status, CUtensorMap* map_slots, uint32_t* sched_counter, const int64_t* row_dest,
+          const int32_t* a_rows, const __nv_bfloat16* a_src,
+          const int64_t a_src_rows, const float* row_scale, const int reduce_add,
+          const int64_t dest_lo, const int64_t dest_hi, const __nv_bfloat16* gate_grad,
+          const PushArgs& push, const InlineSizes& inline_sizes,
+          const int block, const int blocks) {
   static_assert(!SWIGLU || MODE != kTN, "the gated product is a forward product");
   static_assert(!PUSH || (!GATHER && !SWIGLU && MODE != kTN), "push warps exist in the plain forward / dgrad kernels");
   // SWIGLU: two right operands of n columns each, b (gate) and b2 (up).  The
@@ -542,7 +544,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     const int64_t row_vecs = (p.n >> 1) / 8;
     const int64_t first = tail->row_start[p.z];
     const int64_t vecs = (p.tokens - first) * row_vecs;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < 2 * vecs; i += int64_t(gridDim.x) * blockDim.x) {
+    for (int64_t i = int64_t(block) * blockDim.x + threadIdx.x; i < 2 * vecs; i += int64_t(blocks) * blockDim.x) {
       const bool second = i >= vecs;
       uint4* rest = reinterpret_cast<uint4*>(c) + (first + (second ? p.tokens : 0)) * row_vecs;
       rest[second ? i - vecs : i] = make_uint4(0u, 0u, 0u, 0u);
@@ -554,8 +556,8 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
   constexpr uint32_t kIdesc =
       ptx::make_idesc_bf16(kBlockM * CTAS, kBlockN, kAMn ? 1 : 0, kBMn ? 1 : 0);
 
-  const int first_tile = kPair ? (blockIdx.x >> 1) : blockIdx.x;
-  const int tile_stride = kPair ? (gridDim.x >> 1) : gridDim.x;
+  const int first_tile = kPair ? (block >> 1) : block;
+  const int tile_stride = kPair ? (blocks >> 1) : blocks;
   // The ring.  A launch of few tiles is bound by the latency of its loads, one of narrow outputs by
   // their bytes: stages in flight count (one expert of 5788 rows, 792 x 2224, wgrad: 62 us
   // with three stages, 38 with four).
@@ -1067,17 +1069,17 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         const uint32_t stage = ptx::smem_u32(reinterpret_cast<uint8_t*>(tail) + kPushStageOffset);
         const int64_t row_bytes = push.row_vecs * 16;
         const int64_t chunks_per_row = (row_bytes + kPushChunkBytes - 1) / kPushChunkBytes;
-        const int64_t my_items = (push.n_items > blockIdx.x) ? (push.n_items - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+        const int64_t my_items = (push.n_items > block) ? (push.n_items - block + blocks - 1) / blocks : 0;
         const int64_t total = my_items * chunks_per_row;
         const uint64_t t0 = ptx::globaltimer_ns();
-        // chunk q of this block's sequence: item blockIdx.x + (q / chunks_per_row) * gridDim.x, piece q % chunks_per_row
+        // chunk q of this block's sequence: item block + (q / chunks_per_row) * blocks, piece q % chunks_per_row
         auto issue_load = [&](int64_t q) {
           const int64_t it = q / chunks_per_row, piece = q - it * chunks_per_row;
           if (piece == 0 && push.interval_ns > 0) {
             const uint64_t due = t0 + static_cast<uint64_t>(it) * static_cast<uint64_t>(push.interval_ns) / kPushWarps;  // this thread has four warps' shares
             while (ptx::globaltimer_ns() < due) __nanosleep(500);   // bounded: the pacing as a whole stays inside the wait limit
           }
-          const int64_t item = blockIdx.x + it * int64_t(gridDim.x);
+          const int64_t item = block + it * int64_t(blocks);
           const int64_t sr = (push.src_row != nullptr) ? push.src_row[item] : item;
           const int64_t off = piece * kPushChunkBytes;
           const uint32_t bytes = static_cast<uint32_t>(row_bytes - off < kPushChunkBytes ? row_bytes - off : kPushChunkBytes);
@@ -1100,7 +1102,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
           const uint32_t ph = static_cast<uint32_t>((q / kPushChunks) & 1);
           if (!ptx::mbar_wait(ptx::smem_u32(&tail->push_full[b]), ph, wait)) { ok = false; break; }
           const int64_t it = q / chunks_per_row, piece = q - it * chunks_per_row;
-          const int64_t item = blockIdx.x + it * int64_t(gridDim.x);
+          const int64_t item = block + it * int64_t(blocks);
           const int64_t off = piece * kPushChunkBytes;
           const uint32_t bytes = static_cast<uint32_t>(row_bytes - off < kPushChunkBytes ? row_bytes - off : kPushChunkBytes);
           uint8_t* dst = static_cast<uint8_t*>(push.peer_base[push.dst_rank[item]]) + push.dst_row[item] * row_bytes + off;
@@ -1110,8 +1112,8 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
         ptx::bulk_wait_group_all();
       }
     } else {
-    const int64_t first = int64_t(blockIdx.x) * kPushWarps + (warp - (kSchedWarp + 1));
-    const int64_t step = int64_t(gridDim.x) * kPushWarps;
+    const int64_t first = int64_t(block) * kPushWarps + (warp - (kSchedWarp + 1));
+    const int64_t step = int64_t(blocks) * kPushWarps;
     const uint64_t t0 = ptx::globaltimer_ns();
     uint64_t due = t0;
     for (int64_t item = first; item < push.n_items; item += step) {
@@ -1854,6 +1856,48 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
     if (kPair) ptx::tmem_dealloc_pair(tmem_base, kTmemCols);
     else ptx::tmem_dealloc(tmem_base, kTmemCols);
   }
+}
+
+template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false>
+__global__ void __launch_bounds__(GATHER ? GatherWarps<CTAS>::kBlockThreads : (PUSH ? kGemmPushThreads : kThreads), 1)
+gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+           const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_c,
+           const __grid_constant__ CUtensorMap map_a2, __nv_bfloat16* __restrict__ c,
+           const int64_t* batch_sizes, const Problem p,
+           uint32_t* status, CUtensorMap* map_slots, uint32_t* sched_counter, const int64_t* row_dest,
+           const int32_t* a_rows, const __nv_bfloat16* a_src,
+           const int64_t a_src_rows, const float* row_scale, const int reduce_add,
+           const int64_t dest_lo, const int64_t dest_hi, const __nv_bfloat16* gate_grad,
+           const PushArgs push, const __grid_constant__ InlineSizes inline_sizes) {
+  gmm_block<MODE, CTAS, GATHER, SWIGLU, PUSH>(
+      map_a, map_b, map_b2, map_c, map_a2, c, batch_sizes, p, status, map_slots, sched_counter,
+      row_dest, a_rows, a_src, a_src_rows, row_scale, reduce_add, dest_lo, dest_hi, gate_grad, push, inline_sizes,
+      blockIdx.x, gridDim.x);
+}
+
+// Both gradients of a small product in one launch: blocks 0 .. d.blocks - 1 are the input gradient's, the
+// rest the weight gradient's.  Each has one tile at most (Problem::single_wave), so that the
+// two lie side by side on the SMs instead of one after the other, and the host, which bounds
+// such a training step, prepares and launches one kernel less.
+struct ProductArgs {
+  CUtensorMap map_a, map_b, map_c;
+  __nv_bfloat16* c;
+  Problem p;
+  int blocks;
+};
+template <int MODE>
+__global__ void __launch_bounds__(kThreads, 1)
+gmm_gradients_kernel(const __grid_constant__ ProductArgs d, const __grid_constant__ ProductArgs w, const int64_t* batch_sizes,
+                     uint32_t* status, CUtensorMap* map_slots, const __grid_constant__ InlineSizes inline_sizes) {
+  const int block = blockIdx.x;
+  if (block < d.blocks)
+    gmm_block<MODE, 1, false, false, false>(d.map_a, d.map_b, d.map_b, d.map_c, d.map_a, d.c, batch_sizes, d.p, status, map_slots,
+                                            nullptr, nullptr, nullptr, nullptr, 0, nullptr, 0, 0, 0, nullptr, PushArgs{}, inline_sizes,
+                                            block, d.blocks);
+  else
+    gmm_block<kTN, 1, false, false, false>(w.map_a, w.map_b, w.map_b, w.map_c, w.map_a, w.c, batch_sizes, w.p, status, map_slots,
+                                           nullptr, nullptr, nullptr, nullptr, 0, nullptr, 0, 0, 0, nullptr, PushArgs{}, inline_sizes,
+                                           block - d.blocks, w.blocks);
 }
 
 // Zeroes the tile counter for the launch that follows.  A memset between two kernels

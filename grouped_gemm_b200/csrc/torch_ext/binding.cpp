@@ -31,7 +31,9 @@ at::Tensor status_word(const c10::Device& device) {
   return it->second;
 }
 
-void gmm(at::Tensor a, at::Tensor b, at::Tensor c, at::Tensor batch_sizes, bool trans_a, bool trans_b) {
+// Checks a product's arguments and returns the columns of its result.
+int64_t check_product(const at::Tensor& a, const at::Tensor& b, const at::Tensor& c, const at::Tensor& batch_sizes, bool trans_a,
+                      bool trans_b) {
   // Same checks, in the same order, as csrc/grouped_gemm.cu:476-540.
   TORCH_CHECK(!(trans_a && trans_b), "only one of trans_a / trans_b may be set");
   TORCH_CHECK(batch_sizes.is_cuda() || batch_sizes.is_cpu(), "batch_sizes must be a CPU or CUDA tensor");
@@ -68,32 +70,61 @@ void gmm(at::Tensor a, at::Tensor b, at::Tensor c, at::Tensor batch_sizes, bool 
   if (batch_sizes.is_cuda()) {
     TORCH_CHECK(batch_sizes.device() == a.device(), "batch_sizes must be on a's device or on the CPU");
     TORCH_CHECK(batch_sizes.is_contiguous(), "batch_sizes must be contiguous");
-  } else {
-    batch_sizes = batch_sizes.contiguous();
-    // The library reads host batch sizes in pageable memory before the call returns (as
-    // an argument of the launch, or staged by an asynchronous copy).  Pinned memory it
-    // reads later, on the stream, when the caller may already have changed or freed it.
-    // Take a pageable copy.
-    if (batch_sizes.is_pinned()) batch_sizes = batch_sizes.clone();
   }
   TORCH_CHECK(z <= B200GMM_MAX_EXPERTS, b200gmm_strerror(B200GMM_ELIMIT));
+  return n;
+}
 
+// batch_sizes as the library wants it.  It reads host batch sizes in pageable memory before the
+// call returns (as an argument of the launch, or staged by an asynchronous copy).  Pinned
+// memory it reads later, on the stream, when the caller may already have changed or freed
+// it: take a pageable copy.
+at::Tensor readable_sizes(const at::Tensor& batch_sizes) {
+  if (batch_sizes.is_cuda()) return batch_sizes;
+  at::Tensor sizes = batch_sizes.contiguous();
+  return sizes.is_pinned() ? sizes.clone() : sizes;
+}
+
+at::Tensor workspace(const at::Tensor& a, int64_t z, size_t* bytes) {
   // Integers go into the messages below as std::to_string(...): streaming an int
   // into a TORCH_CHECK message has been seen to crash inside the iostream number
   // facets when libstdc++ versions are mixed; strings are always fine.
+  const int rc = b200gmm_workspace_bytes(static_cast<int>(z), bytes);
+  TORCH_CHECK(rc == 0, "b200gmm_workspace_bytes: ", b200gmm_strerror(rc), " (code ", std::to_string(rc), ")");
+  return at::empty({static_cast<int64_t>(*bytes)}, at::TensorOptions().dtype(at::kByte).device(a.device()));
+}
+
+void gmm(at::Tensor a, at::Tensor b, at::Tensor c, at::Tensor batch_sizes, bool trans_a, bool trans_b) {
+  const int64_t n = check_product(a, b, c, batch_sizes, trans_a, trans_b), z = batch_sizes.size(0);
+  batch_sizes = readable_sizes(batch_sizes);
   c10::cuda::CUDAGuard guard(a.device());
   size_t ws_bytes = 0;
-  int rc = b200gmm_workspace_bytes(static_cast<int>(z), &ws_bytes);
-  TORCH_CHECK(rc == 0, "b200gmm_workspace_bytes: ", b200gmm_strerror(rc), " (code ", std::to_string(rc), ")");
-  at::Tensor ws = at::empty({static_cast<int64_t>(ws_bytes)},
-                            at::TensorOptions().dtype(at::kByte).device(a.device()));
+  at::Tensor ws = workspace(a, z, &ws_bytes);
   at::Tensor status = status_word(a.device());
-  rc = b200gmm_run(a.data_ptr(), b.data_ptr(), c.data_ptr(), batch_sizes.data_ptr<int64_t>(),
-                   batch_sizes.is_cuda() ? 1 : 0, static_cast<int>(z), a.size(0), a.size(1), n,
-                   trans_a ? 1 : 0, trans_b ? 1 : 0, ws.data_ptr(), ws_bytes,
-                   reinterpret_cast<uint32_t*>(status.data_ptr<int>()),
-                   at::cuda::getCurrentCUDAStream(a.device().index()).stream());
+  const int rc = b200gmm_run(a.data_ptr(), b.data_ptr(), c.data_ptr(), batch_sizes.data_ptr<int64_t>(),
+                             batch_sizes.is_cuda() ? 1 : 0, static_cast<int>(z), a.size(0), a.size(1), n, trans_a ? 1 : 0,
+                             trans_b ? 1 : 0, ws.data_ptr(), ws_bytes, reinterpret_cast<uint32_t*>(status.data_ptr<int>()),
+                             at::cuda::getCurrentCUDAStream(a.device().index()).stream());
   TORCH_CHECK(rc == 0, "b200gmm_run: ", b200gmm_strerror(rc), " (code ", std::to_string(rc), ")");
+}
+
+// Both gradients of gmm(a, b, .., false, trans_b), given that of its result.
+void gmm_gradients(const at::Tensor& a, const at::Tensor& b, const at::Tensor& grad, const at::Tensor& a_grad,
+                   const at::Tensor& b_grad, const at::Tensor& batch_sizes, bool trans_b) {
+  check_product(grad, b, a_grad, batch_sizes, false, !trans_b);
+  check_product(trans_b ? grad : a, trans_b ? a : grad, b_grad, batch_sizes, true, false);
+  const at::Tensor sizes = readable_sizes(batch_sizes);
+  const int64_t z = sizes.size(0);
+  c10::cuda::CUDAGuard guard(a.device());
+  size_t ws_bytes = 0;
+  at::Tensor ws = workspace(a, z, &ws_bytes);
+  at::Tensor status = status_word(a.device());
+  const int rc = b200gmm_run_gradients(a.data_ptr(), b.data_ptr(), grad.data_ptr(), a_grad.data_ptr(), b_grad.data_ptr(),
+                                       sizes.data_ptr<int64_t>(), sizes.is_cuda() ? 1 : 0, static_cast<int>(z), a.size(0),
+                                       a.size(1), grad.size(1), trans_b ? 1 : 0, ws.data_ptr(), ws_bytes,
+                                       reinterpret_cast<uint32_t*>(status.data_ptr<int>()),
+                                       at::cuda::getCurrentCUDAStream(a.device().index()).stream());
+  TORCH_CHECK(rc == 0, "b200gmm_run_gradients: ", b200gmm_strerror(rc), " (code ", std::to_string(rc), ")");
 }
 
 // The reference's GroupedGemm (grouped_gemm/ops.py:8-29) as a native autograd function.
@@ -120,16 +151,13 @@ struct GmmFunction : public torch::autograd::Function<GmmFunction> {
     at::Tensor agrad, bgrad;
     if (want_a || want_b) {
       const at::Tensor grad = grads[0].contiguous();
-      if (want_a) {  // the other orientation of b (ops.py:19-22)
-        agrad = at::empty({grad.size(0), b.size(trans_b ? 2 : 1)}, grad.options());
-        gmm(grad, b, agrad, batch_sizes, false, !trans_b);
-      }
-      if (want_b) {  // in b's own layout (ops.py:24-28)
-        const at::Tensor& lhs = trans_b ? grad : a;
-        const at::Tensor& rhs = trans_b ? a : grad;
-        bgrad = at::empty({batch_sizes.size(0), lhs.size(1), rhs.size(1)}, lhs.options());
-        gmm(lhs, rhs, bgrad, batch_sizes, true, false);
-      }
+      const at::Tensor& lhs = trans_b ? grad : a;
+      const at::Tensor& rhs = trans_b ? a : grad;
+      if (want_a) agrad = at::empty({grad.size(0), b.size(trans_b ? 2 : 1)}, grad.options());
+      if (want_b) bgrad = at::empty({batch_sizes.size(0), lhs.size(1), rhs.size(1)}, lhs.options());
+      if (want_a && want_b) gmm_gradients(a, b, grad, agrad, bgrad, batch_sizes, trans_b);
+      else if (want_a) gmm(grad, b, agrad, batch_sizes, false, !trans_b);  // the other orientation of b (ops.py:19-22)
+      else gmm(lhs, rhs, bgrad, batch_sizes, true, false);                 // in b's own layout (ops.py:24-28)
     }
     return {agrad, bgrad, at::Tensor(), at::Tensor()};
   }
