@@ -316,8 +316,9 @@ struct Features {
 //     cap adds to it (17 experts of 1548 rows, dgrad 7344 -> 520: 1.67, 309 / 248).
 // Many experts (128 and more) are hardly ever of even size, and swapped tiles take the
 // small ones: z = 256, 256 rows, 7168 x 2048, Zipf routing: ratio 1.67, 2383 / 2244 us, dgrad
-// 2322 / 2152 (even sizes: 3 % slower).  The gathered product has no swapped tiles: from 256 rows on
-// (146 experts of 126 rows, 6712 x 2496: 1185 / 1487).
+// 2322 / 2152 (even sizes: 3 % slower).  The gathered product has no swapped tiles, and its row
+// copies are 16 bytes in any case: from 512 rows on (146 experts of 126 rows, 6712 x 2496: 1185 / 1487; 16 of
+// 386, 1416 x 11392: 258 / 279).
 // A short contraction leaves an accumulator little time to be read out while the other one
 // fills, which a pair's tile does not have: one CTA below 416 (any 16 bytes) and 512 (49 experts, 98681
 // rows, 72 x 2000: 159 / 101 us; 173, 110139, 128 x 856: 113 / 77; 81, 68558, 432 x 2608: 240 / 223),
@@ -346,9 +347,9 @@ int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int t
   const int64_t rounds_pair = nt == 1 ? 2 * ((pair + kPairs - 1) / kPairs)
                                       : 3 * (pair / kPairs) + (left == 0 ? 0 : (2 * left <= kPairs ? 2 : 3));
   const double ratio = double(rounds_one) / double(std::max<int64_t>(rounds_pair, 1));
-  if (trans_a) return rows_from(ragged ? 384 : 512) && d1 >= 256 && ratio >= 1.5 ? 2 : 1;
+  if (trans_a) return rows_from(ragged && !f.gather ? 384 : 512) && d1 >= 256 && ratio >= 1.5 ? 2 : 1;
   if (d1 < (ragged ? 416 : 512) || (one <= kSms && !rows_from(384))) return 1;
-  if (!rows_from(f.gather || f.gated_backward ? 256 : (d1 < 2048 ? 128 : 64))) return 1;
+  if (!rows_from(f.gather ? 512 : f.gated_backward ? 256 : (d1 < 2048 ? 128 : 64))) return 1;
   if (f.scatter && d1 < 8192) return rows_from(512) ? 2 : 1;
   if (nt == 1) return ratio >= 1.25 && (ragged || rows_from(512)) ? 2 : 1;
   if (ragged) return ratio >= 1.25 ? 2 : 1;

@@ -1027,8 +1027,11 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
               ptx::tensormap_set_dim1(ea, rows_end);
               ptx::tensormap_set_dim1(eb, rows_end);
               ptx::fence_tensormap_release();
-              if (kPair) {
-                entry = kMapFresh;  // each producer acquires it for its own SM
+              if (kPair || p.mt * p.nt < tile_stride) {
+                // Each producer of a pair acquires it for its own SM.  So does the producer of
+                // a CTA whose every tile is of another expert: the fences would make this
+                // thread the slower one of the two (172 experts, 2552 x 120: 59.6 / 64.7 us).
+                entry = kMapFresh;
               } else {
                 // The copy is acquired and fetched here, tiles ahead of its use, and handed over with
                 // the tile: in the producer the fence and the first use of a descriptor that no cache
