@@ -466,8 +466,8 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
   // (map_a2: the activations with 32-row boxes; NT also uses map_b2: b with
   // 128-row boxes).
   constexpr bool kLight = (MODE != kTN) && (CTAS == 1) && !GATHER && !SWIGLU;
-  // So do swapped tiles (schedule.cuh), and in the gated product's.  A sum of two products
-  // over one accumulator (Problem::pair_sum) is an option of the plain kernels.
+  // Swapped tiles (schedule.cuh) exist in all forward / dgrad kernels but the gathered ones.  A sum
+  // of two products over one accumulator (Problem::pair_sum) is an option of the plain kernels.
   constexpr bool kSwap = (MODE != kTN) && !GATHER;
   constexpr bool kPairSum = (MODE != kTN) && !GATHER && !SWIGLU && !PUSH;
 
