@@ -316,7 +316,11 @@ __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* 
 // (narrow_tiles); in others what is left over after whole rounds of the grid's
 // `clusters` is taken as halves when the halves fit one round, which then lasts half as
 // long.  A half that does not exist (the last column tile may be one accumulator
-// wide) is a tile of no units.
+// wide) is a tile of no units.  kWide: pairs.  (One-CTA tiles know at compile time that there are no
+// halves: the scheduler decodes before anything else can start, and with the question asked
+// of the Problem launches of one tile a CTA took 0.1 to 0.2 us longer, 6.85 / 7.06 us for the weight
+// gradient of 512 rows in 4 experts of 128 x 128.)
+template <bool kWide>
 struct TileWalker {
   const Problem& p;
   const SmemTail* tail;
@@ -325,7 +329,7 @@ struct TileWalker {
   int pos;
   __device__ TileWalker(const Problem& p_, const SmemTail* tail_, int clusters)
       : p(p_), tail(tail_), whole(tail_->tile_start[p_.z]), total(whole), pos(0) {
-    if (p.tile_n > kBlockN && p.n > kBlockN && clusters > 0) {
+    if (kWide && p.n > kBlockN && clusters > 0) {
       int halves = whole % clusters;
       if (2 * halves > clusters) halves = 0;
       if (narrow_tiles(p, whole, clusters)) halves = whole;
@@ -336,14 +340,14 @@ struct TileWalker {
   __device__ __forceinline__ bool decode(int t, Tile* out) {
     if (t < 0 || t >= total) return false;
     int half = -1;
-    if (t >= whole) {
+    if (kWide && t >= whole) {
       half = (t - whole) & 1;
       t = whole + ((t - whole) >> 1);
     }
     while (t >= tail->tile_start[pos + 1]) ++pos;
     const int e = tail->perm[pos];
     *out = make_tile(p, e, t - tail->tile_start[pos], tail->row_start[e], tail->row_start[e + 1]);
-    if (half >= 0) {
+    if (kWide && half >= 0) {
       out->units = half < out->units ? 1 : 0;
       out->col0 += half * kBlockN;
     }
@@ -975,7 +979,7 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
         __syncwarp();
       }
       if (lane == 0) {
-        TileWalker walk(p, tail, tile_stride);
+        TileWalker<kPair> walk(p, tail, tile_stride);
         TileFeed<kPair> feed(tail, wait, !leader);
         Tile t = {};
         // wgrad: the map slot clipped to the current expert, and for every slot the
@@ -996,7 +1000,7 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
           int entry = 0;
           const bool live = walk.decode(pos, &t);
           if (!live) t.expert = -1;
-          if (live && t.units == 0) {  // a half that does not exist
+          if (kPair && live && t.units == 0) {  // a half that does not exist
             pos = p.single_wave ? walk.total : static_cast<int>(drawn) + tile_stride;
             if (pos < walk.total) drawn = atomicAdd(sched_counter, 1u);
             continue;
@@ -1939,7 +1943,7 @@ schedule_dump_kernel(const int64_t* __restrict__ batch_sizes, const Problem p, i
   build_schedule(p, batch_sizes, InlineSizes{}, &tail, status);
   __syncthreads();
   if (threadIdx.x == 0) {
-    TileWalker walk(p, &tail, 0);
+    TileWalker<true> walk(p, &tail, 0);
     Tile t;
     int n = 0;
     for (int pos = 0; walk.decode(pos, &t); ++pos) {

@@ -131,8 +131,8 @@ B200GMM_HD int tile_stages(const Tile& t) {
 // Returns the rounded row count, 0 for a plain tile.
 B200GMM_HD int swapped_rows(const Problem& p, const Tile& t) {
   if (p.swap_rows == 0 || t.kind != 0 || t.units < p.swap_units) return 0;
-  const int step = p.tile_m == kBlockM ? 16 : 32;
-  const int rows = (t.valid_rows + step - 1) / step * step;
+  const int step = p.tile_m == kBlockM ? 16 : 32;  // (a power of two: no division before every tile)
+  const int rows = (t.valid_rows + step - 1) & ~(step - 1);
   return rows <= p.swap_rows ? rows : 0;
 }
 
