@@ -10,10 +10,11 @@
 //               so the epilogue of tile i overlaps the main loop of tile i+1;
 //   warps 2-9   epilogue: each warp owns 32 rows x 128 columns of an accumulator (TMEM
 //               lane quadrant = warp % 4, column half = (warp - 2) / 4).  It
-//               tcgen05.ld's 32 columns at a time, rounds to bf16, and hands the
-//               accumulator back once all are in registers; then it stages each 32x32
+//               tcgen05.ld's 32 columns at a time, rounds to bf16, stages each 32x32
 //               chunk in swizzled shared memory and writes it with a TMA tensor
-//               store; a warp whose 32 rows do not all exist (ragged last tile of
+//               store (one CTA: while the next chunk is being loaded; a pair, both of whose
+//               accumulators are one tile: once the accumulator is in registers
+//               and handed back); a warp whose 32 rows do not all exist (ragged last tile of
 //               an expert) stores its valid rows directly;
 //   warp 10     scheduler (leader CTA): draws tile positions from a global counter,
 //               several tiles ahead of the other roles, works out the tile of each and
@@ -1448,11 +1449,10 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
       }
     };
 
-    // Swapped tile: 32 rows x 32 columns held transposed, f[c][l] = this lane's fragment of rows
-    // 8 c .. 8 c + 7, columns 8 l .. 8 l + 7 (stmatrix_x4_trans turns it).  The values go through
-    // the staging buffer (row i at 64 i) and leave as a TMA store when all 32 rows exist, as
-    // bulk copies of a row when they are scattered, else as 64 bytes of a row by four lanes.
-    auto emit_swapped = [&](const uint32_t (&f)[4][4], int rows, int64_t row, int col, int out_n) {
+    // Swapped tile: 32 rows x 32 columns, held transposed, go through the staging buffer (row i at
+    // 64 i; stage(buf) puts them there) and leave as a TMA store when all 32 rows exist, as
+    // bulk copies of a row when they are scattered, else row by row.
+    auto emit_swapped = [&](auto stage, int rows, int64_t row, int col, int out_n) {
       const uint32_t buf = scatter_rows ? my_out : stage_buf();
       if (scatter_rows) {
         if (stores > 0) ptx::bulk_wait_group_read<0>();  // this lane's previous copy
@@ -1460,13 +1460,7 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
         ptx::bulk_wait_group_read<G::kOutBufs - 1>();
       }
       __syncwarp();
-      // this lane gives the address of row 8 c + lane % 8, columns 8 (lane / 8) and on: 64-byte
-      // swizzle as in emit(); a scattered row is read linearly by its copy
-      const uint32_t piece = uint32_t(lane) >> 3;
-      const uint32_t sw = scatter_rows ? piece : (piece ^ ((uint32_t(lane) >> 1) & 3u));
-      const uint32_t at = buf + (uint32_t(lane) & 7u) * 64u + (sw << 4);
-#pragma unroll
-      for (int c4 = 0; c4 < 4; ++c4) ptx::stmatrix_x4_trans(at + uint32_t(c4) * 512u, f[c4][0], f[c4][1], f[c4][2], f[c4][3]);
+      stage(buf);
       if (scatter_rows) {
         ptx::fence_proxy_async_smem();
         __syncwarp();
@@ -1495,16 +1489,19 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
         ++stores;
       } else {
         __syncwarp();
-        const int cj = (lane & 3) * 8;
+        // a pair: eight rows at a time by four lanes each; one CTA, whose tiles may have a row or
+        // two: lane i sends row i
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int r = i * 8 + (lane >> 2);
+          const int r = kPair ? i * 8 + (lane >> 2) : lane;
+          const int piece = kPair ? (lane & 3) : i;
+          if (r >= rows) continue;
           uint4 o;
           asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                        : "=r"(o.x), "=r"(o.y), "=r"(o.z), "=r"(o.w)
-                       : "r"(buf + uint32_t(r) * 64u + (((uint32_t(lane) & 3u) ^ ((uint32_t(r) >> 1) & 3u)) << 4))
+                       : "r"(buf + uint32_t(r) * 64u + ((uint32_t(piece) ^ ((uint32_t(r) >> 1) & 3u)) << 4))
                        : "memory");
-          if (r < rows && col + cj < out_n) *reinterpret_cast<uint4*>(c + (row + r) * out_n + col + cj) = o;
+          if (col + piece * 8 < out_n) *reinterpret_cast<uint4*>(c + (row + r) * out_n + col + piece * 8) = o;
         }
         __syncwarp();
       }
@@ -1524,6 +1521,13 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
         constexpr bool kShared = kPair || SWIGLU;
         const int out_n = static_cast<int>(SWIGLU ? (p.n >> 1) : p.n);
         const int r_first = kShared ? half * 32 : 0, r_step = kShared ? 64 : 32;
+        auto gated = [](uint32_t g_bits, uint32_t u_bits) {  // silu(g) * u
+          const float g = __uint_as_float(g_bits);
+          return __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * __uint_as_float(u_bits));
+        };
+        // 16-byte piece of a row in the staging buffer: 64-byte swizzle as in emit(); a scattered
+        // row is read linearly by its copy
+        auto swizzled = [&](uint32_t piece, uint32_t r) { return (scatter_rows ? piece : (piece ^ ((r >> 1) & 3u))) << 4; };
 #pragma unroll 1
         for (int unit = 0; unit < (kPair && !SWIGLU ? t.units : 1); ++unit) {
           const uint32_t ab = it & 1u, ab2 = kPair ? (it + 1u) & 1u : ab;  // (ab2: up columns)
@@ -1538,9 +1542,7 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
           const uint32_t ta = tmem_base + lane_base + ab * kBlockN + (kShared ? 0 : col_base);
           const uint32_t tb = tmem_base + lane_base + ab2 * kBlockN + (kPair ? 0 : kBlockN / 2);
           const bool live = col < out_n;
-          bool held = true;  // the accumulator(s)
           auto release = [&]() {
-            held = false;
             ptx::tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) {
@@ -1550,39 +1552,82 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
               if (kPair && SWIGLU) ptx::mbar_arrive_cluster(ptx::mapa(ptx::smem_u32(&tail->tmem_empty[ab2]), 0));
             }
           };
-#pragma unroll 1
-          for (int r0 = r_first; live && r0 < t.valid_rows; r0 += r_step) {
-            uint32_t f[4][4];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {  // 16 lanes at a time: columns 16 h .. 16 h + 15 of the chunk
-              uint32_t va[16], vb[16];
-              ptx::tmem_ld_16x32_frag(ta + uint32_t(r0) + (uint32_t(h * 16) << 16), va);
-              if (SWIGLU) ptx::tmem_ld_16x32_frag(tb + uint32_t(r0) + (uint32_t(h * 16) << 16), vb);
+          if constexpr (!kPair) {
+            // This lane holds a column of 32 rows: 32 two-byte stores, a warp's to one row 64
+            // consecutive bytes.  (The fragment form below took longer where a tile has few rows and the
+            // epilogue counts, 64 experts of 8 rows, k = 64, n = 4096: scattered 19.5 / 21.5 us, gated
+            // 23.1 / 25.3, and its code cost every small launch 0.1 us.)
+            for (int r0 = r_first; live && r0 < t.valid_rows; r0 += r_step) {
+              uint32_t va[32], vb[32];
+              ptx::tmem_ld_32x32(ta + uint32_t(r0), va);
+              if (SWIGLU) ptx::tmem_ld_32x32(tb + uint32_t(r0), vb);
               ptx::tmem_ld_wait();
-              if (h == 1 && r0 + r_step >= t.valid_rows) release();
               if (SWIGLU) {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                  const float g = __uint_as_float(va[i]);
-                  va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * __uint_as_float(vb[i]));
-                }
+                for (int i = 0; i < 32; ++i) va[i] = gated(va[i], vb[i]);
               }
               if (scatter_rows && row_scale != nullptr) {
                 const float w = r0 + lane < t.valid_rows ? row_scale[int64_t(t.row0) + r0 + lane] : 1.0f;
 #pragma unroll
-                for (int i = 0; i < 16; ++i)  // value i: row 8 (i / 4) + 2 (lane % 4) + i % 2
-                  va[i] = __float_as_uint(__uint_as_float(va[i]) *
-                                          __shfl_sync(0xffffffffu, w, (i >> 2) * 8 + (lane & 3) * 2 + (i & 1)));
+                for (int i = 0; i < 32; ++i)
+                  va[i] = __float_as_uint(__uint_as_float(va[i]) * __shfl_sync(0xffffffffu, w, i));
               }
+              auto stage = [&](uint32_t buf) {
+                const uint32_t at = buf + (uint32_t(lane) & 7u) * 2u;
 #pragma unroll
-              for (int i = 0; i < 16; i += 2) {
-                __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(va[i]), __uint_as_float(va[i + 1]));
-                f[i >> 2][h * 2 + ((i >> 1) & 1)] = *reinterpret_cast<uint32_t*>(&v);
-              }
+                for (int i = 0; i < 32; ++i) {
+                  const __nv_bfloat16 h = __float2bfloat16_rn(__uint_as_float(va[i]));
+                  asm volatile("st.shared.b16 [%0], %1;" ::"r"(at + uint32_t(i) * 64u + swizzled(uint32_t(lane) >> 3, i)),
+                               "h"(__bfloat16_as_ushort(h))
+                               : "memory");
+                }
+              };
+              emit_swapped(stage, t.valid_rows - r0, int64_t(t.row0) + r0, col, out_n);
             }
-            emit_swapped(f, t.valid_rows - r0, int64_t(t.row0) + r0, col, out_n);
+            release();
+          } else {
+            bool held = true;  // the accumulator(s)
+#pragma unroll 1
+            for (int r0 = r_first; live && r0 < t.valid_rows; r0 += r_step) {
+              uint32_t f[4][4];  // f[c][l]: this lane's fragment of rows 8 c .. 8 c + 7, columns 8 l .. 8 l + 7
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {  // 16 lanes at a time: columns 16 h .. 16 h + 15 of the chunk
+                uint32_t va[16], vb[16];
+                ptx::tmem_ld_16x32_frag(ta + uint32_t(r0) + (uint32_t(h * 16) << 16), va);
+                if (SWIGLU) ptx::tmem_ld_16x32_frag(tb + uint32_t(r0) + (uint32_t(h * 16) << 16), vb);
+                ptx::tmem_ld_wait();
+                if (h == 1 && r0 + r_step >= t.valid_rows) {
+                  release();
+                  held = false;
+                }
+                if (SWIGLU) {
+#pragma unroll
+                  for (int i = 0; i < 16; ++i) va[i] = gated(va[i], vb[i]);
+                }
+                if (scatter_rows && row_scale != nullptr) {
+                  const float w = r0 + lane < t.valid_rows ? row_scale[int64_t(t.row0) + r0 + lane] : 1.0f;
+#pragma unroll
+                  for (int i = 0; i < 16; ++i)  // value i: row 8 (i / 4) + 2 (lane % 4) + i % 2
+                    va[i] = __float_as_uint(__uint_as_float(va[i]) *
+                                            __shfl_sync(0xffffffffu, w, (i >> 2) * 8 + (lane & 3) * 2 + (i & 1)));
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) {
+                  __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(va[i]), __uint_as_float(va[i + 1]));
+                  f[i >> 2][h * 2 + ((i >> 1) & 1)] = *reinterpret_cast<uint32_t*>(&v);
+                }
+              }
+              // (a lane gives the address of row 8 c + lane % 8, columns 8 (lane / 8) and on)
+              auto stage = [&](uint32_t buf) {
+                const uint32_t at = buf + (uint32_t(lane) & 7u) * 64u + swizzled(uint32_t(lane) >> 3, lane & 7);
+#pragma unroll
+                for (int c4 = 0; c4 < 4; ++c4)
+                  ptx::stmatrix_x4_trans(at + uint32_t(c4) * 512u, f[c4][0], f[c4][1], f[c4][2], f[c4][3]);
+              };
+              emit_swapped(stage, t.valid_rows - r0, int64_t(t.row0) + r0, col, out_n);
+            }
+            if (held) release();
           }
-          if (held) release();
         }
         continue;
       }
@@ -1700,19 +1745,24 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
           emit(zeros, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
         continue;
       }
-      // Gated backward: a chunk (a pair: both) of this lane's values of the output gradient.  (A pair reads both
-      // before it waits for the accumulator, which is then held for less time.)
-      constexpr int kGradChunks = kPair ? 2 : 1;
-      uint4 d4[4 * kGradChunks] = {};
-      auto load_grad = [&](int first) {
-        if (gate_grad == nullptr || !row_ok) return;
-        const int col = half * 64 + first * 32;
+      // Gated backward: 32 columns of this lane's row of the output gradient.
+      auto load_grad = [&](uint4 (&d4)[4], int col) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d4[j] = make_uint4(0u, 0u, 0u, 0u);
+        if (!row_ok) return;
         const uint4* src = reinterpret_cast<const uint4*>(gate_grad + (out_row0 + r) * out_n + out_col0 + col);
 #pragma unroll
-        for (int j = 0; j < 4 * kGradChunks; ++j)
+        for (int j = 0; j < 4; ++j)
           if (col + j * 8 < cols_left) d4[j] = src[j];
       };
-      if (SWIGLU && kPair) load_grad(0);
+      const bool backward = SWIGLU && gate_grad != nullptr;
+      // (a pair reads both chunks of it before it waits for the accumulator, which is then held for
+      // less time)
+      uint4 d4[kPair ? 2 : 1][4];
+      if (kPair && backward) {
+        load_grad(d4[0], half * 64);
+        load_grad(d4[kPair ? 1 : 0], half * 64 + 32);
+      }
       const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
       ++it;
       if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), aph, wait)) { ok = false; break; }
@@ -1732,99 +1782,148 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
         // This warp's 64 of the tile's 128 output columns: gate from accumulator
         // columns [64 half, +64), up from the same columns of the second half.
         const uint32_t tg = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + half * 64;
-        uint4 o[8 * kGradChunks];  // per chunk: the result, or both gradients
-        auto emit_chunk = [&](int ch) {
-          const int col = half * 64 + ch * 32;
-          const uint4* oc = o + (kPair ? ch * 8 : 0);
-          emit(oc, col, warp_full, row_ok, crow, cols_left, tile_row, out_col0);
-          if (gate_grad != nullptr)
-            emit(oc + 4, col, warp_full, row_ok, crow + p.tokens * out_n, cols_left,
-                 tile_row + static_cast<int>(p.tokens), out_col0);
+        // silu(g) * u of 32 columns, to va
+        auto gated = [&]() {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float g = __uint_as_float(va[i]);
+            const float u = __uint_as_float(vb[i]);
+            va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * u);
+          }
+          if (scaled) scale(va);
         };
-#pragma unroll(kPair ? 2 : 1)
-        for (int ch = 0; ch < 2; ++ch) {
+        // Backward of the gated product: with g, u recomputed in the accumulator and dh the output
+        // gradient, the gradients w.r.t. the two products
+        //   dg = dh * u * silu'(g),  silu'(g) = s (1 + g (1 - s)),  s = 1 / (1 + exp(-g))
+        //   du = dh * silu(g)
+        // (to va and vb) go to rows [0, T) and [T, 2T) of the output.
+        auto gradients = [&](const uint4 (&dh4)[4]) {
+          const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(dh4);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const float g = __uint_as_float(va[i]);
+            const float u = __uint_as_float(vb[i]);
+            const float2 dpair = __bfloat1622float2(d2[i >> 1]);
+            const float dh = (i & 1) ? dpair.y : dpair.x;
+            const float sg = __fdividef(1.0f, 1.0f + __expf(-g));
+            va[i] = __float_as_uint(dh * u * sg * (1.0f + g * (1.0f - sg)));
+            vb[i] = __float_as_uint(dh * g * sg);
+          }
+        };
+        auto emit_gate = [&](const uint4* o, int ch) {
+          emit(o, half * 64 + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, out_col0);
+        };
+        auto emit_up = [&](const uint4* o, int ch) {
+          emit(o, half * 64 + ch * 32, warp_full, row_ok, crow + p.tokens * out_n, cols_left,
+               tile_row + static_cast<int>(p.tokens), out_col0);
+        };
+        auto load = [&](int ch) {
           ptx::tmem_ld_32x32(tg + ch * 32, va);
           ptx::tmem_ld_32x32(tg + kBlockN / 2 + ch * 32, vb);
           ptx::tmem_ld_wait();
           if (ch == 1) release();
-          uint4* oc = o + (kPair ? ch * 8 : 0);
-          if (gate_grad != nullptr) {
-            if (!kPair) load_grad(ch);
-            // Backward of the gated product: with g, u recomputed in the accumulator and
-            // dh = gate_grad[row, col ..], the gradients w.r.t. the two products
-            //   dg = dh * u * silu'(g),  silu'(g) = s (1 + g (1 - s)),  s = 1 / (1 + exp(-g))
-            //   du = dh * silu(g)
-            // go to rows [0, T) and [T, 2T) of the output.
-            const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(d4 + (kPair ? ch * 4 : 0));
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const float g = __uint_as_float(va[i]);
-              const float u = __uint_as_float(vb[i]);
-              const float2 dpair = __bfloat1622float2(d2[i >> 1]);
-              const float dh = (i & 1) ? dpair.y : dpair.x;
-              const float sg = __fdividef(1.0f, 1.0f + __expf(-g));
-              va[i] = __float_as_uint(dh * u * sg * (1.0f + g * (1.0f - sg)));
-              vb[i] = __float_as_uint(dh * g * sg);
+        };
+        if constexpr (!kPair) {
+          uint4 o[4];
+#pragma unroll 1
+          for (int ch = 0; ch < 2; ++ch) {
+            load(ch);
+            if (backward) {
+              load_grad(d4[0], half * 64 + ch * 32);
+              gradients(d4[0]);
+              pack(va, o);
+              emit_gate(o, ch);
+              pack(vb, o);
+              emit_up(o, ch);
+            } else {
+              gated();
+              pack(va, o);
+              emit_gate(o, ch);
             }
-            pack(va, oc);
-            pack(vb, oc + 4);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const float g = __uint_as_float(va[i]);
-              const float u = __uint_as_float(vb[i]);
-              va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * u);  // silu(g) * u
-            }
-            if (scaled) scale(va);
-            pack(va, oc);
           }
-          if (!kPair) emit_chunk(ch);
-        }
-        if (kPair) {
-          emit_chunk(0);
-          emit_chunk(1);
+        } else if (backward) {
+          uint4 og[8], ou[8];
+#pragma unroll
+          for (int ch = 0; ch < 2; ++ch) {
+            load(ch);
+            gradients(d4[kPair ? ch : 0]);
+            pack(va, og + ch * 4);
+            pack(vb, ou + ch * 4);
+          }
+#pragma unroll
+          for (int ch = 0; ch < 2; ++ch) {
+            emit_gate(og + ch * 4, ch);
+            emit_up(ou + ch * 4, ch);
+          }
+        } else {
+          uint4 o[8];
+#pragma unroll
+          for (int ch = 0; ch < 2; ++ch) {
+            load(ch);
+            gated();
+            pack(va, o + ch * 4);
+          }
+          emit_gate(o, 0);
+          emit_gate(o + 4, 1);
         }
         continue;
       }
       const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + col_base;
-      uint4 o[kPair ? 16 : 8];
-      auto emit_chunks = [&](int ch) {  // two of 32 columns
-        const int col = col_base + ch * 32;
-        const uint4* oc = o + (kPair ? ch * 4 : 0);
+      if constexpr (!kPair) {
+        // Chunk by chunk, each as soon as it is read, the next one's load in flight meanwhile: the other
+        // accumulator is being filled, and registers for all of this one would gain nothing.
         if (G::kWideOut && warp_full) {
-          if (col < cols_left) emit64(oc, col, tile_row, unit_col0);
-        } else {
-          emit(oc, col, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
-          emit(oc + 4, col + 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
+#pragma unroll 1
+          for (int ch = 0; ch < kBlockN / 64; ch += 2) {
+            ptx::tmem_ld_32x32(taddr + ch * 32, va);
+            ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
+            ptx::tmem_ld_wait();
+            if (ch + 2 == kBlockN / 64) release();
+            uint4 o[8];
+            pack(va, o);
+            pack(vb, o + 4);
+            if (col_base + ch * 32 < cols_left) emit64(o, col_base + ch * 32, tile_row, unit_col0);
+          }
+          continue;
         }
-      };
-#pragma unroll(kPair ? 2 : 1)
-      for (int ch = 0; ch < kBlockN / 64; ch += 2) {
-        uint4* oc = o + (kPair ? ch * 4 : 0);
-        if (GATHER || PUSH) {  // (128 registers)
-          ptx::tmem_ld_32x32(taddr + ch * 32, va);
+        uint4 o[4];
+        ptx::tmem_ld_32x32(taddr, va);
+#pragma unroll 1
+        for (int ch = 0; ch < kBlockN / 64; ch += 2) {
           ptx::tmem_ld_wait();
-          if (scaled) scale(va);
-          pack(va, oc);
-          ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, va);
-          ptx::tmem_ld_wait();
-          if (ch + 2 == kBlockN / 64) release();
-          if (scaled) scale(va);
-          pack(va, oc + 4);
-        } else {
-          ptx::tmem_ld_32x32(taddr + ch * 32, va);
           ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
+          if (scaled) scale(va);
+          pack(va, o);
+          emit(o, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
           ptx::tmem_ld_wait();
-          if (ch + 2 == kBlockN / 64) release();
-          if (scaled) { scale(va); scale(vb); }
-          pack(va, oc);
-          pack(vb, oc + 4);
+          if (ch + 2 < kBlockN / 64) ptx::tmem_ld_32x32(taddr + (ch + 2) * 32, va);
+          else release();
+          if (scaled) scale(vb);
+          pack(vb, o);
+          emit(o, col_base + (ch + 1) * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
         }
-        if (!kPair) emit_chunks(ch);
-      }
-      if (kPair) {
-        emit_chunks(0);
-        emit_chunks(2);
+      } else {
+        // All of the accumulator is read and rounded before it leaves.
+        uint4 o[16];
+#pragma unroll
+        for (int ch = 0; ch < kBlockN / 64; ch += 2) {
+          ptx::tmem_ld_32x32(taddr + ch * 32, va);
+          if (!GATHER && !PUSH) ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);  // (those have 128 registers)
+          ptx::tmem_ld_wait();
+          if (!GATHER && !PUSH && ch + 2 == kBlockN / 64) release();
+          if (scaled) scale(va);
+          pack(va, o + ch * 4);
+          if (GATHER || PUSH) {
+            ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
+            ptx::tmem_ld_wait();
+            if (ch + 2 == kBlockN / 64) release();
+          }
+          if (scaled) scale(vb);
+          pack(vb, o + (ch + 1) * 4);
+        }
+#pragma unroll
+        for (int ch = 0; ch < kBlockN / 64; ++ch)
+          emit(o + ch * 4, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
       }
       }
     }
