@@ -1756,13 +1756,9 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
           if (col + j * 8 < cols_left) d4[j] = src[j];
       };
       const bool backward = SWIGLU && gate_grad != nullptr;
-      // (a pair reads both chunks of it before it waits for the accumulator, which is then held for
-      // less time)
-      uint4 d4[kPair ? 2 : 1][4];
-      if (kPair && backward) {
-        load_grad(d4[0], half * 64);
-        load_grad(d4[kPair ? 1 : 0], half * 64 + 32);
-      }
+      // (a pair reads it a chunk ahead, the first before it waits for the accumulator)
+      uint4 d4[4];
+      if (kPair && backward) load_grad(d4, half * 64);
       const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
       ++it;
       if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), aph, wait)) { ok = false; break; }
@@ -1829,8 +1825,8 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
           for (int ch = 0; ch < 2; ++ch) {
             load(ch);
             if (backward) {
-              load_grad(d4[0], half * 64 + ch * 32);
-              gradients(d4[0]);
+              load_grad(d4, half * 64 + ch * 32);
+              gradients(d4);
               pack(va, o);
               emit_gate(o, ch);
               pack(vb, o);
@@ -1842,19 +1838,22 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
             }
           }
         } else if (backward) {
-          uint4 og[8], ou[8];
-#pragma unroll
-          for (int ch = 0; ch < 2; ++ch) {
-            load(ch);
-            gradients(d4[kPair ? ch : 0]);
-            pack(va, og + ch * 4);
-            pack(vb, ou + ch * 4);
-          }
-#pragma unroll
-          for (int ch = 0; ch < 2; ++ch) {
-            emit_gate(og + ch * 4, ch);
-            emit_up(ou + ch * 4, ch);
-          }
+          // The accumulator is read before the first chunk's results leave; holding the second's too
+          // took more registers than there are (168: 44 bytes of spill stores, 100 of loads).
+          uint4 o[4], o2[4];
+          load(0);
+          gradients(d4);
+          load_grad(d4, half * 64 + 32);
+          pack(va, o);
+          pack(vb, o2);
+          load(1);
+          emit_gate(o, 0);
+          emit_up(o2, 0);
+          gradients(d4);
+          pack(va, o);
+          pack(vb, o2);
+          emit_gate(o, 1);
+          emit_up(o2, 1);
         } else {
           uint4 o[8];
 #pragma unroll
