@@ -360,7 +360,7 @@ struct TileWalker {
 // tile through sched_tile / sched_full, in its own CTA and in its peer; every other
 // role takes them from there and releases the slot on the leader's sched_empty.
 enum Taken { kTile, kEndOfOrder, kAbandoned };  // kAbandoned: a wait gave up
-constexpr int kMapFresh = 1 << 30;  // TileRecord::map flag: the slot was edited for this tile
+constexpr int kMapFresh = 1 << 30;  // TileRecord::map flag: the slot was edited for this tile, and the producer has to acquire it
 
 template <bool kPair>
 struct TileFeed {
@@ -621,8 +621,8 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
         if (MODE == kTN && nkb > 0) {
           // The scheduler clipped a copy of both maps at this expert's last row, so
           // that the rows a k-block would read from the next expert are out of bounds
-          // for TMA and arrive as zeros.  A freshly edited copy has to be acquired by
-          // the thread that loads through it.
+          // for TMA and arrive as zeros.  A freshly edited copy has to be acquired
+          // before a load through it: by the scheduler, or (kMapFresh) here.
           tn_a = my_maps + (feed.map & (kMapSlots - 1)) * 2;
           tn_b = tn_a + 1;
           if (feed.map & kMapFresh) {
@@ -1032,17 +1032,23 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
               ptx::tensormap_set_dim1(ea, rows_end);
               ptx::tensormap_set_dim1(eb, rows_end);
               ptx::fence_tensormap_release();
-              if (kPair || p.mt * p.nt < tile_stride) {
-                // Each producer of a pair acquires it for its own SM.  So does the producer of
-                // a CTA whose every tile is of another expert: the fences would make this
-                // thread the slower one of the two (172 experts, 2552 x 120: 59.6 / 64.7 us).
+              if (kPair || (p.single_wave ? GATHER : p.mt * p.nt < tile_stride)) {
+                // A pair has two producers, one of them on another SM than this thread: each
+                // acquires the copy for itself.  So does the producer of a CTA whose every tile is of
+                // another expert: the fences would make this thread the slower one of the two (214
+                // experts, 5888 x 72: 163 / 174 us; 172, 2552 x 120: 60.2 / 62.9).  A CTA of one tile has
+                // nothing to be ahead of, but two fences fewer between a thread and its first load
+                // (2048 rows, 16 experts, 256 x 512: 9.06 / 8.86; 1005 rows, 6 experts, 248 x 336: 8.45 /
+                // 8.26); not where the producer only loads b and waits for row copies (9.55 / 9.70).
                 entry = kMapFresh;
               } else {
                 // The copy is acquired and fetched here, tiles ahead of its use, and handed over with
                 // the tile: in the producer the fence and the first use of a descriptor that no cache
                 // holds stood before every tile of another expert, which for experts of few rows is
-                // every third (256 experts, 7168 x 2048, Zipf: 65536 rows 2871 / 2740 us, 1024 rows
-                // 1370 / 1276; with copies never edited the former took 2697).
+                // every third (256 experts, 7168 x 2048, Zipf: 65536 rows 2943 / 2736 us, 1024 rows
+                // 1369 / 1247).  The fences are on this thread's side of the ring's mbarrier, the loads
+                // on the producer's: one chain of causality inside one CTA, which is what a proxy fence
+                // needs.
                 ptx::fence_tensormap_acquire(ea);
                 ptx::fence_tensormap_acquire(eb);
                 ptx::prefetch_tensormap(ea);
