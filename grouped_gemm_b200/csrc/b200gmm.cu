@@ -97,7 +97,7 @@ struct LaunchArgs {
   PushArgs push = {};                     // rows to move while the product runs (src == nullptr: none)
 };
 
-template <int MODE, int CTAS, bool GATHER, bool SWIGLU, bool PUSH = false>
+template <int MODE, int CTAS, bool GATHER, bool SWIGLU, bool PUSH = false, bool PAIR_SWAP = false>
 cudaError_t launch_gmm(const LaunchArgs& a) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.grid);
@@ -113,7 +113,7 @@ cudaError_t launch_gmm(const LaunchArgs& a) {
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = a.overlap ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, gmm_kernel<MODE, CTAS, GATHER, SWIGLU, PUSH>, a.map_a, a.map_b, a.map_b2, a.map_c, a.map_a2, a.c,
+  return cudaLaunchKernelEx(&cfg, gmm_kernel<MODE, CTAS, GATHER, SWIGLU, PUSH, PAIR_SWAP>, a.map_a, a.map_b, a.map_b2, a.map_c, a.map_a2, a.c,
                             a.batch_sizes, a.p, a.status, a.slots, a.sched_counter, a.row_dest, a.a_rows, a.a_src, a.a_src_rows,
                             a.row_scale, a.reduce_add, a.dest_lo, a.dest_hi, a.gate_grad, a.push, a.inline_sizes);
 }
@@ -170,12 +170,16 @@ cudaError_t launch_layout(const LaunchArgs& a) {
 
 template <bool GATHER, bool SWIGLU>
 cudaError_t launch_variant(const LaunchArgs& a, int ctas) {
+  if constexpr (!GATHER) {
+    if (ctas == 2 && a.p.swap_rows > 0)
+      return a.p.mode == kNN ? launch_gmm<kNN, 2, false, SWIGLU, false, true>(a) : launch_gmm<kNT, 2, false, SWIGLU, false, true>(a);
+  }
   return ctas == 2 ? launch_layout<2, GATHER, SWIGLU>(a) : launch_layout<1, GATHER, SWIGLU>(a);
 }
 
-template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false>
+template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false, bool PAIR_SWAP = false>
 cudaError_t set_smem_attr() {
-  return cudaFuncSetAttribute(gmm_kernel<MODE, CTAS, GATHER, SWIGLU, PUSH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(gmm_kernel<MODE, CTAS, GATHER, SWIGLU, PUSH, PAIR_SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               static_cast<int>(PUSH ? kSmemBytesPush : kSmemBytes));
 }
 
@@ -204,7 +208,10 @@ int device_info(DeviceInfo** out) {
         set_smem_attr<kNN, 1, false, true>() != cudaSuccess || set_smem_attr<kNT, 1, false, true>() != cudaSuccess ||
         set_smem_attr<kNN, 2, false, true>() != cudaSuccess || set_smem_attr<kNT, 2, false, true>() != cudaSuccess ||
         set_smem_attr<kNN, 1, false, false, true>() != cudaSuccess || set_smem_attr<kNT, 1, false, false, true>() != cudaSuccess ||
-        set_smem_attr<kNN, 2, false, false, true>() != cudaSuccess || set_smem_attr<kNT, 2, false, false, true>() != cudaSuccess)
+        set_smem_attr<kNN, 2, false, false, true>() != cudaSuccess || set_smem_attr<kNT, 2, false, false, true>() != cudaSuccess ||
+        set_smem_attr<kNN, 2, false, false, false, true>() != cudaSuccess ||
+        set_smem_attr<kNT, 2, false, false, false, true>() != cudaSuccess ||
+        set_smem_attr<kNN, 2, false, true, false, true>() != cudaSuccess || set_smem_attr<kNT, 2, false, true, false, true>() != cudaSuccess)
       return B200GMM_ECUDA;
     if (cudaFuncSetAttribute(gmm_gradients_kernel<kNN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)) != cudaSuccess ||
         cudaFuncSetAttribute(gmm_gradients_kernel<kNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemBytes)) != cudaSuccess)
@@ -627,7 +634,8 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
     if ((rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat)) != B200GMM_OK) return rc;
   }
 
-  p.swap_rows = swap_rows(p, feat, ctas, dev->sm_count);
+  const bool with_push = push != nullptr && push->src != nullptr && push->n_items > 0 && !feat.gather && !swiglu && p.mode != kTN;
+  p.swap_rows = with_push && ctas == 2 ? 0 : swap_rows(p, feat, ctas, dev->sm_count);  // (no such kernels)
   p.swap_units = swiglu ? ctas : 1;
   p.dest_indexed = dest_rows >= 0 ? 1 : 0;
   p.dest_rows = dest_rows;
@@ -751,8 +759,6 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
       return rc;
   }
 
-  const bool with_push = push != nullptr && push->src != nullptr && push->n_items > 0 && !gather && !swiglu &&
-                         p.mode != kTN;
   // A launch that carries a row transfer keeps every CTA, however few its tiles: the
   // items are dealt over the grid.  (6 rows in 4 experts, k = 64, n = 72, beside 4000 rows of
   // 21504 bytes: 6466 us on the tiles' four CTAs, 196 us on all.)

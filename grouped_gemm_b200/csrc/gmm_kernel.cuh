@@ -446,7 +446,7 @@ struct TileFeed {
 // the compiler take the read-only path, whose loads it need not keep behind the
 // grid_dependency_wait() below.
 // What one CTA of a launch does: CTA `block` of `blocks`.
-template <int MODE, int CTAS, bool GATHER, bool SWIGLU, bool PUSH>
+template <int MODE, int CTAS, bool GATHER, bool SWIGLU, bool PUSH, bool PAIR_SWAP>
 __device__ __forceinline__ void
 gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
           const CUtensorMap& map_b2, const CUtensorMap& map_c,
@@ -471,9 +471,12 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
   // (map_a2: the activations with 32-row boxes; NT also uses map_b2: b with
   // 128-row boxes).
   constexpr bool kLight = (MODE != kTN) && (CTAS == 1) && !GATHER && !SWIGLU;
-  // Swapped tiles (schedule.cuh) exist in all forward / dgrad kernels but the gathered ones.  A sum
-  // of two products over one accumulator (Problem::pair_sum) is an option of the plain kernels.
-  constexpr bool kSwap = (MODE != kTN) && !GATHER;
+  // Swapped tiles (schedule.cuh) exist in the one-CTA forward / dgrad kernels but the gathered ones.  On
+  // pairs they are kernels of their own: with the question in front of every k-block plain tiles took up
+  // to 6 % longer (8 experts of 4096 rows, 4096 x 14336, tiles of one accumulator: 3174 / 3013 us, dgrad 3123 /
+  // 2966; 2 of 9300, 4528 x 1440, gated: 403 / 391).  A sum of two products over one accumulator
+  // (Problem::pair_sum) is an option of the plain kernels.
+  constexpr bool kSwap = (MODE != kTN) && !GATHER && (CTAS == 1 || PAIR_SWAP);
   constexpr bool kPairSum = (MODE != kTN) && !GATHER && !SWIGLU && !PUSH;
 
   extern __shared__ uint8_t smem_raw[];
@@ -1969,7 +1972,7 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
   }
 }
 
-template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false>
+template <int MODE, int CTAS, bool GATHER = false, bool SWIGLU = false, bool PUSH = false, bool PAIR_SWAP = false>
 __global__ void __launch_bounds__(GATHER ? GatherWarps<CTAS>::kBlockThreads : (PUSH ? kGemmPushThreads : kThreads), 1)
 gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
            const __grid_constant__ CUtensorMap map_b2, const __grid_constant__ CUtensorMap map_c,
@@ -1980,7 +1983,7 @@ gmm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CU
            const int64_t a_src_rows, const float* row_scale, const int reduce_add,
            const int64_t dest_lo, const int64_t dest_hi, const __nv_bfloat16* gate_grad,
            const PushArgs push, const __grid_constant__ InlineSizes inline_sizes) {
-  gmm_block<MODE, CTAS, GATHER, SWIGLU, PUSH>(
+  gmm_block<MODE, CTAS, GATHER, SWIGLU, PUSH, PAIR_SWAP>(
       map_a, map_b, map_b2, map_c, map_a2, c, batch_sizes, p, status, map_slots, sched_counter,
       row_dest, a_rows, a_src, a_src_rows, row_scale, reduce_add, dest_lo, dest_hi, gate_grad, push, inline_sizes,
       blockIdx.x, gridDim.x);
@@ -2002,11 +2005,11 @@ gmm_gradients_kernel(const __grid_constant__ ProductArgs d, const __grid_constan
                      uint32_t* status, CUtensorMap* map_slots, const __grid_constant__ InlineSizes inline_sizes) {
   const int block = blockIdx.x;
   if (block < d.blocks)
-    gmm_block<MODE, 1, false, false, false>(d.map_a, d.map_b, d.map_b, d.map_c, d.map_a, d.c, batch_sizes, d.p, status, map_slots,
+    gmm_block<MODE, 1, false, false, false, false>(d.map_a, d.map_b, d.map_b, d.map_c, d.map_a, d.c, batch_sizes, d.p, status, map_slots,
                                             nullptr, nullptr, nullptr, nullptr, 0, nullptr, 0, 0, 0, nullptr, PushArgs{}, inline_sizes,
                                             block, d.blocks);
   else
-    gmm_block<kTN, 1, false, false, false>(w.map_a, w.map_b, w.map_b, w.map_c, w.map_a, w.c, batch_sizes, w.p, status, map_slots,
+    gmm_block<kTN, 1, false, false, false, false>(w.map_a, w.map_b, w.map_b, w.map_c, w.map_a, w.c, batch_sizes, w.p, status, map_slots,
                                            nullptr, nullptr, nullptr, nullptr, 0, nullptr, 0, 0, 0, nullptr, PushArgs{}, inline_sizes,
                                            block - d.blocks, w.blocks);
 }

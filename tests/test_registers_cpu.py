@@ -15,7 +15,9 @@ SOURCE = """
 #include "gmm_kernel.cuh"
 using namespace b200gmm;
 const void* kernels[] = {(const void*)gmm_kernel<kNN, 1, false, true>, (const void*)gmm_kernel<kNT, 1, false, true>,
-                         (const void*)gmm_kernel<kNN, 2, false, true>, (const void*)gmm_kernel<kNT, 2, false, true>};
+                         (const void*)gmm_kernel<kNN, 2, false, true>, (const void*)gmm_kernel<kNT, 2, false, true>,
+                         (const void*)gmm_kernel<kNN, 2, false, true, false, true>,
+                         (const void*)gmm_kernel<kNT, 2, false, true, false, true>};
 """
 
 
@@ -28,5 +30,5 @@ def test_gated_kernels_do_not_spill(tmp_path):
     assert done.returncode == 0, done.stderr
     spills = re.findall(r"Compiling entry function '(\w*gmm_kernel\w*)'.*?(\d+) bytes spill stores, (\d+) bytes spill loads",
                         done.stderr, re.S)
-    assert len(spills) == 4
+    assert len(spills) == 6
     assert all(stores == loads == "0" for _, stores, loads in spills), spills
