@@ -3,6 +3,7 @@
 The library is the only compute path: if it cannot be loaded the import of
 ``grouped_gemm_b200.backend`` fails; there is no fallback implementation.
 """
+import collections
 import ctypes
 import os
 
@@ -97,6 +98,9 @@ SIGNATURES = {
     "b200gmm_schedule_device": (_c.c_int, [
         _c.c_void_p, _c.c_int, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int, _c.c_int, _c.c_int,
         _c.c_void_p, _c.c_int64, _c.c_void_p, _c.c_void_p, _c.c_void_p]),
+    "b200gmm_launch_forms": (_c.c_int, [
+        _c.c_void_p, _c.c_int, _c.c_int64, _c.c_int64, _c.c_int64, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
+        _c.c_void_p, _c.c_void_p, _c.c_int64]),
     "b200gmm_selftest_wait_timeout": (_c.c_int, [_c.c_int64, _c.c_void_p, _c.c_void_p]),
     "b200gmm_tile_shape": (_c.c_int, [_c.c_int, _c.POINTER(_c.c_int)]),
     "b200gmm_launch_count": (_c.c_int64, []),
@@ -152,3 +156,20 @@ def tile_shape(cluster_ctas=1):
     out = (ctypes.c_int * 3)()
     check(load().b200gmm_tile_shape(int(cluster_ctas), out), "b200gmm_tile_shape")
     return tuple(out)
+
+
+FORM_GATHER, FORM_GATED, FORM_GATED_BACKWARD, FORM_SCATTER = 1, 2, 4, 8
+LaunchForms = collections.namedtuple("LaunchForms", "ctas wide narrow empty swapped all_narrow single_wave")
+
+
+def launch_forms(sizes, dim_a1, n, trans_a=False, trans_b=False, features=0, tokens=None, sm_count=148, pair_ctas=148,
+                 positions=None):
+    """Forms of tiles that a launch would have (``b200gmm_launch_forms``), on a B200 by default.
+    ``positions``: int64 array [m, 5] for the first m positions of the launch order."""
+    counts = (ctypes.c_int64 * max(len(sizes), 1))(*[int(v) for v in sizes])
+    out = (ctypes.c_int64 * len(LaunchForms._fields))()
+    tokens = sum(int(v) for v in sizes) if tokens is None else int(tokens)
+    check(load().b200gmm_launch_forms(counts, len(sizes), tokens, int(dim_a1), int(n), int(trans_a), int(trans_b), int(features),
+                                      int(sm_count), int(pair_ctas), out, None if positions is None else positions.ctypes.data,
+                                      0 if positions is None else len(positions)), "b200gmm_launch_forms")
+    return LaunchForms(*out)

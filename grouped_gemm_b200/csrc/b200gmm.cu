@@ -406,6 +406,8 @@ int swap_rows(const Problem& p, const Features& f, int ctas, int sm_count) {
   return p.tokens <= kMeanRows * p.z && 2 * tiles >= sm_count ? kBlockM / 2 : 0;
 }
 
+constexpr int kNeverWide = 1000;  // Problem::wide_cost: every tile one accumulator wide
+
 int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b, int ctas,
                   Problem* p, const Features& f = Features()) {
   if (trans_a && trans_b) return B200GMM_EINVAL;
@@ -441,21 +443,24 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   // by streaming their weights from HBM either way, and measured end to end the
   // launch was not faster with them (B200GMM_LIGHT=1 switches them on).
   p->light = (p->mode != kTN && ctas == 1 && !f.gather && !f.swiglu) ? env_int("B200GMM_LIGHT", 0) : 0;
-  // A pair's wide tiles are half as many.  wgrad's are as long as their expert has rows: with
-  // few a CTA and experts of 2048 rows and more the long ones end the launch (11 experts, 126529 rows, 4144 x 576: 712 us with tiles of 256
-  // columns, 872 with 512).  Forward and dgrad: one or two rounds lose more to the last one than the
-  // bytes save (3 experts, 3172 rows, 1936 x 4672: 62.3 / 66.3), unless rows start at any 16 bytes, when
-  // bytes are what bounds them (7 experts, 3001 rows, 1000 x 2504: 26.4 / 23.0).  Scattered rows leave in
-  // 64-byte copies: while an accumulator's are sent the other one has to wait, unless the contraction
-  // is long (16384 rows, 8 experts, 4096 x 14336: 1573 / 1660; 14336 x 4096, 8192 rows: 892 / 855).
-  p->narrow_rounds = trans_a ? (tokens >= 2048 * int64_t(z) ? 8 : 0) : (f.scatter && d1 < 8192 ? 1 << 20 : (ragged_rows(d1, f.swiglu ? n / 2 : n, trans_b) ? 0 : 2));
+  // A pair's tiles two accumulators wide or one (narrow_tiles).  wgrad's are as long as their expert has
+  // rows: with few a CTA and experts of 2048 rows and more the long ones end the launch (11 experts,
+  // 126529 rows, 4144 x 576: 712 us with tiles of 256 columns, 872 with 512).  Rows that start at any 16 bytes
+  // are bound by bytes, which wide tiles save (7 experts, 3001 rows, 1000 x 2504: 26.4 / 23.0).  Scattered
+  // rows leave in 64-byte copies: while an accumulator's are sent the other one has to wait,
+  // unless the contraction is long (16384 rows, 8 experts, 4096 x 14336: 1573 / 1660; 14336 x 4096, 8192
+  // rows: 892 / 855).
+  p->narrow_rounds = trans_a && tokens >= 2048 * int64_t(z) ? 16 : 0;
+  p->wide_cost = 97;
+  if (!trans_a && ragged_rows(d1, f.swiglu ? n / 2 : n, trans_b)) p->wide_cost = 80;
+  if (f.scatter && d1 < 8192) p->wide_cost = kNeverWide;
   p->swap_units = 1;
-  p->swap_rows = 0;  // decided where the device is known (run_impl)
+  p->swap_rows = 0;  // decided where the device is known (settle)
   p->dest_indexed = 0;
   p->dest_rows = 0;
   p->pair_sum = 0;
   p->zero_rest = 0;
-  p->single_wave = 0;  // decided where the grid is (run_impl)
+  p->single_wave = 0;  // decided where the grid is (settle)
   const int64_t wait_ns = env_int64("B200GMM_WAIT_LIMIT_NS", static_cast<int64_t>(ptx::kWaitLimitNs));
   p->wait_ns = wait_ns > 0 ? wait_ns : static_cast<int64_t>(ptx::kWaitLimitNs);
   // Upper bound on the tile count must fit the kernel's 32-bit tile index (twice:
@@ -465,6 +470,23 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
                                     : (tokens / p->tile_m + 3 * int64_t(z));  // + transposed tiles, half as wide
   if (row_tiles * nt >= (int64_t(1) << 30)) return B200GMM_ELIMIT;
   return B200GMM_OK;
+}
+
+// The CTAs of a launch that fills the device.
+int grid_ctas(int ctas, int sm_count, int pair_ctas) { return std::min(ctas == 2 ? pair_ctas : sm_count, kMaxCtas); }
+
+// What check_problem leaves to where the device is known.
+void settle(Problem* p, const Features& f, int ctas, int sm_count, int pair_ctas) {
+  p->swap_rows = swap_rows(*p, f, ctas, sm_count);
+  p->swap_units = f.swiglu ? ctas : 1;
+  // A launch whose every possible tile is the first of some cluster draws no positions:
+  // no counter to zero, and no more CTAs than tiles (run_impl).  Together with the inline
+  // batch_sizes there this leaves a small call with one operation on the stream instead
+  // of two or three; its kernel can then also start while the one before it ends.
+  // A training step of 512 rows (4 experts, 128 x 128, host batch_sizes): 108.9 -> 99.3 us,
+  // host-bound before and after; token generation, where the overlap counts (64 rows, 8
+  // experts of 4096 x 14336): 135.9 -> 129.4 us.
+  p->single_wave = !p->light && max_tiles(*p) * ctas <= grid_ctas(ctas, sm_count, pair_ctas) ? 1 : 0;
 }
 
 // Argument checks alone (no launch): what run_impl would refuse for these sizes.
@@ -540,6 +562,42 @@ int b200gmm_workspace_bytes(int z, size_t* out_bytes) {
 }  // extern "C"
 
 namespace {
+
+// The kernels' build_schedule, replayed: clamped row prefix sums, the order of
+// the experts, tile prefix sums in that order.
+struct HostSchedule {
+  std::vector<int> row_start, perm, tile_start;
+  HostSchedule(const Problem& p, const int64_t* sizes)
+      : row_start(size_t(p.z) + 1), perm(static_cast<size_t>(p.z)), tile_start(size_t(p.z) + 1) {
+    int64_t start = 0;
+    for (int e = 0; e < p.z; ++e) {
+      row_start[e] = static_cast<int>(start < p.tokens ? start : p.tokens);
+      start += sizes[e] < 0 ? 0 : sizes[e];
+    }
+    row_start[p.z] = static_cast<int>(start < p.tokens ? start : p.tokens);
+    for (int e = 0; e < p.z; ++e) perm[e] = e;
+    if (p.order)
+      std::stable_sort(perm.begin(), perm.end(), [&](int x, int y) {
+        return row_start[x + 1] - row_start[x] > row_start[y + 1] - row_start[y];
+      });
+    for (int i = 0; i < p.z; ++i)
+      tile_start[i + 1] = tile_start[i] + expert_tiles(p, row_start[perm[i] + 1] - row_start[perm[i]]);
+  }
+  // The kernels' TileWalker: positions come in increasing order, *pos is the cursor over the experts.
+  TileOrder order(const Problem& p, int clusters) const {
+    if (p.tile_n > kBlockN)
+      return tile_order(p, tile_start.back(), clusters, clusters > 0 && narrow_tiles(p, tile_start.back(), clusters));
+    return TileOrder{TileGrid{p.nt, kBlockN, p.group_m}, tile_start.back(), tile_start.back()};
+  }
+  void decode(const Problem& p, const TileOrder& o, int position, int* pos, Tile* out) const {
+    int half;
+    const int t = tile_of_position(o, position, &half), nt = p.tile_n > kBlockN ? o.grid.nt : 1;
+    while (t >= tile_start[*pos + 1] * nt) ++*pos;
+    const int e = perm[*pos];
+    *out = make_tile(p, o.grid, e, t - tile_start[*pos] * nt, row_start[e], row_start[e + 1]);
+    take_half(out, half);
+  }
+};
 
 // Shared body of b200gmm_run and b200gmm_run_scatter.  row_dest == nullptr: rows
 // go to c.  Otherwise (non-transposed a only) row i of the result goes to the
@@ -635,8 +693,6 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   }
 
   const bool with_push = push != nullptr && push->src != nullptr && push->n_items > 0 && !feat.gather && !swiglu && p.mode != kTN;
-  p.swap_rows = with_push && ctas == 2 ? 0 : swap_rows(p, feat, ctas, dev->sm_count);  // (no such kernels)
-  p.swap_units = swiglu ? ctas : 1;
   p.dest_indexed = dest_rows >= 0 ? 1 : 0;
   p.dest_rows = dest_rows;
   p.pair_sum = pair_sum ? 1 : 0;
@@ -644,6 +700,8 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   if (pair_sum) {
     p.light = 0;  // (transposed tiles know no second part)
   }
+  settle(&p, feat, ctas, dev->sm_count, dev->pair_ctas);
+  if (with_push && ctas == 2) p.swap_rows = 0;  // (no such kernels)
 
   size_t need = 0;
   b200gmm_workspace_bytes(z, &need);
@@ -653,16 +711,8 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   // The tile counter of the kernel's scheduler sits in the 16 bytes after the
   // batch_sizes copy and starts every launch at zero.
   uint32_t* sched_counter = reinterpret_cast<uint32_t*>(static_cast<char*>(workspace) + size_t(z) * sizeof(int64_t));
-  const int max_ctas = std::min(ctas == 2 ? dev->pair_ctas : dev->sm_count, kMaxCtas);
-  // A launch whose every possible tile is the first of some cluster draws no positions:
-  // no counter to zero, and no more CTAs than tiles (below).  Together with the inline
-  // batch_sizes below this leaves a small call with one operation on the stream instead
-  // of two or three; its kernel can then also start while the one before it ends.
-  // A training step of 512 rows (4 experts, 128 x 128, host batch_sizes): 108.9 -> 99.3 us,
-  // host-bound before and after; token generation, where the overlap counts (64 rows, 8
-  // experts of 4096 x 14336): 135.9 -> 129.4 us.
-  const bool single_wave = !p.light && max_tiles(p) * ctas <= max_ctas;
-  p.single_wave = single_wave ? 1 : 0;
+  const int max_ctas = grid_ctas(ctas, dev->sm_count, dev->pair_ctas);
+  const bool single_wave = p.single_wave != 0;
 
   // A capturing stream keeps the copy of host batch_sizes (a replay reads them again)
   // and full dependencies between its kernels.
@@ -1108,30 +1158,13 @@ int b200gmm_schedule_host(const int64_t* batch_sizes_host, int z, int64_t tokens
   const int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, cluster_ctas, &p);
   if (rc != B200GMM_OK) return rc;
   if (n_tiles == nullptr || (z > 0 && batch_sizes_host == nullptr)) return B200GMM_EINVAL;
-  // The kernels' build_schedule, replayed: clamped row prefix sums, the order of
-  // the experts, tile prefix sums in that order.
-  std::vector<int> row_start(size_t(z) + 1), perm(static_cast<size_t>(z)), tile_start(size_t(z) + 1);
-  int64_t start = 0;
-  for (int e = 0; e < z; ++e) {
-    row_start[e] = static_cast<int>(start < tokens ? start : tokens);
-    start += batch_sizes_host[e] < 0 ? 0 : batch_sizes_host[e];
-  }
-  row_start[z] = static_cast<int>(start < tokens ? start : tokens);
-  for (int e = 0; e < z; ++e) perm[e] = e;
-  if (p.order)
-    std::stable_sort(perm.begin(), perm.end(), [&](int x, int y) {
-      return row_start[x + 1] - row_start[x] > row_start[y + 1] - row_start[y];
-    });
-  tile_start[0] = 0;
-  for (int i = 0; i < z; ++i)
-    tile_start[i + 1] = tile_start[i] + expert_tiles(p, row_start[perm[i] + 1] - row_start[perm[i]]);
-  const int total = tile_start[z];
-  int pos = 0;
-  int64_t count = 0;  // tiles of one accumulator: a wide tile is two
-  for (int t = 0; t < total; ++t) {
-    while (t >= tile_start[pos + 1]) ++pos;
-    const int e = perm[pos];
-    const Tile tile = make_tile(p, e, t - tile_start[pos], row_start[e], row_start[e + 1]);
+  const HostSchedule h(p, batch_sizes_host);
+  Tile tile;
+  int64_t count = 0;  // accumulators: a wide tile is two
+  int expert_pos = 0;
+  const TileOrder order = h.order(p, 0);
+  for (int t = 0; t < order.total; ++t) {
+    h.decode(p, order, t, &expert_pos, &tile);
     for (int unit = 0; unit < tile.units; ++unit, ++count) {
       if (out == nullptr || count >= max_tiles) continue;
       int64_t* o = out + count * B200GMM_SCHEDULE_FIELDS;
@@ -1144,6 +1177,50 @@ int b200gmm_schedule_host(const int64_t* batch_sizes_host, int z, int64_t tokens
     }
   }
   *n_tiles = count;
+  return B200GMM_OK;
+}
+
+int b200gmm_launch_forms(const int64_t* batch_sizes_host, int z, int64_t tokens, int64_t dim_a1, int64_t n, int trans_a,
+                         int trans_b, int features, int sm_count, int pair_ctas, int64_t* forms, int64_t* positions,
+                         int64_t max_positions) {
+  if (forms == nullptr || sm_count <= 0 || pair_ctas < 0 || (features & ~0xf) != 0) return B200GMM_EINVAL;
+  for (int i = 0; i < B200GMM_FORM_FIELDS; ++i) forms[i] = 0;
+  Features f;
+  f.gather = (features & B200GMM_FORM_GATHER) != 0;
+  f.gated_backward = (features & B200GMM_FORM_GATED_BACKWARD) != 0;
+  f.swiglu = f.gated_backward || (features & B200GMM_FORM_GATED) != 0;
+  f.scatter = (features & B200GMM_FORM_SCATTER) != 0;
+  if (n < 0 || (f.swiglu && (trans_a || f.gather)) || (f.scatter && trans_a)) return B200GMM_EINVAL;
+  if (f.swiglu) n *= 2;
+  int ctas = choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b, f);
+  if (pair_ctas < 2) ctas = 1;
+  Problem p;
+  const int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, f);
+  if (rc != B200GMM_OK) return rc;
+  if (z > 0 && batch_sizes_host == nullptr) return B200GMM_EINVAL;
+  forms[0] = ctas;
+  if (z == 0 || tokens == 0 || dim_a1 == 0 || n == 0) return B200GMM_OK;
+  settle(&p, f, ctas, sm_count, pair_ctas);
+  const HostSchedule h(p, batch_sizes_host);
+  const int clusters = ctas == 2 ? grid_ctas(2, sm_count, pair_ctas) / 2 : 0;
+  const TileOrder order = h.order(p, clusters);
+  Tile tile;
+  int expert_pos = 0;
+  for (int i = 0; i < order.total; ++i) {
+    h.decode(p, order, i, &expert_pos, &tile);
+    if (positions != nullptr && i < max_positions) {
+      int64_t* o = positions + int64_t(i) * B200GMM_POSITION_FIELDS;
+      o[0] = tile.expert;
+      o[1] = tile.row0;
+      o[2] = tile.col0;
+      o[3] = tile.valid_rows;
+      o[4] = tile.units;
+    }
+    ++forms[tile.units == 2 ? 1 : tile.units == 1 ? 2 : 3];
+    if (tile.units > 0 && p.mode != kTN && swapped_rows(p, tile) != 0) ++forms[4];
+  }
+  forms[5] = ctas == 2 && order.grid.tile_n == kBlockN ? 1 : 0;
+  forms[6] = p.single_wave;
   return B200GMM_OK;
 }
 

@@ -194,7 +194,8 @@ struct __align__(16) SmemTail {
   uint32_t role_sum[16];            // per taking warp: count of positions taken (low 8 bits) + 256 * their sum
   uint64_t push_full[4];            // push variant, bulk-copy form: a staged chunk has landed (kPushChunks used)
   int row_start[kMaxExperts + 1];   // exclusive prefix sum of batch_sizes, by expert
-  int tile_start[kMaxExperts + 1];  // exclusive prefix sum of tile counts, by position in perm
+  bool narrow;                      // a pair's launch: tiles are one accumulator wide
+  int tile_start[kMaxExperts + 1];  // exclusive prefix sum of expert_tiles, by position in perm
   uint16_t perm[kMaxExperts];       // expert at each position of the launch order
 };
 
@@ -250,11 +251,12 @@ __device__ __forceinline__ int64_t scan_step(int64_t v, int lane, int64_t* carry
 //               of rows, largest first, ties by index (the reference sorts its
 //               wgrad problems the same way, csrc/fill_arguments.cuh:80-86), so
 //               that the launch ends on the shortest tiles;
-//   tile_start  exclusive prefix sums of the per-expert tile counts in that order.
+//   tile_start  exclusive prefix sums of the per-expert tile counts in that order;
+//   narrow      how a pair's launch on `clusters` pairs (one-CTA launches: 0) cuts its columns.
 //
 // batch_sizes == nullptr: the sizes are those of `inline_sizes`.
 __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* batch_sizes,
-                                               const InlineSizes& inline_sizes, SmemTail* tail, uint32_t* status) {
+                                               const InlineSizes& inline_sizes, SmemTail* tail, uint32_t* status, int clusters) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int scan_warp = (blockDim.x >= 96) ? 2 : 0;
@@ -306,52 +308,44 @@ __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* 
       if (pos < p.z) tail->tile_start[pos] = carry + incl - tiles;
       carry += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) tail->tile_start[p.z] = carry;
+    if (lane == 0) {
+      tail->tile_start[p.z] = carry;
+      if (clusters > 0) tail->narrow = narrow_tiles(p, carry, clusters);
+    }
   }
 }
 
-// Position of the launch order -> tile (the scheduler's).  Positions come in
-// increasing order, so the expert cursor only ever moves forward.
-//
-// Tiles two accumulators wide are coarse.  A launch of few of them takes all as halves
-// (narrow_tiles); in others what is left over after whole rounds of the grid's
-// `clusters` is taken as halves when the halves fit one round, which then lasts half as
-// long.  A half that does not exist (the last column tile may be one accumulator
-// wide) is a tile of no units.  kWide: pairs.  (One-CTA tiles know at compile time that there are no
-// halves: the scheduler decodes before anything else can start, and with the question asked
-// of the Problem launches of one tile a CTA took 0.1 to 0.2 us longer, 6.85 / 7.06 us for the weight
-// gradient of 512 rows in 4 experts of 128 x 128.)
+// Position of the launch order (schedule.cuh: tile_order) -> tile (the scheduler's).  Positions
+// come in increasing order, so the expert cursor only ever moves forward.  kWide: pairs.
+// (One-CTA tiles know at compile time that there are no halves: the scheduler decodes before
+// anything else can start, and with the question asked of the Problem launches of one
+// tile a CTA took 0.1 to 0.2 us longer, 6.85 / 7.06 us for the weight gradient of 512 rows in 4
+// experts of 128 x 128.)
 template <bool kWide>
 struct TileWalker {
   const Problem& p;
   const SmemTail* tail;
-  int whole;  // positions before the halves
-  int total;
+  TileOrder order;
+  int total;  // positions
   int pos;
   __device__ TileWalker(const Problem& p_, const SmemTail* tail_, int clusters)
-      : p(p_), tail(tail_), whole(tail_->tile_start[p_.z]), total(whole), pos(0) {
-    if (kWide && p.n > kBlockN && clusters > 0) {
-      int halves = whole % clusters;
-      if (2 * halves > clusters) halves = 0;
-      if (narrow_tiles(p, whole, clusters)) halves = whole;
-      whole -= halves;
-      total += halves;
+      : p(p_), tail(tail_), total(tail_->tile_start[p_.z]), pos(0) {
+    if (kWide) {
+      order = tile_order(p, total, clusters, clusters > 0 && tail->narrow);
+      total = order.total;
+    } else {
+      order.grid = TileGrid{p.nt, kBlockN, p.group_m};
     }
   }
   __device__ __forceinline__ bool decode(int t, Tile* out) {
     if (t < 0 || t >= total) return false;
     int half = -1;
-    if (kWide && t >= whole) {
-      half = (t - whole) & 1;
-      t = whole + ((t - whole) >> 1);
-    }
-    while (t >= tail->tile_start[pos + 1]) ++pos;
+    if (kWide) t = tile_of_position(order, t, &half);
+    const int nt = kWide ? order.grid.nt : 1;  // (tile_start counts a pair's row tiles)
+    while (t >= tail->tile_start[pos + 1] * nt) ++pos;
     const int e = tail->perm[pos];
-    *out = make_tile(p, e, t - tail->tile_start[pos], tail->row_start[e], tail->row_start[e + 1]);
-    if (kWide && half >= 0) {
-      out->units = half < out->units ? 1 : 0;
-      out->col0 += half * kBlockN;
-    }
+    *out = make_tile(p, order.grid, e, t - tail->tile_start[pos] * nt, tail->row_start[e], tail->row_start[e + 1]);
+    if (kWide) take_half(out, half);
     return true;
   }
 };
@@ -541,7 +535,7 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
   // The kernel after this one may take over SMs as soon as they fall idle: it waits here too.
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();
-  build_schedule(p, batch_sizes, inline_sizes, tail, status);
+  build_schedule(p, batch_sizes, inline_sizes, tail, status, kPair ? blocks >> 1 : 0);
   ptx::tc_fence_before_sync();
   __syncthreads();
   if (kPair) ptx::cluster_sync();  // the peer's barriers exist before anything arrives on them
@@ -569,7 +563,7 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
   // The ring.  A launch of few tiles is bound by the latency of its loads, one of narrow outputs by
   // their bytes: stages in flight count (one expert of 5788 rows, 792 x 2224, wgrad: 62 us
   // with three stages, 38 with four).
-  const bool narrow = kPair && narrow_tiles(p, tail->tile_start[p.z], tile_stride);
+  const bool narrow = kPair && tail->narrow;
   const uint32_t ring_stages = narrow ? G::kNarrowStages : G::kStages;
   const uint32_t stage_bytes = narrow ? G::kNarrowStageBytes : G::kStageBytes;
   const int row_off = static_cast<int>(cta_rank) * kBlockM;  // this CTA's rows inside a pair tile
@@ -1847,16 +1841,17 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
             }
           }
         } else if (backward) {
-          // The accumulator is read before the first chunk's results leave; holding the second's too
-          // took more registers than there are (168: 44 bytes of spill stores, 100 of loads).
+          // The accumulator is read before all of the first chunk's results have left; holding the
+          // second's too took more registers than there are (168: 44 bytes of spill stores, 100 of
+          // loads).
           uint4 o[4], o2[4];
           load(0);
           gradients(d4);
           load_grad(d4, half * 64 + 32);
           pack(va, o);
           pack(vb, o2);
-          load(1);
           emit_gate(o, 0);
+          load(1);
           emit_up(o2, 0);
           gradients(d4);
           pack(va, o);
@@ -2039,29 +2034,32 @@ fill_offsets_kernel(const int64_t* __restrict__ batch_sizes, const Problem p, in
   }
 }
 
-// The schedule a GEMM launch with this Problem walks, written out for tests: runs
-// the kernels' own build_schedule and TileWalker in one CTA and stores, for every
-// position of the launch order, {expert, row0, col0, valid_rows, stages, kind}.
-// out_count receives the number of tiles; at most max_tiles are written.
+// The schedule of a Problem's tiles, written out for tests: runs the kernels' own build_schedule and
+// TileWalker in one CTA and stores, for every accumulator of every tile in the order of
+// whole tiles (a pair's launch may cut their columns otherwise: tile_order), {expert, row0, col0,
+// valid_rows, stages, kind}.  out_count receives their number; at most max_tiles are written.
 __global__ void __launch_bounds__(kThreads, 1)
 schedule_dump_kernel(const int64_t* __restrict__ batch_sizes, const Problem p, int32_t* __restrict__ out,
                      int max_tiles, int32_t* __restrict__ out_count, uint32_t* status) {
   __shared__ SmemTail tail;
-  build_schedule(p, batch_sizes, InlineSizes{}, &tail, status);
+  build_schedule(p, batch_sizes, InlineSizes{}, &tail, status, 0);
   __syncthreads();
   if (threadIdx.x == 0) {
-    TileWalker<true> walk(p, &tail, 0);
-    Tile t;
-    int n = 0;
-    for (int pos = 0; walk.decode(pos, &t); ++pos) {
-      for (int unit = 0; unit < t.units; ++unit, ++n) {
-        if (n >= max_tiles) continue;
-        int32_t* o = out + int64_t(n) * 6;
-        o[0] = t.expert; o[1] = t.row0; o[2] = t.col0 + unit * kBlockN;
-        o[3] = t.valid_rows; o[4] = tile_stages(t); o[5] = t.kind;
+    auto dump = [&](auto walk) {
+      Tile t;
+      int n = 0;
+      for (int pos = 0; walk.decode(pos, &t); ++pos) {
+        for (int unit = 0; unit < t.units; ++unit, ++n) {
+          if (n >= max_tiles) continue;
+          int32_t* o = out + int64_t(n) * 6;
+          o[0] = t.expert; o[1] = t.row0; o[2] = t.col0 + unit * kBlockN;
+          o[3] = t.valid_rows; o[4] = tile_stages(t); o[5] = t.kind;
+        }
       }
-    }
-    *out_count = n;
+      *out_count = n;
+    };
+    if (p.tile_n > kBlockN) dump(TileWalker<true>(p, &tail, 0));
+    else dump(TileWalker<false>(p, &tail, 0));
   }
 }
 

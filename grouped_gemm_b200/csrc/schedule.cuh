@@ -54,6 +54,7 @@ struct Problem {
   int64_t wait_ns; // limit of every wait inside the kernel, in nanoseconds
   // Derived on the host so that decoding a tile needs no 64-bit division:
   int nt;          // column tiles: ceil(n / tile_n)
+  int nt1;         // column tiles of one accumulator: ceil(n / 256)
   int mt;          // TN: row tiles of c[i]: ceil(d1 / tile_m)
   int lt;          // column tiles of a transposed tile's width: ceil(n / 128)
   int wide_a;      // TN: a's columns are a multiple of 64, one TMA load brings all 64-column boxes of a stage
@@ -68,13 +69,17 @@ struct Problem {
   int64_t dest_rows;
   int zero_rest;   // gated backward: rows past the last expert's of both halves of c become zeros
   int swap_rows;   // NN/NT: a tile of at most this many rows (rounded up, swapped_rows) runs with its operands swapped
-  int narrow_rounds;  // a pair's launch of fewer rounds of wide tiles than this runs halves of them
+  // A pair's launch (narrow_tiles): up to this many rounds of tiles of one accumulator it has no wide ones, and
+  // it has them if they cost less at this percentage.
+  int narrow_rounds;
+  int wide_cost;
   int swap_units;  // ... if it has this many accumulators (a pair's gated tile: 2, gate and up, else 1)
 };
 
 // Fills the derived fields of a Problem whose shape fields are set.
 B200GMM_HD void derive(Problem* p) {
   p->nt = static_cast<int>((p->n + p->tile_n - 1) / p->tile_n);
+  p->nt1 = static_cast<int>((p->n + kBlockN - 1) / kBlockN);
   p->mt = static_cast<int>((p->d1 + p->tile_m - 1) / p->tile_m);
   p->lt = static_cast<int>((p->n + kLightCols - 1) / kLightCols);
 }
@@ -102,19 +107,19 @@ B200GMM_HD int light_rows(const Problem& p, int rows) {
   return (p.light && rows <= kLightRows) ? rows : 0;
 }
 
-// Tiles of one expert.  TN always has the full c[i] grid (empty experts still
-// need their zeros written, csrc/fill_arguments.cuh:100-119).
+// Tiles of one expert; of a pair's launch, whose columns may be cut in two ways (TileGrid), row
+// tiles.  TN always has the full c[i] grid (empty experts still need their zeros written,
+// csrc/fill_arguments.cuh:100-119).
 B200GMM_HD int expert_tiles(const Problem& p, int rows) {
+  if (p.tile_n > kBlockN) return p.mode == kTN ? p.mt : ceil_div_i(rows, p.tile_m);
   if (p.mode == kTN) return p.mt * p.nt;
   return heavy_row_tiles(p, rows) * p.nt + (light_rows(p, rows) > 0 ? p.lt : 0);
 }
 
-// Most tiles a launch can have, whatever batch_sizes holds (B200GMM_LIGHT off).
+// Most tiles of one accumulator a launch can have, whatever batch_sizes holds (B200GMM_LIGHT off).
 B200GMM_HD int64_t max_tiles(const Problem& p) {
-  // (a wide tile may be taken as two positions, whether or not both halves exist)
-  const int64_t nt = p.tile_n > kBlockN && p.n > kBlockN ? 2 * int64_t(p.nt) : (p.n + kBlockN - 1) / kBlockN;
-  if (p.mode == kTN) return int64_t(p.z) * p.mt * nt;
-  return (p.tokens / p.tile_m + (p.z < p.tokens ? p.z : p.tokens)) * nt;
+  if (p.mode == kTN) return int64_t(p.z) * p.mt * p.nt1;
+  return (p.tokens / p.tile_m + (p.z < p.tokens ? p.z : p.tokens)) * p.nt1;
 }
 
 // Pipeline stages (ring slots) one tile consumes.
@@ -148,37 +153,88 @@ B200GMM_HD void decode_in_expert(int local, int row_tiles, int nt, int group_m, 
   *ni = r / gm;
 }
 
-// Whether a pair's launch of `tiles` wide tiles on `clusters` pairs takes all of them as
-// halves of one accumulator: where they are all that wide, where the halves fit one
-// round, or (Problem::narrow_rounds) where there are few rounds.  (single_wave: a pair has no
-// second tile, so only what fits one round may be halved.)
-B200GMM_HD bool narrow_tiles(const Problem& p, int tiles, int clusters) {
-  if (p.n <= kBlockN || 2 * tiles <= clusters) return true;
-  return !p.single_wave && tiles < int64_t(p.narrow_rounds) * clusters;
+// Rounds that `tiles` tiles take on `clusters`; and, counted in rounds of tiles of one accumulator, that
+// `tiles` tiles of two do, where what is left after whole rounds is taken as halves if these fit
+// one round (tile_order).
+template <class Int>
+B200GMM_HD Int rounds_narrow(Int tiles, Int clusters) { return (tiles + clusters - 1) / clusters; }
+template <class Int>
+B200GMM_HD Int rounds_wide(Int tiles, Int clusters) {
+  const Int whole = tiles / clusters, left = tiles - whole * clusters;
+  return 2 * whole + (left == 0 ? 0 : (2 * left <= clusters ? 1 : 2));
 }
 
-// Accumulators that the tile at column col0 fills.
-B200GMM_HD int tile_units(const Problem& p, int col0) {
-  return p.tile_n > kBlockN && p.n - col0 > kBlockN ? 2 : 1;
+// Whether a pair's launch takes its tiles one accumulator wide.  A wide tile brings its rows
+// once for two accumulators, which makes a round of it cost Problem::wide_cost percent of two
+// narrow ones; but it is coarse, and half idle where the last column tile is one accumulator wide.
+B200GMM_HD bool narrow_tiles(const Problem& p, int row_tiles, int clusters) {
+  if (p.n <= kBlockN) return true;
+  const int narrow = rounds_narrow(row_tiles * p.nt1, clusters), wide = rounds_wide(row_tiles * p.nt, clusters);
+  return narrow <= 1 || narrow <= p.narrow_rounds || int64_t(100) * narrow <= int64_t(p.wide_cost) * wide;
+}
+
+// How a launch cuts the columns, and the row tiles swept together.
+struct TileGrid {
+  int nt;
+  int tile_n;
+  int group_m;
+};
+// Launch order of a pair's `row_tiles` in positions, which is what the grid's `clusters` draw: tiles,
+// and what is left over after whole rounds of wide ones as halves when the halves fit one
+// round, which then lasts half as long.  A half that does not exist (the last column tile
+// may be one accumulator wide) is a position of no units; a launch of `narrow` tiles has none, since
+// clusters whose draws hit them are left with fewer tiles than others (11 experts, 16933 rows,
+// 2792 x 592, two wide column tiles of which the second is one accumulator: 71 us as narrow tiles, 87 as
+// halves).  (clusters == 0: whole wide tiles.)
+struct TileOrder {
+  TileGrid grid;
+  int whole;  // positions before the halves
+  int total;
+};
+B200GMM_HD TileOrder tile_order(const Problem& p, int row_tiles, int clusters, bool narrow) {
+  TileOrder o;
+  if (narrow) {
+    // half as many row tiles together keep what is in flight about square
+    o.grid = TileGrid{p.nt1, kBlockN, p.group_m > 1 ? p.group_m / 2 : 1};
+    o.whole = o.total = row_tiles * p.nt1;
+    return o;
+  }
+  o.grid = TileGrid{p.nt, p.tile_n, p.group_m};
+  const int tiles = row_tiles * p.nt;
+  const int left = clusters > 0 ? tiles % clusters : 0;
+  const int halves = 2 * left <= clusters ? left : 0;
+  o.whole = tiles - halves;
+  o.total = tiles + halves;
+  return o;
+}
+// Tile of a position, and which half of it (-1: all).
+B200GMM_HD int tile_of_position(const TileOrder& o, int position, int* half) {
+  *half = position < o.whole ? -1 : (position - o.whole) & 1;
+  return position < o.whole ? position : o.whole + ((position - o.whole) >> 1);
+}
+
+// Accumulators that a tile of tile_n columns fills at column col0.
+B200GMM_HD int tile_units(const Problem& p, int tile_n, int col0) {
+  return tile_n > kBlockN && p.n - col0 > kBlockN ? 2 : 1;
 }
 
 // `local` = tile index relative to the expert's first tile; rs/re = row_start[expert],
 // row_start[expert+1] (already clamped to tokens).
-B200GMM_HD Tile make_tile(const Problem& p, int expert, int local, int rs, int re) {
+B200GMM_HD Tile make_tile(const Problem& p, const TileGrid& grid, int expert, int local, int rs, int re) {
   Tile t;
   t.expert = expert;
   t.kind = 0;
-  const int nt = p.nt;
+  const int nt = grid.nt;
   int mi, ni;
   if (p.mode == kTN) {
-    decode_in_expert(local, p.mt, nt, p.group_m, &mi, &ni);
+    decode_in_expert(local, p.mt, nt, grid.group_m, &mi, &ni);
     t.row0 = mi * p.tile_m;
     const int left = static_cast<int>(p.d1) - t.row0;
     t.valid_rows = left < p.tile_m ? left : p.tile_m;
     t.k_row0 = rs;
     t.k_len = re - rs;
-    t.col0 = ni * p.tile_n;
-    t.units = tile_units(p, t.col0);
+    t.col0 = ni * grid.tile_n;
+    t.units = tile_units(p, grid.tile_n, t.col0);
     return t;
   }
   t.k_row0 = 0;
@@ -187,12 +243,12 @@ B200GMM_HD Tile make_tile(const Problem& p, int expert, int local, int rs, int r
   if (p.pair_sum) t.k_len = (t.k_len + kBlockK - 1) / kBlockK * kBlockK * 2;
   const int mt = heavy_row_tiles(p, re - rs);
   if (local < mt * nt) {
-    decode_in_expert(local, mt, nt, p.group_m, &mi, &ni);
+    decode_in_expert(local, mt, nt, grid.group_m, &mi, &ni);
     t.row0 = rs + mi * p.tile_m;
     const int left = re - t.row0;
     t.valid_rows = left < p.tile_m ? left : p.tile_m;
-    t.col0 = ni * p.tile_n;
-    t.units = tile_units(p, t.col0);
+    t.col0 = ni * grid.tile_n;
+    t.units = tile_units(p, grid.tile_n, t.col0);
   } else {
     t.units = 1;
     t.kind = 1;
@@ -201,6 +257,13 @@ B200GMM_HD Tile make_tile(const Problem& p, int expert, int local, int rs, int r
     t.col0 = (local - mt * nt) * kLightCols;
   }
   return t;
+}
+
+// What a position that is half a tile (tile_of_position) leaves of it.
+B200GMM_HD void take_half(Tile* t, int half) {
+  if (half < 0) return;
+  t->units = half < t->units ? 1 : 0;
+  t->col0 += half * kBlockN;
 }
 
 // The nine per-expert values of the reference's GemmProblem

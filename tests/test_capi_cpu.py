@@ -155,6 +155,39 @@ def test_schedule_covers_rows_and_columns_once(sizes, trans_b, n, ctas, light, m
     assert (cover == 1).all()
 
 
+@pytest.mark.parametrize("sizes", SIZE_SETS + [[256 * (t // 2) - 7, 256 * (t - t // 2) - 100] for t in (25, 37, 62, 150)])
+@pytest.mark.parametrize("n", [256, 264, 776, 1288, 4104])
+@pytest.mark.parametrize("layout", [(0, 0), (0, 1), (1, 0)])
+@pytest.mark.parametrize("pair_ctas", [148, 4])
+def test_positions_of_a_pair_launch_fill_every_accumulator_once(sizes, n, layout, pair_ctas, monkeypatch):
+    """Wide tiles, narrow ones and halves of wide ones, in whatever order the launch has them, and
+    halves that do not exist only where the last column tile is one accumulator wide."""
+    monkeypatch.setenv("B200GMM_CTAS", "2")
+    m = 200 if layout[0] else None
+    positions = np.full((20000, 5), -1, dtype=np.int64)
+    forms = _capi.launch_forms(sizes, 200, n, *layout, pair_ctas=pair_ctas, positions=positions)
+    count = forms.wide + forms.narrow + forms.empty
+    if sum(sizes) == 0:
+        assert count == 0
+        return
+    assert count < len(positions) and (positions[count:] == -1).all()
+    starts = np.concatenate([[0], np.cumsum(sizes)])
+    seen = set()
+    for expert, row0, col0, valid, units in positions[:count]:
+        if units == 0:
+            assert n % 512 in range(1, 257) and col0 >= n
+            continue
+        assert valid == min(256, (m if m else starts[expert + 1]) - row0) and (row0 - (0 if m else starts[expert])) % 256 == 0
+        for unit in range(units):
+            key = (expert, row0, col0 // 256 + unit)
+            assert col0 % 256 == 0 and key[2] * 256 < n and key not in seen
+            seen.add(key)
+    row_tiles = len(sizes) if m else sum((size + 255) // 256 for size in sizes)
+    assert len(seen) == row_tiles * ((n + 255) // 256) == 2 * forms.wide + forms.narrow
+    if forms.all_narrow:
+        assert forms.wide == forms.empty == 0
+
+
 @pytest.mark.parametrize("sizes", SIZE_SETS)
 @pytest.mark.parametrize("ctas", [1, 2])
 def test_schedule_wgrad_full_grid_for_every_expert(sizes, ctas):
