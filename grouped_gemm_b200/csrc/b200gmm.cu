@@ -585,8 +585,7 @@ struct HostSchedule {
   }
   // The kernels' TileWalker: positions come in increasing order, *pos is the cursor over the experts.
   TileOrder order(const Problem& p, int clusters) const {
-    if (p.tile_n > kBlockN)
-      return tile_order(p, tile_start.back(), clusters, clusters > 0 && narrow_tiles(p, tile_start.back(), clusters));
+    if (p.tile_n > kBlockN) return tile_order(p, tile_start.back(), clusters);
     return TileOrder{TileGrid{p.nt, kBlockN, p.group_m}, tile_start.back(), tile_start.back()};
   }
   void decode(const Problem& p, const TileOrder& o, int position, int* pos, Tile* out) const {

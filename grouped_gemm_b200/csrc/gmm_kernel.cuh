@@ -194,7 +194,7 @@ struct __align__(16) SmemTail {
   uint32_t role_sum[16];            // per taking warp: count of positions taken (low 8 bits) + 256 * their sum
   uint64_t push_full[4];            // push variant, bulk-copy form: a staged chunk has landed (kPushChunks used)
   int row_start[kMaxExperts + 1];   // exclusive prefix sum of batch_sizes, by expert
-  bool narrow;                      // a pair's launch: tiles are one accumulator wide
+  TileOrder order;                  // a pair's launch
   int tile_start[kMaxExperts + 1];  // exclusive prefix sum of expert_tiles, by position in perm
   uint16_t perm[kMaxExperts];       // expert at each position of the launch order
 };
@@ -252,7 +252,7 @@ __device__ __forceinline__ int64_t scan_step(int64_t v, int lane, int64_t* carry
 //               wgrad problems the same way, csrc/fill_arguments.cuh:80-86), so
 //               that the launch ends on the shortest tiles;
 //   tile_start  exclusive prefix sums of the per-expert tile counts in that order;
-//   narrow      how a pair's launch on `clusters` pairs (one-CTA launches: 0) cuts its columns.
+//   order       the positions of a pair's launch on `clusters` pairs.
 //
 // batch_sizes == nullptr: the sizes are those of `inline_sizes`.
 __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* batch_sizes,
@@ -310,7 +310,7 @@ __device__ __forceinline__ void build_schedule(const Problem& p, const int64_t* 
     }
     if (lane == 0) {
       tail->tile_start[p.z] = carry;
-      if (clusters > 0) tail->narrow = narrow_tiles(p, carry, clusters);
+      if (p.tile_n > kBlockN) tail->order = tile_order(p, carry, clusters);
     }
   }
 }
@@ -325,26 +325,19 @@ template <bool kWide>
 struct TileWalker {
   const Problem& p;
   const SmemTail* tail;
-  TileOrder order;
   int total;  // positions
   int pos;
-  __device__ TileWalker(const Problem& p_, const SmemTail* tail_, int clusters)
-      : p(p_), tail(tail_), total(tail_->tile_start[p_.z]), pos(0) {
-    if (kWide) {
-      order = tile_order(p, total, clusters, clusters > 0 && tail->narrow);
-      total = order.total;
-    } else {
-      order.grid = TileGrid{p.nt, kBlockN, p.group_m};
-    }
-  }
+  __device__ TileWalker(const Problem& p_, const SmemTail* tail_)
+      : p(p_), tail(tail_), total(kWide ? tail_->order.total : tail_->tile_start[p_.z]), pos(0) {}
   __device__ __forceinline__ bool decode(int t, Tile* out) {
     if (t < 0 || t >= total) return false;
     int half = -1;
-    if (kWide) t = tile_of_position(order, t, &half);
-    const int nt = kWide ? order.grid.nt : 1;  // (tile_start counts a pair's row tiles)
+    if (kWide) t = tile_of_position(tail->order, t, &half);
+    const TileGrid grid = kWide ? tail->order.grid : TileGrid{p.nt, kBlockN, p.group_m};
+    const int nt = kWide ? grid.nt : 1;  // (tile_start counts a pair's row tiles)
     while (t >= tail->tile_start[pos + 1] * nt) ++pos;
     const int e = tail->perm[pos];
-    *out = make_tile(p, order.grid, e, t - tail->tile_start[pos] * nt, tail->row_start[e], tail->row_start[e + 1]);
+    *out = make_tile(p, grid, e, t - tail->tile_start[pos] * nt, tail->row_start[e], tail->row_start[e + 1]);
     if (kWide) take_half(out, half);
     return true;
   }
@@ -563,7 +556,7 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
   // The ring.  A launch of few tiles is bound by the latency of its loads, one of narrow outputs by
   // their bytes: stages in flight count (one expert of 5788 rows, 792 x 2224, wgrad: 62 us
   // with three stages, 38 with four).
-  const bool narrow = kPair && tail->narrow;
+  const bool narrow = kPair && tail->order.grid.tile_n == kBlockN;
   const uint32_t ring_stages = narrow ? G::kNarrowStages : G::kStages;
   const uint32_t stage_bytes = narrow ? G::kNarrowStageBytes : G::kStageBytes;
   const int row_off = static_cast<int>(cta_rank) * kBlockM;  // this CTA's rows inside a pair tile
@@ -977,7 +970,7 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
         __syncwarp();
       }
       if (lane == 0) {
-        TileWalker<kPair> walk(p, tail, tile_stride);
+        TileWalker<kPair> walk(p, tail);
         TileFeed<kPair> feed(tail, wait, !leader);
         Tile t = {};
         // wgrad: the map slot clipped to the current expert, and for every slot the
@@ -1906,27 +1899,29 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
           emit(o, col_base + (ch + 1) * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
         }
       } else {
-        // All of the accumulator is read and rounded before it leaves.
+        // All of the accumulator is read and rounded before it leaves, two chunks at a time, or (gather
+        // and push kernels, which have 128 registers) one, and the first leaves before the last.
+        constexpr int kAtOnce = GATHER || PUSH ? 1 : 2, kChunks = kBlockN / 64;
+        auto emit_chunk = [&](const uint4* oc, int ch) {
+          emit(oc, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
+        };
         uint4 o[16];
 #pragma unroll
-        for (int ch = 0; ch < kBlockN / 64; ch += 2) {
+        for (int ch = 0; ch < kChunks; ch += kAtOnce) {
+          if (kAtOnce == 1 && ch == kChunks - 1) emit_chunk(o, 0);
           ptx::tmem_ld_32x32(taddr + ch * 32, va);
-          if (!GATHER && !PUSH) ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);  // (those have 128 registers)
+          if (kAtOnce == 2) ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
           ptx::tmem_ld_wait();
-          if (!GATHER && !PUSH && ch + 2 == kBlockN / 64) release();
+          if (ch + kAtOnce == kChunks) release();
           if (scaled) scale(va);
           pack(va, o + ch * 4);
-          if (GATHER || PUSH) {
-            ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
-            ptx::tmem_ld_wait();
-            if (ch + 2 == kBlockN / 64) release();
+          if (kAtOnce == 2) {
+            if (scaled) scale(vb);
+            pack(vb, o + (ch + 1) * 4);
           }
-          if (scaled) scale(vb);
-          pack(vb, o + (ch + 1) * 4);
         }
 #pragma unroll
-        for (int ch = 0; ch < kBlockN / 64; ++ch)
-          emit(o + ch * 4, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
+        for (int ch = kAtOnce == 1 ? 1 : 0; ch < kChunks; ++ch) emit_chunk(o + ch * 4, ch);
       }
       }
     }
@@ -2058,8 +2053,8 @@ schedule_dump_kernel(const int64_t* __restrict__ batch_sizes, const Problem p, i
       }
       *out_count = n;
     };
-    if (p.tile_n > kBlockN) dump(TileWalker<true>(p, &tail, 0));
-    else dump(TileWalker<false>(p, &tail, 0));
+    if (p.tile_n > kBlockN) dump(TileWalker<true>(p, &tail));
+    else dump(TileWalker<false>(p, &tail));
   }
 }
 

@@ -182,7 +182,7 @@ struct TileGrid {
 // Launch order of a pair's `row_tiles` in positions, which is what the grid's `clusters` draw: tiles,
 // and what is left over after whole rounds of wide ones as halves when the halves fit one
 // round, which then lasts half as long.  A half that does not exist (the last column tile
-// may be one accumulator wide) is a position of no units; a launch of `narrow` tiles has none, since
+// may be one accumulator wide) is a position of no units; a launch of narrow tiles has none, since
 // clusters whose draws hit them are left with fewer tiles than others (11 experts, 16933 rows,
 // 2792 x 592, two wide column tiles of which the second is one accumulator: 71 us as narrow tiles, 87 as
 // halves).  (clusters == 0: whole wide tiles.)
@@ -191,9 +191,9 @@ struct TileOrder {
   int whole;  // positions before the halves
   int total;
 };
-B200GMM_HD TileOrder tile_order(const Problem& p, int row_tiles, int clusters, bool narrow) {
+B200GMM_HD TileOrder tile_order(const Problem& p, int row_tiles, int clusters) {
   TileOrder o;
-  if (narrow) {
+  if (clusters > 0 && narrow_tiles(p, row_tiles, clusters)) {
     // half as many row tiles together keep what is in flight about square
     o.grid = TileGrid{p.nt1, kBlockN, p.group_m > 1 ? p.group_m / 2 : 1};
     o.whole = o.total = row_tiles * p.nt1;

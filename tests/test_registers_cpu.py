@@ -1,5 +1,6 @@
-"""The kernels of the gated product run at their register limit (168 a thread with 352 threads); a
-form of the epilogue that holds more than that is compiled without complaint, into spills."""
+"""The kernels of the gated product and the gathered ones of pairs run at their register limit (168 a
+thread with 352 threads, 128 with 512); a form of the epilogue that holds more than that is compiled
+without complaint, into spills."""
 import os
 import re
 import shutil
@@ -17,12 +18,13 @@ using namespace b200gmm;
 const void* kernels[] = {(const void*)gmm_kernel<kNN, 1, false, true>, (const void*)gmm_kernel<kNT, 1, false, true>,
                          (const void*)gmm_kernel<kNN, 2, false, true>, (const void*)gmm_kernel<kNT, 2, false, true>,
                          (const void*)gmm_kernel<kNN, 2, false, true, false, true>,
-                         (const void*)gmm_kernel<kNT, 2, false, true, false, true>};
+                         (const void*)gmm_kernel<kNT, 2, false, true, false, true>,
+                         (const void*)gmm_kernel<kTN, 2, true>, (const void*)gmm_kernel<kNN, 2, true>};
 """
 
 
 @pytest.mark.skipif(not os.path.exists(NVCC), reason="needs nvcc")
-def test_gated_kernels_do_not_spill(tmp_path):
+def test_gated_and_gathered_kernels_do_not_spill(tmp_path):
     source = tmp_path / "gated.cu"
     source.write_text(SOURCE)
     done = subprocess.run([NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "-Xptxas", "-v",
@@ -30,5 +32,5 @@ def test_gated_kernels_do_not_spill(tmp_path):
     assert done.returncode == 0, done.stderr
     spills = re.findall(r"Compiling entry function '(\w*gmm_kernel\w*)'.*?(\d+) bytes spill stores, (\d+) bytes spill loads",
                         done.stderr, re.S)
-    assert len(spills) == 6
+    assert len(spills) == 8
     assert all(stores == loads == "0" for _, stores, loads in spills), spills
