@@ -9,8 +9,9 @@ one more rounding.  The gated product multiplies two such sums: its bound is sta
 
 The rule (b200gmm.cu: swap_rows) goes by the mean rows of an expert, the length of the
 contraction and the number of tiles: every case here lies on a stated side of a line, and
-each line has cases on both sides.  Idle experts make the mean.  Kernels of CTA pairs and
-the gathered product do not have the form; they run the same rows here as plain tiles.
+each line has cases on both sides.  Idle experts make the mean.  The gathered product does
+not have the form, and pairs only in launches of more tiles (test_wide_tiles_gpu.py): they run the same
+rows here as plain tiles.
 """
 import pytest
 import torch
