@@ -1676,253 +1676,253 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
       // one accumulator of 256 columns after the other
 #pragma unroll 1
       for (int unit = 0; unit < (kPair ? t.units : 1); ++unit) {
-      const int unit_col0 = t.col0 + unit * kBlockN;
-      const int r = row_off + q * 32 + lane;  // row inside the (pair) tile
-      bool row_ok = r < t.valid_rows;
-      // row_dest != nullptr (expert-parallel combine fused into this epilogue):
-      // output row i does not go to c[i] but to the address row_dest[i], which may
-      // be a row of a buffer on another GPU; such rows are written with plain
-      // stores by the lane that holds them.
-      const bool scatter = (MODE != kTN) && (row_dest != nullptr);
-      const bool warp_full = !scatter && (row_off + q * 32 + 31) < t.valid_rows;
-      const int64_t out_row0 = (MODE == kTN) ? (int64_t(t.expert) * p.d1 + t.row0) : int64_t(t.row0);
-      // Output geometry: the gated product writes half as many columns as it schedules.
-      const int64_t out_n = SWIGLU ? (p.n >> 1) : p.n;
-      const int out_col0 = SWIGLU ? (unit_col0 >> 1) : unit_col0;
-      __nv_bfloat16* crow = c + (out_row0 + r) * out_n + out_col0;
-      if (scatter && row_ok) {
-        int64_t addr;
-        if (dest_of(out_row0 + r, &addr)) {
-          crow = reinterpret_cast<__nv_bfloat16*>(addr) + out_col0;
-        } else {  // never written: skipped and reported
-          row_ok = false;
-          bad_dest = true;
+        const int unit_col0 = t.col0 + unit * kBlockN;
+        const int r = row_off + q * 32 + lane;  // row inside the (pair) tile
+        bool row_ok = r < t.valid_rows;
+        // row_dest != nullptr (expert-parallel combine fused into this epilogue):
+        // output row i does not go to c[i] but to the address row_dest[i], which may
+        // be a row of a buffer on another GPU; such rows are written with plain
+        // stores by the lane that holds them.
+        const bool scatter = (MODE != kTN) && (row_dest != nullptr);
+        const bool warp_full = !scatter && (row_off + q * 32 + 31) < t.valid_rows;
+        const int64_t out_row0 = (MODE == kTN) ? (int64_t(t.expert) * p.d1 + t.row0) : int64_t(t.row0);
+        // Output geometry: the gated product writes half as many columns as it schedules.
+        const int64_t out_n = SWIGLU ? (p.n >> 1) : p.n;
+        const int out_col0 = SWIGLU ? (unit_col0 >> 1) : unit_col0;
+        __nv_bfloat16* crow = c + (out_row0 + r) * out_n + out_col0;
+        if (scatter && row_ok) {
+          int64_t addr;
+          if (dest_of(out_row0 + r, &addr)) {
+            crow = reinterpret_cast<__nv_bfloat16*>(addr) + out_col0;
+          } else {  // never written: skipped and reported
+            row_ok = false;
+            bad_dest = true;
+          }
         }
-      }
-      const int tile_row = static_cast<int>(out_row0) + row_off + q * 32;  // first row of this warp
-      const int cols_left = static_cast<int>(out_n) - out_col0;  // multiple of 8
-      // Scatter mode with per-row weights (the router's top-k weight of this row).
-      const bool scaled = scatter && row_scale != nullptr;
-      const float row_w = (scaled && row_ok) ? row_scale[out_row0 + r] : 1.0f;
-      auto scale = [&](uint32_t (&v)[32]) {
+        const int tile_row = static_cast<int>(out_row0) + row_off + q * 32;  // first row of this warp
+        const int cols_left = static_cast<int>(out_n) - out_col0;  // multiple of 8
+        // Scatter mode with per-row weights (the router's top-k weight of this row).
+        const bool scaled = scatter && row_scale != nullptr;
+        const float row_w = (scaled && row_ok) ? row_scale[out_row0 + r] : 1.0f;
+        auto scale = [&](uint32_t (&v)[32]) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * row_w);
-      };
-      uint32_t va[32], vb[32];
-      if (MODE == kTN && nkb == 0) {  // (forward and dgrad tiles always have k > 0)
-        // Empty wgrad expert: its block of the output is zeros.
-        if (G::kWideOut && warp_full) {
-          // Zeros need staging once: every store of this tile reads the same buffer,
-          // so none of them waits for the one before.
-          const uint32_t buf = stage_buf();
-          if (lane == 0 && stores > 0) ptx::bulk_wait_group_read<G::kOutBufs - 1>();
-          __syncwarp();
-          const uint32_t row_addr = buf + uint32_t(lane) * 128u;
+          for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * row_w);
+        };
+        uint32_t va[32], vb[32];
+        if (MODE == kTN && nkb == 0) {  // (forward and dgrad tiles always have k > 0)
+          // Empty wgrad expert: its block of the output is zeros.
+          if (G::kWideOut && warp_full) {
+            // Zeros need staging once: every store of this tile reads the same buffer,
+            // so none of them waits for the one before.
+            const uint32_t buf = stage_buf();
+            if (lane == 0 && stores > 0) ptx::bulk_wait_group_read<G::kOutBufs - 1>();
+            __syncwarp();
+            const uint32_t row_addr = buf + uint32_t(lane) * 128u;
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(row_addr + (uint32_t(j) << 4)), "r"(0u)
-                         : "memory");
-          ptx::fence_proxy_async_smem();
+            for (int j = 0; j < 8; ++j)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(row_addr + (uint32_t(j) << 4)), "r"(0u)
+                           : "memory");
+            ptx::fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+#pragma unroll 1
+              for (int ch = 0; ch < kBlockN / 128; ++ch) {
+                const int col = col_base + ch * 64;
+                if (col < cols_left) ptx::tma_store_2d(&map_c, buf, unit_col0 + col, tile_row);
+              }
+              ptx::bulk_commit_group();
+            }
+            ++stores;
+            continue;
+          }
+          const uint4 zeros[4] = {};
+#pragma unroll 1
+          for (int ch = 0; ch < kBlockN / 64; ++ch)
+            emit(zeros, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
+          continue;
+        }
+        // Gated backward: 32 columns of this lane's row of the output gradient.
+        auto load_grad = [&](uint4 (&d4)[4], int col) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) d4[j] = make_uint4(0u, 0u, 0u, 0u);
+          if (!row_ok) return;
+          const uint4* src = reinterpret_cast<const uint4*>(gate_grad + (out_row0 + r) * out_n + out_col0 + col);
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (col + j * 8 < cols_left) d4[j] = src[j];
+        };
+        const bool backward = SWIGLU && gate_grad != nullptr;
+        // (a pair reads it a chunk ahead, the first before it waits for the accumulator)
+        uint4 d4[4];
+        if (kPair && backward) load_grad(d4, half * 64);
+        const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
+        ++it;
+        if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), aph, wait)) { ok = false; break; }
+        ptx::tc_fence_after_sync();
+        // A pair's accumulator is read and rounded as a whole and handed back; only then do its values
+        // leave through the staging buffer, where each chunk waits for the store before it.
+        auto release = [&]() {
+          ptx::tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) {
-#pragma unroll 1
-            for (int ch = 0; ch < kBlockN / 128; ++ch) {
-              const int col = col_base + ch * 64;
-              if (col < cols_left) ptx::tma_store_2d(&map_c, buf, unit_col0 + col, tile_row);
-            }
-            ptx::bulk_commit_group();
+            const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
+            if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(te_bar, 0));
+            else ptx::mbar_arrive(te_bar);
           }
-          ++stores;
+        };
+        if (SWIGLU) {
+          // This warp's 64 of the tile's 128 output columns: gate from accumulator
+          // columns [64 half, +64), up from the same columns of the second half.
+          const uint32_t tg = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + half * 64;
+          // silu(g) * u of 32 columns, to va
+          auto gated = [&]() {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const float g = __uint_as_float(va[i]);
+              const float u = __uint_as_float(vb[i]);
+              va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * u);
+            }
+            if (scaled) scale(va);
+          };
+          // Backward of the gated product: with g, u recomputed in the accumulator and dh the output
+          // gradient, the gradients w.r.t. the two products
+          //   dg = dh * u * silu'(g),  silu'(g) = s (1 + g (1 - s)),  s = 1 / (1 + exp(-g))
+          //   du = dh * silu(g)
+          // (to va and vb) go to rows [0, T) and [T, 2T) of the output.
+          auto gradients = [&](const uint4 (&dh4)[4]) {
+            const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(dh4);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const float g = __uint_as_float(va[i]);
+              const float u = __uint_as_float(vb[i]);
+              const float2 dpair = __bfloat1622float2(d2[i >> 1]);
+              const float dh = (i & 1) ? dpair.y : dpair.x;
+              const float sg = __fdividef(1.0f, 1.0f + __expf(-g));
+              va[i] = __float_as_uint(dh * u * sg * (1.0f + g * (1.0f - sg)));
+              vb[i] = __float_as_uint(dh * g * sg);
+            }
+          };
+          auto emit_gate = [&](const uint4* o, int ch) {
+            emit(o, half * 64 + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, out_col0);
+          };
+          auto emit_up = [&](const uint4* o, int ch) {
+            emit(o, half * 64 + ch * 32, warp_full, row_ok, crow + p.tokens * out_n, cols_left,
+                 tile_row + static_cast<int>(p.tokens), out_col0);
+          };
+          auto load = [&](int ch) {
+            ptx::tmem_ld_32x32(tg + ch * 32, va);
+            ptx::tmem_ld_32x32(tg + kBlockN / 2 + ch * 32, vb);
+            ptx::tmem_ld_wait();
+            if (ch == 1) release();
+          };
+          if constexpr (!kPair) {
+            uint4 o[4];
+#pragma unroll 1
+            for (int ch = 0; ch < 2; ++ch) {
+              load(ch);
+              if (backward) {
+                load_grad(d4, half * 64 + ch * 32);
+                gradients(d4);
+                pack(va, o);
+                emit_gate(o, ch);
+                pack(vb, o);
+                emit_up(o, ch);
+              } else {
+                gated();
+                pack(va, o);
+                emit_gate(o, ch);
+              }
+            }
+          } else if (backward) {
+            // The accumulator is read before all of the first chunk's results have left; holding the
+            // second's too took more registers than there are (168: 44 bytes of spill stores, 100 of
+            // loads).
+            uint4 o[4], o2[4];
+            load(0);
+            gradients(d4);
+            load_grad(d4, half * 64 + 32);
+            pack(va, o);
+            pack(vb, o2);
+            emit_gate(o, 0);
+            load(1);
+            emit_up(o2, 0);
+            gradients(d4);
+            pack(va, o);
+            pack(vb, o2);
+            emit_gate(o, 1);
+            emit_up(o2, 1);
+          } else {
+            uint4 o[8];
+#pragma unroll
+            for (int ch = 0; ch < 2; ++ch) {
+              load(ch);
+              gated();
+              pack(va, o + ch * 4);
+            }
+            emit_gate(o, 0);
+            emit_gate(o + 4, 1);
+          }
           continue;
         }
-        const uint4 zeros[4] = {};
-#pragma unroll 1
-        for (int ch = 0; ch < kBlockN / 64; ++ch)
-          emit(zeros, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
-        continue;
-      }
-      // Gated backward: 32 columns of this lane's row of the output gradient.
-      auto load_grad = [&](uint4 (&d4)[4], int col) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) d4[j] = make_uint4(0u, 0u, 0u, 0u);
-        if (!row_ok) return;
-        const uint4* src = reinterpret_cast<const uint4*>(gate_grad + (out_row0 + r) * out_n + out_col0 + col);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (col + j * 8 < cols_left) d4[j] = src[j];
-      };
-      const bool backward = SWIGLU && gate_grad != nullptr;
-      // (a pair reads it a chunk ahead, the first before it waits for the accumulator)
-      uint4 d4[4];
-      if (kPair && backward) load_grad(d4, half * 64);
-      const uint32_t ab = it & 1u, aph = (it >> 1) & 1u;
-      ++it;
-      if (!ptx::mbar_wait<false, 64>(ptx::smem_u32(&tail->tmem_full[ab]), aph, wait)) { ok = false; break; }
-      ptx::tc_fence_after_sync();
-      // A pair's accumulator is read and rounded as a whole and handed back; only then do its values
-      // leave through the staging buffer, where each chunk waits for the store before it.
-      auto release = [&]() {
-        ptx::tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) {
-          const uint32_t te_bar = ptx::smem_u32(&tail->tmem_empty[ab]);
-          if (kPair) ptx::mbar_arrive_cluster(ptx::mapa(te_bar, 0));
-          else ptx::mbar_arrive(te_bar);
-        }
-      };
-      if (SWIGLU) {
-        // This warp's 64 of the tile's 128 output columns: gate from accumulator
-        // columns [64 half, +64), up from the same columns of the second half.
-        const uint32_t tg = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + half * 64;
-        // silu(g) * u of 32 columns, to va
-        auto gated = [&]() {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float g = __uint_as_float(va[i]);
-            const float u = __uint_as_float(vb[i]);
-            va[i] = __float_as_uint(__fdividef(g, 1.0f + __expf(-g)) * u);
-          }
-          if (scaled) scale(va);
-        };
-        // Backward of the gated product: with g, u recomputed in the accumulator and dh the output
-        // gradient, the gradients w.r.t. the two products
-        //   dg = dh * u * silu'(g),  silu'(g) = s (1 + g (1 - s)),  s = 1 / (1 + exp(-g))
-        //   du = dh * silu(g)
-        // (to va and vb) go to rows [0, T) and [T, 2T) of the output.
-        auto gradients = [&](const uint4 (&dh4)[4]) {
-          const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(dh4);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float g = __uint_as_float(va[i]);
-            const float u = __uint_as_float(vb[i]);
-            const float2 dpair = __bfloat1622float2(d2[i >> 1]);
-            const float dh = (i & 1) ? dpair.y : dpair.x;
-            const float sg = __fdividef(1.0f, 1.0f + __expf(-g));
-            va[i] = __float_as_uint(dh * u * sg * (1.0f + g * (1.0f - sg)));
-            vb[i] = __float_as_uint(dh * g * sg);
-          }
-        };
-        auto emit_gate = [&](const uint4* o, int ch) {
-          emit(o, half * 64 + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, out_col0);
-        };
-        auto emit_up = [&](const uint4* o, int ch) {
-          emit(o, half * 64 + ch * 32, warp_full, row_ok, crow + p.tokens * out_n, cols_left,
-               tile_row + static_cast<int>(p.tokens), out_col0);
-        };
-        auto load = [&](int ch) {
-          ptx::tmem_ld_32x32(tg + ch * 32, va);
-          ptx::tmem_ld_32x32(tg + kBlockN / 2 + ch * 32, vb);
-          ptx::tmem_ld_wait();
-          if (ch == 1) release();
-        };
+        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + col_base;
         if constexpr (!kPair) {
-          uint4 o[4];
+          // Chunk by chunk, each as soon as it is read, the next one's load in flight meanwhile: the other
+          // accumulator is being filled, and registers for all of this one would gain nothing.
+          if (G::kWideOut && warp_full) {
 #pragma unroll 1
-          for (int ch = 0; ch < 2; ++ch) {
-            load(ch);
-            if (backward) {
-              load_grad(d4, half * 64 + ch * 32);
-              gradients(d4);
+            for (int ch = 0; ch < kBlockN / 64; ch += 2) {
+              ptx::tmem_ld_32x32(taddr + ch * 32, va);
+              ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
+              ptx::tmem_ld_wait();
+              if (ch + 2 == kBlockN / 64) release();
+              uint4 o[8];
               pack(va, o);
-              emit_gate(o, ch);
-              pack(vb, o);
-              emit_up(o, ch);
-            } else {
-              gated();
-              pack(va, o);
-              emit_gate(o, ch);
+              pack(vb, o + 4);
+              if (col_base + ch * 32 < cols_left) emit64(o, col_base + ch * 32, tile_row, unit_col0);
             }
+            continue;
           }
-        } else if (backward) {
-          // The accumulator is read before all of the first chunk's results have left; holding the
-          // second's too took more registers than there are (168: 44 bytes of spill stores, 100 of
-          // loads).
-          uint4 o[4], o2[4];
-          load(0);
-          gradients(d4);
-          load_grad(d4, half * 64 + 32);
-          pack(va, o);
-          pack(vb, o2);
-          emit_gate(o, 0);
-          load(1);
-          emit_up(o2, 0);
-          gradients(d4);
-          pack(va, o);
-          pack(vb, o2);
-          emit_gate(o, 1);
-          emit_up(o2, 1);
-        } else {
-          uint4 o[8];
-#pragma unroll
-          for (int ch = 0; ch < 2; ++ch) {
-            load(ch);
-            gated();
-            pack(va, o + ch * 4);
-          }
-          emit_gate(o, 0);
-          emit_gate(o + 4, 1);
-        }
-        continue;
-      }
-      const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + ab * kBlockN + col_base;
-      if constexpr (!kPair) {
-        // Chunk by chunk, each as soon as it is read, the next one's load in flight meanwhile: the other
-        // accumulator is being filled, and registers for all of this one would gain nothing.
-        if (G::kWideOut && warp_full) {
+          uint4 o[4];
+          ptx::tmem_ld_32x32(taddr, va);
 #pragma unroll 1
           for (int ch = 0; ch < kBlockN / 64; ch += 2) {
-            ptx::tmem_ld_32x32(taddr + ch * 32, va);
-            ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
             ptx::tmem_ld_wait();
-            if (ch + 2 == kBlockN / 64) release();
-            uint4 o[8];
+            ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
+            if (scaled) scale(va);
             pack(va, o);
-            pack(vb, o + 4);
-            if (col_base + ch * 32 < cols_left) emit64(o, col_base + ch * 32, tile_row, unit_col0);
-          }
-          continue;
-        }
-        uint4 o[4];
-        ptx::tmem_ld_32x32(taddr, va);
-#pragma unroll 1
-        for (int ch = 0; ch < kBlockN / 64; ch += 2) {
-          ptx::tmem_ld_wait();
-          ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
-          if (scaled) scale(va);
-          pack(va, o);
-          emit(o, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
-          ptx::tmem_ld_wait();
-          if (ch + 2 < kBlockN / 64) ptx::tmem_ld_32x32(taddr + (ch + 2) * 32, va);
-          else release();
-          if (scaled) scale(vb);
-          pack(vb, o);
-          emit(o, col_base + (ch + 1) * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
-        }
-      } else {
-        // All of the accumulator is read and rounded before it leaves, two chunks at a time, or (gather
-        // and push kernels, which have 128 registers) one, and the first leaves before the last.
-        constexpr int kAtOnce = GATHER || PUSH ? 1 : 2, kChunks = kBlockN / 64;
-        auto emit_chunk = [&](const uint4* oc, int ch) {
-          emit(oc, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
-        };
-        uint4 o[16];
-#pragma unroll
-        for (int ch = 0; ch < kChunks; ch += kAtOnce) {
-          if (kAtOnce == 1 && ch == kChunks - 1) emit_chunk(o, 0);
-          ptx::tmem_ld_32x32(taddr + ch * 32, va);
-          if (kAtOnce == 2) ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
-          ptx::tmem_ld_wait();
-          if (ch + kAtOnce == kChunks) release();
-          if (scaled) scale(va);
-          pack(va, o + ch * 4);
-          if (kAtOnce == 2) {
+            emit(o, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
+            ptx::tmem_ld_wait();
+            if (ch + 2 < kBlockN / 64) ptx::tmem_ld_32x32(taddr + (ch + 2) * 32, va);
+            else release();
             if (scaled) scale(vb);
-            pack(vb, o + (ch + 1) * 4);
+            pack(vb, o);
+            emit(o, col_base + (ch + 1) * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
           }
-        }
+        } else {
+          // All of the accumulator is read and rounded before it leaves, two chunks at a time, or (gather
+          // and push kernels, which have 128 registers) one, and the first leaves before the last.
+          constexpr int kAtOnce = GATHER || PUSH ? 1 : 2, kChunks = kBlockN / 64;
+          auto emit_chunk = [&](const uint4* oc, int ch) {
+            emit(oc, col_base + ch * 32, warp_full, row_ok, crow, cols_left, tile_row, unit_col0);
+          };
+          uint4 o[16];
 #pragma unroll
-        for (int ch = kAtOnce == 1 ? 1 : 0; ch < kChunks; ++ch) emit_chunk(o + ch * 4, ch);
-      }
+          for (int ch = 0; ch < kChunks; ch += kAtOnce) {
+            if (kAtOnce == 1 && ch == kChunks - 1) emit_chunk(o, 0);
+            ptx::tmem_ld_32x32(taddr + ch * 32, va);
+            if (kAtOnce == 2) ptx::tmem_ld_32x32(taddr + (ch + 1) * 32, vb);
+            ptx::tmem_ld_wait();
+            if (ch + kAtOnce == kChunks) release();
+            if (scaled) scale(va);
+            pack(va, o + ch * 4);
+            if (kAtOnce == 2) {
+              if (scaled) scale(vb);
+              pack(vb, o + (ch + 1) * 4);
+            }
+          }
+#pragma unroll
+          for (int ch = kAtOnce == 1 ? 1 : 0; ch < kChunks; ++ch) emit_chunk(o + ch * 4, ch);
+        }
       }
     }
     // Shared memory must outlive the stores that still read it.
