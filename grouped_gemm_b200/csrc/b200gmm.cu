@@ -306,61 +306,68 @@ struct Features {
   bool scatter = false;  // row_dest: rows of the result go where a table says
 };
 
+constexpr int kNeverWide = 1000;  // Problem::wide_cost: every tile one accumulator wide
+
+// Problem::wide_cost, what two rounds of narrow tiles cost as a round of wide ones, in percent.
+// Rows that start at any 16 bytes are bound by the bytes that enter an SM, of which a
+// wide tile has three quarters (7 experts, 3001 rows, 1000 x 2504: 26.4 / 23.0 us); others by power,
+// and by little else.  The gated backward's epilogue, which reads a gradient and writes two, leaves
+// nothing to gain (16 experts of 1024 rows, 2048 x 4096: wide 561 us, narrow 540).  A gathered product
+// copies its rows 16 bytes at a time, which a wide tile does half as often (67 experts of 206 rows, 13024 x
+// 280: 260 / 211; 18 experts, 34044 rows, 3592 x 552: 250 / 213).  Scattered rows leave in 64-byte
+// copies: while an accumulator's are sent the other one has to wait, unless the contraction is long
+// (16384 rows, 8 experts, 4096 x 14336: 1573 / 1660; 14336 x 4096, 8192 rows: 892 / 855).
+int wide_cost(const Features& f, int64_t d1, bool trans_a, bool ragged) {
+  if (f.scatter && d1 < 8192) return kNeverWide;
+  if (trans_a) return 97;
+  if (f.gather) return 70;
+  return ragged ? 80 : (f.gated_backward ? 100 : 97);
+}
+
 // Which variant a problem runs on.  Only shapes known on the host may decide
 // (batch_sizes can live on the device).  B200GMM_CTAS=1|2 overrides.
 //
-// What bounds the choice is bytes into the SMs: per k-block an SM loads 48 KiB for 128 x 256
-// outputs (one CTA), 48 KiB for 128 x 512 (a pair's tile) or 32 KiB for 128 x 256 (half of one).
-// rounds_one and rounds_pair are these bytes (/ 16 KiB) over the rounds of tiles that the
-// grid makes, for experts of even size, half a row tile of each idle.  Times of the kernels
-// follow their ratio, times a factor for the path (8 or 64 experts, 64 to 1024 rows each):
-//   rows that start at any 16 bytes (a row is then two lines of L2 where it could be one):
-//     about 0.8 to 1; z = 64, 128 rows, 4088 x 8184: ratio 1.5, forward 1351 / 933 us; 512 rows: 1.8, 3769 /
-//     2282; z = 7, 428 rows, 1000 x 2504: 1.2, 28.0 / 23.0 or, other sizes, 31.5; z = 8, 128 rows: 1.0,
-//     17.4 / 21.5.
-//   others: 0.55, the L2 being no bound; z = 64, 512 rows, 2048 x 4096: 1.81, 564 / 608 us; z = 8,
-//     1024 rows: 2.0, 135 / 129; z = 8, 512 rows, dgrad: 1.2, 68 / 90.  From 1024 rows on the power
-//     cap adds to it (17 experts of 1548 rows, dgrad 7344 -> 520: 1.67, 309 / 248).
-// Many experts (128 and more) are hardly ever of even size, and swapped tiles take the
-// small ones: z = 256, 256 rows, 7168 x 2048, Zipf routing: ratio 1.67, 2383 / 2244 us, dgrad
-// 2322 / 2152 (even sizes: 3 % slower).  The gathered product has no swapped tiles, and its row
-// copies are 16 bytes in any case: from 512 rows on (146 experts of 126 rows, 6712 x 2496: 1185 / 1487; 16 of
-// 386, 1416 x 11392: 258 / 279).
-// A short contraction leaves an accumulator little time to be read out while the other one
-// fills, which a pair's tile does not have: one CTA below 416 (any 16 bytes) and 512 (49 experts, 98681
-// rows, 72 x 2000: 159 / 101 us; 173, 110139, 128 x 856: 113 / 77; 81, 68558, 432 x 2608: 240 / 223),
-// and below 128 rows an expert up to 2048 (123 experts, 11149 rows, 528 x 1624: 64 / 81).  Scattered rows
-// run in halves there (narrow_rounds): from 512 rows on.
-// Few tiles: where one-CTA tiles fill no more than one round, experts of less than 384 rows leave
-// too much of a pair's tile idle (one of 322 rows, 5976 x 4736: 37 / 63 us; of 428: 30 / 25).
+// A one-CTA tile and a pair's narrow one are as much work for an SM, 128 x 256 outputs, so the rounds of tiles
+// that the grid makes compare them, for experts of even size, half a row tile of each idle.  What
+// a pair's round costs less for is bytes: per k-block an SM loads 48 KiB for 128 x 256 outputs (one CTA), 32 (a
+// pair's narrow tile) or 24 (wide).  What is saved by that depends on how busy memory and the
+// power supply are.
+//   512 rows an expert and more: pairs, 0.76 to 1 of the time of one-CTA tiles (19 experts, 54879 rows,
+//     9736 x 96: 371 us one-CTA, 284; 2 of 33358, 2248 x 1120: 410 / 339), unless one-CTA tiles make far fewer
+//     rounds (one of 1084, 552 x 1936, gated: 11.2 / 18.7).
+//   128 to 511 rows: pairs only for rows that start at any 16 bytes, which are two lines of L2 where
+//     they could be one (64 experts of 128 rows, 4088 x 8184: 1351 / 933; 7 of 428, dgrad 2504 -> 1000: 29.7 / 25.0), where
+//     they make a tenth less by this reckoning, and not where one-CTA tiles are one round of fewer
+//     than 384 rows each.  Others lose (200 experts of 150 rows, Zipf, 512 x 512: 37.9 / 46.1, gated 59.8 / 80.6;
+//     256 of 256, Zipf, 7168 x 2048: 2123 / 2259, dgrad 2157 / 2176, gated 4055 / 4412).  So do the gathered product
+//     (146 of 126, 6712 x 2496: 1185 / 1487), scattered rows (64 of 116, 1864 x 2872: 199 / 204) and the gated
+//     backward (16 of 386, 1416 x 11392: 547 / 584).
+//   A short contraction leaves an accumulator little time to be read out while the other one
+//     fills, which a pair's wide tile does not have: one CTA below 416 (any 16 bytes) and 512 (49 experts,
+//     98681 rows, 72 x 2000: 101 / 159; 81, 68558, 432 x 2608: 223 / 240; 173, 110139, 128 x 856: 77 / 113).
 // wgrad loads its operands for as many k-blocks as an expert has rows, and writes as much in
-// either form: the line lies at 384 rows (any 16 bytes: 0.98 at 256, 1.17 at 512) and 512
-// (0.9 and 1.02).
-int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b, const Features& f = Features()) {
+// either form: the line lies at 512 rows (0.9 at 256 and 1.02 at 512; 18 experts, 34044 rows, 3592 x 552:
+// 273 / 214; 7, 3001, 1000 x 2504: 34.2 / 35.2).
+int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b, const Features& f = Features(),
+                const DeviceInfo* dev = nullptr) {
   const int forced = env_int("B200GMM_CTAS", 0);
   if (forced == 1 || forced == 2) return forced;
-  if (z <= 0 || tokens <= 0 || d1 <= 0 || n <= 0) return 1;
-  constexpr int64_t kSms = 148, kPairs = kSms / 2;
-  const bool ragged = ragged_rows(d1, f.swiglu ? n / 2 : n, trans_b);
-  const int64_t nt = (n + kBlockN - 1) / kBlockN;
-  const auto tiles = [&](int64_t tile_m, int64_t cols) {
-    return trans_a ? z * ((d1 + tile_m - 1) / tile_m) * cols
-                   : (2 * tokens / tile_m + std::min<int64_t>(z, tokens)) * cols / 2;
-  };
+  if (z <= 0 || tokens <= 0 || d1 <= 0 || n <= 0 || std::max(tokens, n) > (int64_t(1) << 32)) return 1;  // (refused later)
   const auto rows_from = [&](int64_t mean) { return tokens >= mean * int64_t(z); };
-  const int64_t one = tiles(kBlockM, nt), pair = tiles(2 * kBlockM, (nt + 1) / 2);
-  const int64_t left = pair % kPairs;
-  const int64_t rounds_one = 3 * ((one + kSms - 1) / kSms);
-  const int64_t rounds_pair = nt == 1 ? 2 * ((pair + kPairs - 1) / kPairs)
-                                      : 3 * (pair / kPairs) + (left == 0 ? 0 : (2 * left <= kPairs ? 2 : 3));
-  const double ratio = double(rounds_one) / double(std::max<int64_t>(rounds_pair, 1));
-  if (trans_a) return rows_from(ragged && !f.gather ? 384 : 512) && d1 >= 256 && ratio >= 1.5 ? 2 : 1;
-  if (d1 < (ragged ? 416 : 512) || (one <= kSms && !rows_from(384))) return 1;
-  if (!rows_from(f.gather ? 512 : f.gated_backward ? 256 : (d1 < 2048 ? 128 : 64))) return 1;
-  if (f.scatter && d1 < 8192) return rows_from(512) ? 2 : 1;
-  if (nt == 1) return ratio >= 1.25 && (ragged || rows_from(512)) ? 2 : 1;
-  if (ragged) return ratio >= 1.25 ? 2 : 1;
-  return ratio >= (rows_from(1024) || (z >= 128 && !f.gather && !f.gated_backward) ? 1.6 : 1.85) ? 2 : 1;
+  if (trans_a) return rows_from(512) && d1 >= 256 ? 2 : 1;
+  const bool ragged = ragged_rows(d1, f.swiglu ? n / 2 : n, trans_b);
+  if (d1 < (ragged ? 416 : 512)) return 1;
+  if (!rows_from(512) && (!ragged || !rows_from(128) || f.gather || f.scatter || f.gated_backward)) return 1;
+  const int64_t sms = dev != nullptr ? dev->sm_count : 148, pairs = std::max<int64_t>(dev != nullptr ? dev->pair_ctas / 2 : 74, 1);
+  const auto row_tiles = [&](int64_t rows) {  // of experts of even size, half a tile of each idle
+    return z == 1 ? (tokens + rows - 1) / rows : tokens / rows + std::min<int64_t>(z, tokens) / 2;
+  };
+  const int64_t nt = (n + kBlockN - 1) / kBlockN, one_tiles = row_tiles(kBlockM) * nt, pair_rows = row_tiles(2 * kBlockM);
+  if (one_tiles <= sms && !rows_from(384)) return 1;
+  const int64_t one = 125 * rounds_narrow(one_tiles, sms);
+  const int64_t pair = std::min(100 * rounds_narrow(pair_rows * nt, pairs),
+                                wide_cost(f, d1, false, ragged) * rounds_wide(pair_rows * ((nt + 1) / 2), pairs));
+  return rows_from(512) ? (112 * one < 100 * pair ? 1 : 2) : (100 * pair < 90 * one ? 2 : 1);
 }
 
 // Which launches run their tiles of few rows with swapped operands (schedule.cuh), and up
@@ -386,11 +393,12 @@ int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int t
 // which reads its gradient row by row there (104 and 222 us at 40 rows, k = 512).
 // A pair's tiles of up to 192 of 256 rows: the last row tile of an expert, and all of a small
 // expert.  Time without / with:
-//   256 experts of 256 rows on average, Zipf, 7168 x 2048: 2480 / 2244 us, dgrad 2486 / 2152 (one-CTA tiles:
-//     2383, 2322); 64 experts of 64 rows, 4088 x 8184: 942 / 815.
+//   256 experts of 256 rows on average, Zipf, 7168 x 2048: 2480 / 2244 us, dgrad 2486 / 2152; 64 experts of 64
+//     rows, 4088 x 8184: 942 / 815; below 512 rows, over drawn sizes: forward and gated 1.02, dgrad 1.06.
 //   large experts (8 of 1024 rows, 4096 x 14336): gated product 1676 / 1599 us, scattered rows 887 / 867,
-//     forward 815 / 822, dgrad 812 / 844; of 4096: forward 2910 / 2877, dgrad 2934 / 3055.  So NN up to 2048 rows
-//     and NT up to 512.
+//     forward 815 / 822 (1.04 in another run), dgrad 812 / 844; of 4096: forward 2910 / 2877, dgrad 2934 / 3055.
+//     Drawn sizes: forward and gated 1.01 to 1.02 from 512 to 2048 rows, 0.98 to 1.0 above; dgrad even.  So NN up
+//     to 2048 rows and NT up to 512.
 //   few tiles: one pair's pipeline is the bound, as above (322 rows, one expert, 5976 x 4736: 37 us with
 //     one-CTA tiles, 63 with this): a tile for every SM.
 int swap_rows(const Problem& p, const Features& f, int ctas, int sm_count) {
@@ -405,8 +413,6 @@ int swap_rows(const Problem& p, const Features& f, int ctas, int sm_count) {
   if (!f.scatter && p.d1 < kPlainMinK) return 0;
   return p.tokens <= kMeanRows * p.z && 2 * tiles >= sm_count ? kBlockM / 2 : 0;
 }
-
-constexpr int kNeverWide = 1000;  // Problem::wide_cost: every tile one accumulator wide
 
 int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int trans_b, int ctas,
                   Problem* p, const Features& f = Features()) {
@@ -445,15 +451,9 @@ int check_problem(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int
   p->light = (p->mode != kTN && ctas == 1 && !f.gather && !f.swiglu) ? env_int("B200GMM_LIGHT", 0) : 0;
   // A pair's tiles two accumulators wide or one (narrow_tiles).  wgrad's are as long as their expert has
   // rows: with few a CTA and experts of 2048 rows and more the long ones end the launch (11 experts,
-  // 126529 rows, 4144 x 576: 712 us with tiles of 256 columns, 872 with 512).  Rows that start at any 16 bytes
-  // are bound by bytes, which wide tiles save (7 experts, 3001 rows, 1000 x 2504: 26.4 / 23.0).  Scattered
-  // rows leave in 64-byte copies: while an accumulator's are sent the other one has to wait,
-  // unless the contraction is long (16384 rows, 8 experts, 4096 x 14336: 1573 / 1660; 14336 x 4096, 8192
-  // rows: 892 / 855).
+  // 126529 rows, 4144 x 576: 712 us with tiles of 256 columns, 872 with 512).
   p->narrow_rounds = trans_a && tokens >= 2048 * int64_t(z) ? 16 : 0;
-  p->wide_cost = 97;
-  if (!trans_a && ragged_rows(d1, f.swiglu ? n / 2 : n, trans_b)) p->wide_cost = 80;
-  if (f.scatter && d1 < 8192) p->wide_cost = kNeverWide;
+  p->wide_cost = wide_cost(f, d1, trans_a != 0, ragged_rows(d1, f.swiglu ? n / 2 : n, trans_b));
   p->swap_units = 1;
   p->swap_rows = 0;  // decided where the device is known (settle)
   p->dest_indexed = 0;
@@ -644,7 +644,10 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
   feat.swiglu = swiglu;
   feat.gated_backward = gate_grad != nullptr;
   feat.scatter = row_dest != nullptr;
-  int ctas = prepared != nullptr ? 1 : choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b, feat);
+  // (a call that does nothing needs no device)
+  DeviceInfo* dev = nullptr;
+  const int dev_rc = z > 0 && tokens > 0 && dim_a1 > 0 && n > 0 ? device_info(&dev) : B200GMM_OK;
+  int ctas = prepared != nullptr ? 1 : choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b, feat, dev);
   int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, feat);
   if (rc != B200GMM_OK) return rc;
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
@@ -682,9 +685,7 @@ int run_impl(const void* a, const void* b, void* c, const int64_t* batch_sizes,
       (reinterpret_cast<uintptr_t>(c) & 15))
     return B200GMM_EALIGN;
 
-  DeviceInfo* dev = nullptr;
-  rc = device_info(&dev);
-  if (rc != B200GMM_OK) return rc;
+  if (dev_rc != B200GMM_OK) return dev_rc;
 
   if (ctas == 2 && dev->pair_ctas < 2) {
     ctas = 1;
@@ -1191,7 +1192,10 @@ int b200gmm_launch_forms(const int64_t* batch_sizes_host, int z, int64_t tokens,
   f.scatter = (features & B200GMM_FORM_SCATTER) != 0;
   if (n < 0 || (f.swiglu && (trans_a || f.gather)) || (f.scatter && trans_a)) return B200GMM_EINVAL;
   if (f.swiglu) n *= 2;
-  int ctas = choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b, f);
+  DeviceInfo dev;
+  dev.sm_count = sm_count;
+  dev.pair_ctas = pair_ctas;
+  int ctas = choose_ctas(z, tokens, dim_a1, n, trans_a, trans_b, f, &dev);
   if (pair_ctas < 2) ctas = 1;
   Problem p;
   const int rc = check_problem(z, tokens, dim_a1, n, trans_a, trans_b, ctas, &p, f);

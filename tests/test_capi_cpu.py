@@ -155,6 +155,29 @@ def test_schedule_covers_rows_and_columns_once(sizes, trans_b, n, ctas, light, m
     assert (cover == 1).all()
 
 
+# z, rows, k, n, layout, features, CTAs a tile: the faster of the two on a B200 by a tenth and more
+CHOICES = [
+    (200, 30000, 512, 512, "nn", 0, 1), (200, 30000, 512, 512, "nn", _capi.FORM_GATED, 1),
+    (256, 65536, 7168, 2048, "nn", 0, 1), (256, 65536, 7168, 2048, "nn", _capi.FORM_GATED, 1),
+    (1, 1041, 2200, 4120, "nn", 0, 2), (1, 1041, 2200, 4120, "nn", _capi.FORM_GATED, 2),
+    (19, 54879, 9736, 96, "nn", 0, 2), (19, 54879, 9736, 96, "nn", _capi.FORM_SCATTER, 2),
+    (16, 6170, 1416, 11392, "nn", _capi.FORM_GATED_BACKWARD, 1), (16, 6170, 1416, 11392, "nn", _capi.FORM_GATHER, 1),
+    (64, 8192, 4088, 8184, "nn", 0, 2), (64, 8192, 4088, 8184, "nt", 0, 2), (7, 3001, 2504, 1000, "nt", 0, 2),
+    (49, 98681, 72, 2000, "nn", 0, 1), (9, 1966, 952, 128, "nn", 0, 1),
+    (18, 34044, 3592, 552, "tn", 0, 2), (25, 100842, 368, 5768, "tn", 0, 2), (7, 22823, 880, 1344, "tn", 0, 2),
+    (7, 3001, 1000, 2504, "tn", 0, 1), (8, 32768, 4096, 14336, "nn", 0, 2), (8, 32768, 4096, 14336, "tn", 0, 2),
+]
+
+
+@pytest.mark.parametrize("z,rows,k,n,layout,features,ctas", CHOICES)
+def test_choice_between_one_cta_and_pairs(z, rows, k, n, layout, features, ctas, monkeypatch):
+    monkeypatch.delenv("B200GMM_CTAS", raising=False)
+    sizes = [rows // z + (i < rows % z) for i in range(z)]
+    assert _capi.launch_forms(sizes, k, n, layout == "tn", layout == "nt", features).ctas == ctas
+    # a device on which pairs do not fit has none, and the device's own count of pairs is what is asked
+    assert _capi.launch_forms(sizes, k, n, layout == "tn", layout == "nt", features, pair_ctas=0).ctas == 1
+
+
 @pytest.mark.parametrize("sizes", SIZE_SETS + [[256 * (t // 2) - 7, 256 * (t - t // 2) - 100] for t in (25, 37, 62, 150)])
 @pytest.mark.parametrize("n", [256, 264, 776, 1288, 4104])
 @pytest.mark.parametrize("layout", [(0, 0), (0, 1), (1, 0)])
