@@ -1819,9 +1819,12 @@ gmm_block(const CUtensorMap& map_a, const CUtensorMap& map_b,
             uint4 o[4];
 #pragma unroll 1
             for (int ch = 0; ch < 2; ++ch) {
-              load(ch);
+              ptx::tmem_ld_32x32(tg + ch * 32, va);
+              ptx::tmem_ld_32x32(tg + kBlockN / 2 + ch * 32, vb);
+              if (backward) load_grad(d4, half * 64 + ch * 32);  // (in flight with them)
+              ptx::tmem_ld_wait();
+              if (ch == 1) release();
               if (backward) {
-                load_grad(d4, half * 64 + ch * 32);
                 gradients(d4);
                 pack(va, o);
                 emit_gate(o, ch);
