@@ -334,7 +334,8 @@ int wide_cost(const Features& f, int64_t d1, bool trans_a, bool ragged) {
 // power supply are.
 //   512 rows an expert and more: pairs, 0.76 to 1 of the time of one-CTA tiles (19 experts, 54879 rows,
 //     9736 x 96: 371 us one-CTA, 284; 2 of 33358, 2248 x 1120: 410 / 339), unless one-CTA tiles make far fewer
-//     rounds (one of 1084, 552 x 1936, gated: 11.2 / 18.7).
+//     rounds than the fewest a pair's can (one of 1084, 552 x 1936, gated: 11.2 / 18.7; but 6 of 1002, 2016 x 264,
+//     gated, which fit one round of either: 24.2 / 21.8).
 //   128 to 511 rows: pairs only for rows that start at any 16 bytes, which are two lines of L2 where
 //     they could be one (64 experts of 128 rows, 4088 x 8184: 1351 / 933; 7 of 428, dgrad 2504 -> 1000: 29.7 / 25.0), where
 //     they make a tenth less by this reckoning, and not where one-CTA tiles are one round of fewer
@@ -359,10 +360,12 @@ int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int t
   if (d1 < (ragged ? 416 : 512)) return 1;
   if (!rows_from(512) && (!ragged || !rows_from(128) || f.gather || f.scatter || f.gated_backward)) return 1;
   const int64_t sms = dev != nullptr ? dev->sm_count : 148, pairs = std::max<int64_t>(dev != nullptr ? dev->pair_ctas / 2 : 74, 1);
+  const auto fewest = [&](int64_t rows) { return (tokens + rows - 1) / rows; };
   const auto row_tiles = [&](int64_t rows) {  // of experts of even size, half a tile of each idle
-    return z == 1 ? (tokens + rows - 1) / rows : tokens / rows + std::min<int64_t>(z, tokens) / 2;
+    return z == 1 ? fewest(rows) : tokens / rows + std::min<int64_t>(z, tokens) / 2;
   };
-  const int64_t nt = (n + kBlockN - 1) / kBlockN, one_tiles = row_tiles(kBlockM) * nt, pair_rows = row_tiles(2 * kBlockM);
+  const int64_t nt = (n + kBlockN - 1) / kBlockN, one_tiles = row_tiles(kBlockM) * nt;
+  const int64_t pair_rows = rows_from(512) ? fewest(2 * kBlockM) : row_tiles(2 * kBlockM);
   if (one_tiles <= sms && !rows_from(384)) return 1;
   const int64_t one = 125 * rounds_narrow(one_tiles, sms);
   const int64_t pair = std::min(100 * rounds_narrow(pair_rows * nt, pairs),

@@ -159,6 +159,7 @@ def test_schedule_covers_rows_and_columns_once(sizes, trans_b, n, ctas, light, m
 CHOICES = [
     (200, 30000, 512, 512, "nn", 0, 1), (200, 30000, 512, 512, "nn", _capi.FORM_GATED, 1),
     (256, 65536, 7168, 2048, "nn", 0, 1), (256, 65536, 7168, 2048, "nn", _capi.FORM_GATED, 1),
+    (6, 6012, 2016, 264, "nn", _capi.FORM_GATED, 2), (1, 1084, 552, 1936, "nn", _capi.FORM_GATED, 1),
     (1, 1041, 2200, 4120, "nn", 0, 2), (1, 1041, 2200, 4120, "nn", _capi.FORM_GATED, 2),
     (19, 54879, 9736, 96, "nn", 0, 2), (19, 54879, 9736, 96, "nn", _capi.FORM_SCATTER, 2),
     (16, 6170, 1416, 11392, "nn", _capi.FORM_GATED_BACKWARD, 1), (16, 6170, 1416, 11392, "nn", _capi.FORM_GATHER, 1),
