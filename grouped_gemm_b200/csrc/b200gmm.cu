@@ -336,13 +336,15 @@ int wide_cost(const Features& f, int64_t d1, bool trans_a, bool ragged) {
 //     9736 x 96: 371 us one-CTA, 284; 2 of 33358, 2248 x 1120: 410 / 339), unless one-CTA tiles make far fewer
 //     rounds than the fewest a pair's can (one of 1084, 552 x 1936, gated: 11.2 / 18.7; but 6 of 1002, 2016 x 264,
 //     gated, which fit one round of either: 24.2 / 21.8).
-//   128 to 511 rows: pairs only for rows that start at any 16 bytes, which are two lines of L2 where
-//     they could be one (64 experts of 128 rows, 4088 x 8184: 1351 / 933; 7 of 428, dgrad 2504 -> 1000: 29.7 / 25.0), where
+//   128 to 511 rows: pairs for rows that start at any 16 bytes, which are two lines of L2 where they
+//     could be one (64 experts of 128 rows, 4088 x 8184: 1351 / 933; 7 of 428, dgrad 2504 -> 1000: 29.7 / 25.0), where
 //     they make a tenth less by this reckoning, and not where one-CTA tiles are one round of fewer
-//     than 384 rows each.  Others lose (200 experts of 150 rows, Zipf, 512 x 512: 37.9 / 46.1, gated 59.8 / 80.6;
-//     256 of 256, Zipf, 7168 x 2048: 2123 / 2259, dgrad 2157 / 2176, gated 4055 / 4412).  So do the gathered product
-//     (146 of 126, 6712 x 2496: 1185 / 1487), scattered rows (64 of 116, 1864 x 2872: 199 / 204) and the gated
-//     backward (16 of 386, 1416 x 11392: 547 / 584).
+//     than 384 rows each.  Others from 256 rows on in launches of many rounds and a long contraction,
+//     which run into the power cap when they are repeated for a second (200 experts of 256 rows, Zipf, 4096 x 2048:
+//     1060 / 999, dgrad 1067 / 973, gated 2101 / 1970; 256 of 256, 7168 x 2048, Zipf: 2436 / 2382, dgrad 2322 / 2159, even
+//     sizes 2592 / 2602, dgrad 2618 / 2357; in bursts of 10 ms the two are even).  Short ones lose (200 of 150, Zipf,
+//     512 x 512: 37.9 / 46.1, gated 59.8 / 80.6).  So do the gathered product (146 of 126, 6712 x 2496: 1185 / 1487),
+//     scattered rows (64 of 116, 1864 x 2872: 199 / 204) and the gated backward (16 of 386, 1416 x 11392: 547 / 584).
 //   A short contraction leaves an accumulator little time to be read out while the other one
 //     fills, which a pair's wide tile does not have: one CTA below 416 (any 16 bytes) and 512 (49 experts,
 //     98681 rows, 72 x 2000: 101 / 159; 81, 68558, 432 x 2608: 223 / 240; 173, 110139, 128 x 856: 77 / 113).
@@ -358,7 +360,7 @@ int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int t
   if (trans_a) return rows_from(512) && d1 >= 256 ? 2 : 1;
   const bool ragged = ragged_rows(d1, f.swiglu ? n / 2 : n, trans_b);
   if (d1 < (ragged ? 416 : 512)) return 1;
-  if (!rows_from(512) && (!ragged || !rows_from(128) || f.gather || f.scatter || f.gated_backward)) return 1;
+  if (!rows_from(512) && (!rows_from(128) || f.gather || f.scatter || f.gated_backward)) return 1;
   const int64_t sms = dev != nullptr ? dev->sm_count : 148, pairs = std::max<int64_t>(dev != nullptr ? dev->pair_ctas / 2 : 74, 1);
   const auto fewest = [&](int64_t rows) { return (tokens + rows - 1) / rows; };
   const auto row_tiles = [&](int64_t rows) {  // of experts of even size, half a tile of each idle
@@ -367,6 +369,7 @@ int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int t
   const int64_t nt = (n + kBlockN - 1) / kBlockN, one_tiles = row_tiles(kBlockM) * nt;
   const int64_t pair_rows = rows_from(512) ? fewest(2 * kBlockM) : row_tiles(2 * kBlockM);
   if (one_tiles <= sms && !rows_from(384)) return 1;
+  if (!rows_from(512) && !ragged) return rows_from(256) && d1 >= 2048 && one_tiles >= 16 * sms ? 2 : 1;
   const int64_t one = 125 * rounds_narrow(one_tiles, sms);
   const int64_t pair = std::min(100 * rounds_narrow(pair_rows * nt, pairs),
                                 wide_cost(f, d1, false, ragged) * rounds_wide(pair_rows * ((nt + 1) / 2), pairs));

@@ -158,7 +158,7 @@ def test_schedule_covers_rows_and_columns_once(sizes, trans_b, n, ctas, light, m
 # z, rows, k, n, layout, features, CTAs a tile: the faster of the two on a B200 by a tenth and more
 CHOICES = [
     (200, 30000, 512, 512, "nn", 0, 1), (200, 30000, 512, 512, "nn", _capi.FORM_GATED, 1),
-    (256, 65536, 7168, 2048, "nn", 0, 1), (256, 65536, 7168, 2048, "nn", _capi.FORM_GATED, 1),
+    (256, 65536, 7168, 2048, "nn", 0, 2), (256, 65536, 2048, 7168, "nt", 0, 2), (200, 51200, 4096, 2048, "nn", _capi.FORM_GATED, 2),
     (6, 6012, 2016, 264, "nn", _capi.FORM_GATED, 2), (1, 1084, 552, 1936, "nn", _capi.FORM_GATED, 1),
     (1, 1041, 2200, 4120, "nn", 0, 2), (1, 1041, 2200, 4120, "nn", _capi.FORM_GATED, 2),
     (19, 54879, 9736, 96, "nn", 0, 2), (19, 54879, 9736, 96, "nn", _capi.FORM_SCATTER, 2),
