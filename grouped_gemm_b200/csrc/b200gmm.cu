@@ -339,10 +339,11 @@ int wide_cost(const Features& f, int64_t d1, bool trans_a, bool ragged) {
 //   128 to 511 rows: pairs for rows that start at any 16 bytes, which are two lines of L2 where they
 //     could be one (64 experts of 128 rows, 4088 x 8184: 1351 / 933; 7 of 428, dgrad 2504 -> 1000: 29.7 / 25.0), where
 //     they make a tenth less by this reckoning, and not where one-CTA tiles are one round of fewer
-//     than 384 rows each.  Others from 256 rows on in launches of many rounds and a long contraction,
-//     which run into the power cap when they are repeated for a second (200 experts of 256 rows, Zipf, 4096 x 2048:
-//     1060 / 999, dgrad 1067 / 973, gated 2101 / 1970; 256 of 256, 7168 x 2048, Zipf: 2436 / 2382, dgrad 2322 / 2159, even
-//     sizes 2592 / 2602, dgrad 2618 / 2357; in bursts of 10 ms the two are even).  Short ones lose (200 of 150, Zipf,
+//     than 384 rows each.  Others where the contraction is 1536 and more and one-CTA tiles make eight
+//     rounds and more: repeated for a third of a second, under the power cap, one-CTA / pairs (64 experts of 256
+//     rows, 2048 x 4096: 386 / 344, dgrad 402 / 346; 32 of 256, 4096 x 4096: 367 / 323; 128 of 128, Zipf, 4096 x 2048: 480 /
+//     433; 96 of 384, 3072 x 3072: 801 / 769, gated 1527 / 1486; 64 of 384, 1536 x 4096: 379 / 340; 256 of 256, Zipf, 7168 x
+//     2048: 2436 / 2382, dgrad 2322 / 2159); in bursts of 10 ms the two are even.  Short ones lose (200 of 150, Zipf,
 //     512 x 512: 37.9 / 46.1, gated 59.8 / 80.6).  So do the gathered product (146 of 126, 6712 x 2496: 1185 / 1487),
 //     scattered rows (64 of 116, 1864 x 2872: 199 / 204) and the gated backward (16 of 386, 1416 x 11392: 547 / 584).
 //   A short contraction leaves an accumulator little time to be read out while the other one
@@ -369,7 +370,7 @@ int choose_ctas(int z, int64_t tokens, int64_t d1, int64_t n, int trans_a, int t
   const int64_t nt = (n + kBlockN - 1) / kBlockN, one_tiles = row_tiles(kBlockM) * nt;
   const int64_t pair_rows = rows_from(512) ? fewest(2 * kBlockM) : row_tiles(2 * kBlockM);
   if (one_tiles <= sms && !rows_from(384)) return 1;
-  if (!rows_from(512) && !ragged) return rows_from(256) && d1 >= 2048 && one_tiles >= 16 * sms ? 2 : 1;
+  if (!rows_from(512) && !ragged) return d1 >= 1536 && one_tiles >= 8 * sms ? 2 : 1;
   const int64_t one = 125 * rounds_narrow(one_tiles, sms);
   const int64_t pair = std::min(100 * rounds_narrow(pair_rows * nt, pairs),
                                 wide_cost(f, d1, false, ragged) * rounds_wide(pair_rows * ((nt + 1) / 2), pairs));

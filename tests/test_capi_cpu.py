@@ -159,6 +159,7 @@ def test_schedule_covers_rows_and_columns_once(sizes, trans_b, n, ctas, light, m
 CHOICES = [
     (200, 30000, 512, 512, "nn", 0, 1), (200, 30000, 512, 512, "nn", _capi.FORM_GATED, 1),
     (256, 65536, 7168, 2048, "nn", 0, 2), (256, 65536, 2048, 7168, "nt", 0, 2), (200, 51200, 4096, 2048, "nn", _capi.FORM_GATED, 2),
+    (64, 16384, 2048, 4096, "nn", 0, 2), (128, 16384, 4096, 2048, "nn", 0, 2), (64, 16384, 1024, 4096, "nn", 0, 1),
     (6, 6012, 2016, 264, "nn", _capi.FORM_GATED, 2), (1, 1084, 552, 1936, "nn", _capi.FORM_GATED, 1),
     (1, 1041, 2200, 4120, "nn", 0, 2), (1, 1041, 2200, 4120, "nn", _capi.FORM_GATED, 2),
     (19, 54879, 9736, 96, "nn", 0, 2), (19, 54879, 9736, 96, "nn", _capi.FORM_SCATTER, 2),
